@@ -29,6 +29,7 @@ void matmul_gram_impl(grgx_graph* g, int dtype, const void* input, uint64_t in_c
 void set_up_split(long long block, unsigned long long thresholdBytes);
 void set_down_split_mode(int mode);
 void set_staged(bool on);
+void set_pair_mode(int mode);
 void* host_alloc(uint64_t bytes);
 void host_free(void* b);
 std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags);
@@ -452,6 +453,10 @@ extern "C" void grgx_debug_split_forms(int down_mode, int staged) {
     grgx::set_down_split_mode(down_mode);
     grgx::set_staged(staged != 0);
 }
+
+// Test hook (not part of the public header): pair form by its rules (0), wherever possible (1) or
+// never (2); a graph's form is decided on the first call that may use it.
+extern "C" void grgx_debug_pair_form(int mode) { grgx::set_pair_mode(mode); }
 
 grgx_status grgx_collect_timings(grgx_timing* out, uint64_t capacity, uint64_t* count) {
     return guarded([&] {

@@ -8,6 +8,7 @@
 
 #include "grgx_internal.h"
 #include "launch.h"
+#include "pair_plan.h"
 
 namespace grgx {
 
@@ -65,6 +66,7 @@ struct DevicePlan {
     long long n_fin_down = 0;
     bool down_split_built = false;
     std::map<std::pair<int, long long>, bool> down_split_choice;
+    PairPlan pair;                       // pair form of the height-0 edges, on first use (use_pair_form)
     std::vector<int64_t> down_off;       // DOWN row offsets (host copy)
     long long down_h0_row = 0;           // first DOWN row of height 0
     std::vector<int64_t> up_off;         // UP row offsets (host copy)
@@ -170,6 +172,33 @@ void set_staged(bool on);
 bool staged_layout(const Layout& L);
 // DOWN split form: 0 chosen as above, 1 always (where possible), 2 never (tests).
 void set_down_split_mode(int mode);
+
+// Whether a call with layout L runs in pair form (pair_plan.h); builds the form on the first call
+// that may use it.  set_pair_mode: 0 by the rules, 1 wherever possible, 2 never (tests).
+bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L);
+// Scratch the pair form of a call on this thread may take beyond what the other forms need; a
+// server's worker lowers it to what its batch has reserved (PairScratchScope).
+size_t pair_scratch_limit();
+void set_pair_mode(int mode);
+// The launches of a DOWN call in pair form, sized for layout L: a table of pattern rows per range
+// of blocks, and per range the sums of its items.  With several ranges the first sum carries what
+// the ranges before added up.
+struct PairDownRun {
+    struct Range {
+        int g0, g1;  // groups of four blocks
+        long long pat0, count;
+        int items, groups_per_item;
+    };
+    std::vector<Range> ranges;
+    int slots = 0;  // sums per row held at a time (0: the only item writes its rows)
+    size_t table_bytes = 0, part_bytes = 0;
+};
+// `limit`: most bytes of scratch the table and the sums may take; no ranges where that is too little.
+PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit);
+// Adds the height-0 rows' sums onto vals; `work` holds L.ntiles zeroed counters per range.
+// Returns the kernels launched.
+int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
+                     unsigned* work, cudaStream_t s, const int* gate, int gateValue);
 
 // Resolves (once per device, with `device` current) the address of grgx_matmul_noalloc's
 // static scratch, which loads its module and so reserves the array on the device.

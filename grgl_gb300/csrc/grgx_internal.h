@@ -149,6 +149,17 @@ class PlanDeviceScope {
 };
 // Chunks per level the chunker aims for (from the SM count in scope).
 int64_t chunk_target();
+// While alive, calls of this thread keep the pair form's scratch (pair_plan.h) within `bytes`.
+class PairScratchScope {
+  public:
+    explicit PairScratchScope(uint64_t bytes);
+    ~PairScratchScope();
+    PairScratchScope(const PairScratchScope&) = delete;
+    PairScratchScope& operator=(const PairScratchScope&) = delete;
+
+  private:
+    uint64_t saved_;
+};
 // SM count of the current device (looked up once per device, matmul.cu).
 int sm_count();
 void finish_csr(PullCSR& P, const std::vector<int64_t>& off);

@@ -39,6 +39,39 @@ void launch_sweep_staged_xor(const SweepParams<uint32_t>& p, dim3 grid, cudaStre
 void launch_sweep_staged_f32c(const SweepParams<float>& p, dim3 grid, cudaStream_t s);
 void launch_sweep_staged_f32(const SweepParams<float>& p, dim3 grid, cudaStream_t s);
 
+// DOWN in pair form (pair_down.cuh): one launch over `items` shares of the blocks (groups of four,
+// group_begin .. group_end) x `tiles` row tiles.
+template <typename S> struct PairDownParams {
+    const uint2* ids;    // four 16-bit pattern numbers per (row tile of 32, group, row)
+    const uint4* base;   // first pattern of each block, by groups of four
+    const S* table;      // pattern rows, from pattern `base0` on
+    S* vals;             // node values (the height-0 rows first)
+    void* parts;         // one sum per (item, row, column), or null: rows are written at once
+    unsigned* work;      // per column tile: next item (zeroed before the launch)
+    long long rows, stride, groups;
+    unsigned base0, tiles, items;
+    int group_begin, group_end, groups_per_item, part_begin;
+    const int* gate;
+    int gate_value;
+};
+// What a pair_down_* call does, and what its kShape step answers.
+struct PairDownCall {
+    enum Step { kShape, kTable, kGather, kFinish } step = kShape;
+    int rows_per_warp = 0, resident_warps = 0;  // kShape
+    size_t part_bytes = 0;
+    const uint2* nodes = nullptr;  // kTable: the patterns' parents
+    long long count = 0;
+    int parts = 0;      // kFinish: sums per row
+    bool onto = false;  // kFinish: onto the node values (else into the first sum)
+};
+void pair_down_u32(const PairDownParams<uint32_t>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_xor(const PairDownParams<uint32_t>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_u64(const PairDownParams<unsigned long long>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_f64(const PairDownParams<double>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_f32c(const PairDownParams<float>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_f32(const PairDownParams<float>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_f64s(const PairDownParams<DF>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+
 // Column-map modes of the transposing loads/stores.
 enum MapMode { MAP_IDENT = 0, MAP_DIV = 1, MAP_TABLE = 2, MAP_FOLD = 3 };
 

@@ -534,9 +534,10 @@ void validate_matmul(grgx_graph* g, int dtype, uint64_t in_cols, uint64_t rows, 
     }
 }
 
-void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, uint64_t rows, int direction,
-                   void* output, uint64_t output_size, int emit_all, int by_indiv, const void* init, int init_kind,
-                   void* miss, uint32_t flags, void* stream_ptr) {
+namespace {
+void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, uint64_t rows, int direction,
+                 void* output, uint64_t output_size, int emit_all, int by_indiv, const void* init, int init_kind,
+                 void* miss, uint32_t flags, void* stream_ptr, bool pairForm) {
     const HostGraph& hg = *g->host;
     const uint64_t n = hg.num_nodes, N = hg.num_samples, M = hg.num_mutations, P = hg.ploidy;
     validate_matmul(g, dtype, in_cols, rows, direction, output_size, emit_all, by_indiv, init, init_kind, miss);
@@ -592,8 +593,11 @@ void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols
         // UP in split form when the height-0 rows outgrow L2: their edges first, in blocked
         // passes, then the other edges level by level (up_split.cu)
         const bool split = !down && use_up_split(g, dp, L);
-        // DOWN in split form: the height-0 level in parent blocks (up_split.cu)
-        const bool dsplit = down && use_down_split(g, dp, L);
+        // DOWN: the height-0 level over patterns (pair_plan.h), or in parent blocks (up_split.cu)
+        PairDownRun prun;
+        if (down && pairForm && use_pair_form(g, dp, L)) prun = pair_down_run(L, dp, pair_scratch_limit());
+        const bool dpair = !prun.ranges.empty();
+        const bool dsplit = down && !dpair && use_down_split(g, dp, L);
         // coarse or fine chunking for this row width (the split copies are built by now)
         const SweepCSRs cs = sweep_csrs(dp, L);
         const DevCSR& cUp = *cs.up;
@@ -609,7 +613,8 @@ void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols
                                      (dsplit ? cDown0b.n_heavy : 0))
                                   : (split ? cUp0b.n_heavy + cUpInt.n_heavy : cUp.n_heavy);
         const long long nslots = down ? (2 + static_cast<long long>(cDown.lb.size()) +
-                                         (dsplit ? static_cast<long long>(cDown0b.lb.size()) : 0))
+                                         (dsplit ? static_cast<long long>(cDown0b.lb.size()) : 0) +
+                                         static_cast<long long>(prun.ranges.size()))
                                       : static_cast<long long>(split ? cUp0b.lb.size() + cUpInt.lb.size()
                                                                      : cUp.lb.size());
         const long long h0 = static_cast<long long>(dp->level_begin.size() > 1 ? dp->level_begin[1] : 0);
@@ -617,6 +622,8 @@ void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols
                                   : dsplit ? static_cast<size_t>(h0) * L.stride * std::max(L.asize, 8)
                                            : 0;
         void* state = (split || dsplit) ? sc.get(stateBytes) : nullptr;
+        void* ptable = dpair ? sc.get(prun.table_bytes) : nullptr;
+        void* pparts = prun.slots ? sc.get(prun.part_bytes) : nullptr;
         // counters per launch and per heavy row: enough column tiles for any launch shape
         const int TS = max_tiles(L);
         const size_t counterBytes = static_cast<size_t>(nh + nslots) * TS * sizeof(unsigned);
@@ -723,9 +730,11 @@ void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols
                 if (timed && t_timing) GRGX_CUDA(cudaEventRecord(ev[1], s));
                 const size_t nlv = cDown.lb.size();
                 for (size_t lvl = 0; lvl < nlv; lvl++) {
-                    if (dsplit && lvl + 1 == nlv) break;  // the height-0 level runs in split form below
+                    if ((dsplit || dpair) && lvl + 1 == nlv) break;  // the height-0 level runs below
                     launches += level(cDown, lvl, vals, 1, tk, work + (2 + lvl) * TS);
                 }
+                if (dpair)
+                    launches += launch_pair_down(LL, dp, prun, vals, ptable, pparts, work + (2 + nlv) * TS, s, g, gv);
                 if (dsplit) {
                     // parent-block passes merge each height-0 row's sums into its state; then the
                     // rows are written from it, onto their seed / init values
@@ -826,6 +835,23 @@ void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols
     }
     const bool hostWait = !devPtrs && !(flags & GRGX_FLAG_ASYNC);
     if (hostWait || (flags & GRGX_FLAG_SYNC)) GRGX_CUDA(cudaStreamSynchronize(s));
+}
+
+}  // namespace
+
+void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, uint64_t rows, int direction,
+                   void* output, uint64_t output_size, int emit_all, int by_indiv, const void* init, int init_kind,
+                   void* miss, uint32_t flags, void* stream_ptr) {
+    try {
+        matmul_once(g, dtype, input, in_cols, rows, direction, output, output_size, emit_all, by_indiv, init, init_kind,
+                    miss, flags, stream_ptr, true);
+    } catch (const Error& e) {
+        // The pair form's table and sums are scratch that the other forms do without.  (All of a
+        // call's scratch is taken before anything writes its output.)
+        if (e.code != GRGX_ERR_OUT_OF_MEMORY) throw;
+        matmul_once(g, dtype, input, in_cols, rows, direction, output, output_size, emit_all, by_indiv, init, init_kind,
+                    miss, flags, stream_ptr, false);
+    }
 }
 
 // ---- captured CUDA graphs of whole calls (small graphs) ----------------------------------------

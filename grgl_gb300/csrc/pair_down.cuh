@@ -1,0 +1,247 @@
+// DOWN in pair form: the height-0 rows' sums over patterns (pair_plan.h).
+//
+//   pair_table_kernel    pattern row = sum of its parents' rows, for the blocks of one table
+//   pair_down_kernel     height-0 row += one pattern row per block
+//   pair_finish_kernel   rows whose blocks were shared out over several items: the items' sums added
+//                        up in order, onto the row's seed value
+#pragma once
+#include <algorithm>
+#include <stdexcept>
+#include <type_traits>
+
+#include "launch.h"
+
+namespace grgx {
+
+// Accumulated sum of one item as it is kept between kernels: compensated sums stay pairs, a
+// float-pair run becomes the double it stands for.
+template <class Op> struct PairPart {
+    using T = typename Op::A;
+    static __device__ __forceinline__ T of(const typename Op::A& a) { return a; }
+    static __device__ __forceinline__ void merge(typename Op::A& a, const T& x) { Op::merge(a, x); }
+};
+template <> struct PairPart<AddF64S> {
+    using T = double;
+    static __device__ __forceinline__ T of(const F64Run& a) { return a.acc + AddF64S::run_value(a); }
+    static __device__ __forceinline__ void merge(F64Run& a, const T& x) { a.acc += x; }
+};
+
+// a + b of two node values, in storage precision.  Compensated float32 rounds the pair once, like
+// the first level of the plain pre-sums of the sweep (vecacc.cuh); float pairs keep 48 bits.
+template <class Op> __device__ __forceinline__ typename Op::S pair_sum(typename Op::S a, typename Op::S b) {
+    typename Op::A t = Op::zero();
+    Op::add(t, a);
+    Op::add(t, b);
+    return Op::finish(t);
+}
+template <> __device__ __forceinline__ float pair_sum<AddF32C>(float a, float b) { return __fadd_rn(a, b); }
+template <> __device__ __forceinline__ DF pair_sum<AddF64S>(DF a, DF b) {
+    AddF64S::run_add(a.hi, a.lo, b.hi, b.lo);
+    return a;
+}
+
+template <class Op, int VW>
+__global__ void pair_table_kernel(const uint2* __restrict__ nodes, long long count, const typename Op::S* __restrict__ vals,
+                                  long long stride, typename Op::S* __restrict__ table, const int* gate, int gate_value) {
+    using S = typename Op::S;
+    if (gate != nullptr && *gate != gate_value) return;
+    const unsigned vecs = static_cast<unsigned>(stride / VW);
+    const unsigned long long total = (unsigned long long)count * vecs;
+    for (unsigned long long x = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
+         x += (unsigned long long)gridDim.x * blockDim.x) {
+        const unsigned long long pat = x / vecs;
+        const int col = static_cast<int>(x - pat * vecs) * VW;
+        const uint2 nd = __ldg(nodes + pat);
+        S a[VW], b[VW];
+#pragma unroll
+        for (int i = 0; i < VW; i++) a[i] = b[i] = S{};
+        if (nd.x != 0x7fffffffu) Vec<S, VW>::ld(vals + (long long)nd.x * stride + col, a);
+        if (nd.y != 0x7fffffffu) Vec<S, VW>::ld(vals + (long long)nd.y * stride + col, b);
+#pragma unroll
+        for (int i = 0; i < VW; i++) a[i] = pair_sum<Op>(a[i], b[i]);
+        Vec<S, VW>::st(table + (long long)pat * stride + col, a);
+    }
+}
+
+// Rows per group of lanes: a warp covers (32 / G) * kPairRows rows, four blocks of each at a time,
+// so eight gathers are in flight per lane.  Four rows (sixteen gathers, two blocks of threads per
+// SM instead of three) ran within 3% either way for int32 and wide float64 and slower for the rest
+// (float32 K=64 4.29 against 4.11 ms, float64 K=8 1.92 against 1.66 ms; N=200,000, M=250,000).
+constexpr int kPairRows = 2;
+
+// Bound by the L2 -> SM reads of its gathers when rows are wide (float32 K=64: 16-17 TB/s of pattern
+// rows, the read probe's rate), by the packed float32 additions for float pairs, and by the rate
+// of gather instructions for the narrowest rows, whose tables mostly sit in L1.  It takes half the
+// gathers of a sweep over edges, has no row boundaries to look for (each row has exactly one
+// pattern per block), and reads one byte of ids per edge.  DOWN products on N=200,000, M=250,000
+// before and after: int32 K=1 0.65 -> 0.34 ms (staged split passes before), float32 K=9 2.38 ->
+// 1.32, float32 K=64 7.87 -> 4.1, float64 K=64 16.6 -> 9.3 ms.
+//
+// One warp per item (a share of the blocks x a tile of rows).  A row's columns are spread over G
+// lanes as in the sweep; each lane loads its rows' ids of four blocks (8 bytes) and gathers the
+// four pattern rows of each of its kRows rows before adding them.
+template <class Op, int VW, int G>
+__global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<typename Op::S> p) {
+    using S = typename Op::S;
+    using Acc = VecAcc<Op, VW>;
+    using Part = PairPart<Op>;
+    constexpr int NG = 32 / G, ROWS = kPairRows;
+    constexpr bool kChains = ChainTraits<Op>::kChains;
+    if (p.gate != nullptr && *p.gate != p.gate_value) return;
+    const int lane = threadIdx.x & 31;
+    const int lg = lane / G;
+    const int col = blockIdx.y * (G * VW) + (lane % G) * VW;
+    const bool colok = col < p.stride;
+    const unsigned rowBytes = static_cast<unsigned>(p.stride * sizeof(S));
+    const char* table = reinterpret_cast<const char*>(p.table + (colok ? col : 0));
+    unsigned* counter = p.work + blockIdx.y;
+    for (;;) {
+        unsigned c = 0;
+        if (lane == 0) c = atomicAdd(counter, 1u);
+        c = __shfl_sync(FULL_MASK, c, 0);
+        if (c >= p.tiles * p.items) return;
+        const unsigned item = c / p.tiles;
+        const long long row0 = (long long)(c - item * p.tiles) * (NG * ROWS) + lg;
+        const int q0 = p.group_begin + static_cast<int>(item) * p.groups_per_item;
+        const int q1 = min(p.group_end, q0 + p.groups_per_item);
+        const uint2* idp[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const long long row = row0 + r * NG;
+            idp[r] = p.ids + ((row >> 5) * p.groups + q0) * 32 + (row & 31);
+        }
+        Acc acc[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) acc[r].zero();
+        uint2 next[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) next[r] = __ldg(idp[r]);
+        for (int q = q0; q < q1; q++) {
+            const uint4 b = __ldg(p.base + q);
+            uint2 id[ROWS];
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) {
+                id[r] = next[r];
+                idp[r] += 32;
+                if (q + 1 < q1) next[r] = __ldg(idp[r]);
+            }
+            S v[ROWS][4][VW];
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) {
+                const unsigned k[4] = {b.x - p.base0 + (id[r].x & 0xffffu), b.y - p.base0 + (id[r].x >> 16),
+                                       b.z - p.base0 + (id[r].y & 0xffffu), b.w - p.base0 + (id[r].y >> 16)};
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    Vec<S, VW>::ld(reinterpret_cast<const S*>(table + (unsigned long long)k[u] * rowBytes), v[r][u]);
+            }
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) acc[r].add_pairs(v[r]);
+            if (kChains && ((q - q0) & 7) == 7) {
+#pragma unroll
+                for (int r = 0; r < ROWS; r++) acc[r].flush();
+            }
+        }
+        if (!colok) continue;
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const long long row = row0 + r * NG;
+            if (row >= p.rows) continue;
+            if (p.parts == nullptr) {
+                S base[VW], out[VW];
+                S* d = p.vals + row * p.stride + col;
+                ld_plain<S, VW>(d, base);
+#pragma unroll
+                for (int i = 0; i < VW; i++) out[i] = Op::finish_onto(base[i], acc[r].get(i));
+                Vec<S, VW>::st(d, out);
+            } else {
+                typename Part::T* d = static_cast<typename Part::T*>(p.parts) +
+                                      ((long long)(p.part_begin + item) * p.rows + row) * p.stride + col;
+#pragma unroll
+                for (int i = 0; i < VW; i++) d[i] = Part::of(acc[r].get(i));
+            }
+        }
+    }
+}
+
+// Adds up `count` sums per row, in order: into the first one (vals null), or onto the node values.
+template <class Op>
+__global__ void pair_finish_kernel(typename PairPart<Op>::T* __restrict__ parts, int count, long long rows,
+                                   long long stride, typename Op::S* __restrict__ vals, const int* gate, int gate_value) {
+    if (gate != nullptr && *gate != gate_value) return;
+    const long long total = rows * stride;
+    for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
+        typename Op::A a = Op::zero();
+        for (int j = 0; j < count; j++) PairPart<Op>::merge(a, parts[j * total + x]);
+        if (vals == nullptr) {
+            parts[x] = PairPart<Op>::of(a);
+            continue;
+        }
+        if constexpr (std::is_same<typename Op::S, DF>::value)
+            df_put(vals, x, stride, Op::finish_onto(df_get(vals, x, stride), a));
+        else
+            vals[x] = Op::finish_onto(vals[x], a);
+    }
+}
+
+template <class Op, int VW, int G>
+int pair_blocks_per_sm() {
+    static int n = 0;
+    if (n == 0) {
+        int v = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, pair_down_kernel<Op, VW, G>, 256, 0);
+        n = v > 0 ? v : 1;
+    }
+    return n;
+}
+
+template <class Op, int VW, int G> void pair_down_as(PairDownParams<typename Op::S> p, PairDownCall& c, int sms, cudaStream_t s) {
+    if (c.step == PairDownCall::kShape) {
+        c.rows_per_warp = (32 / G) * kPairRows;
+        c.resident_warps = pair_blocks_per_sm<Op, VW, G>() * 8 * sms;
+        c.part_bytes = sizeof(typename PairPart<Op>::T);
+        return;
+    }
+    if (c.step == PairDownCall::kTable) {
+        const unsigned long long total = (unsigned long long)c.count * (p.stride / VW);
+        const unsigned grid = static_cast<unsigned>(std::min<unsigned long long>((total + 255) / 256, sms * 64ull));
+        pair_table_kernel<Op, VW><<<grid, 256, 0, s>>>(c.nodes, c.count, p.vals, p.stride, const_cast<typename Op::S*>(p.table),
+                                                       p.gate, p.gate_value);
+        return;
+    }
+    if (c.step == PairDownCall::kFinish) {
+        const unsigned long long total = (unsigned long long)p.rows * p.stride;
+        const unsigned grid = static_cast<unsigned>(std::min<unsigned long long>((total + 255) / 256, sms * 64ull));
+        pair_finish_kernel<Op><<<grid, 256, 0, s>>>(static_cast<typename PairPart<Op>::T*>(p.parts), c.parts, p.rows, p.stride,
+                                                    c.onto ? p.vals : nullptr, p.gate, p.gate_value);
+        return;
+    }
+    const unsigned warps = p.tiles * p.items;
+    const unsigned most = static_cast<unsigned>(pair_blocks_per_sm<Op, VW, G>() * sms);
+    const unsigned tilesY = static_cast<unsigned>((p.stride / VW + G - 1) / G);
+    pair_down_kernel<Op, VW, G><<<dim3(std::min((warps + 7) / 8, most), tilesY), 256, 0, s>>>(p);
+}
+
+#define GRGX_PAIR_CASE(OP, VWV, GV)               \
+    if (vw == VWV && g == GV) {                   \
+        pair_down_as<OP, VWV, GV>(p, c, sms, s);  \
+        return;                                   \
+    }
+#define GRGX_PAIR4(OP)                                                                              \
+    GRGX_PAIR_CASE(OP, 1, 1)                                                                        \
+    GRGX_PAIR_CASE(OP, 2, 1)                                                                        \
+    GRGX_PAIR_CASE(OP, 4, 1)                                                                        \
+    GRGX_PAIR_CASE(OP, 4, 2)                                                                        \
+    GRGX_PAIR_CASE(OP, 4, 4)                                                                        \
+    GRGX_PAIR_CASE(OP, 4, 8)                                                                        \
+    GRGX_PAIR_CASE(OP, 4, 16)                                                                       \
+    GRGX_PAIR_CASE(OP, 4, 32)
+#define GRGX_PAIR8(OP)                                                                              \
+    GRGX_PAIR_CASE(OP, 1, 1)                                                                        \
+    GRGX_PAIR_CASE(OP, 2, 1)                                                                        \
+    GRGX_PAIR_CASE(OP, 2, 2)                                                                        \
+    GRGX_PAIR_CASE(OP, 2, 4)                                                                        \
+    GRGX_PAIR_CASE(OP, 2, 8)                                                                        \
+    GRGX_PAIR_CASE(OP, 2, 16)                                                                       \
+    GRGX_PAIR_CASE(OP, 2, 32)
+
+}  // namespace grgx

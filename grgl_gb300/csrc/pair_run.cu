@@ -1,0 +1,133 @@
+// Host side of the pair form: how a call's products are cut into tables and items, and the launches.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "device_plan.h"
+
+namespace grgx {
+
+namespace {
+
+// Pattern rows held at a time: a table is written and gathered from before the next one.
+constexpr size_t kPairTableBytes = 1ULL << 30;
+// A share of the blocks (item) covers at most this much of a table.  The warps of a launch take
+// the items of one share before those of the next, so about this much is gathered from at a time
+// and mostly stays in L2 (float32 K=64, N=200,000, M=250,000, a 650 MB table: 4.08 ms at 96 MB,
+// 4.29 at 48 MB, 4.57 unshared).
+constexpr long long kPairItemBytes = 96LL << 20;
+// Items per resident warp that even out the launch's end, and the fewest groups of four blocks
+// that make an item worth its sum's trip through memory.
+constexpr long long kPairItemsPerWarp = 8;
+constexpr int kPairMinGroups = 16;
+// Most of a call's scratch unless a scope says less.
+constexpr uint64_t kPairScratch = 6ULL << 30;
+
+thread_local uint64_t t_limit = kPairScratch;
+
+template <typename F> void by_kind(const Layout& L, F&& f) {
+    switch (L.kind) {
+    case Kind::U32: f(PairDownParams<uint32_t>{}, pair_down_u32); break;
+    case Kind::XOR: f(PairDownParams<uint32_t>{}, pair_down_xor); break;
+    case Kind::U64: f(PairDownParams<unsigned long long>{}, pair_down_u64); break;
+    case Kind::F64: f(PairDownParams<double>{}, pair_down_f64); break;
+    case Kind::F32C: f(PairDownParams<float>{}, pair_down_f32c); break;
+    case Kind::F32: f(PairDownParams<float>{}, pair_down_f32); break;
+    case Kind::F64S: f(PairDownParams<DF>{}, pair_down_f64s); break;
+    }
+}
+
+}  // namespace
+
+PairScratchScope::PairScratchScope(uint64_t bytes) : saved_(t_limit) { t_limit = std::min(bytes, kPairScratch); }
+PairScratchScope::~PairScratchScope() { t_limit = saved_; }
+size_t pair_scratch_limit() { return static_cast<size_t>(t_limit); }
+
+PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit) {
+    const PairPlan& P = dp->pair;
+    PairDownRun run;
+    PairDownCall shape;
+    by_kind(L, [&](auto p, auto fn) { fn(p, shape, L.vw, L.g, sm_count(), nullptr); });
+    const size_t rowBytes = static_cast<size_t>(L.stride) * L.ssize;
+    const size_t slotBytes = static_cast<size_t>(P.h0) * L.stride * shape.part_bytes;
+    const size_t tableMost = std::min(kPairTableBytes, limit / 3);
+    // sums held at a time: what the rest of the limit holds, one of them carried between ranges
+    const long long slotsMost = static_cast<long long>((limit - tableMost) / slotBytes);
+    const long long tiles = (P.h0 + shape.rows_per_warp - 1) / shape.rows_per_warp;
+    const int groups = static_cast<int>((P.nblk + 3) / 4);
+    auto patterns = [&](int g) { return P.pat_base[std::min<long long>(4LL * g, P.nblk)]; };
+    for (int g0 = 0; g0 < groups;) {
+        int g1 = g0 + 1;
+        while (g1 < groups && static_cast<size_t>(patterns(g1 + 1) - patterns(g0)) * rowBytes <= tableMost) g1++;
+        PairDownRun::Range r{};
+        r.g0 = g0;
+        r.g1 = g1;
+        r.pat0 = patterns(g0);
+        r.count = patterns(g1) - r.pat0;
+        const long long carried = g0 > 0 ? 1 : 0;
+        // (the columns of a tile are gathered together, so a share spans rowBytes / ntiles per row)
+        const long long share = static_cast<long long>(r.count * rowBytes / L.ntiles) / kPairItemBytes + 1;
+        const long long even = (kPairItemsPerWarp * shape.resident_warps + tiles - 1) / tiles;
+        const long long most = std::min<long long>((g1 - g0) / kPairMinGroups, slotsMost - carried);
+        const long long items = std::max(1LL, std::min(std::max(share, even), most));
+        r.groups_per_item = static_cast<int>((g1 - g0 + items - 1) / items);
+        r.items = (g1 - g0 + r.groups_per_item - 1) / r.groups_per_item;
+        run.slots = std::max(run.slots, r.items + static_cast<int>(carried));
+        run.table_bytes = std::max(run.table_bytes, static_cast<size_t>(r.count) * rowBytes);
+        run.ranges.push_back(r);
+        g0 = g1;
+    }
+    if (run.slots == 1) run.slots = 0;
+    run.part_bytes = static_cast<size_t>(run.slots) * slotBytes;
+    if (run.table_bytes + run.part_bytes > limit) run.ranges.clear();
+    return run;
+}
+
+int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
+                     unsigned* work, cudaStream_t s, const int* gate, int gateValue) {
+    const PairPlan& P = dp->pair;
+    int launches = 0;
+    by_kind(L, [&](auto p, auto fn) {
+        PairDownCall c;
+        fn(p, c, L.vw, L.g, sm_count(), s);
+        p.ids = reinterpret_cast<const uint2*>(P.ids);
+        p.base = reinterpret_cast<const uint4*>(P.base);
+        p.table = static_cast<decltype(p.table)>(table);
+        p.vals = static_cast<decltype(p.vals)>(vals);
+        p.parts = run.slots ? parts : nullptr;
+        p.rows = P.h0;
+        p.stride = L.stride;
+        p.groups = (P.nblk + 3) / 4;
+        p.tiles = static_cast<unsigned>((P.h0 + c.rows_per_warp - 1) / c.rows_per_warp);
+        p.gate = gate;
+        p.gate_value = gateValue;
+        for (size_t i = 0; i < run.ranges.size(); i++) {
+            const PairDownRun::Range& r = run.ranges[i];
+            c.step = PairDownCall::kTable;
+            c.nodes = P.pat_nodes + r.pat0;
+            c.count = r.count;
+            fn(p, c, L.vw, L.g, sm_count(), s);
+            c.step = PairDownCall::kGather;
+            p.base0 = static_cast<unsigned>(r.pat0);
+            p.group_begin = r.g0;
+            p.group_end = r.g1;
+            p.items = static_cast<unsigned>(r.items);
+            p.groups_per_item = r.groups_per_item;
+            p.part_begin = i > 0 ? 1 : 0;
+            p.work = work + i * L.ntiles;
+            fn(p, c, L.vw, L.g, sm_count(), s);
+            launches += 2;
+            if (run.slots == 0) continue;
+            c.step = PairDownCall::kFinish;
+            c.parts = r.items + p.part_begin;
+            c.onto = i + 1 == run.ranges.size();
+            if (c.onto || c.parts > 1) {
+                fn(p, c, L.vw, L.g, sm_count(), s);
+                launches++;
+            }
+        }
+    });
+    return launches;
+}
+
+}  // namespace grgx

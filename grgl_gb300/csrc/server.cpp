@@ -67,6 +67,9 @@ struct grgx_server {
         }
     }
 
+    // Its share for the state of the split forms, which the pair form's scratch stays within.
+    static uint64_t state_bytes(const grgx::HostGraph& h, uint64_t rows) { return h.num_nodes * rows * 16; }
+
     // Conservative device bytes of one batch: node values and per-mutation rows in the widest
     // storage (8 bytes), the stacked input/output, plus a quarter for partials and the pool.
     uint64_t estimate(const grgx::HostGraph& h, int dtype, uint64_t rows) const {
@@ -74,7 +77,7 @@ struct grgx_server {
         // node values and the DOWN input rows (8 bytes an element at most), the split-form UP
         // state (16 bytes an element at most), heavy-row partials (a quarter more), and the I/O
         const uint64_t valueBytes = (h.num_nodes + h.num_mutations) * rows * 8;
-        const uint64_t stateBytes = h.num_nodes * rows * 16;
+        const uint64_t stateBytes = state_bytes(h, rows);
         const uint64_t ioBytes = rows * (h.num_samples + h.num_mutations) * es * 2;
         return valueBytes + valueBytes / 4 + stateBytes + ioBytes;
     }
@@ -161,6 +164,7 @@ struct grgx_server {
             int status = GRGX_OK;
             std::string err;
             try {
+                const grgx::PairScratchScope scratch(state_bytes(*graphs[batch[0]->graph]->host, rows));
                 grgx::matmul_batch_impl(graphs[batch[0]->graph], reqs.data(), reqs.size(), rows, GRGX_FLAG_SYNC,
                                         stream);
             } catch (const grgx::Error& e) {

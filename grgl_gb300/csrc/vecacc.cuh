@@ -47,6 +47,8 @@ template <class Op, int VW> struct ScalarAcc {
 #pragma unroll
         for (int u = 0; u < N; u++) add(v[u]);
     }
+    // Four pattern rows of the pair form, each the sum of two edges' rows.
+    __device__ __forceinline__ void add_pairs(const S (*v)[VW]) { add_block<4>(v); }
     __device__ __forceinline__ void merge(const ScalarAcc& o) {
 #pragma unroll
         for (int i = 0; i < VW; i++) Op::merge(a[i], o.a[i]);
@@ -102,6 +104,7 @@ template <> struct VecAcc<AddF32C, 1> {
         }
         if (N & 1) add(v[N - 1]);
     }
+    __device__ __forceinline__ void add_pairs(const float (*v)[1]) { add_block<4>(v); }
     __device__ __forceinline__ void merge(const VecAcc& o) {
         float2 sum, err;
         two_sum2(hi, o.hi, sum, err);
@@ -147,6 +150,7 @@ template <> struct VecAcc<AddF64S, 1> {
             if ((u & 3) == 3) settle();
         }
     }
+    __device__ __forceinline__ void add_pairs(const DF (*v)[1]) { add_block<4>(v); }
     __device__ __forceinline__ void merge(const VecAcc& o) { AddF64S::merge(a[0], o.a[0]); }
     __device__ __forceinline__ VecAcc shfl_xor(int m) const { return {{AddF64S::shfl_xor(a[0], m)}}; }
     __device__ __forceinline__ VecAcc shfl_up(int d) const { return {{AddF64S::shfl_up(a[0], d)}}; }
@@ -197,6 +201,17 @@ template <int NP> struct PackedF32C {
                 }
                 add_pair2(j, t);
             }
+        }
+    }
+    // Four pattern rows, each the rounded sum of two edges: two at a time in plain float32, so the
+    // edges pass the same two rounding levels before a TwoSum as four edges do in add_block.
+    __device__ __forceinline__ void add_pairs(const float (*v)[2 * NP]) {
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+#pragma unroll
+            for (int j = 0; j < NP; j++)
+                add_pair2(j, add2(make_float2(v[u][2 * j], v[u][2 * j + 1]),
+                                  make_float2(v[u + 1][2 * j], v[u + 1][2 * j + 1])));
         }
     }
     __device__ __forceinline__ void merge(const PackedF32C& o) {
@@ -273,6 +288,7 @@ template <int NP> struct PackedF64S {
             if ((u & 3) == 3) settle();
         }
     }
+    __device__ __forceinline__ void add_pairs(const DF (*v)[2 * NP]) { add_block<4>(v); }
     __device__ __forceinline__ void settle() {
 #pragma unroll
         for (int j = 0; j < NP; j++) {

@@ -1,0 +1,175 @@
+"""The pair form (height-0 nodes that share their pair of parents in two consecutive runs share one
+pattern row) gives the oracle's results: integers bit-exact, floats within the tolerances of the
+other forms, with the options of each direction, at the edges of its tiles and tables."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+from tests.conftest import abs_scale, assert_matches
+
+pytestmark = pytest.mark.gpu
+DOWN, UP = 1, 2
+
+
+def _pair_mode(mode):
+    from grgl_gb300 import _lib
+
+    fn = _lib.lib().grgx_debug_pair_form
+    fn.restype = None
+    fn.argtypes = [ctypes.c_int]
+    fn(mode)
+
+
+def _both(gx, g, ploidy=2, miss=None):
+    """The graph again from its arrays, decided in pair form, and the oracle's."""
+    a = g.export_arrays()
+    kw = {} if miss is None else {"miss_node": miss}
+    pg = gx.from_csr(g.num_samples, ploidy, a["down_off"], a["down_adj"], a["mut_node"], **kw).upload()
+    og = oracle.OracleGraph(num_samples=g.num_samples, ploidy=ploidy, down_off=a["down_off"], down_adj=a["down_adj"],
+                            mut_node=a["mut_node"], **kw)
+    return pg, og
+
+
+@pytest.fixture(scope="module")
+def env(cuda_ok):
+    import grgl_gb300 as gx
+
+    _pair_mode(1)
+    gx.set_graph_replay(False)
+    try:
+        # odd numbers of haplotypes (tiles of 32 and 128 end early) and of runs (a block of one run)
+        g = gx.window_tree_grg(3001, 20300, seed=97)
+        rng = np.random.default_rng(1)
+        miss = np.full(g.num_mutations, gx.INVALID_NODE, dtype=np.uint32)
+        miss[::7] = rng.integers(0, g.num_nodes, size=len(miss[::7]))
+        yield (gx, *_both(gx, g, ploidy=1, miss=miss))
+    finally:
+        gx.set_graph_replay(True)
+        _pair_mode(0)
+
+
+def _rand(rng, dt, shape):
+    if np.dtype(dt).kind == "f":
+        return rng.standard_normal(shape).astype(dt)
+    if np.dtype(dt) == np.bool_:
+        return rng.integers(0, 2, size=shape).astype(bool)
+    return rng.integers(0, 50, size=shape).astype(dt)
+
+
+def _check(og, V, direction, got, **kw):
+    rtol = 1e-12
+    if V.dtype == np.float32:  # compensated float32 against the float64 product of the same inputs
+        V, got = V.astype(np.float64), got.astype(np.float64)
+        kw = {k: (v.astype(np.float64) if isinstance(v, np.ndarray) else v) for k, v in kw.items()}
+        rtol = 1e-6
+    ref = oracle.matmul(og, V, direction, **{k: (v.copy() if isinstance(v, np.ndarray) else v) for k, v in kw.items()})
+    if V.dtype.kind == "f":
+        assert_matches(got, ref, abs_scale(og, V, direction, kw), rtol=rtol)
+    else:
+        assert_matches(got, ref)
+
+
+# every lane count of both element sizes, with and without a last vector or column tile in part
+@pytest.mark.parametrize("dt", [np.int32, np.int64, np.uint8, np.float32, np.float64, np.bool_])
+@pytest.mark.parametrize("K", [1, 2, 3, 8, 17, 33, 64, 130])
+def test_pair_down_matches_oracle(env, dt, K):
+    gx, g, og = env
+    V = _rand(np.random.default_rng(K), dt, (K, g.num_mutations))
+    _check(og, V, DOWN, gx.matmul(g, V, DOWN))
+
+
+@pytest.mark.parametrize("flag", ["f32_compensated", "f64_native"])
+def test_pair_down_other_accumulations(env, flag):
+    gx, g, og = env
+    rng = np.random.default_rng(9)
+    if flag == "f64_native":
+        V = rng.standard_normal((5, g.num_mutations))
+        _check(og, V, DOWN, gx.matmul(g, V, DOWN, f64_native=True))
+        V[0, 0], V[1, 1] = 1e300, 1e-300  # beyond the float-pair range: the FP64 path inside the same call
+        _check(og, V, DOWN, gx.matmul(g, V, DOWN))
+    else:
+        V = rng.standard_normal((5, g.num_mutations)).astype(np.float32)
+        ref = oracle.matmul(og, V.astype(np.float64), DOWN)
+        got = gx.matmul(g, V, DOWN, f32_compensated=False).astype(np.float64)
+        assert np.all(np.abs(got - ref) <= 2e-5 * oracle.matmul(og, np.abs(V).astype(np.float64), DOWN))
+
+
+def test_pair_down_options(env):
+    gx, g, og = env
+    rng = np.random.default_rng(3)
+    V = rng.standard_normal((5, g.num_mutations))
+    init, miss = rng.standard_normal(5), rng.standard_normal((5, g.num_mutations))
+    _check(og, V, DOWN, gx.matmul(g, V, DOWN, emit_all_nodes=True, init=init), emit_all_nodes=True, init=init)
+    _check(og, V, DOWN, gx.matmul(g, V, DOWN, miss=miss), miss=miss)
+    Vi = rng.integers(0, 9, size=(3, g.num_mutations)).astype(np.int32)
+    _check(og, Vi, DOWN, gx.matmul(g, Vi, DOWN, by_individual=True), by_individual=True)
+    initm = rng.standard_normal((1, g.num_nodes)).astype(np.float32)
+    V1 = rng.standard_normal((1, g.num_mutations)).astype(np.float32)
+    _check(og, V1, DOWN, gx.matmul(g, V1, DOWN, init=initm), init=initm)
+
+
+def test_pair_down_repeats_bit_for_bit(env):
+    gx, g, _ = env
+    V = np.random.default_rng(4).standard_normal((20, g.num_mutations))
+    assert np.array_equal(gx.matmul(g, V, DOWN), gx.matmul(g, V, DOWN))
+
+
+# graphs whose runs are short, uneven or single, with nodes and haplotypes left over
+@pytest.mark.parametrize("shape", ["one run", "nested", "duplicate child", "no low edges"])
+def test_pair_form_other_graphs(env, shape):
+    gx = env[0]
+    if shape == "one run":
+        N, kids = 40, {40: range(0, 20), 41: range(20, 39)}
+    elif shape == "nested":  # every node conflicts with the one before it; the last haplotype has no parent
+        N, kids = 33, {33: range(0, 32), 34: range(0, 16), 35: [33, 34], 36: [1, 3, 5, 35], 37: range(1, 32, 2)}
+    elif shape == "duplicate child":
+        N, kids = 34, {34: [0, 1, 1, 2], 35: [1, 33], 36: [3, 34, 35]}
+    else:
+        N, kids = 4, {4: [0, 1], 5: [4], 6: [5], 7: [6], 8: [4, 7], 9: [8]}
+    n = max(kids) + 1
+    off, adj = [0], []
+    for v in range(n):
+        adj += list(kids.get(v, []))
+        off.append(len(adj))
+    arrays = dict(down_off=np.array(off, dtype=np.uint64), down_adj=np.array(adj, dtype=np.uint32),
+                  mut_node=np.arange(n, dtype=np.uint32))
+    g = gx.from_csr(N, 1, *arrays.values())
+    og = oracle.OracleGraph(num_samples=N, ploidy=1, **arrays)
+    rng = np.random.default_rng(5)
+    for dt in (np.int32, np.float64):
+        for K in (1, 6):
+            V = _rand(rng, dt, (K, n))
+            _check(og, V, DOWN, gx.matmul(g, V, DOWN))
+            V = _rand(rng, dt, (K, N))
+            _check(og, V, UP, gx.matmul(g, V, UP))
+
+
+def test_large_graph_takes_the_pair_form_by_rule(cuda_ok):
+    """N=20,000, M=30,000 (6e6 edges) is over the rule's size: the same integers as without it."""
+    import grgl_gb300 as gx
+
+    g = gx.window_tree_grg(20_000, 30_000, seed=5).upload()
+    V = np.random.default_rng(2).integers(0, 3, size=(6, g.num_mutations)).astype(np.int32)
+    before = g.info()["device_bytes"]
+    got = gx.matmul(g, V, DOWN)
+    assert g.info()["device_bytes"] > before  # the form was built
+    gx.set_graph_replay(False)
+    _pair_mode(2)
+    try:
+        assert np.array_equal(got, gx.matmul(g, V, DOWN))
+    finally:
+        _pair_mode(0)
+        gx.set_graph_replay(True)
+
+
+@pytest.mark.parametrize("dt", [np.int32, np.float32, np.float64])
+def test_pair_down_within_a_servers_memory(env, dt):
+    """A server's batch has scratch for a part of the patterns at a time: several tables, their
+    sums carried from one to the next."""
+    gx, g, og = env
+    V = _rand(np.random.default_rng(6), dt, (12, g.num_mutations))
+    with gx.Server(workers=1) as srv:
+        got, _ = srv.result(srv.submit(srv.add_graph(g), V, DOWN), timeout=60.0)
+    _check(og, V, DOWN, got)
