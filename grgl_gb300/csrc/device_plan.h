@@ -32,6 +32,9 @@ struct DevCSR {
     HeavyDev* heavy = nullptr;
     std::vector<int32_t> lb, le;
     std::vector<long long> level_rows, level_edges;  // per level, for the launch-shape table
+    // per level of short rows: its rows' first edges, relative to level_e0 (else null)
+    std::vector<unsigned*> level_short;
+    std::vector<long long> level_r0, level_e0;
     long long n_heavy = 0, n_pieces = 0, n_edges = 0, n_rows = 0;
 };
 
@@ -125,6 +128,9 @@ struct SweepCSRs {
 };
 bool fine_chunks(const Layout& L);
 SweepCSRs sweep_csrs(const DevicePlan* dp, const Layout& L);
+// Finds the levels of `r` whose rows are short (rows' offsets `off`, chunks of `c`) and uploads their
+// offsets.
+void mark_short_levels(DevicePlan& d, DevCSR& r, const PullCSR& c, const std::vector<int64_t>& off);
 // `coarse` with the chunks, heavy rows and level ranges of `fine` (uploaded; the adjacency and
 // rows are shared).
 DevCSR fine_view(DevicePlan& d, const DevCSR& coarse, const PullCSR& fine);

@@ -44,7 +44,7 @@ void launch_sweep_staged_f32(const SweepParams<float>& p, dim3 grid, cudaStream_
 template <typename S> struct PairDownParams {
     const uint2* ids;    // four 16-bit pattern numbers per (row tile of 32, group, row)
     const uint4* base;   // first pattern of each block, by groups of four
-    const S* table;      // pattern rows, from pattern `base0` on
+    void* table;         // pattern rows, from pattern `base0` on
     S* vals;             // node values (the height-0 rows first)
     void* parts;         // one sum per (item, row, column), or null: rows are written at once
     unsigned* work;      // per column tile: next item (zeroed before the launch)
@@ -58,7 +58,7 @@ template <typename S> struct PairDownParams {
 struct PairDownCall {
     enum Step { kShape, kTable, kGather, kFinish } step = kShape;
     int rows_per_warp = 0, resident_warps = 0;  // kShape
-    size_t part_bytes = 0;
+    size_t part_bytes = 0, table_bytes = 0;     // per element of a sum and of a pattern row
     const uint2* nodes = nullptr;  // kTable: the patterns' parents
     long long count = 0;
     int parts = 0;      // kFinish: sums per row

@@ -49,6 +49,42 @@ template <typename T> T* upload(DevicePlan& d, const std::vector<T>& v) {
     return static_cast<T*>(p);
 }
 
+// Levels with at most this many edges per row on average, and in any one row, run on
+// short_rows_kernel.  Measured on one level of R random rows of d edges, short_rows_kernel against
+// sweep_kernel in microseconds (int32 K=1, float32 K=64, float64 K=20):
+//   R=30,000   d=1  7 / 10 / 14 against 9 / 30 / 106     d=8  7 / 12 / 21 against 11 / 20 / 53
+//              d=16 9 / 19 / 37 against 15 / 22 / 48     d=32 13 / 31 / 67 against 20 / 31 / 54
+//   R=200,000  d=1  7 / 39 / 53 against 11 / 47 / 252    d=8  9 / 55 / 100 against 24 / 76 / 241
+//              d=16 16 / 86 / 194 against 29 / 94 / 256  d=32 36 / 155 / 383 against 34 / 145 / 270
+// (float64 K=64 turns between d=8, 193 against 229, and d=16, 379 against 258).  A row walked by
+// one group of lanes takes about 0.2 us per four edges: the longest allowed ends with the level.
+constexpr long long kShortMean = 8, kShortMost = 128;
+
+}  // namespace
+
+void mark_short_levels(DevicePlan& d, DevCSR& r, const PullCSR& c, const std::vector<int64_t>& off) {
+    r.level_short.assign(c.level_chunk_begin.size(), nullptr);
+    r.level_r0.assign(c.level_chunk_begin.size(), 0);
+    r.level_e0.assign(c.level_chunk_begin.size(), 0);
+    for (size_t l = 0; l < c.level_chunk_begin.size(); l++) {
+        const int64_t rb = c.chunks[static_cast<size_t>(c.level_chunk_begin[l])].r0;
+        const int64_t re = c.chunks[static_cast<size_t>(c.level_chunk_end[l])].r0;
+        if (re <= rb || off[re] - off[rb] > kShortMean * (re - rb) || off[re] - off[rb] > 0x7fffffff) continue;
+        std::vector<unsigned> rel(static_cast<size_t>(re - rb) + 1);
+        bool fits = true;
+        for (int64_t i = rb; i <= re && fits; i++) {
+            rel[static_cast<size_t>(i - rb)] = static_cast<unsigned>(off[i] - off[rb]);
+            fits = i == rb || off[i] - off[i - 1] <= kShortMost;
+        }
+        if (!fits) continue;
+        r.level_short[l] = upload(d, rel);
+        r.level_r0[l] = rb;
+        r.level_e0[l] = off[rb];
+    }
+}
+
+namespace {
+
 DevCSR upload_csr(DevicePlan& d, const PullCSR& c) {
     DevCSR r;
     r.adj = upload(d, c.adj);  // null when the adjacency is built on the device
@@ -67,6 +103,7 @@ DevCSR upload_csr(DevicePlan& d, const PullCSR& c) {
         r.level_rows.push_back(static_cast<long long>(b.r0) - a.r0);
         r.level_edges.push_back(static_cast<long long>(b.e0 - a.e0));
     }
+    if (!c.off.empty()) mark_short_levels(d, r, c, c.off);
     return r;
 }
 
@@ -225,6 +262,8 @@ SweepParams<S> make_params(const DevCSR& c, long long cb, long long ce, const vo
     p.id_base = 0;
     p.src_rows = 0;
     p.col_base = 0;
+    p.short_off = nullptr;
+    p.short_row0 = p.short_rows = 0;
     return p;
 }
 
@@ -244,8 +283,10 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
     const long long base = c.id16 ? c.level_base[level] : 0;
     // One launch of `tiles` column tiles of g lanes from column colBase; its work counters and
     // heavy-row tickets are those of tile slot `slot` onwards.
+    const bool isShort = level < c.level_short.size() && c.level_short[level] != nullptr;
     auto launch = [&](int g, int tiles, int variant, int colBase, int slot) {
-        const dim3 grid(static_cast<unsigned>((ce - cb + 7) / 8), static_cast<unsigned>(tiles));
+        const long long blocks = isShort ? (c.level_rows[level] * g + 255) / 256 : (ce - cb + 7) / 8;
+        const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(tiles));
         auto prm = [&](auto tag) {
             using S = decltype(tag);
             SweepParams<S> p = make_params<S>(c, cb, ce, src, dst, L.stride, rmw, partials, tickets + slot,
@@ -259,6 +300,12 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
             // a split block: 16-bit ids relative to the block's first source id
             p.id16 = c.id16 ? 1 : 0;
             p.id_base = base;
+            if (isShort) {
+                p.adj += c.level_e0[level];
+                p.short_off = c.level_short[level];
+                p.short_row0 = c.level_r0[level];
+                p.short_rows = c.level_rows[level];
+            }
             return p;
         };
         const int vw = L.vw;
@@ -301,6 +348,10 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
             }
             return 1;
         }
+    }
+    if (isShort) {
+        launch(L.g, L.ntiles, 0, 0, 0);
+        return 1;
     }
     // A last column tile under a quarter full costs nearly a full pass at g lanes per row (its
     // warps gather one or two edges per sub-step): it runs as a launch of its own with as few

@@ -160,6 +160,22 @@ __device__ __forceinline__ void df_put(DF* base, long long e, long long stride, 
     f[2] = v.lo;
 }
 
+// a + b of two float pairs with one rounding of the low part, as rounding the float64 sum into a
+// pair has: the high parts' and the low parts' errors are carried exactly until then.
+__device__ __forceinline__ DF df_add(DF a, DF b) {
+    auto two_sum = [](float x, float y, float& s, float& e) {
+        s = __fadd_rn(x, y);
+        const float yy = __fsub_rn(s, x);
+        e = __fadd_rn(__fsub_rn(x, __fsub_rn(s, yy)), __fsub_rn(y, yy));
+    };
+    float s, e, t, f, g, h;
+    two_sum(a.hi, b.hi, s, e);
+    two_sum(a.lo, b.lo, t, f);
+    two_sum(e, t, g, h);
+    const float hi = __fadd_rn(s, g);
+    return {hi, __fadd_rn(__fsub_rn(g, __fsub_rn(hi, s)), __fadd_rn(h, f))};
+}
+
 struct F64Run {
     double acc;
     float hi, lo;

@@ -26,24 +26,47 @@ template <> struct PairPart<AddF64S> {
     static __device__ __forceinline__ void merge(F64Run& a, const T& x) { a.acc += x; }
 };
 
-// a + b of two node values, in storage precision.  Compensated float32 rounds the pair once, like
-// the first level of the plain pre-sums of the sweep (vecacc.cuh); float pairs keep 48 bits.
-template <class Op> __device__ __forceinline__ typename Op::S pair_sum(typename Op::S a, typename Op::S b) {
-    typename Op::A t = Op::zero();
-    Op::add(t, a);
-    Op::add(t, b);
-    return Op::finish(t);
-}
-template <> __device__ __forceinline__ float pair_sum<AddF32C>(float a, float b) { return __fadd_rn(a, b); }
-template <> __device__ __forceinline__ DF pair_sum<AddF64S>(DF a, DF b) {
-    AddF64S::run_add(a.hi, a.lo, b.hi, b.lo);
-    return a;
-}
+// Pattern row elements.  A pair of rows is summed in storage precision: compensated float32 rounds
+// it once, like the first level of the sweep's plain pre-sums (vecacc.cuh); float pairs keep 48
+// bits.  A single compensated column has no pre-sums in the sweep and keeps the pair's error here.
+template <class Op, int VW> struct PairTable {
+    using T = typename Op::S;
+    static __device__ __forceinline__ T sum(typename Op::S a, typename Op::S b) {
+        if constexpr (std::is_same<Op, AddF64S>::value) return df_add(a, b);
+        else if constexpr (std::is_same<Op, AddF32C>::value) return __fadd_rn(a, b);
+        else {
+            typename Op::A t = Op::zero();
+            Op::add(t, a);
+            Op::add(t, b);
+            return Op::finish(t);
+        }
+    }
+};
+template <> struct PairTable<AddF32C, 1> {
+    using T = F32Pair;
+    static __device__ __forceinline__ T sum(float a, float b) {
+        T t;
+        AddF32C::two_sum(a, b, t.hi, t.lo);
+        return t;
+    }
+};
+template <typename T, int VW> struct TableVec : Vec<T, VW> {};
+template <> struct TableVec<F32Pair, 1> {
+    static __device__ __forceinline__ void ld(const F32Pair* p, F32Pair* v) {
+        const float2 t = __ldg(reinterpret_cast<const float2*>(p));
+        v[0] = {t.x, t.y};
+    }
+    static __device__ __forceinline__ void st(F32Pair* p, const F32Pair* v) {
+        *reinterpret_cast<float2*>(p) = make_float2(v[0].hi, v[0].lo);
+    }
+};
 
 template <class Op, int VW>
 __global__ void pair_table_kernel(const uint2* __restrict__ nodes, long long count, const typename Op::S* __restrict__ vals,
-                                  long long stride, typename Op::S* __restrict__ table, const int* gate, int gate_value) {
+                                  long long stride, typename PairTable<Op, VW>::T* __restrict__ table, const int* gate,
+                                  int gate_value) {
     using S = typename Op::S;
+    using T = typename PairTable<Op, VW>::T;
     if (gate != nullptr && *gate != gate_value) return;
     const unsigned vecs = static_cast<unsigned>(stride / VW);
     const unsigned long long total = (unsigned long long)count * vecs;
@@ -57,9 +80,10 @@ __global__ void pair_table_kernel(const uint2* __restrict__ nodes, long long cou
         for (int i = 0; i < VW; i++) a[i] = b[i] = S{};
         if (nd.x != 0x7fffffffu) Vec<S, VW>::ld(vals + (long long)nd.x * stride + col, a);
         if (nd.y != 0x7fffffffu) Vec<S, VW>::ld(vals + (long long)nd.y * stride + col, b);
+        T t[VW];
 #pragma unroll
-        for (int i = 0; i < VW; i++) a[i] = pair_sum<Op>(a[i], b[i]);
-        Vec<S, VW>::st(table + (long long)pat * stride + col, a);
+        for (int i = 0; i < VW; i++) t[i] = PairTable<Op, VW>::sum(a[i], b[i]);
+        TableVec<T, VW>::st(table + (long long)pat * stride + col, t);
     }
 }
 
@@ -83,6 +107,7 @@ constexpr int kPairRows = 2;
 template <class Op, int VW, int G>
 __global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<typename Op::S> p) {
     using S = typename Op::S;
+    using T = typename PairTable<Op, VW>::T;
     using Acc = VecAcc<Op, VW>;
     using Part = PairPart<Op>;
     constexpr int NG = 32 / G, ROWS = kPairRows;
@@ -92,8 +117,8 @@ __global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<
     const int lg = lane / G;
     const int col = blockIdx.y * (G * VW) + (lane % G) * VW;
     const bool colok = col < p.stride;
-    const unsigned rowBytes = static_cast<unsigned>(p.stride * sizeof(S));
-    const char* table = reinterpret_cast<const char*>(p.table + (colok ? col : 0));
+    const unsigned rowBytes = static_cast<unsigned>(p.stride * sizeof(T));
+    const char* table = reinterpret_cast<const char*>(static_cast<const T*>(p.table) + (colok ? col : 0));
     unsigned* counter = p.work + blockIdx.y;
     for (;;) {
         unsigned c = 0;
@@ -125,14 +150,14 @@ __global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<
                 idp[r] += 32;
                 if (q + 1 < q1) next[r] = __ldg(idp[r]);
             }
-            S v[ROWS][4][VW];
+            T v[ROWS][4][VW];
 #pragma unroll
             for (int r = 0; r < ROWS; r++) {
                 const unsigned k[4] = {b.x - p.base0 + (id[r].x & 0xffffu), b.y - p.base0 + (id[r].x >> 16),
                                        b.z - p.base0 + (id[r].y & 0xffffu), b.w - p.base0 + (id[r].y >> 16)};
 #pragma unroll
                 for (int u = 0; u < 4; u++)
-                    Vec<S, VW>::ld(reinterpret_cast<const S*>(table + (unsigned long long)k[u] * rowBytes), v[r][u]);
+                    TableVec<T, VW>::ld(reinterpret_cast<const T*>(table + (unsigned long long)k[u] * rowBytes), v[r][u]);
             }
 #pragma unroll
             for (int r = 0; r < ROWS; r++) acc[r].add_pairs(v[r]);
@@ -199,13 +224,15 @@ template <class Op, int VW, int G> void pair_down_as(PairDownParams<typename Op:
         c.rows_per_warp = (32 / G) * kPairRows;
         c.resident_warps = pair_blocks_per_sm<Op, VW, G>() * 8 * sms;
         c.part_bytes = sizeof(typename PairPart<Op>::T);
+        c.table_bytes = sizeof(typename PairTable<Op, VW>::T);
         return;
     }
     if (c.step == PairDownCall::kTable) {
         const unsigned long long total = (unsigned long long)c.count * (p.stride / VW);
         const unsigned grid = static_cast<unsigned>(std::min<unsigned long long>((total + 255) / 256, sms * 64ull));
-        pair_table_kernel<Op, VW><<<grid, 256, 0, s>>>(c.nodes, c.count, p.vals, p.stride, const_cast<typename Op::S*>(p.table),
-                                                       p.gate, p.gate_value);
+        pair_table_kernel<Op, VW><<<grid, 256, 0, s>>>(c.nodes, c.count, p.vals, p.stride,
+                                                       static_cast<typename PairTable<Op, VW>::T*>(p.table), p.gate,
+                                                       p.gate_value);
         return;
     }
     if (c.step == PairDownCall::kFinish) {

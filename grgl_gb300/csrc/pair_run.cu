@@ -48,7 +48,7 @@ PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit) {
     PairDownRun run;
     PairDownCall shape;
     by_kind(L, [&](auto p, auto fn) { fn(p, shape, L.vw, L.g, sm_count(), nullptr); });
-    const size_t rowBytes = static_cast<size_t>(L.stride) * L.ssize;
+    const size_t rowBytes = static_cast<size_t>(L.stride) * shape.table_bytes;
     const size_t slotBytes = static_cast<size_t>(P.h0) * L.stride * shape.part_bytes;
     const size_t tableMost = std::min(kPairTableBytes, limit / 3);
     // sums held at a time: what the rest of the limit holds, one of them carried between ranges
@@ -92,7 +92,7 @@ int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& r
         fn(p, c, L.vw, L.g, sm_count(), s);
         p.ids = reinterpret_cast<const uint2*>(P.ids);
         p.base = reinterpret_cast<const uint4*>(P.base);
-        p.table = static_cast<decltype(p.table)>(table);
+        p.table = table;
         p.vals = static_cast<decltype(p.vals)>(vals);
         p.parts = run.slots ? parts : nullptr;
         p.rows = P.h0;

@@ -138,6 +138,7 @@ void single_level_csr(PullCSR& P, const std::vector<std::pair<uint32_t, uint32_t
     if (!pairs.empty()) off.push_back(static_cast<int64_t>(pairs.size()));
     if (!P.rows.empty()) chunk_level(P, off, 0, static_cast<int64_t>(P.rows.size()));
     finish_csr(P, off);
+    P.off = std::move(off);
 }
 
 namespace {

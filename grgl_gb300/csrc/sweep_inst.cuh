@@ -9,6 +9,10 @@
 // (split block passes) and the 32-bit one are separate kernels.
 #define GRGX_SWEEP_CASE(OP, VWV, GV, DV)                                              \
     if (vw == VWV && g == GV && variant == DV - 1) {                                  \
+        if (DV == 1 && p.short_off != nullptr) {                                      \
+            short_rows_kernel<OP, VWV, GV><<<grid, 256, 0, s>>>(p);                   \
+            return;                                                                   \
+        }                                                                             \
         static int perSm = 0;                                                         \
         if (perSm == 0) {                                                             \
             int nb = 0;                                                               \

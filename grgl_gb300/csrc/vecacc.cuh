@@ -104,7 +104,16 @@ template <> struct VecAcc<AddF32C, 1> {
         }
         if (N & 1) add(v[N - 1]);
     }
-    __device__ __forceinline__ void add_pairs(const float (*v)[1]) { add_block<4>(v); }
+    // Four pattern rows of the pair form with their errors.
+    __device__ __forceinline__ void add_pairs(const F32Pair (*v)[1]) {
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+            float2 sum, err;
+            two_sum2(hi, make_float2(v[u][0].hi, v[u + 1][0].hi), sum, err);
+            hi = sum;
+            lo = add2(lo, add2(err, make_float2(v[u][0].lo, v[u + 1][0].lo)));
+        }
+    }
     __device__ __forceinline__ void merge(const VecAcc& o) {
         float2 sum, err;
         two_sum2(hi, o.hi, sum, err);
