@@ -35,6 +35,7 @@ struct DevCSR {
     // per level of short rows: its rows' first edges, relative to level_e0 (else null)
     std::vector<unsigned*> level_short;
     std::vector<long long> level_r0, level_e0;
+    std::vector<int> level_most;  // its longest row
     long long n_heavy = 0, n_pieces = 0, n_edges = 0, n_rows = 0;
 };
 
@@ -55,6 +56,7 @@ struct DevicePlan {
     DevCSR up0b, up_int, up0b_f, up_int_f;
     int* fin = nullptr;
     std::vector<long long> fin_begin;
+    bool up_int_built = false;                 // (up_int, fin: also used by the pair form)
     long long split_block = 0, split_src = 0;  // split_src = height-0 ids = first UP row's node id
     bool split_built = false;
     std::map<std::pair<int, long long>, bool> split_choice;  // (storage kind, stride) -> measured choice
@@ -128,6 +130,10 @@ struct SweepCSRs {
 };
 bool fine_chunks(const Layout& L);
 SweepCSRs sweep_csrs(const DevicePlan* dp, const Layout& L);
+// Uploads rows, chunks and heavy rows of P; `adj` (E ids) is on the device already.  blockBase and
+// blockRows set: 16-bit ids, level j = the block of blockRows[j] source ids from blockBase[j] on.
+DevCSR upload_pull(DevicePlan& d, const PullCSR& P, void* adj, long long E,
+                   const std::vector<long long>* blockBase = nullptr, const std::vector<long long>* blockRows = nullptr);
 // Finds the levels of `r` whose rows are short (rows' offsets `off`, chunks of `c`) and uploads their
 // offsets.
 void mark_short_levels(DevicePlan& d, DevCSR& r, const PullCSR& c, const std::vector<int64_t>& off);
@@ -153,6 +159,7 @@ void launch_state_finish(Kind kind, const void* state, void* vals, const int* no
                          int gateValue);
 // Height-0 row bytes (height-0 ids x stride x element size) above which UP runs in split form,
 // and the block of height-0 ids each split pass covers; both adjustable for tests.
+constexpr unsigned long long kDefaultSplitThreshold = 64ull << 20;
 uint64_t split_threshold_bytes();
 long long split_block_size();
 // Whether a call with layout L runs UP in split form: the choice grgx_autotune measured for
@@ -178,10 +185,11 @@ void set_staged(bool on);
 bool staged_layout(const Layout& L);
 // DOWN split form: 0 chosen as above, 1 always (where possible), 2 never (tests).
 void set_down_split_mode(int mode);
+bool down_split_forced();
 
 // Whether a call with layout L runs in pair form (pair_plan.h); builds the form on the first call
 // that may use it.  set_pair_mode: 0 by the rules, 1 wherever possible, 2 never (tests).
-bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L);
+bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
 // Scratch the pair form of a call on this thread may take beyond what the other forms need; a
 // server's worker lowers it to what its batch has reserved (PairScratchScope).
 size_t pair_scratch_limit();
@@ -205,6 +213,25 @@ PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit);
 // Returns the kernels launched.
 int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
                      unsigned* work, cudaStream_t s, const int* gate, int gateValue);
+
+// The launches of an UP call in pair form: ranges of segments, with a table of pattern rows at a
+// time.
+struct PairUpRun {
+    struct Range {
+        size_t s0, s1;  // segments
+    };
+    std::vector<Range> ranges;
+    size_t table_bytes = 0;
+};
+PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit);
+// Writes every node's sum over its height-0 children to vals (onto it when rmw), or leaves it in
+// `state` where one is given.
+int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, void* vals, void* table, void* state,
+                   int rmw, cudaStream_t s, const int* gate, int gateValue);
+// Builds the UP edges to children of height >= 1 (up_int and the finish lists), once: `low` = each
+// UP row's children of height 0.  The caller holds the graph's lock.
+void build_up_internal(DevicePlan& d, const std::vector<unsigned>& low);
+std::vector<unsigned> count_low_children(DevicePlan& d);
 
 // Resolves (once per device, with `device` current) the address of grgx_matmul_noalloc's
 // static scratch, which loads its module and so reserves the array on the device.

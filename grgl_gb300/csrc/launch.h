@@ -72,6 +72,34 @@ void pair_down_f32c(const PairDownParams<float>& p, PairDownCall& c, int vw, int
 void pair_down_f32(const PairDownParams<float>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
 void pair_down_f64s(const PairDownParams<DF>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
 
+// UP in pair form (pair_up.cuh): sums over `count` lists of source rows.
+struct PairList {
+    long long e0;  // first id
+    int len;
+    int out;       // destination row; ~row for a row of the table
+};
+template <typename S> struct PairUpParams {
+    const PairList* lists;
+    long long count;
+    const uint32_t* adj;
+    const S* src;
+    S* table;      // pattern rows
+    S* dst;        // the nodes' rows of sums (added onto when rmw), or
+    int rmw;
+    void* state;   // when set, accumulators (Op::A)
+    int second;    // the sources are rows of the table
+    long long stride;
+    const int* gate;
+    int gate_value;
+};
+void pair_up_u32(const PairUpParams<uint32_t>& p, int vw, int g, cudaStream_t s);
+void pair_up_xor(const PairUpParams<uint32_t>& p, int vw, int g, cudaStream_t s);
+void pair_up_u64(const PairUpParams<unsigned long long>& p, int vw, int g, cudaStream_t s);
+void pair_up_f64(const PairUpParams<double>& p, int vw, int g, cudaStream_t s);
+void pair_up_f32c(const PairUpParams<float>& p, int vw, int g, cudaStream_t s);
+void pair_up_f32(const PairUpParams<float>& p, int vw, int g, cudaStream_t s);
+void pair_up_f64s(const PairUpParams<DF>& p, int vw, int g, cudaStream_t s);
+
 // Column-map modes of the transposing loads/stores.
 enum MapMode { MAP_IDENT = 0, MAP_DIV = 1, MAP_TABLE = 2, MAP_FOLD = 3 };
 

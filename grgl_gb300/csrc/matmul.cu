@@ -11,6 +11,7 @@
 // stream-ordered memory pool and is released on the same stream.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <map>
@@ -66,6 +67,7 @@ void mark_short_levels(DevicePlan& d, DevCSR& r, const PullCSR& c, const std::ve
     r.level_short.assign(c.level_chunk_begin.size(), nullptr);
     r.level_r0.assign(c.level_chunk_begin.size(), 0);
     r.level_e0.assign(c.level_chunk_begin.size(), 0);
+    r.level_most.assign(c.level_chunk_begin.size(), 0);
     for (size_t l = 0; l < c.level_chunk_begin.size(); l++) {
         const int64_t rb = c.chunks[static_cast<size_t>(c.level_chunk_begin[l])].r0;
         const int64_t re = c.chunks[static_cast<size_t>(c.level_chunk_end[l])].r0;
@@ -74,7 +76,9 @@ void mark_short_levels(DevicePlan& d, DevCSR& r, const PullCSR& c, const std::ve
         bool fits = true;
         for (int64_t i = rb; i <= re && fits; i++) {
             rel[static_cast<size_t>(i - rb)] = static_cast<unsigned>(off[i] - off[rb]);
-            fits = i == rb || off[i] - off[i - 1] <= kShortMost;
+            const int64_t len = i == rb ? 0 : off[i] - off[i - 1];
+            fits = len <= kShortMost;
+            r.level_most[l] = std::max(r.level_most[l], static_cast<int>(len));
         }
         if (!fits) continue;
         r.level_short[l] = upload(d, rel);
@@ -264,6 +268,7 @@ SweepParams<S> make_params(const DevCSR& c, long long cb, long long ce, const vo
     p.col_base = 0;
     p.short_off = nullptr;
     p.short_row0 = p.short_rows = 0;
+    p.short_split = 1;
     return p;
 }
 
@@ -285,7 +290,12 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
     // heavy-row tickets are those of tile slot `slot` onwards.
     const bool isShort = level < c.level_short.size() && c.level_short[level] != nullptr;
     auto launch = [&](int g, int tiles, int variant, int colBase, int slot) {
-        const long long blocks = isShort ? (c.level_rows[level] * g + 255) / 256 : (ce - cb + 7) / 8;
+        // one group of lanes per row, more (as many as a warp has) where some row has more than four
+        // batches of edges: at K=1 a row of 50 edges takes one lane 9 us (ten levels of 3 to 50
+        // children, UP K=1 on N=200,000, M=250,000: 40 us of 910)
+        int split = 1;
+        while (isShort && g * split < 32 && c.level_most[level] > 16 * split) split *= 2;
+        const long long blocks = isShort ? (c.level_rows[level] * g * split + 255) / 256 : (ce - cb + 7) / 8;
         const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(tiles));
         auto prm = [&](auto tag) {
             using S = decltype(tag);
@@ -305,6 +315,7 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
                 p.short_off = c.level_short[level];
                 p.short_row0 = c.level_r0[level];
                 p.short_rows = c.level_rows[level];
+                p.short_split = split;
             }
             return p;
         };
@@ -643,10 +654,21 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
         void* vals = sc.get(valBytes);
         // UP in split form when the height-0 rows outgrow L2: their edges first, in blocked
         // passes, then the other edges level by level (up_split.cu)
-        const bool split = !down && use_up_split(g, dp, L);
+        // UP in pair form: the height-0 edges over patterns first (pair_plan.h), the others level by
+        // level from the sums, as in split form
+        PairUpRun urun;
+        size_t upStateBytes = 0;
+        if (!down && pairForm && use_pair_form(g, dp, L, false)) {
+            // compensated float32 keeps the sums as pairs until a node's other children are added;
+            // every other kind adds them onto the node's value
+            upStateBytes = L.kind == Kind::F32C ? static_cast<size_t>(n - dp->pair.h0) * L.stride * L.asize : 0;
+            if (upStateBytes < pair_scratch_limit()) urun = pair_up_run(L, dp, pair_scratch_limit() - upStateBytes);
+        }
+        const bool upair = !urun.ranges.empty();
+        const bool split = !down && !upair && use_up_split(g, dp, L);
         // DOWN: the height-0 level over patterns (pair_plan.h), or in parent blocks (up_split.cu)
         PairDownRun prun;
-        if (down && pairForm && use_pair_form(g, dp, L)) prun = pair_down_run(L, dp, pair_scratch_limit());
+        if (down && pairForm && use_pair_form(g, dp, L, true)) prun = pair_down_run(L, dp, pair_scratch_limit());
         const bool dpair = !prun.ranges.empty();
         const bool dsplit = down && !dpair && use_down_split(g, dp, L);
         // coarse or fine chunking for this row width (the split copies are built by now)
@@ -657,23 +679,29 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
         const DevCSR& cUpInt = *cs.up_int;
         const DevCSR& cDown0b = *cs.down0b;
         long long pieces = down ? std::max(cDown.n_pieces, std::max(dp->seed.n_pieces, dp->miss.n_pieces))
-                                : (split ? std::max(cUp0b.n_pieces, cUpInt.n_pieces) : cUp.n_pieces);
+                                : (split   ? std::max(cUp0b.n_pieces, cUpInt.n_pieces)
+                                   : upair ? cUpInt.n_pieces
+                                           : cUp.n_pieces);
         if (dsplit) pieces = std::max(pieces, cDown0b.n_pieces);
         void* partials = sc.get(static_cast<size_t>(pieces) * L.stride * L.asize);
         const long long nh = down ? (cDown.n_heavy + dp->seed.n_heavy + dp->miss.n_heavy +
                                      (dsplit ? cDown0b.n_heavy : 0))
-                                  : (split ? cUp0b.n_heavy + cUpInt.n_heavy : cUp.n_heavy);
+                                  : (split   ? cUp0b.n_heavy + cUpInt.n_heavy
+                                     : upair ? cUpInt.n_heavy
+                                             : cUp.n_heavy);
         const long long nslots = down ? (2 + static_cast<long long>(cDown.lb.size()) +
                                          (dsplit ? static_cast<long long>(cDown0b.lb.size()) : 0) +
                                          static_cast<long long>(prun.ranges.size()))
-                                      : static_cast<long long>(split ? cUp0b.lb.size() + cUpInt.lb.size()
-                                                                     : cUp.lb.size());
+                                      : static_cast<long long>(split   ? cUp0b.lb.size() + cUpInt.lb.size()
+                                                               : upair ? cUpInt.lb.size()
+                                                                       : cUp.lb.size());
         const long long h0 = static_cast<long long>(dp->level_begin.size() > 1 ? dp->level_begin[1] : 0);
         const size_t stateBytes = split    ? static_cast<size_t>(n - dp->split_src) * L.stride * std::max(L.asize, 8)
+                                  : upair  ? upStateBytes
                                   : dsplit ? static_cast<size_t>(h0) * L.stride * std::max(L.asize, 8)
                                            : 0;
-        void* state = (split || dsplit) ? sc.get(stateBytes) : nullptr;
-        void* ptable = dpair ? sc.get(prun.table_bytes) : nullptr;
+        void* state = stateBytes ? sc.get(stateBytes) : nullptr;
+        void* ptable = (dpair || upair) ? sc.get(dpair ? prun.table_bytes : urun.table_bytes) : nullptr;
         void* pparts = prun.slots ? sc.get(prun.part_bytes) : nullptr;
         // counters per launch and per heavy row: enough column tiles for any launch shape
         const int TS = max_tiles(L);
@@ -813,25 +841,24 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
                 // UP seed: samples <- input columns
                 load_rows(dIn, in_cols, N, by_indiv ? MAP_DIV : MAP_IDENT, P, nullptr, vals, hasInit);
                 if (timed && t_timing) GRGX_CUDA(cudaEventRecord(ev[1], s));
-                if (split) {
-                    GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
-                    unsigned* t0b = tickets;
-                    unsigned* tIn = tickets + cUp0b.n_heavy * TS;
-                    unsigned* w0b = work;
-                    unsigned* wIn = work + cUp0b.lb.size() * TS;
-                    const long long base = dp->split_src;
-                    for (size_t j = 0; j < cUp0b.lb.size(); j++) {
+                if (split || upair) {
+                    if (state) GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
+                    unsigned* tIn = tickets + (upair ? 0 : cUp0b.n_heavy) * TS;
+                    unsigned* wIn = work + (upair ? 0 : cUp0b.lb.size()) * TS;
+                    if (upair)
+                        launches += launch_pair_up(LL, dp, urun, vals, ptable, state, hasInit, s, g, gv);
+                    for (size_t j = 0; split && j < cUp0b.lb.size(); j++) {
                         const LevelShape sh = level_shape(LL, cUp0b, j);
-                        launches += launch_level(LL, cUp0b, j, vals, vals, 0, partials, t0b, w0b + j * TS, s, g,
-                                                 gv, &sh, TS, state, base, 1);
+                        launches += launch_level(LL, cUp0b, j, vals, vals, 0, partials, tickets, work + j * TS, s, g, gv,
+                                                 &sh, TS, state, h0, 1);
                     }
                     for (size_t lvl = 0; lvl < cUpInt.lb.size(); lvl++) {
                         const LevelShape sh = level_shape(LL, cUpInt, lvl);
-                        launches += launch_level(LL, cUpInt, lvl, vals, vals, hasInit, partials, tIn,
-                                                 wIn + lvl * TS, s, g, gv, &sh, TS, state, base, 2);
+                        launches += launch_level(LL, cUpInt, lvl, vals, vals, state ? hasInit : 1, partials, tIn,
+                                                 wIn + lvl * TS, s, g, gv, &sh, TS, state, h0, 2);
                         const long long f0 = dp->fin_begin[lvl], f1 = dp->fin_begin[lvl + 1];
-                        if (f1 > f0) {
-                            launch_state_finish(LL.kind, state, vals, dp->fin + f0, f1 - f0, base, LL.stride, hasInit,
+                        if (state && f1 > f0) {
+                            launch_state_finish(LL.kind, state, vals, dp->fin + f0, f1 - f0, h0, LL.stride, hasInit,
                                                 s, g, gv);
                             launches++;
                         }

@@ -127,6 +127,10 @@ struct AddF32C {
     }
 };
 
+// The same with PRE edges pre-summed in plain float32 where the sweep's block path pre-sums
+// kF32PreSum (vecacc.cuh).
+template <int PRE> struct AddF32CPre : AddF32C {};
+
 // Float64 on GB300 without the FP64 pipe in the inner loop.  Node values are stored as a
 // float pair (hi + lo, 48 significant bits) of the value scaled by 2^-e_k per input row k, so
 // each row's largest input sits in [2^60, 2^61) and every sum stays well inside float range.
@@ -252,5 +256,10 @@ struct AddF64S {
         return split(value(base) + (a.acc + run_value(a)));
     }
 };
+
+// The same with the runs folded into a float pair instead of a double (VecAcc, vecacc.cuh).
+struct AddF64SD : AddF64S {};
+// ... and with no runs: every addition is normalised (df_add).
+struct AddF64SN : AddF64SD {};
 
 }  // namespace grgx

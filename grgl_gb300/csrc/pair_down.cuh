@@ -20,7 +20,7 @@ template <class Op> struct PairPart {
     static __device__ __forceinline__ T of(const typename Op::A& a) { return a; }
     static __device__ __forceinline__ void merge(typename Op::A& a, const T& x) { Op::merge(a, x); }
 };
-template <> struct PairPart<AddF64S> {
+template <> struct PairPart<AddF64SD> {
     using T = double;
     static __device__ __forceinline__ T of(const F64Run& a) { return a.acc + AddF64S::run_value(a); }
     static __device__ __forceinline__ void merge(F64Run& a, const T& x) { a.acc += x; }
@@ -32,7 +32,7 @@ template <> struct PairPart<AddF64S> {
 template <class Op, int VW> struct PairTable {
     using T = typename Op::S;
     static __device__ __forceinline__ T sum(typename Op::S a, typename Op::S b) {
-        if constexpr (std::is_same<Op, AddF64S>::value) return df_add(a, b);
+        if constexpr (std::is_base_of<AddF64S, Op>::value) return df_add(a, b);
         else if constexpr (std::is_same<Op, AddF32C>::value) return __fadd_rn(a, b);
         else {
             typename Op::A t = Op::zero();

@@ -17,6 +17,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cub/device/device_radix_sort.cuh>
+#include <thread>
 #include <vector>
 
 #include "device_plan.h"
@@ -48,6 +50,10 @@ struct Temps {
     void keep(DevicePlan& d, void* p, size_t bytes) {
         d.allocs.push_back(p);
         d.bytes += bytes;
+        ptrs.erase(std::remove(ptrs.begin(), ptrs.end(), p), ptrs.end());
+    }
+    void release(void* p) {
+        cudaFree(p);
         ptrs.erase(std::remove(ptrs.begin(), ptrs.end(), p), ptrs.end());
     }
     ~Temps() {
@@ -89,11 +95,18 @@ __global__ void __launch_bounds__(kThreads) prev_kernel(const uint32_t* __restri
     for (long long q = warm[blockIdx.x]; q < q1; q++) {
         const long long r = seqRow[q], e = off[r + 1];
         int m = -1;
-        for (long long x = off[r] + threadIdx.x; x < e; x += kThreads) {
-            const uint32_t c = adj[x] & 0x7fffffffu;
-            if (c < h0) {
-                m = max(m, last[c]);
-                last[c] = static_cast<int>(q);
+        // (a node's children are distinct: the loads of a batch need not wait for its stores)
+        for (long long x = off[r] + threadIdx.x; x < e; x += 8 * kThreads) {
+            uint32_t c[8];
+            int l[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) c[u] = (x + u * kThreads < e) ? adj[x + u * kThreads] & 0x7fffffffu : 0xffffffffu;
+#pragma unroll
+            for (int u = 0; u < 8; u++) l[u] = c[u] < h0 ? last[c[u]] : -1;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                m = max(m, l[u]);
+                if (c[u] < h0) last[c[u]] = static_cast<int>(q);
             }
         }
         for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -128,12 +141,6 @@ __global__ void fill_parents_kernel(const uint32_t* __restrict__ adj, const long
         }
     }
 }
-
-struct PairBlock {
-    int run;      // first run
-    int q0, q1;   // first position of its runs (q1: of the second)
-    int n0, n1;   // nodes in each (n1 = 0: a block of one run)
-};
 
 // Counts of the block's pairs in `cnt` (n0+1 x n1+1 entries; the empty pair is not counted);
 // returns this thread's count of entries set in the matrix.
@@ -174,20 +181,29 @@ __global__ void __launch_bounds__(kThreads) distinct_kernel(const PairBlock* __r
     }
 }
 
-// Numbers the block's pairs in (first, second) order and writes the patterns' nodes and every
-// height-0 node's pattern.
+// What emit_kernel writes (null: left out).  Patterns are numbered from patBase[block] on.
+struct PairOut {
+    const unsigned* patBase;
+    const int* seqNode;     // new id at each position
+    uint2* nodes;           // each pattern's parents
+    unsigned* count;        // ... and height-0 nodes
+    unsigned short* ids;    // DOWN: each height-0 node's pattern in each block
+    long long groups;
+    unsigned *keys, *vals;  // UP: (pattern, height-0 node), block by block
+};
+
+// Numbers the block's pairs in (first, second) order.
 __global__ void __launch_bounds__(kThreads) emit_kernel(const PairBlock* __restrict__ blocks, int run0, long long blk0,
                                                         unsigned h0, const unsigned short* __restrict__ par,
-                                                        const unsigned* __restrict__ patBase, const int* __restrict__ seqNode,
-                                                        long long groups, uint2* __restrict__ patNodes,
-                                                        unsigned short* __restrict__ ids) {
+                                                        const PairOut out) {
     extern __shared__ unsigned cnt[];
     __shared__ unsigned sums[kThreads / 32];
     const PairBlock B = blocks[blockIdx.x];
-    count_pairs(B, run0, h0, par, cnt);
+    const unsigned set = count_pairs(B, run0, h0, par, cnt);
+    (void)set;
     const int w = B.n1 + 1, size = (B.n0 + 1) * w;
     const long long blk = blk0 + blockIdx.x;
-    const unsigned base = patBase[blockIdx.x];
+    const unsigned base = out.patBase[blockIdx.x];
     // exclusive count of distinct pairs before each thread's contiguous share of the table
     const int per = (size + kThreads - 1) / kThreads, k0 = threadIdx.x * per, k1 = min(size, k0 + per);
     unsigned mine = 0;
@@ -201,12 +217,14 @@ __global__ void __launch_bounds__(kThreads) emit_kernel(const PairBlock* __restr
     __syncthreads();
     unsigned at = 1 + inc - mine;  // number 0 is the empty pair
     for (unsigned v = 0; v < (threadIdx.x >> 5); v++) at += sums[v];
-    if (threadIdx.x == 0) patNodes[base] = make_uint2(INVALID_NODE, INVALID_NODE);
+    if (threadIdx.x == 0 && out.nodes) out.nodes[base] = make_uint2(INVALID_NODE, INVALID_NODE);
     for (int k = k0; k < k1; k++) {
         if (cnt[k] == 0) continue;
         const int i = k / w, j = k % w;
-        patNodes[base + at] = make_uint2(i ? static_cast<unsigned>(seqNode[B.q0 + i - 1]) : INVALID_NODE,
-                                         j ? static_cast<unsigned>(seqNode[B.q1 + j - 1]) : INVALID_NODE);
+        if (out.nodes)
+            out.nodes[base + at] = make_uint2(i ? static_cast<unsigned>(out.seqNode[B.q0 + i - 1]) : INVALID_NODE,
+                                              j ? static_cast<unsigned>(out.seqNode[B.q1 + j - 1]) : INVALID_NODE);
+        if (out.count) out.count[base + at] = cnt[k];
         cnt[k] = at++;
     }
     __syncthreads();
@@ -215,7 +233,25 @@ __global__ void __launch_bounds__(kThreads) emit_kernel(const PairBlock* __restr
     for (unsigned s = threadIdx.x; s < h0; s += kThreads) {
         const int i = a[s], j = B.n1 ? b[s] : 0;
         const unsigned p = (i | j) ? cnt[i * w + j] : 0u;
-        ids[(((long long)(s >> 5) * groups + (blk >> 2)) * 32 + (s & 31)) * 4 + (blk & 3)] = static_cast<unsigned short>(p);
+        if (out.ids)
+            out.ids[(((long long)(s >> 5) * out.groups + (blk >> 2)) * 32 + (s & 31)) * 4 + (blk & 3)] =
+                static_cast<unsigned short>(p);
+        if (out.keys) {
+            // height-0 nodes with the empty pair are sorted past the others
+            out.keys[(long long)blockIdx.x * h0 + s] = p ? base + p : 0x7fffffffu;
+            out.vals[(long long)blockIdx.x * h0 + s] = s;
+        }
+    }
+}
+
+// (position, table row) pairs: the rows' first parents, then their second ones; none = `none`.
+__global__ void node_pairs_kernel(const uint2* __restrict__ nodes, long long rows, unsigned none,
+                                  unsigned* __restrict__ keys, unsigned* __restrict__ vals) {
+    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < rows; p += (long long)gridDim.x * blockDim.x) {
+        const uint2 nd = nodes[p];
+        keys[p] = min(nd.x, none);
+        keys[rows + p] = min(nd.y, none);
+        vals[p] = vals[rows + p] = static_cast<unsigned>(p);
     }
 }
 
@@ -230,91 +266,250 @@ std::vector<int> cut_runs(const std::vector<int>& pv) {
     return start;
 }
 
-void build_pair_plan(DevicePlan& d) {
+// Pairs sorted by key (stable), on the legacy stream; returns the sorted keys and values.
+void sort_pairs(Temps& tmp, unsigned*& keys, unsigned*& vals, unsigned* keys2, unsigned* vals2, long long count, int bits) {
+    cub::DoubleBuffer<unsigned> k(keys, keys2), v(vals, vals2);
+    size_t bytes = 0;
+    GRGX_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, k, v, count, 0, bits));
+    unsigned char* t = tmp.get<unsigned char>(bytes);
+    GRGX_CUDA(cub::DeviceRadixSort::SortPairs(t, bytes, k, v, count, 0, bits));
+    keys = k.Current();
+    vals = v.Current();
+    tmp.release(t);
+}
+
+// The UP lists, by segments: the patterns' pieces (a table row each), the nodes' table rows.
+void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& patBase, const std::vector<unsigned>& counts,
+                    uint32_t* patAdj, long long patEdges, const uint2* nodes) {
     PairPlan& P = d.pair;
+    const long long h0 = static_cast<long long>(d.level_begin[1]);
+    const long long Q = static_cast<long long>(P.seq.size()), nblk = static_cast<long long>(P.blocks.size());
+    std::vector<uint2> patNodes(patBase.back());
+    GRGX_CUDA(cudaMemcpy(patNodes.data(), nodes, patNodes.size() * sizeof(uint2), cudaMemcpyDeviceToHost));
+
+    // Stable sort of lists by length, longest first (a counting sort).
+    auto longest_first = [](PairList* v, size_t count) {
+        int most = 0;
+        for (size_t i = 0; i < count; i++) most = std::max(most, v[i].len);
+        std::vector<size_t> at(most + 2, 0);
+        for (size_t i = 0; i < count; i++) at[most - v[i].len + 1]++;
+        for (int l = 0; l <= most; l++) at[l + 1] += at[l];
+        std::vector<PairList> sorted(count);
+        for (size_t i = 0; i < count; i++) sorted[at[most - v[i].len]++] = v[i];
+        std::copy(sorted.begin(), sorted.end(), v);
+    };
+    const long long nseg = (nblk + kPairSegment - 1) / kPairSegment;
+    auto first_pattern = [&](long long s) { return patBase[std::min(nblk, s * kPairSegment)]; };
+    auto first_position = [&](long long s) {
+        return s * kPairSegment < nblk ? static_cast<long long>(P.blocks[s * kPairSegment].q0) : Q;
+    };
+    auto pieces_of = [](long long c) { return (c + kPairPiece - 1) / kPairPiece; };
+    auto threaded = [&](auto&& fn) {
+        const long long T = std::min<long long>(nseg, std::max(1u, std::min(32u, std::thread::hardware_concurrency())));
+        std::vector<std::thread> pool;
+        for (long long t = 1; t < T; t++)
+            pool.emplace_back([&, t] {
+                for (long long s = t; s < nseg; s += T) fn(s);
+            });
+        for (long long s = 0; s < nseg; s += T) fn(s);
+        for (std::thread& th : pool) th.join();
+    };
+    // position of each UP row in the sequence; a node's patterns are all of its own segment
+    std::vector<unsigned> posOf(d.up_off.size(), 0);
+    for (long long q = 0; q < Q; q++) posOf[P.seq[q]] = static_cast<unsigned>(q);
+    auto position = [&](unsigned node) { return node == INVALID_NODE ? INVALID_NODE : posOf[node - h0]; };
+    std::vector<PairPlan::Segment> segments(nseg + 1);
+    std::vector<long long> edge0(nseg + 1, 0), sub0(nseg + 1, 0), nedge0(nseg + 1, 0);
+    std::vector<unsigned> deg(Q, 0);
+    threaded([&](long long s) {
+        PairPlan::Segment& next = segments[s + 1];
+        for (long long p = first_pattern(s); p < first_pattern(s + 1); p++) {
+            const long long n = pieces_of(counts[p]);
+            edge0[s + 1] += counts[p];
+            next.pat0 += n;
+            for (unsigned q : {position(patNodes[p].x), position(patNodes[p].y)})
+                if (q != INVALID_NODE) deg[q] += static_cast<unsigned>(n);
+        }
+        for (long long q = first_position(s); q < first_position(s + 1); q++) {
+            const long long n = pieces_of(deg[q]);
+            nedge0[s + 1] += deg[q];
+            next.node0 += n;
+            next.top0 += n > 1;
+            sub0[s + 1] += n > 1 ? n : 0;
+        }
+        next.row0 = next.pat0 + sub0[s + 1];
+    });
+    for (long long s = 0; s < nseg; s++) {
+        edge0[s + 1] += edge0[s];
+        nedge0[s + 1] += nedge0[s];
+        sub0[s + 1] += sub0[s];
+        segments[s + 1].row0 += segments[s].row0;
+        segments[s + 1].pat0 += segments[s].pat0;
+        segments[s + 1].node0 += segments[s].node0;
+        segments[s + 1].top0 += segments[s].top0;
+    }
+    const long long rows = segments.back().row0, ne = nedge0.back();
+    GRGX_CHECK(edge0.back() == patEdges && rows < 0x3fffffffLL, GRGX_ERR_UNSUPPORTED, "pair form too large");
+    std::vector<PairList> patLists(segments.back().pat0), nodeLists(segments.back().node0), topLists(segments.back().top0);
+    std::vector<uint2> rowNodes(rows, uint2{INVALID_NODE, INVALID_NODE});
+    std::vector<uint32_t> topAdj(sub0.back());
+    threaded([&](long long s) {
+        const PairPlan::Segment& a = segments[s];
+        long long e = edge0[s], row = a.row0, at = a.pat0;
+        auto cut = [](PairList* out, long long e, long long c, long long n, long long i, int dst) {
+            const long long k0 = c * i / n, k1 = c * (i + 1) / n;
+            *out = {e + k0, static_cast<int>(k1 - k0), dst};
+        };
+        for (long long p = first_pattern(s); p < first_pattern(s + 1); p++) {
+            const long long n = pieces_of(counts[p]);
+            for (long long i = 0; i < n; i++, row++) {
+                cut(&patLists[at++], e, counts[p], n, i, ~static_cast<int>(row));
+                rowNodes[row] = uint2{position(patNodes[p].x), position(patNodes[p].y)};
+            }
+            e += counts[p];
+        }
+        e = nedge0[s];
+        long long node = a.node0, top = a.top0, sub = sub0[s];
+        for (long long q = first_position(s); q < first_position(s + 1); q++) {
+            const long long n = pieces_of(deg[q]);
+            if (n > 1) topLists[top++] = {sub, static_cast<int>(n), P.seq[q]};
+            for (long long i = 0; i < n; i++) {
+                cut(&nodeLists[node++], e, deg[q], n, i, n > 1 ? ~static_cast<int>(row) : P.seq[q]);
+                if (n > 1) topAdj[sub++] = static_cast<uint32_t>(row++);
+            }
+            e += deg[q];
+        }
+        longest_first(patLists.data() + a.pat0, static_cast<size_t>(at - a.pat0));
+        longest_first(nodeLists.data() + a.node0, static_cast<size_t>(node - a.node0));
+    });
+
+    const uint2* dRowNodes = tmp.copy(rowNodes);
+    unsigned *keys = tmp.get<unsigned>(2 * rows), *vals = tmp.get<unsigned>(2 * rows);
+    unsigned *keys2 = tmp.get<unsigned>(2 * rows), *vals2 = tmp.get<unsigned>(2 * rows);
+    node_pairs_kernel<<<blocks_for(rows, 256), 256>>>(dRowNodes, rows, static_cast<unsigned>(Q), keys, vals);
+    GRGX_CUDA(cudaGetLastError());
+    int bits = 1;
+    while ((1LL << bits) <= Q) bits++;
+    sort_pairs(tmp, keys, vals, keys2, vals2, 2 * rows, bits);
+    uint32_t* adj = tmp.get<uint32_t>(ne);
+    GRGX_CUDA(cudaMemcpyAsync(adj, vals, ne * sizeof(uint32_t), cudaMemcpyDeviceToDevice, cudaStreamLegacy));
+    P.pat_lists = tmp.copy(patLists);
+    P.node_lists = tmp.copy(nodeLists);
+    P.top_lists = tmp.copy(topLists);
+    P.top_adj = tmp.copy(topAdj);
+    P.pat_adj = patAdj;
+    P.node_adj = adj;
+    GRGX_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    tmp.keep(d, patAdj, patEdges * sizeof(uint32_t));
+    tmp.keep(d, adj, ne * sizeof(uint32_t));
+    tmp.keep(d, P.top_adj, topAdj.size() * sizeof(uint32_t));
+    tmp.keep(d, P.pat_lists, patLists.size() * sizeof(PairList));
+    tmp.keep(d, P.node_lists, nodeLists.size() * sizeof(PairList));
+    tmp.keep(d, P.top_lists, topLists.size() * sizeof(PairList));
+    P.segments = std::move(segments);
+}
+
+// Everything about the form that needs one pass over the height-0 edges: the analysis on the first
+// call (which may find the form not worth using), and the arrays of the direction asked for.
+void build_pair_plan(DevicePlan& d, bool down) {
+    PairPlan& P = d.pair;
+    const bool first = !P.tried, forced = g_pair_mode.load() == 1;
+    P.tried = true;
     if (d.num_levels < 2 || d.up_off.size() < 2) return;
     const long long h0 = static_cast<long long>(d.level_begin[1]);
     const long long n = static_cast<long long>(d.level_begin[d.num_levels]);
     const long long R = n - h0;
-    const bool forced = g_pair_mode.load() == 1;
     // 16-bit matrix entries and 32-bit positions; small graphs stay as they are
     if (d.up_off.back() < (forced ? 1 : kPairMinEdges) || h0 > 0x3fffffff) return;
+    const unsigned H = static_cast<unsigned>(h0);
     Temps tmp;
-    long long* dOff = reinterpret_cast<long long*>(tmp.copy(d.up_off));
-    unsigned* dLow = tmp.get<unsigned>(R);
-    low_count_kernel<<<blocks_for(R, 8), 256>>>(d.up.adj, dOff, R, static_cast<unsigned>(h0), dLow);
-    GRGX_CUDA(cudaGetLastError());
-    std::vector<unsigned> low(R);
-    std::vector<uint32_t> old2new(n);
-    GRGX_CUDA(cudaMemcpy(low.data(), dLow, R * sizeof(unsigned), cudaMemcpyDeviceToHost));
-    GRGX_CUDA(cudaMemcpy(old2new.data(), d.old2new, n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-
-    // ---- the nodes with height-0 children, in original id order --------------------------------
-    std::vector<int> seqRow, seqNode;
-    std::vector<long long> cum(1, 0);
-    for (long long v = 0; v < n; v++) {
-        const long long r = static_cast<long long>(old2new[v]) - h0;
-        if (r < 0 || low[r] == 0) continue;
-        seqRow.push_back(static_cast<int>(r));
-        seqNode.push_back(static_cast<int>(old2new[v]));
-        cum.push_back(cum.back() + low[r]);
-    }
-    const long long Q = static_cast<long long>(seqRow.size()), E0 = cum.back();
-    if (Q == 0 || E0 < (forced ? 1 : kPairMinEdges) || 2 * E0 < d.up_off.back()) return;
-
-    // ---- runs ------------------------------------------------------------------------------------
-    // stretches of at least 16 average haplotype sets, one thread block each
-    const long long S = std::max<long long>(1, std::min<long long>({2LL * sm_count(), E0 / h0 / 16, (1LL << 30) / h0 + 1, Q}));
-    std::vector<long long> seg, warm;
-    for (long long b = 0; b <= S; b++)
-        seg.push_back(b == S ? Q : std::lower_bound(cum.begin(), cum.end(), E0 * b / S) - cum.begin());
-    for (long long b = 0; b < S; b++)
-        warm.push_back(std::lower_bound(cum.begin(), cum.end(), std::max<long long>(0, cum[seg[b]] - h0)) -
-                       cum.begin());
-    const int* dRow = tmp.copy(seqRow);
-    const int* dNode = tmp.copy(seqNode);
-    std::vector<int> pv(Q);
-    {
-        Temps t2;
-        const long long* dSeg = t2.copy(seg);
-        const long long* dWarm = t2.copy(warm);
-        int* last = t2.get<int>(S * h0);
-        int* dPv = t2.get<int>(Q);
-        GRGX_CUDA(cudaMemsetAsync(last, 0xff, S * h0 * sizeof(int), cudaStreamLegacy));
-        prev_kernel<<<static_cast<unsigned>(S), kThreads>>>(d.up.adj, dOff, dRow, dSeg, dWarm, static_cast<unsigned>(h0), last,
-                                                            dPv);
-        GRGX_CUDA(cudaGetLastError());
-        GRGX_CUDA(cudaMemcpy(pv.data(), dPv, Q * sizeof(int), cudaMemcpyDeviceToHost));
-    }
-    const std::vector<int> run = cut_runs(pv);
-    const int nruns = static_cast<int>(run.size()) - 1;
-
-    // ---- blocks ----------------------------------------------------------------------------------
-    std::vector<PairBlock> blocks;
-    for (int r = 0; r < nruns;) {
-        PairBlock B{r, run[r], 0, run[r + 1] - run[r], 0};
-        if (r + 1 < nruns && (B.n0 + 1LL) * (run[r + 2] - run[r + 1] + 1) <= kMaxPairs) {
-            B.q1 = run[r + 1];
-            B.n1 = run[r + 2] - run[r + 1];
+    const long long* dOff = reinterpret_cast<long long*>(tmp.copy(d.up_off));
+    if (first) {
+        P.low = count_low_children(d);
+        std::vector<uint32_t> old2new(n);
+        GRGX_CUDA(cudaMemcpy(old2new.data(), d.old2new, n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+        // the nodes with height-0 children, in original id order
+        for (long long v = 0; v < n; v++) {
+            const long long r = static_cast<long long>(old2new[v]) - h0;
+            if (r >= 0 && P.low[r]) P.seq.push_back(static_cast<int>(r));
         }
-        r += B.n1 ? 2 : 1;
-        blocks.push_back(B);
     }
-    const long long nblk = static_cast<long long>(blocks.size());
-    if (!forced && static_cast<double>(nblk) * h0 > kPairMaxCost * static_cast<double>(E0)) return;
+    const long long Q = static_cast<long long>(P.seq.size());
+    std::vector<long long> cum(1, 0);
+    for (int r : P.seq) cum.push_back(cum.back() + P.low[r]);
+    const long long E0 = cum.back();
+    if (Q == 0 || E0 < (forced ? 1 : kPairMinEdges) || 2 * E0 < d.up_off.back()) return;
+    const int* dRow = tmp.copy(P.seq);
 
-    // ---- patterns, a batch of blocks at a time -----------------------------------------------------
-    std::vector<int> runOf(Q);
+    if (first) {
+        // ---- runs: stretches of at least 6 average haplotype sets, one thread block each -----------
+        const long long S =
+            std::max<long long>(1, std::min<long long>({2LL * sm_count(), E0 / h0 / 6, (1LL << 30) / h0 + 1, Q}));
+        std::vector<long long> seg, warm;
+        for (long long b = 0; b <= S; b++)
+            seg.push_back(b == S ? Q : std::lower_bound(cum.begin(), cum.end(), E0 * b / S) - cum.begin());
+        for (long long b = 0; b < S; b++)
+            warm.push_back(std::lower_bound(cum.begin(), cum.end(), std::max<long long>(0, cum[seg[b]] - h0)) - cum.begin());
+        std::vector<int> pv(Q);
+        {
+            Temps t2;
+            const long long* dSeg = t2.copy(seg);
+            const long long* dWarm = t2.copy(warm);
+            int* last = t2.get<int>(S * h0);
+            int* dPv = t2.get<int>(Q);
+            GRGX_CUDA(cudaMemsetAsync(last, 0xff, S * h0 * sizeof(int), cudaStreamLegacy));
+            prev_kernel<<<static_cast<unsigned>(S), kThreads>>>(d.up.adj, dOff, dRow, dSeg, dWarm, H, last, dPv);
+            GRGX_CUDA(cudaGetLastError());
+            GRGX_CUDA(cudaMemcpy(pv.data(), dPv, Q * sizeof(int), cudaMemcpyDeviceToHost));
+        }
+        P.run = cut_runs(pv);
+        // ---- blocks --------------------------------------------------------------------------------
+        const int nruns = static_cast<int>(P.run.size()) - 1;
+        for (int r = 0; r < nruns;) {
+            PairBlock B{r, P.run[r], 0, P.run[r + 1] - P.run[r], 0};
+            if (r + 1 < nruns && (B.n0 + 1LL) * (P.run[r + 2] - P.run[r + 1] + 1) <= kMaxPairs) {
+                B.q1 = P.run[r + 1];
+                B.n1 = P.run[r + 2] - P.run[r + 1];
+            }
+            r += B.n1 ? 2 : 1;
+            P.blocks.push_back(B);
+        }
+    }
+    const std::vector<int>& run = P.run;
+    const std::vector<PairBlock>& blocks = P.blocks;
+    const int nruns = static_cast<int>(run.size()) - 1;
+    const long long nblk = static_cast<long long>(blocks.size());
+    const double edges = static_cast<double>(E0);
+    if (!forced && static_cast<double>(nblk) * h0 > kPairMaxCost * edges) return;
+
+    // ---- patterns, a batch of blocks at a time -------------------------------------------------------
+    std::vector<int> runOf(Q), seqNode(Q);
     for (int r = 0; r < nruns; r++) std::fill(runOf.begin() + run[r], runOf.begin() + run[r + 1], r);
+    for (long long q = 0; q < Q; q++) seqNode[q] = static_cast<int>(P.seq[q] + h0);
     const int* dRunOf = tmp.copy(runOf);
     const int* dRun = tmp.copy(run);
+    const int* dNode = tmp.copy(seqNode);
     const PairBlock* dBlocks = tmp.copy(blocks);
     const long long groups = (nblk + 3) / 4;
     const long long tiles = (h0 + 127) / 128 * 4;  // whole groups of 128 nodes: a warp's largest share
-    const size_t idBytes = static_cast<size_t>(tiles) * groups * 128 * sizeof(unsigned short);
-    unsigned short* ids = tmp.get<unsigned short>(idBytes / sizeof(unsigned short));
-    GRGX_CUDA(cudaMemsetAsync(ids, 0, idBytes, cudaStreamLegacy));
     const long long batch = std::max<long long>(1, std::min(nblk, (1LL << 27) / h0));
+    const size_t idBytes = static_cast<size_t>(tiles) * groups * 128 * sizeof(unsigned short);
+    PairOut out{};
+    out.seqNode = dNode;
+    out.groups = groups;
+    uint32_t* upAdj = nullptr;
+    unsigned *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr;
+    long long upEdges = 0;
+    if (down) {
+        out.ids = tmp.get<unsigned short>(idBytes / sizeof(unsigned short));
+        GRGX_CUDA(cudaMemsetAsync(out.ids, 0, idBytes, cudaStreamLegacy));
+    } else {
+        upAdj = tmp.get<uint32_t>(nblk * h0);
+        keys = tmp.get<unsigned>(batch * h0);
+        vals = tmp.get<unsigned>(batch * h0);
+        keys2 = tmp.get<unsigned>(batch * h0);
+        vals2 = tmp.get<unsigned>(batch * h0);
+    }
     unsigned short* par = tmp.get<unsigned short>(2 * batch * h0);
     unsigned* dNpat = tmp.get<unsigned>(batch);
     unsigned* dBase = tmp.get<unsigned>(batch);
@@ -328,11 +523,11 @@ void build_pair_plan(DevicePlan& d) {
         long long count;
     };
     std::vector<Part> parts;
+    std::vector<unsigned> counts;  // UP: each pattern's height-0 nodes
     for (long long b0 = 0; b0 < nblk; b0 += batch) {
         const long long b1 = std::min(nblk, b0 + batch), nb = b1 - b0;
         const PairBlock& last = blocks[b1 - 1];
         const int run0 = blocks[b0].run, run1 = last.run + (last.n1 ? 2 : 1);
-        const unsigned H = static_cast<unsigned>(h0);
         GRGX_CUDA(cudaMemsetAsync(par, 0, static_cast<size_t>(run1 - run0) * h0 * sizeof(unsigned short), cudaStreamLegacy));
         fill_parents_kernel<<<blocks_for(run[run1] - run[run0], 8), 256>>>(d.up.adj, dOff, dRow, dRunOf, dRun, run[run0],
                                                                            run[run1], run0, H, par);
@@ -343,7 +538,7 @@ void build_pair_plan(DevicePlan& d) {
         GRGX_CUDA(cudaGetLastError());
         std::vector<unsigned> npat(nb), rel(nb);
         GRGX_CUDA(cudaMemcpy(npat.data(), dNpat, nb * sizeof(unsigned), cudaMemcpyDeviceToHost));
-        unsigned long long total = 0;
+        long long total = 0;
         for (long long b = 0; b < nb; b++) {
             rel[b] = static_cast<unsigned>(total);
             total += npat[b];
@@ -355,60 +550,110 @@ void build_pair_plan(DevicePlan& d) {
                                        kPairMaxCost * static_cast<double>(cum[run[run1]] - cum[run[run0]])))
             return;
         GRGX_CUDA(cudaMemcpy(dBase, rel.data(), nb * sizeof(unsigned), cudaMemcpyHostToDevice));
-        parts.push_back({tmp.get<uint2>(total), static_cast<long long>(total)});
-        emit_kernel<<<static_cast<unsigned>(nb), kThreads, most>>>(dBlocks + b0, run0, b0, H, par, dBase, dNode, groups,
-                                                                   parts.back().nodes, ids);
+        out.patBase = dBase;
+        parts.push_back({tmp.get<uint2>(total), total});
+        out.nodes = parts.back().nodes;
+        if (!down) {
+            out.keys = keys;
+            out.vals = vals;
+            out.count = tmp.get<unsigned>(total);
+            GRGX_CUDA(cudaMemsetAsync(out.count, 0, total * sizeof(unsigned), cudaStreamLegacy));
+        }
+        emit_kernel<<<static_cast<unsigned>(nb), kThreads, most>>>(dBlocks + b0, run0, b0, H, par, out);
         GRGX_CUDA(cudaGetLastError());
+        if (!down) {
+            const size_t at = counts.size();
+            counts.resize(at + total);
+            GRGX_CUDA(cudaMemcpy(counts.data() + at, out.count, total * sizeof(unsigned), cudaMemcpyDeviceToHost));
+            long long have = 0;
+            for (size_t p = at; p < counts.size(); p++) have += counts[p];
+            unsigned *k = keys, *v = vals;
+            int bits = 1;
+            while ((1LL << bits) <= total) bits++;
+            // (the empty pair's key has every bit set: it sorts last within any number of bits)
+            sort_pairs(tmp, k, v, keys2, vals2, nb * h0, bits);
+            GRGX_CUDA(cudaMemcpyAsync(upAdj + upEdges, v, have * sizeof(uint32_t), cudaMemcpyDeviceToDevice, cudaStreamLegacy));
+            upEdges += have;
+            tmp.release(out.count);
+        }
     }
     unsigned long long set = 0;
     GRGX_CUDA(cudaMemcpy(&set, dSet, sizeof(set), cudaMemcpyDeviceToHost));
     // every edge has its entry: no height-0 node has two parents in one run, or the same one twice
     if (static_cast<long long>(set) != E0) return;
-    P.npat = patBase.back();
-    if (!forced && nblk * h0 + kPairPatternCost * static_cast<double>(P.npat) > kPairMaxCost * static_cast<double>(E0)) return;
+    const long long npat = patBase.back();
+    if (!forced && nblk * h0 + kPairPatternCost * static_cast<double>(npat) > kPairMaxCost * edges) return;
 
-    uint2* nodes = tmp.get<uint2>(P.npat);
+    uint2* nodes = tmp.get<uint2>(npat);
     long long at = 0;
     for (const Part& p : parts) {
         GRGX_CUDA(cudaMemcpyAsync(nodes + at, p.nodes, p.count * sizeof(uint2), cudaMemcpyDeviceToDevice, cudaStreamLegacy));
         at += p.count;
     }
-    std::vector<unsigned> base(groups * 4, 0);  // padding blocks point at an empty pair
-    for (long long b = 0; b < nblk; b++) base[b] = static_cast<unsigned>(patBase[b]);
-    for (long long b = nblk; b < groups * 4; b++) base[b] = base[nblk - 1];
-    unsigned* dB = tmp.copy(base);
-    GRGX_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
-    tmp.keep(d, ids, idBytes);
-    tmp.keep(d, nodes, P.npat * sizeof(uint2));
-    tmp.keep(d, dB, base.size() * sizeof(unsigned));
+    if (down) {
+        std::vector<unsigned> base(groups * 4);
+        for (long long b = 0; b < groups * 4; b++)  // padding blocks point at an empty pair
+            base[b] = static_cast<unsigned>(patBase[std::min(b, nblk - 1)]);
+        unsigned* dB = tmp.copy(base);
+        GRGX_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+        tmp.keep(d, out.ids, idBytes);
+        tmp.keep(d, nodes, npat * sizeof(uint2));
+        tmp.keep(d, dB, base.size() * sizeof(unsigned));
+        P.base = dB;
+        P.pat_nodes = nodes;
+        P.ids = out.ids;
+        P.down_built = true;
+    } else {
+        build_up_internal(d, P.low);
+        build_up_lists(d, tmp, patBase, counts, upAdj, upEdges, nodes);
+        P.up_built = true;
+    }
     P.h0 = h0;
     P.nblk = nblk;
+    P.npat = npat;
     P.pat_base = std::move(patBase);
-    P.base = dB;
-    P.pat_nodes = nodes;
-    P.ids = ids;
     P.usable = true;
 }
 
 }  // namespace
 
+std::vector<unsigned> count_low_children(DevicePlan& d) {
+    Temps tmp;
+    const long long R = static_cast<long long>(d.up_off.size()) - 1;
+    std::vector<unsigned> low(R);
+    const long long* dOff = reinterpret_cast<long long*>(tmp.copy(d.up_off));
+    unsigned* dLow = tmp.get<unsigned>(R);
+    low_count_kernel<<<blocks_for(R, 8), 256>>>(d.up.adj, dOff, R, static_cast<unsigned>(d.level_begin[1]), dLow);
+    GRGX_CUDA(cudaGetLastError());
+    GRGX_CUDA(cudaMemcpy(low.data(), dLow, R * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    return low;
+}
+
 void set_pair_mode(int mode) { g_pair_mode.store(mode); }
 
-bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout&) {
+bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
     const int mode = g_pair_mode.load();
     if (mode == 2) return false;
+    // (a split form asked for by its test hooks)
+    if (mode == 0 && (down ? down_split_forced() : split_threshold_bytes() != kDefaultSplitThreshold)) return false;
+    // UP, a single 4-byte column: gathers from the height-0 values run at about one per SM clock
+    // however narrow, and the staged split passes at two edges per clock (int32 0.62 ms against
+    // 1.0, N=200,000, M=250,000); compensated sums would lose the pattern rows' roundings.
+    if (!down && L.stride == 1 && (L.kind == Kind::F32C || (staged_layout(L) && up_split_possible(dp)))) return false;
     std::lock_guard<std::mutex> lk(g->mu);
-    if (!dp->pair.tried) {
-        dp->pair.tried = true;
+    PairPlan& P = dp->pair;
+    bool& built = down ? P.down_built : P.up_built;
+    if (!P.tried || (P.usable && !built)) {
         try {
-            build_pair_plan(*dp);
+            build_pair_plan(*dp, down);
         } catch (const Error& e) {
             // no memory for it: the other forms need none of this
             if (e.code != GRGX_ERR_OUT_OF_MEMORY) throw;
             cudaGetLastError();
+            P.usable = P.usable && (P.down_built || P.up_built);
         }
     }
-    return dp->pair.usable;
+    return P.usable && built;
 }
 
 }  // namespace grgx

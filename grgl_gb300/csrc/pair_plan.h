@@ -16,14 +16,31 @@
 #include <cstdint>
 #include <vector>
 
+#include "launch.h"
+
 namespace grgx {
 
-// Graphs with fewer edges between height-0 nodes and parents keep the other forms.
-constexpr long long kPairMinEdges = 1LL << 22;
+// Graphs with fewer edges between height-0 nodes and parents keep the other forms: their calls are
+// a chain of launches either way (N=20,000, M=5,000, 1e6 edges: int32 K=5 UP 77 us against 56 in
+// pair form, DOWN 57 against 47; building it takes 4 ms).
+constexpr long long kPairMinEdges = 1000000;
 // The form is used when its gathers -- one per block and height-0 node, kPairPatternCost per
 // pattern (two reads, a write and the table's own traffic) -- are at most this share of one per edge.
 constexpr double kPairPatternCost = 4.0;
-constexpr double kPairMaxCost = 0.75;
+// (N=5,000, M=50,000: 0.86; float64 K=20 UP 0.32 against 0.20 ms, DOWN 0.172 against 0.160.)
+constexpr double kPairMaxCost = 0.9;
+
+// UP: lists (a pattern's height-0 nodes, a node's table rows) are summed in pieces of at most this
+// many, each with a row of its own in the table; it bounds how long one group of lanes works on one.
+constexpr long long kPairPiece = 256;
+// Blocks whose lists are sorted by length together, longest first (the order they are launched in).
+constexpr long long kPairSegment = 64;
+
+// One block: its runs' first positions in the sequence of nodes with height-0 children, and their
+// node counts (n1 = 0: a block of one run).
+struct PairBlock {
+    int run, q0, q1, n0, n1;
+};
 
 struct PairPlan {
     bool tried = false;   // the analysis ran (once per graph)
@@ -32,11 +49,29 @@ struct PairPlan {
     long long nblk = 0;
     long long npat = 0;
     std::vector<long long> pat_base;  // first pattern of each block (nblk + 1)
-    unsigned* base = nullptr;         // the same on the device, padded to whole groups of four blocks
+    // kept for the second direction's arrays: the sequence (UP rows), its runs and blocks, and
+    // each UP row's height-0 children
+    std::vector<int> seq, run;
+    std::vector<PairBlock> blocks;
+    std::vector<unsigned> low;
+    // DOWN, on the first DOWN call:
+    bool down_built = false;
+    unsigned* base = nullptr;         // pat_base on the device, padded to whole groups of four blocks
     uint2* pat_nodes = nullptr;       // the pattern's two parents (new ids, INVALID_NODE = none)
-    // DOWN: each height-0 node's pattern within each block (0: the empty pair), 16 bits, ordered
+    // each height-0 node's pattern within each block (0: the empty pair), 16 bits, ordered
     // [tile of 32 nodes][group of four blocks][node][block]: a node's four ids are one 8-byte load
     unsigned short* ids = nullptr;
+    // UP, on the first UP call: lists of height-0 nodes (the patterns' pieces, a table row each), of
+    // table rows (the nodes, and the pieces of nodes with many), and of such pieces' rows (those
+    // nodes), by segments of blocks.
+    bool up_built = false;
+    struct Segment {
+        long long row0 = 0;                       // first table row
+        long long pat0 = 0, node0 = 0, top0 = 0;  // first list of each kind
+    };
+    std::vector<Segment> segments;                // + the end
+    PairList *pat_lists = nullptr, *node_lists = nullptr, *top_lists = nullptr;
+    uint32_t *pat_adj = nullptr, *node_adj = nullptr, *top_adj = nullptr;
 };
 
 }  // namespace grgx

@@ -64,6 +64,7 @@ template <typename S> struct SweepParams {
     // `adj` (short_rows + 1 entries), and the level's first row.
     const unsigned* short_off;
     long long short_row0, short_rows;
+    int short_split;           // groups of lanes that share a row's edges (a power of two)
     // First column of the launch's tile 0 (a launch of the last, narrow tile starts past the
     // full tiles of another launch).
     int col_base;
@@ -181,6 +182,7 @@ template <class Op> struct ChainTraits {
 template <> struct ChainTraits<AddF64S> {
     static constexpr bool kChains = true;
 };
+template <> struct ChainTraits<AddF64SD> : ChainTraits<AddF64S> {};
 
 // Edge-id ring of a staged warp (16-bit ids): kRingStages steps of 256 ids in flight, each step's
 // ids copied global -> shared by cp.async (16 bytes per lane, 16-byte aligned, so a step's copy
@@ -530,20 +532,28 @@ __global__ void __launch_bounds__(256, SweepOccupancy<Op, VW, G, D>::kBlocks) sw
 // rows one boundary after the other within a chunk, a chain of dependent steps that sets the
 // launch's time however few edges the level has: float64 K=20 on N=20,000, M=50,000, 130-150 us for
 // a DOWN level of a few thousand one-edge rows.  Bound by the latency of three dependent loads.
+// A level with longer rows among them has `short_split` groups of lanes to a row, which take its
+// edges in turns of four and merge their sums at the end.
 template <class Op, int VW, int G>
 __global__ void __launch_bounds__(256) short_rows_kernel(const SweepParams<typename Op::S> p) {
     using S = typename Op::S;
     constexpr bool kPairs = std::is_same<Op, AddF64S>::value;
     constexpr int BATCH = 4;
     if (p.gate != nullptr && *p.gate != p.gate_value) return;
-    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int split = p.short_split;
+    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long row = thread / (G * split);
+    const int sub = static_cast<int>(thread / G) & (split - 1);
     const int col = blockIdx.y * (G * VW) + (threadIdx.x % G) * VW;
-    if (row >= p.short_rows || col >= p.stride) return;
-    unsigned e = __ldg(p.short_off + row);
-    const unsigned end = __ldg(p.short_off + row + 1);
+    const bool live = row < p.short_rows && col < p.stride;
+    unsigned e = 0, end = 0;
+    if (live) {
+        e = __ldg(p.short_off + row) + BATCH * sub;
+        end = __ldg(p.short_off + row + 1);
+    }
     ScalarAcc<Op, VW> acc;
     acc.zero();
-    for (; e < end; e += BATCH) {
+    for (; e < end; e += BATCH * split) {
         uint32_t id[BATCH];
         S v[BATCH][VW];
 #pragma unroll
@@ -572,6 +582,20 @@ __global__ void __launch_bounds__(256) short_rows_kernel(const SweepParams<typen
                 if (e + u < end) acc.add(v[u]);
         }
     }
+    for (int m = G; m < G * split; m <<= 1) {
+        const ScalarAcc<Op, VW> t = acc.shfl_xor(m);
+        if constexpr (kPairs) {
+#pragma unroll
+            for (int i = 0; i < VW; i++) {
+                const DF r = df_add(DF{acc.a[i].hi, acc.a[i].lo}, DF{t.a[i].hi, t.a[i].lo});
+                acc.a[i].hi = r.hi;
+                acc.a[i].lo = r.lo;
+            }
+        } else {
+            acc.merge(t);
+        }
+    }
+    if (!live || sub != 0) return;
     if constexpr (kPairs) {
         if (p.state == nullptr) {
             DF* d = p.dst + (long long)p.rows[p.short_row0 + row] * p.stride + col;

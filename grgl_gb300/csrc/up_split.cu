@@ -51,7 +51,7 @@ namespace {
                         std::string(#call) + ": " + cudaGetErrorString(e__));                        \
     } while (0)
 
-std::atomic<unsigned long long> g_threshold{64ull << 20};
+std::atomic<unsigned long long> g_threshold{kDefaultSplitThreshold};
 std::atomic<long long> g_block{32768};  // at most 32768: block-relative ids fit in 15 bits
 std::atomic<bool> g_staged{true};
 std::atomic<int> g_down_mode{0};  // DOWN split form: 0 by the rule below, 1 always, 2 never
@@ -89,28 +89,42 @@ __global__ void segment_kernel(const uint32_t* __restrict__ adj, const long long
 }
 
 // One warp per row: every edge of the row's block segments to its place in the block passes'
-// copy, as a 16-bit id relative to its block (bit 15 on the first edge of each segment), and
-// (UP) the rest of the row to its internal run, HEAD_BIT on the run's first edge.
+// copy, as a 16-bit id relative to its block (bit 15 on the first edge of each segment).
 __global__ void scatter_kernel(const uint32_t* __restrict__ adj, const long long* __restrict__ off, long long R,
                                int nb, long long block, long long key0, const uint32_t* __restrict__ seg,
-                               const long long* __restrict__ dst0, const long long* __restrict__ dstI,
-                               unsigned short* __restrict__ out0, uint32_t* __restrict__ outI) {
+                               const long long* __restrict__ dst0, unsigned short* __restrict__ out0) {
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < R; i += warps) {
-        const long long b0 = off[i], deg = off[i + 1] - b0;
-        const long long p = seg[i * (nb + 1) + nb];
-        for (long long k = lane; k < deg; k += 32) {
+        const long long b0 = off[i], p = seg[i * (nb + 1) + nb];
+        for (long long k = lane; k < p; k += 32) {
             const uint32_t c = adj[b0 + k] & 0x7fffffffu;
-            if (k < p) {
-                const int b = static_cast<int>((static_cast<long long>(c) - key0) / block);
-                const long long rel = k - seg[i * (nb + 1) + b];
-                const uint32_t id = static_cast<uint32_t>(static_cast<long long>(c) - key0 - b * block);
-                out0[dst0[i * nb + b] + rel] = static_cast<unsigned short>(id | (rel == 0 ? 0x8000u : 0u));
-            } else {
-                const long long rel = k - p;
-                outI[dstI[i] + rel] = c | (rel == 0 ? HEAD_BIT : 0u);
-            }
+            const int b = static_cast<int>((static_cast<long long>(c) - key0) / block);
+            const long long rel = k - seg[i * (nb + 1) + b];
+            const uint32_t id = static_cast<uint32_t>(static_cast<long long>(c) - key0 - b * block);
+            out0[dst0[i * nb + b] + rel] = static_cast<unsigned short>(id | (rel == 0 ? 0x8000u : 0u));
+        }
+    }
+}
+
+// One warp per row: its edges to children of height >= 1 (ids from h0 on), in order, to the row's
+// internal run; HEAD_BIT on the run's first edge.
+__global__ void internal_kernel(const uint32_t* __restrict__ adj, const long long* __restrict__ off, long long R,
+                                uint32_t h0, const long long* __restrict__ dst, uint32_t* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < R; i += warps) {
+        long long w = dst[i];
+        if (w < 0) continue;
+        bool first = true;
+        for (long long k = off[i]; k < off[i + 1]; k += 32) {
+            const uint32_t c = (k + lane < off[i + 1]) ? adj[k + lane] & 0x7fffffffu : 0u;
+            const bool mine = k + lane < off[i + 1] && c >= h0;
+            const unsigned m = __ballot_sync(0xffffffffu, mine);
+            const int rank = __popc(m & ((1u << lane) - 1u));
+            if (mine) out[w + rank] = c | (first && rank == 0 ? HEAD_BIT : 0u);
+            w += __popc(m);
+            first = first && m == 0;
         }
     }
 }
@@ -145,9 +159,10 @@ void finish_as(const void* state, void* vals, const int* nodes, long long count,
         rmw, gate, gateValue);
 }
 
-// `blockBase`/`blockRows` set: 16-bit ids, level j = the block starting at blockBase[j].
-DevCSR upload_pull(DevicePlan& d, PullCSR& P, void* adj, long long E, const std::vector<long long>* blockBase = nullptr,
-                   const std::vector<long long>* blockRows = nullptr) {
+}  // namespace
+
+DevCSR upload_pull(DevicePlan& d, const PullCSR& P, void* adj, long long E, const std::vector<long long>* blockBase,
+                   const std::vector<long long>* blockRows) {
     auto up = [&](const auto& v) -> void* {
         if (v.empty()) return nullptr;
         void* p = nullptr;
@@ -182,8 +197,6 @@ DevCSR upload_pull(DevicePlan& d, PullCSR& P, void* adj, long long E, const std:
     return r;
 }
 
-}  // namespace
-
 uint64_t split_threshold_bytes() { return g_threshold.load(); }
 long long split_block_size() { return g_block.load(); }
 
@@ -198,6 +211,7 @@ bool staged_layout(const Layout& L) {
            (L.kind == Kind::U32 || L.kind == Kind::XOR || L.kind == Kind::F32C || L.kind == Kind::F32);
 }
 void set_staged(bool on) { g_staged.store(on); }
+bool down_split_forced() { return g_down_mode.load() != 0; }
 void set_down_split_mode(int mode) { g_down_mode.store(mode); }
 
 void launch_state_finish(Kind kind, const void* state, void* vals, const int* nodes, long long count,
@@ -243,7 +257,73 @@ long long block_layout(PullCSR& P0, const std::vector<uint32_t>& seg, long long 
     return off0.back();
 }
 
-// Builds d.up0b / d.up_int / d.fin from the resident UP CSR (rows = nodes level_begin[1] .. n-1
+}  // namespace
+
+// Internal edges: one level per UP level (heights 1..H-1), plus the finish lists.
+void build_up_internal(DevicePlan& d, const std::vector<unsigned>& low) {
+    if (d.up_int_built) return;
+    const long long src0 = static_cast<long long>(d.level_begin[1]);
+    const long long R = static_cast<long long>(d.level_begin[d.num_levels]) - src0;
+    const std::vector<int64_t>& off = d.up_off;
+    PullCSR PI;
+    std::vector<int64_t> offI(1, 0), rowBeginI;
+    std::vector<long long> dstI(static_cast<size_t>(R), -1);
+    std::vector<int> fin;
+    std::vector<long long> finBegin;
+    for (uint64_t h = 1; h < d.num_levels; h++) {
+        rowBeginI.push_back(static_cast<int64_t>(PI.rows.size()));
+        finBegin.push_back(static_cast<long long>(fin.size()));
+        for (long long node = static_cast<long long>(d.level_begin[h]);
+             node < static_cast<long long>(d.level_begin[h + 1]); node++) {
+            const long long i = node - src0;
+            const long long len = (off[i + 1] - off[i]) - low[static_cast<size_t>(i)];
+            if (len <= 0) {
+                fin.push_back(static_cast<int>(node));
+                continue;
+            }
+            dstI[static_cast<size_t>(i)] = offI.back();
+            PI.rows.push_back(static_cast<int32_t>(node));
+            offI.push_back(offI.back() + len);
+        }
+    }
+    rowBeginI.push_back(static_cast<int64_t>(PI.rows.size()));
+    finBegin.push_back(static_cast<long long>(fin.size()));
+    for (size_t h = 0; h + 1 < rowBeginI.size(); h++) chunk_level(PI, offI, rowBeginI[h], rowBeginI[h + 1]);
+    finish_csr(PI, offI);
+    const long long EI = offI.back();
+    void *dOff = nullptr, *dDst = nullptr, *out = nullptr, *dFin = nullptr;
+    try {
+        BL_CUDA(cudaMalloc(&dOff, (R + 1) * sizeof(long long)));
+        BL_CUDA(cudaMalloc(&dDst, std::max<long long>(R, 1) * sizeof(long long)));
+        BL_CUDA(cudaMalloc(&out, std::max<long long>(EI, 1) * sizeof(uint32_t)));
+        BL_CUDA(cudaMalloc(&dFin, std::max<size_t>(fin.size(), 1) * sizeof(int)));
+        BL_CUDA(cudaMemcpy(dOff, off.data(), (R + 1) * sizeof(long long), cudaMemcpyHostToDevice));
+        BL_CUDA(cudaMemcpy(dDst, dstI.data(), R * sizeof(long long), cudaMemcpyHostToDevice));
+        if (!fin.empty()) BL_CUDA(cudaMemcpy(dFin, fin.data(), fin.size() * sizeof(int), cudaMemcpyHostToDevice));
+        internal_kernel<<<blocks_for(R, 8), 256>>>(d.up.adj, static_cast<const long long*>(dOff), R,
+                                                   static_cast<uint32_t>(src0), static_cast<const long long*>(dDst),
+                                                   static_cast<uint32_t*>(out));
+        BL_CUDA(cudaGetLastError());
+        BL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the legacy-stream kernel above, not the device
+    } catch (...) {
+        for (void* p : {dOff, dDst, out, dFin}) cudaFree(p);
+        throw;
+    }
+    cudaFree(dOff);
+    cudaFree(dDst);
+    d.allocs.push_back(out);
+    d.allocs.push_back(dFin);
+    d.bytes += static_cast<uint64_t>(EI) * sizeof(uint32_t) + fin.size() * sizeof(int);
+    d.up_int = upload_pull(d, PI, out, EI);
+    mark_short_levels(d, d.up_int, PI, offI);
+    d.up_int_f = fine_view(d, d.up_int, rechunk(PI, offI, kFineChunkFactor));
+    d.fin = static_cast<int*>(dFin);
+    d.fin_begin = finBegin;
+    d.up_int_built = true;
+}
+
+namespace {
+// Builds d.up0b (and d.up_int / d.fin) from the resident UP CSR (rows = nodes level_begin[1] .. n-1
 // in order, children ascending).
 void build_up_split(DevicePlan& d) {
     const PlanDeviceScope planSms(sm_count());
@@ -267,7 +347,6 @@ void build_up_split(DevicePlan& d) {
         tmp.clear();
     };
     unsigned short* out0 = nullptr;
-    uint32_t* outI = nullptr;
     try {
         long long* dOff = static_cast<long long*>(dmalloc((R + 1) * sizeof(long long)));
         BL_CUDA(cudaMemcpy(dOff, off.data(), (R + 1) * sizeof(long long), cudaMemcpyHostToDevice));
@@ -286,77 +365,42 @@ void build_up_split(DevicePlan& d) {
         const long long E0 = block_layout(P0, seg, R, nb, [&](long long i) { return static_cast<int32_t>(src0 + i); },
                                           dst0, off0);
 
-        // internal edges: one level per UP level (heights 1..H-1), plus the finish lists
-        PullCSR PI;
-        std::vector<int64_t> offI(1, 0), rowBeginI;
-        std::vector<long long> dstI(static_cast<size_t>(R), -1);
-        std::vector<int> fin;
-        std::vector<long long> finBegin;
-        for (uint64_t h = 1; h < d.num_levels; h++) {
-            rowBeginI.push_back(static_cast<int64_t>(PI.rows.size()));
-            finBegin.push_back(static_cast<long long>(fin.size()));
-            for (long long node = static_cast<long long>(d.level_begin[h]);
-                 node < static_cast<long long>(d.level_begin[h + 1]); node++) {
-                const long long i = node - src0;
-                const long long len = (off[i + 1] - off[i]) - S(i, nb);
-                if (len <= 0) {
-                    fin.push_back(static_cast<int>(node));
-                    continue;
-                }
-                dstI[static_cast<size_t>(i)] = offI.back();
-                PI.rows.push_back(static_cast<int32_t>(node));
-                offI.push_back(offI.back() + len);
+        // (children out of order: a row's height-0 children are no prefix of it, and the graph runs
+        // unsplit)
+        const std::vector<unsigned> low = count_low_children(d);
+        for (long long i = 0; i < R; i++) {
+            if (low[static_cast<size_t>(i)] != static_cast<unsigned long long>(S(i, nb))) {
+                freeTmp();
+                return;
             }
         }
-        rowBeginI.push_back(static_cast<int64_t>(PI.rows.size()));
-        finBegin.push_back(static_cast<long long>(fin.size()));
-        for (size_t h = 0; h + 1 < rowBeginI.size(); h++) chunk_level(PI, offI, rowBeginI[h], rowBeginI[h + 1]);
-        finish_csr(PI, offI);
-        const long long EI = offI.back();
-        GRGX_CHECK(E0 + EI == E, GRGX_ERR_CUDA, "split edge count mismatch");
+        build_up_internal(d, low);
+        GRGX_CHECK(E0 + d.up_int.n_edges == E, GRGX_ERR_CUDA, "split edge count mismatch");
 
         long long* dDst0 = static_cast<long long*>(dmalloc(dst0.size() * sizeof(long long)));
-        long long* dDstI = static_cast<long long*>(dmalloc(dstI.size() * sizeof(long long)));
         BL_CUDA(cudaMemcpy(dDst0, dst0.data(), dst0.size() * sizeof(long long), cudaMemcpyHostToDevice));
-        BL_CUDA(cudaMemcpy(dDstI, dstI.data(), dstI.size() * sizeof(long long), cudaMemcpyHostToDevice));
         // padded for the staged passes' id ring, whose last copy may reach kRingIds ids past the end
         BL_CUDA(cudaMalloc(reinterpret_cast<void**>(&out0), (E0 + kRingIds) * sizeof(unsigned short)));
-        BL_CUDA(cudaMalloc(reinterpret_cast<void**>(&outI), (EI ? EI : 1) * sizeof(uint32_t)));
-        scatter_kernel<<<blocks_for(R, 8), 256>>>(d.up.adj, dOff, R, nb, block, 0, dSeg, dDst0, dDstI, out0, outI);
+        scatter_kernel<<<blocks_for(R, 8), 256>>>(d.up.adj, dOff, R, nb, block, 0, dSeg, dDst0, out0);
         BL_CUDA(cudaGetLastError());
         BL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the legacy-stream kernels above, not the device
         freeTmp();
         void* a0 = out0;
-        uint32_t* aI = outI;
         d.allocs.push_back(a0);
         out0 = nullptr;
-        d.allocs.push_back(aI);
-        outI = nullptr;
-        d.bytes += static_cast<uint64_t>(E0 + kRingIds) * sizeof(unsigned short) + static_cast<uint64_t>(EI) * sizeof(uint32_t);
+        d.bytes += static_cast<uint64_t>(E0 + kRingIds) * sizeof(unsigned short);
         std::vector<long long> base(nb), rows(nb);
         for (int b = 0; b < nb; b++) {
             base[b] = static_cast<long long>(b) * block;
             rows[b] = std::min(block, src0 - base[b]);
         }
         d.up0b = upload_pull(d, P0, a0, E0, &base, &rows);
-        d.up_int = upload_pull(d, PI, aI, EI);
         d.up0b_f = fine_view(d, d.up0b, rechunk(P0, off0, kFineChunkFactor));
-        d.up_int_f = fine_view(d, d.up_int, rechunk(PI, offI, kFineChunkFactor));
-        if (!fin.empty()) {
-            void* p = nullptr;
-            BL_CUDA(cudaMalloc(&p, fin.size() * sizeof(int)));
-            d.allocs.push_back(p);
-            d.bytes += fin.size() * sizeof(int);
-            BL_CUDA(cudaMemcpy(p, fin.data(), fin.size() * sizeof(int), cudaMemcpyHostToDevice));
-            d.fin = static_cast<int*>(p);
-        }
-        d.fin_begin = finBegin;
         d.split_block = block;
         d.split_src = src0;
     } catch (...) {
         freeTmp();
         if (out0) cudaFree(out0);
-        if (outI) cudaFree(outI);
         throw;
     }
 }
@@ -415,8 +459,7 @@ void build_down_split(DevicePlan& d) {
         BL_CUDA(cudaMemcpy(dDst0, dst0.data(), dst0.size() * sizeof(long long), cudaMemcpyHostToDevice));
         // padded for the staged passes' id ring, whose last copy may reach kRingIds ids past the end
         BL_CUDA(cudaMalloc(reinterpret_cast<void**>(&out0), (E0 + kRingIds) * sizeof(unsigned short)));
-        scatter_kernel<<<blocks_for(R, 8), 256>>>(adj, dOff, R, nb, block, src0, dSeg, dDst0, nullptr, out0,
-                                                  nullptr);
+        scatter_kernel<<<blocks_for(R, 8), 256>>>(adj, dOff, R, nb, block, src0, dSeg, dDst0, out0);
         BL_CUDA(cudaGetLastError());
         BL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the legacy-stream kernels above, not the device
         freeTmp();

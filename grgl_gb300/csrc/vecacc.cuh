@@ -176,8 +176,8 @@ template <> struct VecAcc<AddF64S, 1> {
 // TwoSum per edge.
 constexpr int kF32PreSum = 4;
 
-// Compensated float32, columns in pairs.
-template <int NP> struct PackedF32C {
+// Compensated float32, columns in pairs; PRE edges are pre-summed in add_block.
+template <int NP, int PRE = kF32PreSum> struct PackedF32C {
     float2 hi[NP], lo[NP];
     __device__ __forceinline__ void zero() {
 #pragma unroll
@@ -194,15 +194,15 @@ template <int NP> struct PackedF32C {
         for (int j = 0; j < NP; j++) add_pair2(j, make_float2(v[2 * j], v[2 * j + 1]));
     }
     template <int N> __device__ __forceinline__ void add_block(const float (*v)[2 * NP]) {
-        static_assert(N % kF32PreSum == 0, "block of whole pre-sums");
+        static_assert(N % PRE == 0 && (PRE == 1 || PRE == 2 || PRE == 4), "block of whole pre-sums");
 #pragma unroll
-        for (int u = 0; u < N; u += kF32PreSum) {
+        for (int u = 0; u < N; u += PRE) {
 #pragma unroll
             for (int j = 0; j < NP; j++) {
                 float2 t = make_float2(v[u][2 * j], v[u][2 * j + 1]);
-                if (kF32PreSum == 2) {
+                if constexpr (PRE == 2) {
                     t = add2(t, make_float2(v[u + 1][2 * j], v[u + 1][2 * j + 1]));
-                } else if (kF32PreSum == 4) {
+                } else if constexpr (PRE == 4) {
                     const float2 b = make_float2(v[u + 1][2 * j], v[u + 1][2 * j + 1]);
                     const float2 c = make_float2(v[u + 2][2 * j], v[u + 2][2 * j + 1]);
                     const float2 d = make_float2(v[u + 3][2 * j], v[u + 3][2 * j + 1]);
@@ -267,6 +267,9 @@ template <int NP> struct PackedF32C {
 };
 template <> struct VecAcc<AddF32C, 2> : PackedF32C<1> {};
 template <> struct VecAcc<AddF32C, 4> : PackedF32C<2> {};
+template <int PRE> struct VecAcc<AddF32CPre<PRE>, 1> : VecAcc<AddF32C, 1> {};
+template <int PRE> struct VecAcc<AddF32CPre<PRE>, 2> : PackedF32C<1, PRE> {};
+template <int PRE> struct VecAcc<AddF32CPre<PRE>, 4> : PackedF32C<2, PRE> {};
 
 // float64 as float pairs, columns in pairs: double run folds, float2 (hi, lo) state.
 template <int NP> struct PackedF64S {
@@ -364,5 +367,168 @@ template <int NP> struct PackedF64S {
     }
 };
 template <> struct VecAcc<AddF64S, 2> : PackedF64S<1> {};
+
+// df_add on pairs of columns.
+__device__ __forceinline__ void df_add2(float2& ahi, float2& alo, float2 bhi, float2 blo) {
+    float2 s, e, t, f, g, h;
+    two_sum2(ahi, bhi, s, e);
+    two_sum2(alo, blo, t, f);
+    two_sum2(e, t, g, h);
+    ahi = add2(s, g);
+    alo = add2(sub2(g, sub2(ahi, s)), add2(h, f));
+}
+
+// float64 as float pairs with the runs folded into a normalised float pair: no FP64 instruction
+// until the sum is read.  The low part is renormalised every two additions, not four (2% of the
+// time of a wide product): mean errors of products in pair form stay 15-20% below the sweep's.
+template <int NP> struct PackedF64SD {
+    float2 hi[NP], lo[NP], thi[NP], tlo[NP];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int j = 0; j < NP; j++) hi[j] = lo[j] = thi[j] = tlo[j] = make_float2(0.0f, 0.0f);
+    }
+    __device__ __forceinline__ void add(const DF* v) {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            float2 s, e;
+            two_sum2(hi[j], make_float2(v[2 * j].hi, v[2 * j + 1].hi), s, e);
+            lo[j] = add2(lo[j], add2(e, make_float2(v[2 * j].lo, v[2 * j + 1].lo)));
+            hi[j] = s;
+        }
+    }
+    template <int N> __device__ __forceinline__ void add_block(const DF (*v)[2 * NP]) {
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+            add(v[u]);
+            if (u & 1) settle();
+        }
+    }
+    __device__ __forceinline__ void add_pairs(const DF (*v)[2 * NP]) { add_block<4>(v); }
+    __device__ __forceinline__ void settle() {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            const float2 h = add2(hi[j], lo[j]);
+            lo[j] = sub2(lo[j], sub2(h, hi[j]));
+            hi[j] = h;
+        }
+    }
+    __device__ __forceinline__ void flush() {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            df_add2(thi[j], tlo[j], hi[j], lo[j]);
+            hi[j] = lo[j] = make_float2(0.0f, 0.0f);
+        }
+    }
+    __device__ __forceinline__ void merge(const PackedF64SD& o) {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            df_add2(thi[j], tlo[j], o.thi[j], o.tlo[j]);
+            df_add2(thi[j], tlo[j], o.hi[j], o.lo[j]);
+        }
+    }
+    __device__ __forceinline__ PackedF64SD shfl_xor(int m) const {
+        PackedF64SD r;
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            r.hi[j] = shfl_xor2(hi[j], m);
+            r.lo[j] = shfl_xor2(lo[j], m);
+            r.thi[j] = shfl_xor2(thi[j], m);
+            r.tlo[j] = shfl_xor2(tlo[j], m);
+        }
+        return r;
+    }
+    // The sum as one float pair.
+    __device__ __forceinline__ DF pair(int i) const {
+        return df_add(DF{lane_of(thi[i >> 1], i), lane_of(tlo[i >> 1], i)}, DF{lane_of(hi[i >> 1], i), lane_of(lo[i >> 1], i)});
+    }
+    __device__ __forceinline__ F64Run get(int i) const {
+        return {static_cast<double>(lane_of(thi[i >> 1], i)) + static_cast<double>(lane_of(tlo[i >> 1], i)),
+                lane_of(hi[i >> 1], i), lane_of(lo[i >> 1], i)};
+    }
+};
+template <> struct VecAcc<AddF64SD, 2> : PackedF64SD<1> {};
+// One column: the pair form of the accumulator with an unused second half.
+template <> struct VecAcc<AddF64SD, 1> : PackedF64SD<1> {
+    using Base = PackedF64SD<1>;
+    __device__ __forceinline__ VecAcc() = default;
+    __device__ __forceinline__ VecAcc(const Base& b) : Base(b) {}
+    template <int N> __device__ __forceinline__ void add_block(const DF (*v)[1]) {
+        // two rows at a time, one in each half
+#pragma unroll
+        for (int u = 0; u < N; u += 2) {
+            const DF w[2] = {v[u][0], v[u + 1][0]};
+            Base::add(w);
+            if ((u & 2) != 0) settle();
+        }
+    }
+    __device__ __forceinline__ void add_pairs(const DF (*v)[1]) { add_block<4>(v); }
+    __device__ __forceinline__ DF pair(int) const { return df_add(Base::pair(0), Base::pair(1)); }
+    __device__ __forceinline__ F64Run get(int) const {
+        const F64Run a = Base::get(0), b = Base::get(1);
+        return {a.acc + b.acc + AddF64S::run_value(b), a.hi, a.lo};
+    }
+};
+
+// Every addition normalised: four rows as a two-level tree, then onto the sum.
+template <int NP> struct PackedF64SN {
+    float2 hi[NP], lo[NP];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int j = 0; j < NP; j++) hi[j] = lo[j] = make_float2(0.0f, 0.0f);
+    }
+    template <int N> __device__ __forceinline__ void add_block(const DF (*v)[2 * NP]) {
+        static_assert(N % 4 == 0, "block of whole trees");
+#pragma unroll
+        for (int u = 0; u < N; u += 4) {
+#pragma unroll
+            for (int j = 0; j < NP; j++) {
+                float2 h[4], l[4];
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    h[t] = make_float2(v[u + t][2 * j].hi, v[u + t][2 * j + 1].hi);
+                    l[t] = make_float2(v[u + t][2 * j].lo, v[u + t][2 * j + 1].lo);
+                }
+                df_add2(h[0], l[0], h[1], l[1]);
+                df_add2(h[2], l[2], h[3], l[3]);
+                df_add2(h[0], l[0], h[2], l[2]);
+                df_add2(hi[j], lo[j], h[0], l[0]);
+            }
+        }
+    }
+    __device__ __forceinline__ void flush() {}
+    __device__ __forceinline__ void merge(const PackedF64SN& o) {
+#pragma unroll
+        for (int j = 0; j < NP; j++) df_add2(hi[j], lo[j], o.hi[j], o.lo[j]);
+    }
+    __device__ __forceinline__ PackedF64SN shfl_xor(int m) const {
+        PackedF64SN r;
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            r.hi[j] = shfl_xor2(hi[j], m);
+            r.lo[j] = shfl_xor2(lo[j], m);
+        }
+        return r;
+    }
+    __device__ __forceinline__ DF pair(int i) const { return {lane_of(hi[i >> 1], i), lane_of(lo[i >> 1], i)}; }
+    __device__ __forceinline__ F64Run get(int i) const { return {0.0, lane_of(hi[i >> 1], i), lane_of(lo[i >> 1], i)}; }
+};
+template <> struct VecAcc<AddF64SN, 2> : PackedF64SN<1> {};
+template <> struct VecAcc<AddF64SN, 1> : PackedF64SN<1> {
+    __device__ __forceinline__ VecAcc() = default;
+    template <int N> __device__ __forceinline__ void add_block(const DF (*v)[1]) {
+        DF w[N / 2][2];
+#pragma unroll
+        for (int u = 0; u < N / 2; u++) {
+            w[u][0] = v[2 * u][0];
+            w[u][1] = v[2 * u + 1][0];
+        }
+        PackedF64SN<1>::template add_block<N / 2>(w);
+    }
+    __device__ __forceinline__ DF pair(int) const { return df_add(PackedF64SN<1>::pair(0), PackedF64SN<1>::pair(1)); }
+    __device__ __forceinline__ F64Run get(int) const {
+        const DF r = pair(0);
+        return {0.0, r.hi, r.lo};
+    }
+};
 
 }  // namespace grgx

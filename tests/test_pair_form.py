@@ -80,6 +80,30 @@ def test_pair_down_matches_oracle(env, dt, K):
     _check(og, V, DOWN, gx.matmul(g, V, DOWN))
 
 
+@pytest.mark.parametrize("dt", [np.int32, np.int64, np.uint8, np.float32, np.float64, np.bool_])
+@pytest.mark.parametrize("K", [1, 2, 3, 8, 17, 33, 64, 130])
+def test_pair_up_matches_oracle(env, dt, K):
+    gx, g, og = env
+    V = _rand(np.random.default_rng(K), dt, (K, g.num_samples))
+    _check(og, V, UP, gx.matmul(g, V, UP))
+
+
+def test_pair_up_options(env):
+    gx, g, og = env
+    rng = np.random.default_rng(3)
+    V = rng.standard_normal((5, g.num_samples))
+    init = rng.standard_normal((5, g.num_nodes))
+    _check(og, V, UP, gx.matmul(g, V, UP, emit_all_nodes=True, init=init), emit_all_nodes=True, init=init)
+    for dt in (np.float32, np.int32):
+        Vm = _rand(rng, dt, (3, g.num_samples))
+        got_miss, ref_miss = (np.zeros((3, g.num_mutations), dtype=dt) for _ in range(2))
+        got = gx.matmul(g, Vm, UP, by_individual=True, miss=got_miss)
+        assert_matches(got, oracle.matmul(og, Vm, UP, by_individual=True, miss=ref_miss),
+                       oracle.matmul(og, np.abs(Vm), UP, by_individual=True), rtol=2e-5)
+        assert_matches(got_miss, ref_miss, np.full(ref_miss.shape, np.abs(Vm).sum()), rtol=2e-5)
+    assert np.array_equal(gx.matmul(g, V, UP), gx.matmul(g, V, UP))
+
+
 @pytest.mark.parametrize("flag", ["f32_compensated", "f64_native"])
 def test_pair_down_other_accumulations(env, flag):
     gx, g, og = env
@@ -165,11 +189,13 @@ def test_large_graph_takes_the_pair_form_by_rule(cuda_ok):
 
 
 @pytest.mark.parametrize("dt", [np.int32, np.float32, np.float64])
-def test_pair_down_within_a_servers_memory(env, dt):
+def test_pair_form_within_a_servers_memory(env, dt):
     """A server's batch has scratch for a part of the patterns at a time: several tables, their
     sums carried from one to the next."""
     gx, g, og = env
-    V = _rand(np.random.default_rng(6), dt, (12, g.num_mutations))
     with gx.Server(workers=1) as srv:
-        got, _ = srv.result(srv.submit(srv.add_graph(g), V, DOWN), timeout=60.0)
-    _check(og, V, DOWN, got)
+        gid = srv.add_graph(g)
+        for direction, cols in ((DOWN, g.num_mutations), (UP, g.num_samples)):
+            V = _rand(np.random.default_rng(6), dt, (12, cols))
+            got, _ = srv.result(srv.submit(gid, V, direction), timeout=60.0)
+            _check(og, V, direction, got)
