@@ -122,3 +122,17 @@ def test_gram_products_match_dense(env, standardized):
     Vi = rng.integers(-3, 4, size=(2, g.num_samples)).astype(np.int64)
     if not standardized:
         assert np.array_equal(gx.matmul_gram(g, Vi, UP), Vi @ og.dense_X().astype(np.int64) @ og.dense_X().T)
+
+
+@pytest.mark.parametrize("K", [1, 3, 700])
+def test_standardized_rows_in_shares(env, K):
+    """Row sums are taken by several blocks per row when rows are few and longer than 1,024."""
+    gx = env[0]
+    g = gx.window_tree_grg(1025, 2049, seed=43)
+    a = g.export_arrays()
+    og = oracle.OracleGraph(num_samples=1025, ploidy=1, down_off=a["down_off"], down_adj=a["down_adj"],
+                            mut_node=a["mut_node"])
+    for direction, cols in ((UP, g.num_samples), (DOWN, g.num_mutations)):
+        V = np.random.default_rng(K).standard_normal((K, cols)) + 3.0
+        ref, scale = oracle.standardized(og, V, direction, return_scale=True)
+        assert np.all(np.abs(gx.matmul_standardized(g, V, direction) - ref) <= 1e-12 * scale)
