@@ -39,6 +39,9 @@ void launch_sweep_staged_xor(const SweepParams<uint32_t>& p, dim3 grid, cudaStre
 void launch_sweep_staged_f32c(const SweepParams<float>& p, dim3 grid, cudaStream_t s);
 void launch_sweep_staged_f32(const SweepParams<float>& p, dim3 grid, cudaStream_t s);
 
+// The pair form's ids are padded to whole groups of this many height-0 rows: no warp takes more.
+constexpr int kPairTile = 128;
+
 // DOWN in pair form (pair_down.cuh): one launch over `items` shares of the blocks (groups of four,
 // group_begin .. group_end) x `tiles` row tiles.
 template <typename S> struct PairDownParams {

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<
     using Acc = VecAcc<Op, VW>;
     using Part = PairPart<Op>;
     constexpr int NG = 32 / G, ROWS = kPairRows;
+    static_assert(NG * ROWS <= kPairTile, "a warp's rows end within the padded ids");
     constexpr bool kChains = ChainTraits<Op>::kChains;
     if (p.gate != nullptr && *p.gate != p.gate_value) return;
     const int lane = threadIdx.x & 31;

@@ -491,9 +491,9 @@ void build_pair_plan(DevicePlan& d, bool down) {
     const int* dNode = tmp.copy(seqNode);
     const PairBlock* dBlocks = tmp.copy(blocks);
     const long long groups = (nblk + 3) / 4;
-    const long long tiles = (h0 + 127) / 128 * 4;  // whole groups of 128 nodes: a warp's largest share
+    const long long tiles = (h0 + kPairTile - 1) / kPairTile * (kPairTile / 32);
     const long long batch = std::max<long long>(1, std::min(nblk, (1LL << 27) / h0));
-    const size_t idBytes = static_cast<size_t>(tiles) * groups * 128 * sizeof(unsigned short);
+    const size_t idBytes = static_cast<size_t>(tiles) * groups * 32 * 4 * sizeof(unsigned short);
     PairOut out{};
     out.seqNode = dNode;
     out.groups = groups;
