@@ -147,14 +147,17 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
     const bool down = (direction == GRGX_DIRECTION_DOWN);
     // the CSRs a call of this shape sweeps; for UP both forms when the split form is possible,
     // so the faster one is recorded for this graph
-    // (for DOWN too: the height-0 level in parent blocks, the levels above it as usual)
+    // (for DOWN too: the height-0 level in parent blocks, the levels above it as usual; a single
+    // 4-byte column's split form runs on lists in shared memory, which has one shape)
     struct Pass {
         const DevCSR* c;
         int mode;
         const char* name;
         long long stateBase;
         bool skipLast;  // the CSR's last level is left to the next pass
+        bool staged = false;  // the CSR's levels are one launch of staged lists
     };
+    const bool staged = staged_layout(L);
     std::vector<std::vector<Pass>> forms;
     const long long h0 = static_cast<long long>(dp->level_begin.size() > 1 ? dp->level_begin[1] : 0);
     // (on the chunking calls of this row width run on)
@@ -164,13 +167,13 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
         forms.push_back({{cs.down, 0, "level", 0, false}});
         if (cs.down0b->n_rows > 0)
             forms.push_back({{cs.down, 0, "split: level", 0, true},
-                             {cs.down0b, 1, "split: height-0 parent block", 0, false}});
+                             {cs.down0b, 1, "split: height-0 parent block", 0, false, staged && dp->down_staged.slots > 0}});
     } else {
         if (up_split_possible(dp)) ensure_up_split(g, dp);
         const SweepCSRs cs = sweep_csrs(dp, L);
         forms.push_back({{cs.up, 0, "level", 0, false}});
         if (cs.up0b->n_rows > 0)
-            forms.push_back({{cs.up0b, 1, "split: height-0 block", dp->split_src, false},
+            forms.push_back({{cs.up0b, 1, "split: height-0 block", dp->split_src, false, staged && dp->up_staged.slots > 0},
                              {cs.up_int, 2, "split: level", dp->split_src, false}});
     }
     long long maxPieces = 0, maxHeavy = 0;
@@ -184,7 +187,7 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
     const size_t n = g->host->num_nodes;
     cudaStream_t s = nullptr;
     GRGX_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    void *vals = nullptr, *partials = nullptr, *state = nullptr;
+    void *vals = nullptr, *partials = nullptr, *state = nullptr, *slots = nullptr;
     unsigned* counters = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     std::ostringstream rep;
@@ -192,6 +195,7 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
         if (vals) cudaFree(vals);
         if (partials) cudaFree(partials);
         if (state) cudaFree(state);
+        if (slots) cudaFree(slots);
         if (counters) cudaFree(counters);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
@@ -234,6 +238,22 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
             }
             return best;
         };
+        const StagedLists& lists = down ? dp->down_staged : dp->up_staged;
+        if (staged && lists.slots > 0) GRGX_CUDA(cudaMalloc(&slots, static_cast<size_t>(lists.slots) * L.asize));
+        auto time_staged = [&] {
+            float best = 1e30f;
+            for (int rep_i = 0; rep_i < 3; rep_i++) {
+                GRGX_CUDA(cudaEventRecord(e0, s));
+                launch_staged(L.kind, lists, vals, slots, nullptr, 0, rmw, s);
+                GRGX_CUDA(cudaEventRecord(e1, s));
+                GRGX_CUDA(cudaEventSynchronize(e1));
+                GRGX_CUDA(cudaGetLastError());
+                float ms = 0;
+                GRGX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+                if (rep_i > 0) best = std::min(best, ms);
+            }
+            return best;
+        };
         const std::vector<int> gs = candidate_g(L);
         std::vector<double> formBest;
         for (const auto& form : forms) {
@@ -245,6 +265,12 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
                 curMode = ps.mode;
                 curBase = ps.stateBase;
                 const DevCSR& c = *ps.c;
+                if (ps.staged) {
+                    const float t = time_staged();
+                    totDefault += t;
+                    totBest += t;
+                    continue;
+                }
                 for (size_t lvl = 0; lvl + (ps.skipLast ? 1 : 0) < c.lb.size(); lvl++) {
                     if (c.le[lvl] <= c.lb[lvl]) continue;
                     const LevelShape def = default_shape(L);

@@ -39,6 +39,24 @@ struct DevCSR {
     long long n_heavy = 0, n_pieces = 0, n_edges = 0, n_rows = 0;
 };
 
+// A share of one split block's lists (staged.cu): parts `part` of `parts`.
+struct StagedPart {
+    long long src;  // the block's first source id
+    int rows;       // its source ids
+    int list0, list1;
+    int part, parts;
+};
+// The lists of a split copy for single-column products.
+struct StagedLists {
+    StagedPart* parts = nullptr;
+    unsigned nparts = 0;
+    PairList* lists = nullptr;              // out = slot
+    unsigned* slot0 = nullptr;              // first slot of each row (+ the end)
+    int* nodes = nullptr;
+    const unsigned short* adj = nullptr;
+    long long rows = 0, slots = 0;
+};
+
 struct DevicePlan {
     int device = -1;
     DevCSR up, down, seed, miss;
@@ -67,6 +85,7 @@ struct DevicePlan {
     //   fin_down the height-0 DOWN rows, finished from their state after the block passes
     // Built on the first call that runs DOWN in split form (use_down_split).
     DevCSR down0b, down0b_f;
+    StagedLists up_staged, down_staged;  // built with the split copies
     int* fin_down = nullptr;
     long long n_fin_down = 0;
     bool down_split_built = false;
@@ -176,13 +195,21 @@ bool use_down_split(grgx_graph* g, DevicePlan* dp, const Layout& L);
 bool down_split_possible(const DevicePlan* dp);
 void ensure_down_split(grgx_graph* g, DevicePlan* dp);
 void set_down_split_choice(grgx_graph* g, DevicePlan* dp, const Layout& L, bool split);
-// Whether single-column 4-byte split passes stage their block's source values in shared memory
-// (sweep_kernel_staged); on by default, switchable for tests.
+// Whether layout L runs its split form staged: a single 4-byte column (K = 1 for the 4-byte dtypes,
+// bool up to 32 columns), whose source blocks fit in shared memory (staged.cu); on by default,
+// switchable for tests.
+constexpr long long kStagedRows = 32768;
 bool staged_enabled();
 void set_staged(bool on);
-// Whether split block passes of layout L run staged: a single 4-byte column (K = 1 for the
-// 4-byte dtypes, bool up to 32 columns), staging on.
 bool staged_layout(const Layout& L);
+// The rows' sums over their height-0 children (UP) or parents (DOWN) on T's lists: into `state` (from
+// node stateBase on) or onto / into vals; `sums` holds T.slots accumulators.
+int launch_staged(Kind kind, const StagedLists& T, void* vals, void* sums, void* state, long long stateBase, int rmw,
+                  cudaStream_t s);
+// The lists of a split copy: per row (R) and block (nb) its segment bounds `seg` and place `start`.
+void build_staged(DevicePlan& d, StagedLists& T, const std::vector<uint32_t>& seg, const std::vector<long long>& start,
+                  long long R, int nb, const std::vector<long long>& base, const std::vector<long long>& srcRows,
+                  const std::vector<int>& nodeOf, const unsigned short* adj);
 // DOWN split form: 0 chosen as above, 1 always (where possible), 2 never (tests).
 void set_down_split_mode(int mode);
 bool down_split_forced();

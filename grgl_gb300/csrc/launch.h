@@ -32,13 +32,6 @@ void launch_sweep_f32(const SweepParams<float>& p, int vw, int g, int variant, d
 void launch_sweep_f64s(const SweepParams<DF>& p, int vw, int g, int variant, dim3 grid,
                       int sms, cudaStream_t s);
 
-// Staged single-column sweeps of one split block (sweep_kernel_staged; p.src = the block's first
-// source value, p.src_rows <= kStagedRows values), 4-byte storage kinds.
-void launch_sweep_staged_u32(const SweepParams<uint32_t>& p, dim3 grid, cudaStream_t s);
-void launch_sweep_staged_xor(const SweepParams<uint32_t>& p, dim3 grid, cudaStream_t s);
-void launch_sweep_staged_f32c(const SweepParams<float>& p, dim3 grid, cudaStream_t s);
-void launch_sweep_staged_f32(const SweepParams<float>& p, dim3 grid, cudaStream_t s);
-
 // The pair form's ids are padded to whole groups of this many height-0 rows: no warp takes more.
 constexpr int kPairTile = 128;
 

@@ -264,7 +264,6 @@ SweepParams<S> make_params(const DevCSR& c, long long cb, long long ce, const vo
     p.state_mode = 0;
     p.id16 = 0;
     p.id_base = 0;
-    p.src_rows = 0;
     p.col_base = 0;
     p.short_off = nullptr;
     p.short_row0 = p.short_rows = 0;
@@ -330,36 +329,6 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
         case Kind::F64S: launch_sweep_f64s(prm(DF{}), vw, g, variant, grid, sms, s); break;
         }
     };
-    if (c.id16) {
-        // single-column 4-byte rows stage the block's sources in shared memory (one 1024-thread
-        // block per SM)
-        const long long srows = c.level_src_rows[level];
-        if (staged_layout(L) && srows <= kStagedRows && sh.ntiles == 1) {
-            const dim3 sgrid(static_cast<unsigned>(std::min<long long>((ce - cb + 7) / 8, sms)), 1);
-            auto sp = [&](auto tag) {
-                using S = decltype(tag);
-                SweepParams<S> p = make_params<S>(c, cb, ce, src, dst, L.stride, rmw, partials, tickets, work, ts);
-                p.gate = gate;
-                p.gate_value = gateValue;
-                p.state = state;
-                p.state_base = stateBase;
-                p.state_mode = stateMode;
-                p.id16 = 1;
-                p.id_base = 0;
-                p.src = static_cast<const S*>(src) + base;
-                p.src_rows = srows;
-                return p;
-            };
-            switch (L.kind) {
-            case Kind::U32: launch_sweep_staged_u32(sp(uint32_t{}), sgrid, s); break;
-            case Kind::XOR: launch_sweep_staged_xor(sp(uint32_t{}), sgrid, s); break;
-            case Kind::F32C: launch_sweep_staged_f32c(sp(float{}), sgrid, s); break;
-            case Kind::F32: launch_sweep_staged_f32(sp(float{}), sgrid, s); break;
-            default: break;
-            }
-            return 1;
-        }
-    }
     if (isShort) {
         launch(L.g, L.ntiles, 0, 0, 0);
         return 1;
@@ -696,7 +665,14 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
                                                                : upair ? cUpInt.lb.size()
                                                                        : cUp.lb.size());
         const long long h0 = static_cast<long long>(dp->level_begin.size() > 1 ? dp->level_begin[1] : 0);
-        const size_t stateBytes = split    ? static_cast<size_t>(n - dp->split_src) * L.stride * std::max(L.asize, 8)
+        // a single 4-byte column in split form: the blocks' values staged in shared memory (staged.cu);
+        // only compensated float32 keeps per-node state between its sums and the UP levels
+        const StagedLists& stl = down ? dp->down_staged : dp->up_staged;
+        const size_t slotBytes = static_cast<size_t>(stl.slots) * L.asize;
+        const bool staged = (split || dsplit) && pairForm && staged_layout(L) && stl.slots > 0 && slotBytes <= pair_scratch_limit();
+        void* slots = staged ? sc.get(slotBytes) : nullptr;
+        const size_t stateBytes = staged   ? (split && L.kind == Kind::F32C ? static_cast<size_t>(n - h0) * L.asize : 0)
+                                  : split  ? static_cast<size_t>(n - dp->split_src) * L.stride * std::max(L.asize, 8)
                                   : upair  ? upStateBytes
                                   : dsplit ? static_cast<size_t>(h0) * L.stride * std::max(L.asize, 8)
                                            : 0;
@@ -814,7 +790,9 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
                 }
                 if (dpair)
                     launches += launch_pair_down(LL, dp, prun, vals, ptable, pparts, work + (2 + nlv) * TS, s, g, gv);
-                if (dsplit) {
+                if (dsplit && staged) {
+                    launches += launch_staged(LL.kind, stl, vals, slots, nullptr, 0, 1, s);
+                } else if (dsplit) {
                     // parent-block passes merge each height-0 row's sums into its state; then the
                     // rows are written from it, onto their seed / init values
                     GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
@@ -847,7 +825,8 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
                     unsigned* wIn = work + (upair ? 0 : cUp0b.lb.size()) * TS;
                     if (upair)
                         launches += launch_pair_up(LL, dp, urun, vals, ptable, state, hasInit, s, g, gv);
-                    for (size_t j = 0; split && j < cUp0b.lb.size(); j++) {
+                    if (staged) launches += launch_staged(LL.kind, stl, vals, slots, state, h0, hasInit, s);
+                    for (size_t j = 0; split && !staged && j < cUp0b.lb.size(); j++) {
                         const LevelShape sh = level_shape(LL, cUp0b, j);
                         launches += launch_level(LL, cUp0b, j, vals, vals, 0, partials, tickets, work + j * TS, s, g, gv,
                                                  &sh, TS, state, h0, 1);

@@ -164,7 +164,8 @@ struct grgx_server {
             int status = GRGX_OK;
             std::string err;
             try {
-                const grgx::PairScratchScope scratch(state_bytes(*graphs[batch[0]->graph]->host, rows));
+                // (a single column's slots are a few MB more than its state)
+                const grgx::PairScratchScope scratch(state_bytes(*graphs[batch[0]->graph]->host, rows) + (32ULL << 20));
                 grgx::matmul_batch_impl(graphs[batch[0]->graph], reqs.data(), reqs.size(), rows, GRGX_FLAG_SYNC,
                                         stream);
             } catch (const grgx::Error& e) {

@@ -25,7 +25,7 @@
 // Inside a block every source id is below 32,768 past the block's first id, so the block
 // passes' edge ids are stored in 16 bits (bit 15 marks a row's first edge): half the edge-id
 // bytes a traversal streams from HBM.  Single-column 4-byte products stage a block's source
-// values in shared memory (sweep_kernel_staged) and gather from there.
+// values in shared memory and gather from there (staged.cu).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,6 +55,8 @@ std::atomic<unsigned long long> g_threshold{kDefaultSplitThreshold};
 std::atomic<long long> g_block{32768};  // at most 32768: block-relative ids fit in 15 bits
 std::atomic<bool> g_staged{true};
 std::atomic<int> g_down_mode{0};  // DOWN split form: 0 by the rule below, 1 always, 2 never
+
+constexpr long long kIdPadding = 72;  // ids
 
 unsigned blocks_for(unsigned long long items, unsigned perBlock) {
     unsigned long long b = (items + perBlock - 1) / perBlock;
@@ -207,7 +209,7 @@ void set_up_split(long long block, unsigned long long thresholdBytes) {
 
 bool staged_enabled() { return g_staged.load(); }
 bool staged_layout(const Layout& L) {
-    return staged_enabled() && L.stride == 1 && L.ssize == 4 &&
+    return staged_enabled() && split_block_size() <= kStagedRows && L.stride == 1 && L.ssize == 4 &&
            (L.kind == Kind::U32 || L.kind == Kind::XOR || L.kind == Kind::F32C || L.kind == Kind::F32);
 }
 void set_staged(bool on) { g_staged.store(on); }
@@ -379,8 +381,8 @@ void build_up_split(DevicePlan& d) {
 
         long long* dDst0 = static_cast<long long*>(dmalloc(dst0.size() * sizeof(long long)));
         BL_CUDA(cudaMemcpy(dDst0, dst0.data(), dst0.size() * sizeof(long long), cudaMemcpyHostToDevice));
-        // padded for the staged passes' id ring, whose last copy may reach kRingIds ids past the end
-        BL_CUDA(cudaMalloc(reinterpret_cast<void**>(&out0), (E0 + kRingIds) * sizeof(unsigned short)));
+        // padded for the staged lists, whose last load may reach 7 ids past a step of 64
+        BL_CUDA(cudaMalloc(reinterpret_cast<void**>(&out0), (E0 + kIdPadding) * sizeof(unsigned short)));
         scatter_kernel<<<blocks_for(R, 8), 256>>>(d.up.adj, dOff, R, nb, block, 0, dSeg, dDst0, out0);
         BL_CUDA(cudaGetLastError());
         BL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the legacy-stream kernels above, not the device
@@ -388,13 +390,16 @@ void build_up_split(DevicePlan& d) {
         void* a0 = out0;
         d.allocs.push_back(a0);
         out0 = nullptr;
-        d.bytes += static_cast<uint64_t>(E0 + kRingIds) * sizeof(unsigned short);
+        d.bytes += static_cast<uint64_t>(E0 + kIdPadding) * sizeof(unsigned short);
         std::vector<long long> base(nb), rows(nb);
         for (int b = 0; b < nb; b++) {
             base[b] = static_cast<long long>(b) * block;
             rows[b] = std::min(block, src0 - base[b]);
         }
         d.up0b = upload_pull(d, P0, a0, E0, &base, &rows);
+        std::vector<int> nodes(static_cast<size_t>(R));
+        for (long long i = 0; i < R; i++) nodes[static_cast<size_t>(i)] = static_cast<int>(src0 + i);
+        build_staged(d, d.up_staged, seg, dst0, R, nb, base, rows, nodes, static_cast<const unsigned short*>(a0));
         d.up0b_f = fine_view(d, d.up0b, rechunk(P0, off0, kFineChunkFactor));
         d.split_block = block;
         d.split_src = src0;
@@ -457,8 +462,8 @@ void build_down_split(DevicePlan& d) {
         GRGX_CHECK(E0 == E, GRGX_ERR_CUDA, "split edge count mismatch");
         long long* dDst0 = static_cast<long long*>(dmalloc(dst0.size() * sizeof(long long)));
         BL_CUDA(cudaMemcpy(dDst0, dst0.data(), dst0.size() * sizeof(long long), cudaMemcpyHostToDevice));
-        // padded for the staged passes' id ring, whose last copy may reach kRingIds ids past the end
-        BL_CUDA(cudaMalloc(reinterpret_cast<void**>(&out0), (E0 + kRingIds) * sizeof(unsigned short)));
+        // padded for the staged lists, whose last load may reach 7 ids past a step of 64
+        BL_CUDA(cudaMalloc(reinterpret_cast<void**>(&out0), (E0 + kIdPadding) * sizeof(unsigned short)));
         scatter_kernel<<<blocks_for(R, 8), 256>>>(adj, dOff, R, nb, block, src0, dSeg, dDst0, out0);
         BL_CUDA(cudaGetLastError());
         BL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the legacy-stream kernels above, not the device
@@ -466,13 +471,14 @@ void build_down_split(DevicePlan& d) {
         void* a0 = out0;
         d.allocs.push_back(a0);
         out0 = nullptr;
-        d.bytes += static_cast<uint64_t>(E0 + kRingIds) * sizeof(unsigned short);
+        d.bytes += static_cast<uint64_t>(E0 + kIdPadding) * sizeof(unsigned short);
         std::vector<long long> base(nb), rows(nb);
         for (int b = 0; b < nb; b++) {
             base[b] = src0 + static_cast<long long>(b) * block;
             rows[b] = std::min(block, n - base[b]);
         }
         d.down0b = upload_pull(d, P0, a0, E0, &base, &rows);
+        build_staged(d, d.down_staged, seg, dst0, R, nb, base, rows, rowNode, static_cast<const unsigned short*>(a0));
         d.down0b_f = fine_view(d, d.down0b, rechunk(P0, off0, kFineChunkFactor));
         void* p = nullptr;
         BL_CUDA(cudaMalloc(&p, rowNode.size() * sizeof(int)));
