@@ -227,7 +227,7 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
             for (int rep_i = 0; rep_i < 3; rep_i++) {
                 GRGX_CUDA(cudaMemsetAsync(counters, 0, counterBytes, s));
                 GRGX_CUDA(cudaEventRecord(e0, s));
-                launch_level(L, *cur, lvl, vals, vals, curMode == 1 ? 0 : rmw, partials, tickets, work, s, nullptr, 0,
+                launch_level(L, *cur, lvl, vals, vals, curMode == 1 ? 0 : rmw, partials, tickets, work, s, nullptr,
                              &sh, maxT, curMode ? state : nullptr, curBase, curMode ? curMode : 1);
                 GRGX_CUDA(cudaEventRecord(e1, s));
                 GRGX_CUDA(cudaEventSynchronize(e1));

@@ -168,14 +168,13 @@ DevCSR fine_view(DevicePlan& d, const DevCSR& coarse, const PullCSR& fine);
 // from the accumulator merged with the row's sum.
 int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src, void* dst, int rmw,
                  void* partials, unsigned* tickets, unsigned* work, cudaStream_t s, const int* gate = nullptr,
-                 int gateValue = 0, const LevelShape* shape = nullptr, int tileStride = 0, void* state = nullptr,
+                 const LevelShape* shape = nullptr, int tileStride = 0, void* state = nullptr,
                  long long stateBase = 0, int stateMode = 1);
 
 // UP in split form (up_split.cu): writes vals[node] from its accumulator state (added onto the
 // value when rmw) for the `count` nodes listed at `nodes`.
 void launch_state_finish(Kind kind, const void* state, void* vals, const int* nodes, long long count,
-                         long long stateBase, long long stride, int rmw, cudaStream_t s, const int* gate,
-                         int gateValue);
+                         long long stateBase, long long stride, int rmw, cudaStream_t s, const int* gate);
 // Height-0 row bytes (height-0 ids x stride x element size) above which UP runs in split form,
 // and the block of height-0 ids each split pass covers; both adjustable for tests.
 constexpr unsigned long long kDefaultSplitThreshold = 64ull << 20;
@@ -239,7 +238,7 @@ PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit);
 // Adds the height-0 rows' sums onto vals; `work` holds L.ntiles zeroed counters per range.
 // Returns the kernels launched.
 int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
-                     unsigned* work, cudaStream_t s, const int* gate, int gateValue);
+                     unsigned* work, cudaStream_t s, const int* gate);
 
 // The launches of an UP call in pair form: ranges of segments, with a table of pattern rows at a
 // time.
@@ -254,7 +253,7 @@ PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit);
 // Writes every node's sum over its height-0 children to vals (onto it when rmw), or leaves it in
 // `state` where one is given.
 int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, void* vals, void* table, void* state,
-                   int rmw, cudaStream_t s, const int* gate, int gateValue);
+                   int rmw, cudaStream_t s, const int* gate);
 // Builds the UP edges to children of height >= 1 (up_int and the finish lists), once: `low` = each
 // UP row's children of height 0.  The caller holds the graph's lock.
 void build_up_internal(DevicePlan& d, const std::vector<unsigned>& low);

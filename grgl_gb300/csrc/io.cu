@@ -63,10 +63,8 @@ template <typename S> __device__ __forceinline__ S s_add(S a, S b) { return a + 
 template <typename IO>
 __global__ void load_rows_kernel(const IO* __restrict__ src, long long K, long long ld, long long R, int mode,
                                  long long div, const uint32_t* __restrict__ tab,
-                                 typename Store<IO>::S* __restrict__ dst, long long stride, int add,
-                                 const int* gate, int gate_value) {
+                                 typename Store<IO>::S* __restrict__ dst, long long stride, int add) {
     using S = typename Store<IO>::S;
-    if (gate != nullptr && *gate != gate_value) return;
     __shared__ S tile[32][33];
     const long long i0 = (long long)blockIdx.x * 32, k0 = (long long)blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -96,9 +94,8 @@ __global__ void load_rows_kernel(const IO* __restrict__ src, long long K, long l
 template <typename IO>
 __global__ void store_cols_kernel(const typename Store<IO>::S* __restrict__ vals, long long stride, long long K,
                                   long long C, int mode, long long fold, const uint32_t* __restrict__ tab,
-                                  IO* __restrict__ out, long long ld, int add, const int* gate, int gate_value) {
+                                  IO* __restrict__ out, long long ld, int add) {
     using S = typename Store<IO>::S;
-    if (gate != nullptr && *gate != gate_value) return;
     __shared__ S tile[32][33];
     const long long c0 = (long long)blockIdx.x * 32, k0 = (long long)blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -131,10 +128,8 @@ __global__ void store_cols_kernel(const typename Store<IO>::S* __restrict__ vals
 
 template <typename IO>
 __global__ void init_vector_kernel(const IO* __restrict__ init, long long K, long long n,
-                                   typename Store<IO>::S* __restrict__ vals, long long stride, const int* gate,
-                                   int gate_value) {
+                                   typename Store<IO>::S* __restrict__ vals, long long stride) {
     using S = typename Store<IO>::S;
-    if (gate != nullptr && *gate != gate_value) return;
     const long long total = n * stride;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
          x += (long long)gridDim.x * blockDim.x) {
@@ -145,10 +140,8 @@ __global__ void init_vector_kernel(const IO* __restrict__ init, long long K, lon
 
 template <typename IO>
 __global__ void init_xtx_kernel(const uint32_t* __restrict__ xtx, long long K, long long n,
-                                typename Store<IO>::S* __restrict__ vals, long long stride, const int* gate,
-                                int gate_value) {
+                                typename Store<IO>::S* __restrict__ vals, long long stride) {
     using S = typename Store<IO>::S;
-    if (gate != nullptr && *gate != gate_value) return;
     const long long total = n * stride;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
          x += (long long)gridDim.x * blockDim.x) {
@@ -197,20 +190,20 @@ __global__ void store_bits_kernel(const uint32_t* __restrict__ vals, long long s
 
 template <typename IO>
 void load_rows_t(const void* src, long long K, long long ld, long long R, int mode, long long div, const uint32_t* tab,
-                 void* dst, long long stride, int add, const int* gate, int gv, cudaStream_t s) {
+                 void* dst, long long stride, int add, cudaStream_t s) {
     if (R <= 0) return;
     const dim3 grid((unsigned)((R + 31) / 32), (unsigned)((stride + 31) / 32));
     load_rows_kernel<IO><<<grid, dim3(32, 8), 0, s>>>(static_cast<const IO*>(src), K, ld, R, mode, div, tab,
-                                                      static_cast<typename Store<IO>::S*>(dst), stride, add, gate, gv);
+                                                      static_cast<typename Store<IO>::S*>(dst), stride, add);
 }
 
 template <typename IO>
 void store_cols_t(const void* vals, long long stride, long long K, long long C, int mode, long long fold,
-                  const uint32_t* tab, void* out, long long ld, int add, const int* gate, int gv, cudaStream_t s) {
+                  const uint32_t* tab, void* out, long long ld, int add, cudaStream_t s) {
     if (C <= 0 || K <= 0) return;
     const dim3 grid((unsigned)((C + 31) / 32), (unsigned)((K + 31) / 32));
     store_cols_kernel<IO><<<grid, dim3(32, 8), 0, s>>>(static_cast<const typename Store<IO>::S*>(vals), stride, K,
-                                                       C, mode, fold, tab, static_cast<IO*>(out), ld, add, gate, gv);
+                                                       C, mode, fold, tab, static_cast<IO*>(out), ld, add);
 }
 
 unsigned grid_for(long long total) {
@@ -238,8 +231,7 @@ unsigned grid_for(long long total) {
     }
 
 void launch_load_rows(int dtype, const void* src, long long K, long long ld, long long R, int mode, long long div,
-                      const uint32_t* tab, void* dst, long long stride, int add, cudaStream_t s, const int* gate,
-                      int gv) {
+                      const uint32_t* tab, void* dst, long long stride, int add, cudaStream_t s) {
     if (dtype == GRGX_BOOL) {
         if (R <= 0) return;
         const dim3 grid((unsigned)((R + 127) / 128), (unsigned)stride);
@@ -247,14 +239,13 @@ void launch_load_rows(int dtype, const void* src, long long K, long long ld, lon
                                               static_cast<uint32_t*>(dst), stride, add);
         return;
     }
-#define CALL(T) load_rows_t<T>(src, K, ld, R, mode, div, tab, dst, stride, add, gate, gv, s)
+#define CALL(T) load_rows_t<T>(src, K, ld, R, mode, div, tab, dst, stride, add, s)
     GRGX_IO_DISPATCH(dtype, CALL)
 #undef CALL
 }
 
 void launch_store_cols(int dtype, const void* vals, long long stride, long long K, long long C, int mode,
-                       long long fold, const uint32_t* tab, void* out, long long ld, int add, cudaStream_t s,
-                       const int* gate, int gv) {
+                       long long fold, const uint32_t* tab, void* out, long long ld, int add, cudaStream_t s) {
     if (dtype == GRGX_BOOL) {
         if (C <= 0 || K <= 0) return;
         const dim3 grid((unsigned)((C + 127) / 128), (unsigned)K);
@@ -262,26 +253,26 @@ void launch_store_cols(int dtype, const void* vals, long long stride, long long 
                                                static_cast<uint8_t*>(out), ld, add);
         return;
     }
-#define CALL(T) store_cols_t<T>(vals, stride, K, C, mode, fold, tab, out, ld, add, gate, gv, s)
+#define CALL(T) store_cols_t<T>(vals, stride, K, C, mode, fold, tab, out, ld, add, s)
     GRGX_IO_DISPATCH(dtype, CALL)
 #undef CALL
 }
 
 void launch_init_vector(int dtype, const void* init, long long K, long long n, void* vals, long long stride,
-                        cudaStream_t s, const int* gate, int gv) {
+                        cudaStream_t s) {
     const unsigned grid = grid_for(n * stride);
 #define CALL(T)                                                                                            \
     init_vector_kernel<T><<<grid, 256, 0, s>>>(static_cast<const T*>(init), K, n,                          \
-                                               static_cast<typename Store<T>::S*>(vals), stride, gate, gv)
+                                               static_cast<typename Store<T>::S*>(vals), stride)
     GRGX_IO_DISPATCH(dtype, CALL)
 #undef CALL
 }
 
 void launch_init_xtx(int dtype, const uint32_t* xtx, long long K, long long n, void* vals, long long stride,
-                     cudaStream_t s, const int* gate, int gv) {
+                     cudaStream_t s) {
     const unsigned grid = grid_for(n * stride);
 #define CALL(T) \
-    init_xtx_kernel<T><<<grid, 256, 0, s>>>(xtx, K, n, static_cast<typename Store<T>::S*>(vals), stride, gate, gv)
+    init_xtx_kernel<T><<<grid, 256, 0, s>>>(xtx, K, n, static_cast<typename Store<T>::S*>(vals), stride)
     GRGX_IO_DISPATCH(dtype, CALL)
 #undef CALL
 }

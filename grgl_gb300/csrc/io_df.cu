@@ -1,4 +1,6 @@
-// Seed and gather kernels for float64 carried as scaled float pairs (AddF64S, ops.cuh).
+// Seed and gather kernels for float64 carried as scaled float pairs (AddF64S, ops.cuh), or as plain
+// doubles in the same buffers when the call's gate is set (rows spanning too many binades, infinities
+// or nans: the FP64 path).
 //
 // Each input row k is scaled by the exact power of two 2^-e_k (e_k = exponent of the row's
 // largest finite magnitude, clamped to the normal range) before it is split into hi + lo floats,
@@ -104,8 +106,9 @@ __global__ void load_rows_df_kernel(const double* __restrict__ src, long long K,
                                     long long div, const uint32_t* __restrict__ tab, DF* __restrict__ dst,
                                     long long stride, int add, const unsigned long long* __restrict__ rowmax,
                                     const int* gate) {
-    if (gate != nullptr && *gate != 0) return;
-    __shared__ DF tile[32][33];
+    const bool native = gate != nullptr && *gate != 0;
+    double* const plain = reinterpret_cast<double*>(dst);
+    __shared__ double tile[32][33];  // a double's or a float pair's 8 bytes
     const long long i0 = (long long)blockIdx.x * 32, k0 = (long long)blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const long long i = i0 + tx;
@@ -114,7 +117,9 @@ __global__ void load_rows_df_kernel(const double* __restrict__ src, long long K,
 #pragma unroll
     for (int j = ty; j < 32; j += 8) {
         const long long k = k0 + j;
-        tile[j][tx] = (k < K && colIdx >= 0) ? split_scaled(src[k * ld + colIdx], row_exp(rowmax, k)) : DF{0.f, 0.f};
+        const double x = (k < K && colIdx >= 0) ? src[k * ld + colIdx] : 0.0;
+        if (native) tile[j][tx] = x;
+        else reinterpret_cast<DF&>(tile[j][tx]) = (k < K) ? split_scaled(x, row_exp(rowmax, k)) : DF{0.f, 0.f};
     }
     __syncthreads();
 #pragma unroll
@@ -122,12 +127,14 @@ __global__ void load_rows_df_kernel(const double* __restrict__ src, long long K,
         const long long r = i0 + j, k = k0 + tx;
         if (r < R && k < stride) {
             const long long e = r * stride + k;
-            if (add) {
-                if (k < K)
-                    df_put(dst, e, stride,
-                           AddF64S::split(AddF64S::value(df_get(dst, e, stride)) + AddF64S::value(tile[tx][j])));
+            const DF t = reinterpret_cast<const DF&>(tile[tx][j]);
+            if (native) {
+                if (!add) plain[e] = tile[tx][j];
+                else if (k < K) plain[e] += tile[tx][j];
+            } else if (add) {
+                if (k < K) df_put(dst, e, stride, AddF64S::split(AddF64S::value(df_get(dst, e, stride)) + AddF64S::value(t)));
             } else {
-                df_put(dst, e, stride, tile[tx][j]);
+                df_put(dst, e, stride, t);
             }
         }
     }
@@ -137,7 +144,9 @@ __global__ void store_cols_df_kernel(const DF* __restrict__ vals, long long stri
                                      int mode, long long fold, const uint32_t* __restrict__ tab,
                                      double* __restrict__ out, long long ld, int add,
                                      const unsigned long long* __restrict__ rowmax, const int* gate) {
-    if (gate != nullptr && *gate != 0) return;
+    const bool native = gate != nullptr && *gate != 0;
+    const double* const plain = reinterpret_cast<const double*>(vals);
+    auto value = [&](long long e) { return native ? plain[e] : AddF64S::value(df_get(vals, e, stride)); };
     __shared__ double tile[32][33];
     const long long c0 = (long long)blockIdx.x * 32, k0 = (long long)blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -147,12 +156,12 @@ __global__ void store_cols_df_kernel(const DF* __restrict__ vals, long long stri
         double v = 0.0;
         if (c < C && k < K) {
             if (mode == MAP_FOLD) {
-                for (long long p = 0; p < fold; p++) v += AddF64S::value(df_get(vals, (c * fold + p) * stride + k, stride));
+                for (long long p = 0; p < fold; p++) v = (p == 0) ? value((c * fold) * stride + k) : v + value((c * fold + p) * stride + k);
             } else {
                 const long long node = (mode == MAP_TABLE) ? (long long)tab[c] : c;
-                if (node != (long long)kInvalid) v = AddF64S::value(df_get(vals, node * stride + k, stride));
+                if (node != (long long)kInvalid) v = value(node * stride + k);
             }
-            v *= pow2(row_exp(rowmax, k));
+            if (!native) v *= pow2(row_exp(rowmax, k));
         }
         tile[j][tx] = v;
     }
@@ -170,23 +179,25 @@ __global__ void store_cols_df_kernel(const DF* __restrict__ vals, long long stri
 __global__ void init_vector_df_kernel(const double* __restrict__ init, long long K, long long n, DF* __restrict__ vals,
                                       long long stride, const unsigned long long* __restrict__ rowmax,
                                       const int* gate) {
-    if (gate != nullptr && *gate != 0) return;
+    const bool native = gate != nullptr && *gate != 0;
     const long long total = n * stride;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
          x += (long long)gridDim.x * blockDim.x) {
         const long long k = x % stride;
-        df_put(vals, x, stride, (k < K) ? split_scaled(init[k], row_exp(rowmax, k)) : DF{0.f, 0.f});
+        if (native) reinterpret_cast<double*>(vals)[x] = (k < K) ? init[k] : 0.0;
+        else df_put(vals, x, stride, (k < K) ? split_scaled(init[k], row_exp(rowmax, k)) : DF{0.f, 0.f});
     }
 }
 
 __global__ void init_xtx_df_kernel(const uint32_t* __restrict__ xtx, long long K, long long n, DF* __restrict__ vals,
                                    long long stride, const unsigned long long* __restrict__ rowmax, const int* gate) {
-    if (gate != nullptr && *gate != 0) return;
+    const bool native = gate != nullptr && *gate != 0;
     const long long total = n * stride;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
          x += (long long)gridDim.x * blockDim.x) {
         const long long k = x % stride, v = x / stride;
-        df_put(vals, x, stride, (k < K) ? split_scaled(static_cast<double>(xtx[v]), row_exp(rowmax, k)) : DF{0.f, 0.f});
+        if (native) reinterpret_cast<double*>(vals)[x] = (k < K) ? static_cast<double>(xtx[v]) : 0.0;
+        else df_put(vals, x, stride, (k < K) ? split_scaled(static_cast<double>(xtx[v]), row_exp(rowmax, k)) : DF{0.f, 0.f});
     }
 }
 

@@ -47,8 +47,7 @@ template <typename S> struct PairDownParams {
     long long rows, stride, groups;
     unsigned base0, tiles, items;
     int group_begin, group_end, groups_per_item, part_begin;
-    const int* gate;
-    int gate_value;
+    const int* gate;  // as SweepParams::gate
 };
 // What a pair_down_* call does, and what its kShape step answers.
 struct PairDownCall {
@@ -85,8 +84,7 @@ template <typename S> struct PairUpParams {
     void* state;   // when set, accumulators (Op::A)
     int second;    // the sources are rows of the table
     long long stride;
-    const int* gate;
-    int gate_value;
+    const int* gate;  // as SweepParams::gate
 };
 void pair_up_u32(const PairUpParams<uint32_t>& p, int vw, int g, cudaStream_t s);
 void pair_up_xor(const PairUpParams<uint32_t>& p, int vw, int g, cudaStream_t s);
@@ -101,30 +99,27 @@ enum MapMode { MAP_IDENT = 0, MAP_DIV = 1, MAP_TABLE = 2, MAP_FOLD = 3 };
 
 // dst[i*stride + k] (=, or += when add) IO->S(src[k*ld + col(i)]) for i < R, k < K; columns
 // K..stride-1 are zeroed when assigning.  col(i) = i, i/div, or tab[i].
-// `gate`: when non-null the kernel runs only if *gate == gate_value (device-side path choice).
 void launch_load_rows(int dtype, const void* src, long long K, long long ld, long long R, int mode, long long div,
-                      const uint32_t* tab, void* dst, long long stride, int add, cudaStream_t s,
-                      const int* gate = nullptr, int gate_value = 0);
+                      const uint32_t* tab, void* dst, long long stride, int add, cudaStream_t s);
 
 // out[k*ld + c] (=, or += when add) S->IO(vals[map(c)]) for c < C, k < K; map(c) = c, tab[c]
 // (INVALID -> 0), or the sum of rows c*fold .. c*fold+fold-1.
 void launch_store_cols(int dtype, const void* vals, long long stride, long long K, long long C, int mode,
-                       long long fold, const uint32_t* tab, void* out, long long ld, int add, cudaStream_t s,
-                       const int* gate = nullptr, int gate_value = 0);
+                       long long fold, const uint32_t* tab, void* out, long long ld, int add, cudaStream_t s);
 
 // Node-value initialisation: VECTOR (vals[v][k] = init[k]) and XTX (vals[v][k] = xtx[v]).
 void launch_init_vector(int dtype, const void* init, long long K, long long n, void* vals, long long stride,
-                        cudaStream_t s, const int* gate = nullptr, int gate_value = 0);
+                        cudaStream_t s);
 void launch_init_xtx(int dtype, const uint32_t* xtx, long long K, long long n, void* vals, long long stride,
-                     cudaStream_t s, const int* gate = nullptr, int gate_value = 0);
+                     cudaStream_t s);
 
 // ---- float64 as scaled float pairs (AddF64S) ----------------------------------------------
 // rowmax[k] = max over finite |x| of row k, as IEEE bits (0 for an all-zero row); callers
 // fill it first (0, or a floor such as the largest XTX init value) and may fold several
 // matrices into it.  Row k is scaled by 2^(60 - e_k), e_k the exponent of rowmax[k], so the
 // row's largest value sits in [2^60, 2^61) and values down to 2^-126 of float range (186
-// binades below the maximum) keep full precision.  The float-pair kernels run when
-// gate[0] == 0.
+// binades below the maximum) keep full precision.  When gate[0] != 0 the same launches move plain
+// doubles instead (the call takes the FP64 path).
 void launch_fill_u64(unsigned long long* p, long long n, unsigned long long v, cudaStream_t s);
 // Also folds the smallest nonzero finite magnitude into rowmin[k] (filled with ~0 first).
 void launch_rowmax(const double* src, long long K, long long ld, long long cols, unsigned long long* rowmax,

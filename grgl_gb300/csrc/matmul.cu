@@ -258,7 +258,6 @@ SweepParams<S> make_params(const DevCSR& c, long long cb, long long ce, const vo
     p.work = work;
     p.ntiles = ntiles;
     p.gate = nullptr;
-    p.gate_value = 0;
     p.state = nullptr;
     p.state_base = 0;
     p.state_mode = 0;
@@ -276,7 +275,7 @@ SweepParams<S> make_params(const DevCSR& c, long long cb, long long ce, const vo
 // by this level.
 int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src, void* dst, int rmw,
                  void* partials, unsigned* tickets, unsigned* work, cudaStream_t s, const int* gate,
-                 int gateValue, const LevelShape* shape, int tileStride, void* state, long long stateBase,
+                 const LevelShape* shape, int tileStride, void* state, long long stateBase,
                  int stateMode) {
     const long long cb = c.lb[level], ce = c.le[level];
     if (ce <= cb) return 0;
@@ -301,7 +300,6 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
             SweepParams<S> p = make_params<S>(c, cb, ce, src, dst, L.stride, rmw, partials, tickets + slot,
                                               work + slot, ts);
             p.gate = gate;
-            p.gate_value = gateValue;
             p.state = state;
             p.state_base = stateBase;
             p.state_mode = stateMode;
@@ -721,147 +719,135 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
         const int hasInit = (init_kind != GRGX_INIT_ZERO);
         const int add = overwrite ? 0 : 1;
         if (init_kind == GRGX_INIT_ZERO) GRGX_CUDA(cudaMemsetAsync(vals, 0, valBytes, s));
-        // Scratch shared by both float64 paths (same 8-byte elements).
         void* vt = (down && dp->seed.n_edges > 0) ? sc.get(static_cast<size_t>(M) * L.stride * L.ssize) : nullptr;
         void* mt = (down && useMiss && dp->miss.n_edges > 0) ? sc.get(static_cast<size_t>(M) * L.stride * L.ssize)
                                                               : nullptr;
 
-        // One full pipeline (init, seed, level sweep, gather) for layout LL; `pdf` selects the
-        // float-pair I/O kernels; kernels run only where *g == gv when g is set.
-        auto pipeline = [&](const Layout& LL, bool pdf, const int* g, int gv, bool timed) {
-            auto load_rows = [&](const void* src, long long ld, long long R, int mode, long long div,
-                                 const uint32_t* tab, void* dst, int addTo) {
-                if (pdf)
-                    launch_load_rows_df(static_cast<const double*>(src), K, ld, R, mode, div, tab, dst, LL.stride,
-                                        addTo, rowmax, s, g);
-                else
-                    launch_load_rows(dtype, src, K, ld, R, mode, div, tab, dst, LL.stride, addTo, s, g, gv);
-                launches++;
-            };
-            auto store_cols = [&](long long C, int mode, long long fold, const uint32_t* tab, void* out, long long ld,
-                                  int addTo) {
-                if (pdf)
-                    launch_store_cols_df(vals, LL.stride, K, C, mode, fold, tab, static_cast<double*>(out), ld, addTo,
-                                         rowmax, s, g);
-                else
-                    launch_store_cols(dtype, vals, LL.stride, K, C, mode, fold, tab, out, ld, addTo, s, g, gv);
-                launches++;
-            };
-            auto level = [&](const DevCSR& c, size_t lvl, const void* src, int rmw, unsigned* tk, unsigned* wk) {
-                const LevelShape sh = level_shape(LL, c, lvl);
-                return launch_level(LL, c, lvl, src, vals, rmw, partials, tk, wk, s, g, gv, &sh, TS);
-            };
-            switch (init_kind) {
-            case GRGX_INIT_VECTOR:
-                if (pdf)
-                    launch_init_vector_df(static_cast<const double*>(dInit), K, n, vals, LL.stride, rowmax, s, g);
-                else
-                    launch_init_vector(dtype, dInit, K, n, vals, LL.stride, s, g, gv);
-                launches++;
-                break;
-            case GRGX_INIT_MATRIX: load_rows(dInit, n, n, MAP_TABLE, 1, dp->new2old, vals, 0); break;
-            case GRGX_INIT_XTX:
-                if (pdf)
-                    launch_init_xtx_df(dp->xtx_new, K, n, vals, LL.stride, rowmax, s, g);
-                else
-                    launch_init_xtx(dtype, dp->xtx_new, K, n, vals, LL.stride, s, g, gv);
-                launches++;
-                break;
-            default: break;
+        // Init, seed, level sweep, gather.  float64 launches look at the gate: float pairs, or doubles
+        // in the same buffers.
+        auto load_rows = [&](const void* src, long long ld, long long R, int mode, long long div,
+                             const uint32_t* tab, void* dst, int addTo) {
+            if (df)
+                launch_load_rows_df(static_cast<const double*>(src), K, ld, R, mode, div, tab, dst, L.stride,
+                                    addTo, rowmax, s, gate);
+            else
+                launch_load_rows(dtype, src, K, ld, R, mode, div, tab, dst, L.stride, addTo, s);
+            launches++;
+        };
+        auto store_cols = [&](long long C, int mode, long long fold, const uint32_t* tab, void* out, long long ld,
+                              int addTo) {
+            if (df)
+                launch_store_cols_df(vals, L.stride, K, C, mode, fold, tab, static_cast<double*>(out), ld, addTo,
+                                     rowmax, s, gate);
+            else
+                launch_store_cols(dtype, vals, L.stride, K, C, mode, fold, tab, out, ld, addTo, s);
+            launches++;
+        };
+        auto level = [&](const DevCSR& c, size_t lvl, const void* src, int rmw, unsigned* tk, unsigned* wk) {
+            const LevelShape sh = level_shape(L, c, lvl);
+            return launch_level(L, c, lvl, src, vals, rmw, partials, tk, wk, s, gate, &sh, TS);
+        };
+        switch (init_kind) {
+        case GRGX_INIT_VECTOR:
+            if (df)
+                launch_init_vector_df(static_cast<const double*>(dInit), K, n, vals, L.stride, rowmax, s, gate);
+            else
+                launch_init_vector(dtype, dInit, K, n, vals, L.stride, s);
+            launches++;
+            break;
+        case GRGX_INIT_MATRIX: load_rows(dInit, n, n, MAP_TABLE, 1, dp->new2old, vals, 0); break;
+        case GRGX_INIT_XTX:
+            if (df)
+                launch_init_xtx_df(dp->xtx_new, K, n, vals, L.stride, rowmax, s, gate);
+            else
+                launch_init_xtx(dtype, dp->xtx_new, K, n, vals, L.stride, s);
+            launches++;
+            break;
+        default: break;
+        }
+        if (down) {
+            // DOWN seed: mutation rows, then node <- sum of its mutations (and missingness)
+            unsigned* tk = tickets;
+            if (vt) {
+                load_rows(dIn, in_cols, M, MAP_IDENT, 1, nullptr, vt, 0);
+                launches += level(dp->seed, 0, vt, hasInit, tk, work);
             }
-            if (down) {
-                // DOWN seed: mutation rows, then node <- sum of its mutations (and missingness)
-                unsigned* tk = tickets;
-                if (vt) {
-                    load_rows(dIn, in_cols, M, MAP_IDENT, 1, nullptr, vt, 0);
-                    launches += level(dp->seed, 0, vt, hasInit, tk, work);
+            tk += dp->seed.n_heavy * TS;
+            if (mt) {
+                load_rows(dMiss, M, M, MAP_IDENT, 1, nullptr, mt, 0);
+                launches += level(dp->miss, 0, mt, 1, tk, work + TS);
+            }
+            tk += dp->miss.n_heavy * TS;
+            if (t_timing) GRGX_CUDA(cudaEventRecord(ev[1], s));
+            const size_t nlv = cDown.lb.size();
+            for (size_t lvl = 0; lvl < nlv; lvl++) {
+                if ((dsplit || dpair) && lvl + 1 == nlv) break;  // the height-0 level runs below
+                launches += level(cDown, lvl, vals, 1, tk, work + (2 + lvl) * TS);
+            }
+            if (dpair)
+                launches += launch_pair_down(L, dp, prun, vals, ptable, pparts, work + (2 + nlv) * TS, s, gate);
+            if (dsplit && staged) {
+                launches += launch_staged(L.kind, stl, vals, slots, nullptr, 0, 1, s);
+            } else if (dsplit) {
+                // parent-block passes merge each height-0 row's sums into its state; then the
+                // rows are written from it, onto their seed / init values
+                GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
+                unsigned* tS = tk + cDown.n_heavy * TS;
+                unsigned* wS = work + (2 + nlv) * TS;
+                for (size_t j = 0; j < cDown0b.lb.size(); j++) {
+                    const LevelShape sh = level_shape(L, cDown0b, j);
+                    launches += launch_level(L, cDown0b, j, vals, vals, 0, partials, tS, wS + j * TS, s, gate, &sh,
+                                             TS, state, 0, 1);
                 }
-                tk += dp->seed.n_heavy * TS;
-                if (mt) {
-                    load_rows(dMiss, M, M, MAP_IDENT, 1, nullptr, mt, 0);
-                    launches += level(dp->miss, 0, mt, 1, tk, work + TS);
+                launch_state_finish(L.kind, state, vals, dp->fin_down, dp->n_fin_down, 0, L.stride, 1, s, gate);
+                launches++;
+            }
+            if (t_timing) GRGX_CUDA(cudaEventRecord(ev[2], s));
+            if (emit_all) {
+                store_cols(n, MAP_TABLE, 1, dp->old2new, dOut, out_cols, add);
+            } else if (by_indiv) {
+                store_cols(out_cols, MAP_FOLD, P, nullptr, dOut, out_cols, add);
+            } else {
+                store_cols(out_cols, MAP_IDENT, 1, nullptr, dOut, out_cols, add);
+            }
+        } else {
+            // UP seed: samples <- input columns
+            load_rows(dIn, in_cols, N, by_indiv ? MAP_DIV : MAP_IDENT, P, nullptr, vals, hasInit);
+            if (t_timing) GRGX_CUDA(cudaEventRecord(ev[1], s));
+            if (split || upair) {
+                if (state) GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
+                unsigned* tIn = tickets + (upair ? 0 : cUp0b.n_heavy) * TS;
+                unsigned* wIn = work + (upair ? 0 : cUp0b.lb.size()) * TS;
+                if (upair)
+                    launches += launch_pair_up(L, dp, urun, vals, ptable, state, hasInit, s, gate);
+                if (staged) launches += launch_staged(L.kind, stl, vals, slots, state, h0, hasInit, s);
+                for (size_t j = 0; split && !staged && j < cUp0b.lb.size(); j++) {
+                    const LevelShape sh = level_shape(L, cUp0b, j);
+                    launches += launch_level(L, cUp0b, j, vals, vals, 0, partials, tickets, work + j * TS, s, gate,
+                                             &sh, TS, state, h0, 1);
                 }
-                tk += dp->miss.n_heavy * TS;
-                if (timed && t_timing) GRGX_CUDA(cudaEventRecord(ev[1], s));
-                const size_t nlv = cDown.lb.size();
-                for (size_t lvl = 0; lvl < nlv; lvl++) {
-                    if ((dsplit || dpair) && lvl + 1 == nlv) break;  // the height-0 level runs below
-                    launches += level(cDown, lvl, vals, 1, tk, work + (2 + lvl) * TS);
-                }
-                if (dpair)
-                    launches += launch_pair_down(LL, dp, prun, vals, ptable, pparts, work + (2 + nlv) * TS, s, g, gv);
-                if (dsplit && staged) {
-                    launches += launch_staged(LL.kind, stl, vals, slots, nullptr, 0, 1, s);
-                } else if (dsplit) {
-                    // parent-block passes merge each height-0 row's sums into its state; then the
-                    // rows are written from it, onto their seed / init values
-                    GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
-                    unsigned* tS = tk + cDown.n_heavy * TS;
-                    unsigned* wS = work + (2 + nlv) * TS;
-                    for (size_t j = 0; j < cDown0b.lb.size(); j++) {
-                        const LevelShape sh = level_shape(LL, cDown0b, j);
-                        launches += launch_level(LL, cDown0b, j, vals, vals, 0, partials, tS, wS + j * TS, s, g,
-                                                 gv, &sh, TS, state, 0, 1);
+                for (size_t lvl = 0; lvl < cUpInt.lb.size(); lvl++) {
+                    const LevelShape sh = level_shape(L, cUpInt, lvl);
+                    launches += launch_level(L, cUpInt, lvl, vals, vals, state ? hasInit : 1, partials, tIn,
+                                             wIn + lvl * TS, s, gate, &sh, TS, state, h0, 2);
+                    const long long f0 = dp->fin_begin[lvl], f1 = dp->fin_begin[lvl + 1];
+                    if (state && f1 > f0) {
+                        launch_state_finish(L.kind, state, vals, dp->fin + f0, f1 - f0, h0, L.stride, hasInit,
+                                            s, gate);
+                        launches++;
                     }
-                    launch_state_finish(LL.kind, state, vals, dp->fin_down, dp->n_fin_down, 0, LL.stride, 1, s, g,
-                                        gv);
-                    launches++;
-                }
-                if (timed && t_timing) GRGX_CUDA(cudaEventRecord(ev[2], s));
-                if (emit_all) {
-                    store_cols(n, MAP_TABLE, 1, dp->old2new, dOut, out_cols, add);
-                } else if (by_indiv) {
-                    store_cols(out_cols, MAP_FOLD, P, nullptr, dOut, out_cols, add);
-                } else {
-                    store_cols(out_cols, MAP_IDENT, 1, nullptr, dOut, out_cols, add);
                 }
             } else {
-                // UP seed: samples <- input columns
-                load_rows(dIn, in_cols, N, by_indiv ? MAP_DIV : MAP_IDENT, P, nullptr, vals, hasInit);
-                if (timed && t_timing) GRGX_CUDA(cudaEventRecord(ev[1], s));
-                if (split || upair) {
-                    if (state) GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
-                    unsigned* tIn = tickets + (upair ? 0 : cUp0b.n_heavy) * TS;
-                    unsigned* wIn = work + (upair ? 0 : cUp0b.lb.size()) * TS;
-                    if (upair)
-                        launches += launch_pair_up(LL, dp, urun, vals, ptable, state, hasInit, s, g, gv);
-                    if (staged) launches += launch_staged(LL.kind, stl, vals, slots, state, h0, hasInit, s);
-                    for (size_t j = 0; split && !staged && j < cUp0b.lb.size(); j++) {
-                        const LevelShape sh = level_shape(LL, cUp0b, j);
-                        launches += launch_level(LL, cUp0b, j, vals, vals, 0, partials, tickets, work + j * TS, s, g, gv,
-                                                 &sh, TS, state, h0, 1);
-                    }
-                    for (size_t lvl = 0; lvl < cUpInt.lb.size(); lvl++) {
-                        const LevelShape sh = level_shape(LL, cUpInt, lvl);
-                        launches += launch_level(LL, cUpInt, lvl, vals, vals, state ? hasInit : 1, partials, tIn,
-                                                 wIn + lvl * TS, s, g, gv, &sh, TS, state, h0, 2);
-                        const long long f0 = dp->fin_begin[lvl], f1 = dp->fin_begin[lvl + 1];
-                        if (state && f1 > f0) {
-                            launch_state_finish(LL.kind, state, vals, dp->fin + f0, f1 - f0, h0, LL.stride, hasInit,
-                                                s, g, gv);
-                            launches++;
-                        }
-                    }
-                } else {
-                    for (size_t lvl = 0; lvl < cUp.lb.size(); lvl++)
-                        launches += level(cUp, lvl, vals, hasInit, tickets, work + lvl * TS);
-                }
-                if (timed && t_timing) GRGX_CUDA(cudaEventRecord(ev[2], s));
-                if (emit_all) {
-                    store_cols(n, MAP_TABLE, 1, dp->old2new, dOut, out_cols, add);
-                } else {
-                    store_cols(M, MAP_TABLE, 1, dp->mut_new, dOut, out_cols, add);
-                    if (useMiss) store_cols(M, MAP_TABLE, 1, dp->miss_new, dMiss, M, 1);
-                }
+                for (size_t lvl = 0; lvl < cUp.lb.size(); lvl++)
+                    launches += level(cUp, lvl, vals, hasInit, tickets, work + lvl * TS);
             }
-        };
-        if (df) {
-            Layout LN = L;
-            LN.kind = Kind::F64;
-            pipeline(L, true, gate, 0, true);
-            pipeline(LN, false, gate, 1, false);
-        } else {
-            pipeline(L, false, nullptr, 0, true);
+            if (t_timing) GRGX_CUDA(cudaEventRecord(ev[2], s));
+            if (emit_all) {
+                store_cols(n, MAP_TABLE, 1, dp->old2new, dOut, out_cols, add);
+            } else {
+                store_cols(M, MAP_TABLE, 1, dp->mut_new, dOut, out_cols, add);
+                if (useMiss) store_cols(M, MAP_TABLE, 1, dp->miss_new, dMiss, M, 1);
+            }
         }
         GRGX_CUDA(cudaGetLastError());
         if (!devPtrs) {

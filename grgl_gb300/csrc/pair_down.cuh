@@ -61,13 +61,15 @@ template <> struct TableVec<F32Pair, 1> {
     }
 };
 
+// The operator a float-pair kernel stands in for when its call takes the FP64 path.
+template <class Op> constexpr bool kHasF64 = std::is_base_of<AddF64S, Op>::value;
+
 template <class Op, int VW>
-__global__ void pair_table_kernel(const uint2* __restrict__ nodes, long long count, const typename Op::S* __restrict__ vals,
-                                  long long stride, typename PairTable<Op, VW>::T* __restrict__ table, const int* gate,
-                                  int gate_value) {
+__device__ __forceinline__ void pair_table(const uint2* __restrict__ nodes, long long count,
+                                           const typename Op::S* __restrict__ vals, long long stride,
+                                           typename PairTable<Op, VW>::T* __restrict__ table) {
     using S = typename Op::S;
     using T = typename PairTable<Op, VW>::T;
-    if (gate != nullptr && *gate != gate_value) return;
     const unsigned vecs = static_cast<unsigned>(stride / VW);
     const unsigned long long total = (unsigned long long)count * vecs;
     for (unsigned long long x = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
@@ -87,6 +89,18 @@ __global__ void pair_table_kernel(const uint2* __restrict__ nodes, long long cou
     }
 }
 
+template <class Op, int VW>
+__global__ void pair_table_kernel(const uint2* nodes, long long count, const typename Op::S* vals, long long stride,
+                                  typename PairTable<Op, VW>::T* table, const int* gate) {
+    if constexpr (kHasF64<Op>) {
+        if (gate != nullptr && *gate != 0) {
+            pair_table<AddF64, VW>(nodes, count, reinterpret_cast<const double*>(vals), stride, reinterpret_cast<double*>(table));
+            return;
+        }
+    }
+    pair_table<Op, VW>(nodes, count, vals, stride, table);
+}
+
 // Rows per group of lanes: a warp covers (32 / G) * kPairRows rows, four blocks of each at a time,
 // so eight gathers are in flight per lane.  Four rows (sixteen gathers, two blocks of threads per
 // SM instead of three) ran within 3% either way for int32 and wide float64 and slower for the rest
@@ -104,8 +118,7 @@ constexpr int kPairRows = 2;
 // One warp per item (a share of the blocks x a tile of rows).  A row's columns are spread over G
 // lanes as in the sweep; each lane loads its rows' ids of four blocks (8 bytes) and gathers the
 // four pattern rows of each of its kRows rows before adding them.
-template <class Op, int VW, int G>
-__global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<typename Op::S> p) {
+template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(const PairDownParams<typename Op::S>& p) {
     using S = typename Op::S;
     using T = typename PairTable<Op, VW>::T;
     using Acc = VecAcc<Op, VW>;
@@ -113,7 +126,6 @@ __global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<
     constexpr int NG = 32 / G, ROWS = kPairRows;
     static_assert(NG * ROWS <= kPairTile, "a warp's rows end within the padded ids");
     constexpr bool kChains = ChainTraits<Op>::kChains;
-    if (p.gate != nullptr && *p.gate != p.gate_value) return;
     const int lane = threadIdx.x & 31;
     const int lg = lane / G;
     const int col = blockIdx.y * (G * VW) + (lane % G) * VW;
@@ -189,11 +201,21 @@ __global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<
     }
 }
 
+template <class Op, int VW, int G>
+__global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<typename Op::S> p) {
+    if constexpr (kHasF64<Op>) {
+        if (p.gate != nullptr && *p.gate != 0) {
+            pair_down<AddF64, VW, G>(as_f64(p));
+            return;
+        }
+    }
+    pair_down<Op, VW, G>(p);
+}
+
 // Adds up `count` sums per row, in order: into the first one (vals null), or onto the node values.
 template <class Op>
-__global__ void pair_finish_kernel(typename PairPart<Op>::T* __restrict__ parts, int count, long long rows,
-                                   long long stride, typename Op::S* __restrict__ vals, const int* gate, int gate_value) {
-    if (gate != nullptr && *gate != gate_value) return;
+__device__ __forceinline__ void pair_finish(typename PairPart<Op>::T* __restrict__ parts, int count, long long rows,
+                                            long long stride, typename Op::S* __restrict__ vals) {
     const long long total = rows * stride;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
         typename Op::A a = Op::zero();
@@ -207,6 +229,18 @@ __global__ void pair_finish_kernel(typename PairPart<Op>::T* __restrict__ parts,
         else
             vals[x] = Op::finish_onto(vals[x], a);
     }
+}
+
+template <class Op>
+__global__ void pair_finish_kernel(typename PairPart<Op>::T* parts, int count, long long rows, long long stride,
+                                   typename Op::S* vals, const int* gate) {
+    if constexpr (kHasF64<Op>) {
+        if (gate != nullptr && *gate != 0) {
+            pair_finish<AddF64>(parts, count, rows, stride, reinterpret_cast<double*>(vals));
+            return;
+        }
+    }
+    pair_finish<Op>(parts, count, rows, stride, vals);
 }
 
 template <class Op, int VW, int G>
@@ -232,15 +266,14 @@ template <class Op, int VW, int G> void pair_down_as(PairDownParams<typename Op:
         const unsigned long long total = (unsigned long long)c.count * (p.stride / VW);
         const unsigned grid = static_cast<unsigned>(std::min<unsigned long long>((total + 255) / 256, sms * 64ull));
         pair_table_kernel<Op, VW><<<grid, 256, 0, s>>>(c.nodes, c.count, p.vals, p.stride,
-                                                       static_cast<typename PairTable<Op, VW>::T*>(p.table), p.gate,
-                                                       p.gate_value);
+                                                       static_cast<typename PairTable<Op, VW>::T*>(p.table), p.gate);
         return;
     }
     if (c.step == PairDownCall::kFinish) {
         const unsigned long long total = (unsigned long long)p.rows * p.stride;
         const unsigned grid = static_cast<unsigned>(std::min<unsigned long long>((total + 255) / 256, sms * 64ull));
         pair_finish_kernel<Op><<<grid, 256, 0, s>>>(static_cast<typename PairPart<Op>::T*>(p.parts), c.parts, p.rows, p.stride,
-                                                    c.onto ? p.vals : nullptr, p.gate, p.gate_value);
+                                                    c.onto ? p.vals : nullptr, p.gate);
         return;
     }
     const unsigned warps = p.tiles * p.items;

@@ -86,7 +86,7 @@ PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit) {
 }
 
 int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
-                     unsigned* work, cudaStream_t s, const int* gate, int gateValue) {
+                     unsigned* work, cudaStream_t s, const int* gate) {
     const PairPlan& P = dp->pair;
     int launches = 0;
     by_kind(L, [&](auto p, auto fn) {
@@ -102,7 +102,6 @@ int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& r
         p.groups = (P.nblk + 3) / 4;
         p.tiles = static_cast<unsigned>((P.h0 + c.rows_per_warp - 1) / c.rows_per_warp);
         p.gate = gate;
-        p.gate_value = gateValue;
         for (size_t i = 0; i < run.ranges.size(); i++) {
             const PairDownRun::Range& r = run.ranges[i];
             c.step = PairDownCall::kTable;
@@ -148,7 +147,7 @@ PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit) {
 }
 
 int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, void* vals, void* table, void* state,
-                   int rmw, cudaStream_t s, const int* gate, int gateValue) {
+                   int rmw, cudaStream_t s, const int* gate) {
     const PairPlan& P = dp->pair;
     int launches = 0;
     // Lanes per row for the gathers from the height-0 rows: as many as leave the columns of one tile
@@ -175,8 +174,7 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
                 p.second = second ? 1 : 0;
                 p.stride = L.stride;
                 p.gate = gate;
-                p.gate_value = gateValue;
-                fn(p, L.vw, second ? L.g : g, s);
+                        fn(p, L.vw, second ? L.g : g, s);
             };
             switch (L.kind) {
             case Kind::U32: go(PairUpParams<uint32_t>{}, pair_up_u32); break;

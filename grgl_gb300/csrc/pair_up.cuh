@@ -23,8 +23,7 @@ namespace grgx {
 // without the pair form and 4.4 here, float64 K=32 11.9, 9.4 and 5.1, int32 K=48 3.7, 6.5 and 3.8.
 // Four blocks of threads per SM against three: float32 K=64 4.43 against 4.83 ms; batches of four
 // gathers instead of eight: within 3% either way.
-template <class Op, int VW, int G>
-__global__ void __launch_bounds__(256, 4) pair_up_kernel(const PairUpParams<typename Op::S> p) {
+template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const PairUpParams<typename Op::S>& p) {
     using S = typename Op::S;
     using Acc = VecAcc<Op, VW>;
     constexpr int L = G < 8 ? 8 : G;           // lanes per list
@@ -32,7 +31,6 @@ __global__ void __launch_bounds__(256, 4) pair_up_kernel(const PairUpParams<type
     constexpr int SLOTS = G * STEPS;           // rows a lane gathers from them
     constexpr int FLUSH_EVERY = SLOTS >= 32 ? 1 : 32 / SLOTS;
     constexpr bool kChains = ChainTraits<Op>::kChains;
-    if (p.gate != nullptr && *p.gate != p.gate_value) return;
     const int lane = threadIdx.x & 31;
     const int gl = lane % L, sub = gl / G;
     const int col = blockIdx.y * (G * VW) + (lane % G) * VW;
@@ -104,6 +102,17 @@ __global__ void __launch_bounds__(256, 4) pair_up_kernel(const PairUpParams<type
         else out[i] = onto ? Op::finish_onto(out[i], acc.get(i)) : Op::finish(acc.get(i));
     }
     Vec<S, VW>::st(d, out);
+}
+
+template <class Op, int VW, int G>
+__global__ void __launch_bounds__(256, 4) pair_up_kernel(const PairUpParams<typename Op::S> p) {
+    if constexpr (std::is_base_of<AddF64S, Op>::value) {
+        if (p.gate != nullptr && *p.gate != 0) {
+            pair_up<AddF64, VW, G>(as_f64(p));
+            return;
+        }
+    }
+    pair_up<Op, VW, G>(p);
 }
 
 template <class Op, int VW, int G> void pair_up_as(const PairUpParams<typename Op::S>& p, cudaStream_t s) {

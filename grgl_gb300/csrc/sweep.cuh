@@ -15,6 +15,7 @@
 // ticket) adds them up in piece order, so results do not depend on scheduling.
 #pragma once
 #include <cstdint>
+#include <cstring>
 #include <type_traits>
 
 #include "ops.cuh"
@@ -47,8 +48,7 @@ template <typename S> struct SweepParams {
     unsigned* tickets;         // per (heavy row, column tile)
     unsigned* work;            // per column tile: next chunk to take (zeroed before the launch)
     int ntiles;
-    const int* gate;           // when set, the launch runs only if *gate == gate_value
-    int gate_value;
+    const int* gate;           // float64 as float pairs: when set and *gate != 0, the buffers hold doubles
     void* state;               // per-node Op::A carried between launches (UP split passes), or null
     long long state_base;      // node id of the first state row
     int state_mode;            // 1: merge each row sum into its state; 2: write state + row sum
@@ -66,6 +66,17 @@ template <typename S> struct SweepParams {
     // full tiles of another launch).
     int col_base;
 };
+
+// The parameters of a float64 call for its FP64 path: the same buffers, of doubles.  Every kernel of
+// the float-pair pipeline carries this path and takes it when the call's gate says so (io_df.cu):
+// a pipeline of its own behind it was a launch per step that did nothing, a third of the time of a
+// small product (one float64 score on N=1,000, M=10,000: 28 launches before, 16 now).
+template <template <typename> class Params> __device__ __forceinline__ Params<double> as_f64(const Params<DF>& p) {
+    static_assert(sizeof(Params<double>) == sizeof(Params<DF>), "same layout");
+    Params<double> q;
+    memcpy(&q, &p, sizeof(q));
+    return q;
+}
 
 // Edge id e of a chunk as stored (32-bit, or 16-bit zero-extended).  The load is issued a step
 // ahead of its use; decode_id turns it into the 32-bit form the sweep works with (source id |
@@ -377,8 +388,7 @@ template <class Op, int VW, int G, int D> struct SweepOccupancy {
 };
 
 template <class Op, int VW, int G, int D, bool ID16>
-__global__ void __launch_bounds__(256, SweepOccupancy<Op, VW, G, D>::kBlocks) sweep_kernel(const SweepParams<typename Op::S> p) {
-    if (p.gate != nullptr && *p.gate != p.gate_value) return;
+__device__ __forceinline__ void sweep_level(const SweepParams<typename Op::S>& p) {
     const int lane = threadIdx.x & 31;
     unsigned* counter = p.work + blockIdx.y;
     for (;;) {
@@ -390,6 +400,17 @@ __global__ void __launch_bounds__(256, SweepOccupancy<Op, VW, G, D>::kBlocks) sw
     }
 }
 
+template <class Op, int VW, int G, int D, bool ID16>
+__global__ void __launch_bounds__(256, SweepOccupancy<Op, VW, G, D>::kBlocks) sweep_kernel(const SweepParams<typename Op::S> p) {
+    if constexpr (std::is_same<Op, AddF64S>::value) {
+        if (p.gate != nullptr && *p.gate != 0) {
+            sweep_level<AddF64, VW, G, D, ID16>(as_f64(p));
+            return;
+        }
+    }
+    sweep_level<Op, VW, G, D, ID16>(p);
+}
+
 // A level of short rows (most with one edge: a node's only parent, a node's only mutation): G lanes
 // per row walk the row's edges from its offset, many rows at a time.  sweep_kernel would walk such
 // rows one boundary after the other within a chunk, a chain of dependent steps that sets the
@@ -398,11 +419,10 @@ __global__ void __launch_bounds__(256, SweepOccupancy<Op, VW, G, D>::kBlocks) sw
 // A level with longer rows among them has `short_split` groups of lanes to a row, which take its
 // edges in turns of four and merge their sums at the end.
 template <class Op, int VW, int G>
-__global__ void __launch_bounds__(256) short_rows_kernel(const SweepParams<typename Op::S> p) {
+__device__ __forceinline__ void short_rows(const SweepParams<typename Op::S>& p) {
     using S = typename Op::S;
     constexpr bool kPairs = std::is_same<Op, AddF64S>::value;
     constexpr int BATCH = 4;
-    if (p.gate != nullptr && *p.gate != p.gate_value) return;
     const int split = p.short_split;
     const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long row = thread / (G * split);
@@ -474,6 +494,17 @@ __global__ void __launch_bounds__(256) short_rows_kernel(const SweepParams<typen
         }
     }
     write_row<Op, VW>(p, p.short_row0 + row, col, acc);
+}
+
+template <class Op, int VW, int G>
+__global__ void __launch_bounds__(256) short_rows_kernel(const SweepParams<typename Op::S> p) {
+    if constexpr (std::is_same<Op, AddF64S>::value) {
+        if (p.gate != nullptr && *p.gate != 0) {
+            short_rows<AddF64, VW, G>(as_f64(p));
+            return;
+        }
+    }
+    short_rows<Op, VW, G>(p);
 }
 
 }  // namespace grgx

@@ -132,10 +132,9 @@ __global__ void internal_kernel(const uint32_t* __restrict__ adj, const long lon
 }
 
 template <class Op>
-__global__ void state_finish_kernel(const typename Op::A* __restrict__ state, typename Op::S* __restrict__ vals,
-                                    const int* __restrict__ nodes, long long count, long long base, long long stride,
-                                    int rmw, const int* gate, int gateValue) {
-    if (gate != nullptr && *gate != gateValue) return;
+__device__ __forceinline__ void state_finish(const typename Op::A* __restrict__ state, typename Op::S* __restrict__ vals,
+                                             const int* __restrict__ nodes, long long count, long long base,
+                                             long long stride, int rmw) {
     const long long total = count * stride;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
          x += (long long)gridDim.x * blockDim.x) {
@@ -152,13 +151,26 @@ __global__ void state_finish_kernel(const typename Op::A* __restrict__ state, ty
 }
 
 template <class Op>
+__global__ void state_finish_kernel(const typename Op::A* state, typename Op::S* vals, const int* nodes, long long count,
+                                    long long base, long long stride, int rmw, const int* gate) {
+    if constexpr (std::is_same<Op, AddF64S>::value) {
+        if (gate != nullptr && *gate != 0) {
+            state_finish<AddF64>(reinterpret_cast<const double*>(state), reinterpret_cast<double*>(vals), nodes, count, base,
+                                 stride, rmw);
+            return;
+        }
+    }
+    state_finish<Op>(state, vals, nodes, count, base, stride, rmw);
+}
+
+template <class Op>
 void finish_as(const void* state, void* vals, const int* nodes, long long count, long long base, long long stride,
-               int rmw, cudaStream_t s, const int* gate, int gateValue) {
+               int rmw, cudaStream_t s, const int* gate) {
     const long long total = count * stride;
     if (total <= 0) return;
     state_finish_kernel<Op><<<blocks_for(static_cast<unsigned long long>(total), 256), 256, 0, s>>>(
         static_cast<const typename Op::A*>(state), static_cast<typename Op::S*>(vals), nodes, count, base, stride,
-        rmw, gate, gateValue);
+        rmw, gate);
 }
 
 }  // namespace
@@ -217,9 +229,8 @@ bool down_split_forced() { return g_down_mode.load() != 0; }
 void set_down_split_mode(int mode) { g_down_mode.store(mode); }
 
 void launch_state_finish(Kind kind, const void* state, void* vals, const int* nodes, long long count,
-                         long long stateBase, long long stride, int rmw, cudaStream_t s, const int* gate,
-                         int gateValue) {
-#define GRGX_FIN(OP) finish_as<OP>(state, vals, nodes, count, stateBase, stride, rmw, s, gate, gateValue)
+                         long long stateBase, long long stride, int rmw, cudaStream_t s, const int* gate) {
+#define GRGX_FIN(OP) finish_as<OP>(state, vals, nodes, count, stateBase, stride, rmw, s, gate)
     switch (kind) {
     case Kind::U32: GRGX_FIN(AddU32); break;
     case Kind::XOR: GRGX_FIN(XorU32); break;
