@@ -32,8 +32,11 @@ struct DevCSR {
     HeavyDev* heavy = nullptr;
     std::vector<int32_t> lb, le;
     std::vector<long long> level_rows, level_edges;  // per level, for the launch-shape table
-    // per level of short rows: its rows' first edges, relative to level_e0 (else null)
+    // per level of short rows, or small enough for a chain: its rows' first edges, relative to
+    // level_e0 (else null)
     std::vector<unsigned*> level_short;
+    // ... and whether short_rows_kernel takes it (else the offsets serve chains only)
+    std::vector<char> level_alone;
     std::vector<long long> level_r0, level_e0;
     std::vector<int> level_most;  // its longest row
     long long n_heavy = 0, n_pieces = 0, n_edges = 0, n_rows = 0;
@@ -170,6 +173,25 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
                  void* partials, unsigned* tickets, unsigned* work, cudaStream_t s, const int* gate = nullptr,
                  const LevelShape* shape = nullptr, int tileStride = 0, void* state = nullptr,
                  long long stateBase = 0, int stateMode = 1);
+
+// Levels first .. last-1 of a CSR, launched one by one or, where consecutive ones are short and small,
+// as chains (chain.cuh).  `seed` set: its level 0 (gathering from seedSrc, seedRmw) goes first.
+// `tickets` and `work` as for launch_level, level lvl's counters at work + lvl * tileStride (the
+// seed's own: seedTickets, seedWork).
+struct LevelRun {
+    const DevCSR* csr = nullptr;
+    size_t first = 0, last = 0;
+    int rmw = 0;
+    unsigned *tickets = nullptr, *work = nullptr;
+    const DevCSR* seed = nullptr;
+    const void* seedSrc = nullptr;
+    int seedRmw = 0;
+    unsigned *seedTickets = nullptr, *seedWork = nullptr;
+    void* state = nullptr;  // mode 2
+    long long stateBase = 0;
+};
+int launch_levels(const Layout& L, const LevelRun& run, void* vals, void* partials, int tileStride, cudaStream_t s,
+                  const int* gate);
 
 // UP in split form (up_split.cu): writes vals[node] from its accumulator state (added onto the
 // value when rmw) for the `count` nodes listed at `nodes`.

@@ -32,6 +32,34 @@ void launch_sweep_f32(const SweepParams<float>& p, int vw, int g, int variant, d
 void launch_sweep_f64s(const SweepParams<DF>& p, int vw, int g, int variant, dim3 grid,
                       int sms, cudaStream_t s);
 
+// Chains of small levels (chain.cuh): up to kChainMost levels in one launch of one cluster.
+constexpr int kChainMost = 24, kChainBlocks = 16, kChainThreads = 1024;
+struct ChainLevel {
+    const unsigned* off;   // first edge of each row (rows + 1), relative to adj
+    const uint32_t* adj;
+    const int* nodes;      // destination of each row
+    const void* src;       // rows gathered from
+    unsigned rows;
+    int split, rmw;
+};
+struct ChainParams {
+    ChainLevel level[kChainMost];
+    int count, tiles;      // tiles: of G x VW columns
+    void* vals;
+    long long stride;
+    void* state;           // as SweepParams::state, mode 2
+    long long state_base;
+    const int* gate;       // as SweepParams::gate
+};
+bool chain_supported();  // the device takes a cluster of that size
+void launch_chain_u32(const ChainParams& p, int vw, int g, cudaStream_t s);
+void launch_chain_xor(const ChainParams& p, int vw, int g, cudaStream_t s);
+void launch_chain_u64(const ChainParams& p, int vw, int g, cudaStream_t s);
+void launch_chain_f64(const ChainParams& p, int vw, int g, cudaStream_t s);
+void launch_chain_f32c(const ChainParams& p, int vw, int g, cudaStream_t s);
+void launch_chain_f32(const ChainParams& p, int vw, int g, cudaStream_t s);
+void launch_chain_f64s(const ChainParams& p, int vw, int g, cudaStream_t s);
+
 // The pair form's ids are padded to whole groups of this many height-0 rows: no warp takes more.
 constexpr int kPairTile = 128;
 

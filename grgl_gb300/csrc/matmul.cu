@@ -60,6 +60,15 @@ template <typename T> T* upload(DevicePlan& d, const std::vector<T>& v) {
 // (float64 K=64 turns between d=8, 193 against 229, and d=16, 379 against 258).  A row walked by
 // one group of lanes takes about 0.2 us per four edges: the longest allowed ends with the level.
 constexpr long long kShortMean = 8, kShortMost = 128;
+// Other levels of few edges, and none in a row that would hold up the rest, may join a chain.
+constexpr long long kChainEdges = 1 << 17, kChainRow = 512;
+// A level joins a chain when the cluster's threads get through its rows in at most kChainRounds rounds
+// and its gathers, kChainGathers lanes at most, do not need the other SMs.  On N=1,000, M=10,000 (all
+// levels in one chain against a launch each): int32 K=1 UP 43 against 57 us, float64 K=5 UP 99
+// against 131, float64 K=1 DOWN 55 against 60; past the line float32 K=20 DOWN (800,000 lanes in its
+// last level) 64 against 52 and float64 K=64 UP 249 against 183.  With 4 or 8 rounds float64 K=20
+// DOWN on N=20,000, M=50,000 loses 2-7%.
+constexpr long long kChainRounds = 2, kChainGathers = 1 << 18;
 
 }  // namespace
 
@@ -68,20 +77,23 @@ void mark_short_levels(DevicePlan& d, DevCSR& r, const PullCSR& c, const std::ve
     r.level_r0.assign(c.level_chunk_begin.size(), 0);
     r.level_e0.assign(c.level_chunk_begin.size(), 0);
     r.level_most.assign(c.level_chunk_begin.size(), 0);
+    r.level_alone.assign(c.level_chunk_begin.size(), 0);
     for (size_t l = 0; l < c.level_chunk_begin.size(); l++) {
         const int64_t rb = c.chunks[static_cast<size_t>(c.level_chunk_begin[l])].r0;
         const int64_t re = c.chunks[static_cast<size_t>(c.level_chunk_end[l])].r0;
-        if (re <= rb || off[re] - off[rb] > kShortMean * (re - rb) || off[re] - off[rb] > 0x7fffffff) continue;
+        const bool shortRows = off[re] - off[rb] <= kShortMean * (re - rb), small = off[re] - off[rb] <= kChainEdges;
+        if (re <= rb || !(shortRows || small) || off[re] - off[rb] > 0x7fffffff) continue;
         std::vector<unsigned> rel(static_cast<size_t>(re - rb) + 1);
         bool fits = true;
         for (int64_t i = rb; i <= re && fits; i++) {
             rel[static_cast<size_t>(i - rb)] = static_cast<unsigned>(off[i] - off[rb]);
             const int64_t len = i == rb ? 0 : off[i] - off[i - 1];
-            fits = len <= kShortMost;
+            fits = len <= (small ? kChainRow : kShortMost);
             r.level_most[l] = std::max(r.level_most[l], static_cast<int>(len));
         }
         if (!fits) continue;
         r.level_short[l] = upload(d, rel);
+        r.level_alone[l] = shortRows && r.level_most[l] <= kShortMost;
         r.level_r0[l] = rb;
         r.level_e0[l] = off[rb];
     }
@@ -270,6 +282,14 @@ SweepParams<S> make_params(const DevCSR& c, long long cb, long long ce, const vo
     return p;
 }
 
+namespace {
+int short_split(const DevCSR& c, size_t level, int g) {
+    int split = 1;
+    while (g * split < 32 && c.level_most[level] > 4 * kShortBatch * split) split *= 2;
+    return split;
+}
+}  // namespace
+
 // Launches one level of a CSR; returns the number of kernels launched (0, 1, or 2 when a nearly
 // empty last column tile runs on its own).  `work` points at `tileStride` zeroed counters owned
 // by this level.
@@ -286,13 +306,12 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
     const long long base = c.id16 ? c.level_base[level] : 0;
     // One launch of `tiles` column tiles of g lanes from column colBase; its work counters and
     // heavy-row tickets are those of tile slot `slot` onwards.
-    const bool isShort = level < c.level_short.size() && c.level_short[level] != nullptr;
+    const bool isShort = level < c.level_short.size() && c.level_short[level] != nullptr && c.level_alone[level];
     auto launch = [&](int g, int tiles, int variant, int colBase, int slot) {
         // one group of lanes per row, more (as many as a warp has) where some row has more than four
         // batches of edges: at K=1 a row of 50 edges takes one lane 9 us (ten levels of 3 to 50
         // children, UP K=1 on N=200,000, M=250,000: 40 us of 910)
-        int split = 1;
-        while (isShort && g * split < 32 && c.level_most[level] > 16 * split) split *= 2;
+        const int split = isShort ? short_split(c, level, g) : 1;
         const long long blocks = isShort ? (c.level_rows[level] * g * split + 255) / 256 : (ce - cb + 7) / 8;
         const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(tiles));
         auto prm = [&](auto tag) {
@@ -344,6 +363,70 @@ int launch_level(const Layout& L, const DevCSR& c, size_t level, const void* src
     }
     launch(sh.g, sh.ntiles, sh.variant, 0, 0);
     return 1;
+}
+
+int launch_levels(const Layout& L, const LevelRun& run, void* vals, void* partials, int tileStride, cudaStream_t s,
+                  const int* gate) {
+    int launches = 0;
+    ChainParams chain{};
+    chain.tiles = L.ntiles;
+    chain.vals = vals;
+    chain.stride = L.stride;
+    chain.state = run.state;
+    chain.state_base = run.stateBase;
+    chain.gate = gate;
+    std::vector<std::pair<const DevCSR*, size_t>> held;  // the chain's levels
+    const bool chains = chain_supported();
+    const LevelShape plain = default_shape(L);
+    auto single = [&](const DevCSR* c, size_t lvl) {
+        const bool seed = c == run.seed;
+        const LevelShape sh = level_shape(L, *c, lvl);
+        launches += launch_level(L, *c, lvl, seed ? run.seedSrc : vals, vals, seed ? run.seedRmw : run.rmw, partials,
+                                 seed ? run.seedTickets : run.tickets, seed ? run.seedWork : run.work + lvl * tileStride, s, gate,
+                                 &sh, tileStride, seed ? nullptr : run.state, run.stateBase, 2);
+    };
+    auto flush = [&] {
+        if (held.size() == 1) {
+            single(held[0].first, held[0].second);
+        } else if (!held.empty()) {
+            chain.count = static_cast<int>(held.size());
+            switch (L.kind) {
+            case Kind::U32: launch_chain_u32(chain, L.vw, L.g, s); break;
+            case Kind::XOR: launch_chain_xor(chain, L.vw, L.g, s); break;
+            case Kind::U64: launch_chain_u64(chain, L.vw, L.g, s); break;
+            case Kind::F64: launch_chain_f64(chain, L.vw, L.g, s); break;
+            case Kind::F32C: launch_chain_f32c(chain, L.vw, L.g, s); break;
+            case Kind::F32: launch_chain_f32(chain, L.vw, L.g, s); break;
+            case Kind::F64S: launch_chain_f64s(chain, L.vw, L.g, s); break;
+            }
+            launches++;
+        }
+        held.clear();
+    };
+    auto take = [&](const DevCSR* c, size_t lvl) {
+        if (c->le[lvl] <= c->lb[lvl]) return;
+        const bool seed = c == run.seed;
+        const unsigned* off = lvl < c->level_short.size() ? c->level_short[lvl] : nullptr;
+        const int split = off ? short_split(*c, lvl, L.g) : 1;
+        // rounds of the cluster's threads
+        const long long rounds =
+            off ? (c->level_rows[lvl] * L.g * split * L.ntiles + kChainBlocks * kChainThreads - 1) / (kChainBlocks * kChainThreads) : 0;
+        const LevelShape sh = level_shape(L, *c, lvl);  // (a tuned shape stays a launch of its own)
+        const bool few = off && c->level_edges[lvl] * L.g * L.ntiles <= kChainGathers && rounds <= kChainRounds;
+        if (!chains || !few || sh.g != plain.g || sh.variant != plain.variant) {
+            flush();
+            single(c, lvl);
+            return;
+        }
+        if (held.size() == kChainMost) flush();
+        chain.level[held.size()] = {off, c->adj + c->level_e0[lvl], c->rows + c->level_r0[lvl], seed ? run.seedSrc : vals,
+                                    static_cast<unsigned>(c->level_rows[lvl]), split, seed ? run.seedRmw : run.rmw};
+        held.push_back({c, lvl});
+    };
+    if (run.seed) take(run.seed, 0);
+    for (size_t lvl = run.first; lvl < run.last; lvl++) take(run.csr, lvl);
+    flush();
+    return launches;
 }
 
 namespace {
@@ -770,8 +853,9 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
             unsigned* tk = tickets;
             if (vt) {
                 load_rows(dIn, in_cols, M, MAP_IDENT, 1, nullptr, vt, 0);
-                launches += level(dp->seed, 0, vt, hasInit, tk, work);
+                if (mt) launches += level(dp->seed, 0, vt, hasInit, tk, work);
             }
+            unsigned* seedTickets = tk;
             tk += dp->seed.n_heavy * TS;
             if (mt) {
                 load_rows(dMiss, M, M, MAP_IDENT, 1, nullptr, mt, 0);
@@ -780,10 +864,20 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
             tk += dp->miss.n_heavy * TS;
             if (t_timing) GRGX_CUDA(cudaEventRecord(ev[1], s));
             const size_t nlv = cDown.lb.size();
-            for (size_t lvl = 0; lvl < nlv; lvl++) {
-                if ((dsplit || dpair) && lvl + 1 == nlv) break;  // the height-0 level runs below
-                launches += level(cDown, lvl, vals, 1, tk, work + (2 + lvl) * TS);
+            LevelRun levels;
+            levels.csr = &cDown;
+            levels.last = (dsplit || dpair) && nlv ? nlv - 1 : nlv;  // the height-0 level runs below
+            levels.rmw = 1;
+            levels.tickets = tk;
+            levels.work = work + 2 * TS;
+            if (vt && !mt) {
+                levels.seed = &dp->seed;
+                levels.seedSrc = vt;
+                levels.seedRmw = hasInit;
+                levels.seedTickets = seedTickets;
+                levels.seedWork = work;
             }
+            launches += launch_levels(L, levels, vals, partials, TS, s, gate);
             if (dpair)
                 launches += launch_pair_down(L, dp, prun, vals, ptable, pparts, work + (2 + nlv) * TS, s, gate);
             if (dsplit && staged) {
@@ -826,20 +920,28 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
                     launches += launch_level(L, cUp0b, j, vals, vals, 0, partials, tickets, work + j * TS, s, gate,
                                              &sh, TS, state, h0, 1);
                 }
-                for (size_t lvl = 0; lvl < cUpInt.lb.size(); lvl++) {
-                    const LevelShape sh = level_shape(L, cUpInt, lvl);
-                    launches += launch_level(L, cUpInt, lvl, vals, vals, state ? hasInit : 1, partials, tIn,
-                                             wIn + lvl * TS, s, gate, &sh, TS, state, h0, 2);
-                    const long long f0 = dp->fin_begin[lvl], f1 = dp->fin_begin[lvl + 1];
-                    if (state && f1 > f0) {
-                        launch_state_finish(L.kind, state, vals, dp->fin + f0, f1 - f0, h0, L.stride, hasInit,
-                                            s, gate);
-                        launches++;
-                    }
+                // (a node without children above height 0 is final before any level)
+                if (state && dp->fin_begin.back() > 0) {
+                    launch_state_finish(L.kind, state, vals, dp->fin, dp->fin_begin.back(), h0, L.stride, hasInit, s, gate);
+                    launches++;
                 }
+                LevelRun levels;
+                levels.csr = &cUpInt;
+                levels.last = cUpInt.lb.size();
+                levels.rmw = state ? hasInit : 1;
+                levels.tickets = tIn;
+                levels.work = wIn;
+                levels.state = state;
+                levels.stateBase = h0;
+                launches += launch_levels(L, levels, vals, partials, TS, s, gate);
             } else {
-                for (size_t lvl = 0; lvl < cUp.lb.size(); lvl++)
-                    launches += level(cUp, lvl, vals, hasInit, tickets, work + lvl * TS);
+                LevelRun levels;
+                levels.csr = &cUp;
+                levels.last = cUp.lb.size();
+                levels.rmw = hasInit;
+                levels.tickets = tickets;
+                levels.work = work;
+                launches += launch_levels(L, levels, vals, partials, TS, s, gate);
             }
             if (t_timing) GRGX_CUDA(cudaEventRecord(ev[2], s));
             if (emit_all) {

@@ -118,6 +118,25 @@ template <typename S, int VW> __device__ __forceinline__ void ld_plain(const S* 
     }
 }
 
+// The same from L2, past an L1 line that may be older than another SM's store.
+template <typename S, int VW> __device__ __forceinline__ void ld_l2(const S* p, S* v) {
+    if constexpr (VW * sizeof(S) == 16) {
+        const uint4 t = __ldcg(reinterpret_cast<const uint4*>(p));
+        if constexpr (std::is_same<S, DF>::value) {
+            v[0] = {__uint_as_float(t.x), __uint_as_float(t.z)};
+            v[1] = {__uint_as_float(t.y), __uint_as_float(t.w)};
+        } else {
+            memcpy(v, &t, 16);
+        }
+    } else if constexpr (VW * sizeof(S) == 8) {
+        const uint2 t = __ldcg(reinterpret_cast<const uint2*>(p));
+        memcpy(v, &t, 8);
+    } else {
+        const unsigned t = __ldcg(reinterpret_cast<const unsigned*>(p));
+        memcpy(v, &t, 4);
+    }
+}
+
 // Sum of a lane's accumulator over the 32/G groups of the warp (every group gets the result).
 template <class Op, int VW, int G, class Acc> __device__ __forceinline__ void group_allreduce(Acc& x) {
 #pragma unroll
@@ -143,7 +162,8 @@ __device__ __forceinline__ F32Pair ld_cg(const F32Pair* p) {
     return {t.x, t.y};
 }
 
-template <class Op, int VW, class Acc>
+// CG: the row's value may have been written by another SM earlier in the same launch.
+template <class Op, int VW, bool CG = false, class Acc>
 __device__ __forceinline__ void write_row(const SweepParams<typename Op::S>& p, long long row, int col,
                                           const Acc& tot) {
     using S = typename Op::S;
@@ -172,7 +192,8 @@ __device__ __forceinline__ void write_row(const SweepParams<typename Op::S>& p, 
     S out[VW];
     if (p.rmw) {
         S base[VW];
-        ld_plain<S, VW>(d, base);
+        if constexpr (CG) ld_l2<S, VW>(d, base);
+        else ld_plain<S, VW>(d, base);
 #pragma unroll
         for (int i = 0; i < VW; i++) out[i] = Op::finish_onto(base[i], sum[i]);
     } else {
@@ -418,38 +439,36 @@ __global__ void __launch_bounds__(256, SweepOccupancy<Op, VW, G, D>::kBlocks) sw
 // a DOWN level of a few thousand one-edge rows.  Bound by the latency of three dependent loads.
 // A level with longer rows among them has `short_split` groups of lanes to a row, which take its
 // edges in turns of four and merge their sums at the end.
-template <class Op, int VW, int G>
-__device__ __forceinline__ void short_rows(const SweepParams<typename Op::S>& p) {
+constexpr int kShortBatch = 4;
+
+// Row `row` of such a level, from its edges e, e + split batches on, ..: `id` holds the first batch's
+// ids (past `end`: any).  The warp's lanes call it together; `live` lanes have a row and a column.
+template <class Op, int VW, int G, bool CG>
+__device__ __forceinline__ void short_row(const SweepParams<typename Op::S>& p, const uint32_t* __restrict__ adj, long long row,
+                                          int col, int split, int sub, bool live, unsigned e, unsigned end,
+                                          uint32_t (&id)[kShortBatch]) {
     using S = typename Op::S;
     constexpr bool kPairs = std::is_same<Op, AddF64S>::value;
-    constexpr int BATCH = 4;
-    const int split = p.short_split;
-    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long row = thread / (G * split);
-    const int sub = static_cast<int>(thread / G) & (split - 1);
-    const int col = blockIdx.y * (G * VW) + (threadIdx.x % G) * VW;
-    const bool live = row < p.short_rows && col < p.stride;
-    unsigned e = 0, end = 0;
-    if (live) {
-        e = __ldg(p.short_off + row) + BATCH * sub;
-        end = __ldg(p.short_off + row + 1);
-    }
     ScalarAcc<Op, VW> acc;
     acc.zero();
-    for (; e < end; e += BATCH * split) {
-        uint32_t id[BATCH];
-        S v[BATCH][VW];
+    while (e < end) {
+        S v[kShortBatch][VW];
 #pragma unroll
-        for (int u = 0; u < BATCH; u++) id[u] = (e + u < end) ? __ldg(p.adj + e + u) & 0x7fffffffu : 0u;
-#pragma unroll
-        for (int u = 0; u < BATCH; u++) {
+        for (int u = 0; u < kShortBatch; u++) {
             if (e + u < end) {
-                Vec<S, VW>::ld(p.src + (long long)id[u] * p.stride + col, v[u]);
+                const S* from = p.src + (long long)(id[u] & 0x7fffffffu) * p.stride + col;
+                if constexpr (CG) ld_l2<S, VW>(from, v[u]);
+                else Vec<S, VW>::ld(from, v[u]);
             } else {
 #pragma unroll
                 for (int i = 0; i < VW; i++) v[u][i] = S{};
             }
         }
+        const unsigned at = e;
+        e += kShortBatch * split;
+#pragma unroll
+        for (int u = 0; u < kShortBatch; u++)
+            if (e + u < end) id[u] = __ldg(adj + e + u);
         if constexpr (kPairs) {
             // normalised float pairs throughout: no run to fold, and no FP64 pipe
 #pragma unroll
@@ -461,8 +480,8 @@ __device__ __forceinline__ void short_rows(const SweepParams<typename Op::S>& p)
             }
         } else {
 #pragma unroll
-            for (int u = 0; u < BATCH; u++)
-                if (e + u < end) acc.add(v[u]);
+            for (int u = 0; u < kShortBatch; u++)
+                if (at + u < end) acc.add(v[u]);
         }
     }
     for (int m = G; m < G * split; m <<= 1) {
@@ -481,9 +500,12 @@ __device__ __forceinline__ void short_rows(const SweepParams<typename Op::S>& p)
     if (!live || sub != 0) return;
     if constexpr (kPairs) {
         if (p.state == nullptr) {
-            DF* d = p.dst + (long long)p.rows[p.short_row0 + row] * p.stride + col;
+            DF* d = p.dst + (long long)p.rows[row] * p.stride + col;
             DF out[VW];
-            if (p.rmw) ld_plain<DF, VW>(d, out);
+            if (p.rmw) {
+                if constexpr (CG) ld_l2<DF, VW>(d, out);
+                else ld_plain<DF, VW>(d, out);
+            }
 #pragma unroll
             for (int i = 0; i < VW; i++) {
                 const DF r{acc.a[i].hi, acc.a[i].lo};
@@ -493,7 +515,26 @@ __device__ __forceinline__ void short_rows(const SweepParams<typename Op::S>& p)
             return;
         }
     }
-    write_row<Op, VW>(p, p.short_row0 + row, col, acc);
+    write_row<Op, VW, CG>(p, row, col, acc);
+}
+
+template <class Op, int VW, int G>
+__device__ __forceinline__ void short_rows(const SweepParams<typename Op::S>& p) {
+    const int split = p.short_split;
+    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long row = thread / (G * split);
+    const int sub = static_cast<int>(thread / G) & (split - 1);
+    const int col = blockIdx.y * (G * VW) + (threadIdx.x % G) * VW;
+    const bool live = row < p.short_rows && col < p.stride;
+    unsigned e = 0, end = 0;
+    if (live) {
+        e = __ldg(p.short_off + row) + kShortBatch * sub;
+        end = __ldg(p.short_off + row + 1);
+    }
+    uint32_t id[kShortBatch];
+#pragma unroll
+    for (int u = 0; u < kShortBatch; u++) id[u] = (e + u < end) ? __ldg(p.adj + e + u) : 0u;
+    short_row<Op, VW, G, false>(p, p.adj, p.short_row0 + row, col, split, sub, live, e, end, id);
 }
 
 template <class Op, int VW, int G>
