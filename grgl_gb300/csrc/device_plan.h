@@ -252,12 +252,13 @@ struct PairDownRun {
         int items, groups_per_item;
     };
     std::vector<Range> ranges;
+    int tiles = 1;  // column tiles: counters per range
     int slots = 0;  // sums per row held at a time (0: the only item writes its rows)
     size_t table_bytes = 0, part_bytes = 0;
 };
 // `limit`: most bytes of scratch the table and the sums may take; no ranges where that is too little.
 PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit);
-// Adds the height-0 rows' sums onto vals; `work` holds L.ntiles zeroed counters per range.
+// Adds the height-0 rows' sums onto vals; `work` holds run.tiles zeroed counters per range.
 // Returns the kernels launched.
 int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
                      unsigned* work, cudaStream_t s, const int* gate);

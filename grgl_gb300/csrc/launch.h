@@ -60,7 +60,7 @@ void launch_chain_f32c(const ChainParams& p, int vw, int g, cudaStream_t s);
 void launch_chain_f32(const ChainParams& p, int vw, int g, cudaStream_t s);
 void launch_chain_f64s(const ChainParams& p, int vw, int g, cudaStream_t s);
 
-// The pair form's ids are padded to whole groups of this many height-0 rows: no warp takes more.
+// The pair form's ids are padded by at least this many height-0 rows: no warp takes more at a time.
 constexpr int kPairTile = 128;
 
 // DOWN in pair form (pair_down.cuh): one launch over `items` shares of the blocks (groups of four,

@@ -761,7 +761,7 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
         void* ptable = (dpair || upair) ? sc.get(dpair ? prun.table_bytes : urun.table_bytes) : nullptr;
         void* pparts = prun.slots ? sc.get(prun.part_bytes) : nullptr;
         // counters per launch and per heavy row: enough column tiles for any launch shape
-        const int TS = max_tiles(L);
+        const int TS = std::max(max_tiles(L), prun.tiles);
         const size_t counterBytes = static_cast<size_t>(nh + nslots) * TS * sizeof(unsigned);
         unsigned* tickets = static_cast<unsigned*>(sc.get(counterBytes));
         GRGX_CUDA(cudaMemsetAsync(tickets, 0, counterBytes, s));

@@ -127,11 +127,12 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(con
     static_assert(NG * ROWS <= kPairTile, "a warp's rows end within the padded ids");
     constexpr bool kChains = ChainTraits<Op>::kChains;
     const int lane = threadIdx.x & 31;
-    const int lg = lane / G;
+    // (lanes without a column or past the last whole row follow along on the warp's first row)
     const int col = blockIdx.y * (G * VW) + (lane % G) * VW;
-    const bool colok = col < p.stride;
+    const bool active = (NG * G == 32 || lane < NG * G) && col < p.stride;
+    const int lg = (NG * G == 32 || lane < NG * G) ? lane / G : 0;
     const unsigned rowBytes = static_cast<unsigned>(p.stride * sizeof(T));
-    const char* table = reinterpret_cast<const char*>(static_cast<const T*>(p.table) + (colok ? col : 0));
+    const char* table = reinterpret_cast<const char*>(static_cast<const T*>(p.table) + (active ? col : 0));
     unsigned* counter = p.work + blockIdx.y;
     for (;;) {
         unsigned c = 0;
@@ -179,7 +180,7 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(con
                 for (int r = 0; r < ROWS; r++) acc[r].flush();
             }
         }
-        if (!colok) continue;
+        if (!active) continue;
 #pragma unroll
         for (int r = 0; r < ROWS; r++) {
             const long long row = row0 + r * NG;
@@ -287,6 +288,11 @@ template <class Op, int VW, int G> void pair_down_as(PairDownParams<typename Op:
         pair_down_as<OP, VWV, GV>(p, c, sms, s);  \
         return;                                   \
     }
+// (lane counts that are no power of two fit more rows into a warp: see pair_lanes)
+#define GRGX_PAIR_ODD(OP, VWV)                                                                      \
+    GRGX_PAIR_CASE(OP, VWV, 5)                                                                      \
+    GRGX_PAIR_CASE(OP, VWV, 6)                                                                      \
+    GRGX_PAIR_CASE(OP, VWV, 10)
 #define GRGX_PAIR4(OP)                                                                              \
     GRGX_PAIR_CASE(OP, 1, 1)                                                                        \
     GRGX_PAIR_CASE(OP, 2, 1)                                                                        \
@@ -295,7 +301,8 @@ template <class Op, int VW, int G> void pair_down_as(PairDownParams<typename Op:
     GRGX_PAIR_CASE(OP, 4, 4)                                                                        \
     GRGX_PAIR_CASE(OP, 4, 8)                                                                        \
     GRGX_PAIR_CASE(OP, 4, 16)                                                                       \
-    GRGX_PAIR_CASE(OP, 4, 32)
+    GRGX_PAIR_CASE(OP, 4, 32)                                                                       \
+    GRGX_PAIR_ODD(OP, 4)
 #define GRGX_PAIR8(OP)                                                                              \
     GRGX_PAIR_CASE(OP, 1, 1)                                                                        \
     GRGX_PAIR_CASE(OP, 2, 1)                                                                        \
@@ -303,6 +310,7 @@ template <class Op, int VW, int G> void pair_down_as(PairDownParams<typename Op:
     GRGX_PAIR_CASE(OP, 2, 4)                                                                        \
     GRGX_PAIR_CASE(OP, 2, 8)                                                                        \
     GRGX_PAIR_CASE(OP, 2, 16)                                                                       \
-    GRGX_PAIR_CASE(OP, 2, 32)
+    GRGX_PAIR_CASE(OP, 2, 32)                                                                       \
+    GRGX_PAIR_ODD(OP, 2)
 
 }  // namespace grgx

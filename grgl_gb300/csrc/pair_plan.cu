@@ -491,7 +491,7 @@ void build_pair_plan(DevicePlan& d, bool down) {
     const int* dNode = tmp.copy(seqNode);
     const PairBlock* dBlocks = tmp.copy(blocks);
     const long long groups = (nblk + 3) / 4;
-    const long long tiles = (h0 + kPairTile - 1) / kPairTile * (kPairTile / 32);
+    const long long tiles = (h0 / kPairTile + 2) * (kPairTile / 32);  // padded: see kPairTile
     const long long batch = std::max<long long>(1, std::min(nblk, (1LL << 27) / h0));
     const size_t idBytes = static_cast<size_t>(tiles) * groups * 32 * 4 * sizeof(unsigned short);
     PairOut out{};

@@ -27,6 +27,29 @@ constexpr uint64_t kPairScratch = 6ULL << 30;
 
 thread_local uint64_t t_limit = kPairScratch;
 
+// Lanes per row.  A gather instruction costs the L1 about the same whichever of its lanes do nothing, so
+// what counts is the instructions per row: its column tiles over the rows a warp's 32 lanes hold.  Ten
+// lanes hold three rows where sixteen hold two, six hold five, five hold six; they are taken where they
+// need at most 0.7 of the instructions of the layout's power of two, 0.8 where the additions of the
+// idle lanes weigh too (compensated kinds; float32 DOWN only in a single tile).  Milliseconds on
+// N=200,000, M=250,000, power of two against these:
+//   float64 K=20 (10 vectors) UP 5.09 / 3.20  DOWN 4.00 / 3.01    K=36 (18) UP 10.1 / 6.2  DOWN 7.6 / 5.7
+//   float64 K=24 (12)         UP 5.12 / 4.25  DOWN 4.07 / 3.89    float32 K=40 (10) UP 4.30 / 3.05  DOWN 3.55 / 2.85
+//   int32 K=72 (18)           UP 7.20 / 6.01  DOWN 5.81 / 5.31    K=80 (20) UP 7.32 / 6.08  DOWN 5.78 / 5.41
+// and past the line int32 K=20 (5) UP 1.86 / 2.10, K=48 (12) UP 3.74 / 4.12, float32 K=48 DOWN 3.58 / 3.85.
+int pair_lanes(const Layout& L, bool up) {
+    const long long vecs = L.stride / L.vw;
+    auto cost = [&](int g) { return static_cast<double>((vecs + g - 1) / g) / (32 / g); };
+    int best = L.g;
+    for (int g : {10, 6, 5}) {
+        if (L.vw * L.ssize != 16 || (g == 5 && up)) continue;
+        const bool one = vecs <= g;
+        const bool both = L.kind == Kind::F64S || (L.kind == Kind::F32C && (up || one));
+        if (cost(g) <= (both ? 0.801 : 0.701) * cost(L.g) && cost(g) < cost(best)) best = g;
+    }
+    return best;
+}
+
 template <typename F> void by_kind(const Layout& L, F&& f) {
     switch (L.kind) {
     case Kind::U32: f(PairDownParams<uint32_t>{}, pair_down_u32); break;
@@ -48,8 +71,10 @@ size_t pair_scratch_limit() { return static_cast<size_t>(t_limit); }
 PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit) {
     const PairPlan& P = dp->pair;
     PairDownRun run;
+    const int lanes = pair_lanes(L, false);
+    run.tiles = static_cast<int>((L.stride / L.vw + lanes - 1) / lanes);
     PairDownCall shape;
-    by_kind(L, [&](auto p, auto fn) { fn(p, shape, L.vw, L.g, sm_count(), nullptr); });
+    by_kind(L, [&](auto p, auto fn) { fn(p, shape, L.vw, pair_lanes(L, false), sm_count(), nullptr); });
     const size_t rowBytes = static_cast<size_t>(L.stride) * shape.table_bytes;
     const size_t slotBytes = static_cast<size_t>(P.h0) * L.stride * shape.part_bytes;
     const size_t tableMost = std::min(kPairTableBytes, limit / 3);
@@ -67,8 +92,8 @@ PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit) {
         r.pat0 = patterns(g0);
         r.count = patterns(g1) - r.pat0;
         const long long carried = g0 > 0 ? 1 : 0;
-        // (the columns of a tile are gathered together, so a share spans rowBytes / ntiles per row)
-        const long long share = static_cast<long long>(r.count * rowBytes / L.ntiles) / kPairItemBytes + 1;
+        // (the columns of a tile are gathered together, so a share spans rowBytes / tiles per row)
+        const long long share = static_cast<long long>(r.count * rowBytes / run.tiles) / kPairItemBytes + 1;
         const long long even = (kPairItemsPerWarp * shape.resident_warps + tiles - 1) / tiles;
         const long long most = std::min<long long>((g1 - g0) / kPairMinGroups, slotsMost - carried);
         const long long items = std::max(1LL, std::min(std::max(share, even), most));
@@ -91,7 +116,7 @@ int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& r
     int launches = 0;
     by_kind(L, [&](auto p, auto fn) {
         PairDownCall c;
-        fn(p, c, L.vw, L.g, sm_count(), s);
+        fn(p, c, L.vw, pair_lanes(L, false), sm_count(), s);
         p.ids = reinterpret_cast<const uint2*>(P.ids);
         p.base = reinterpret_cast<const uint4*>(P.base);
         p.table = table;
@@ -107,7 +132,7 @@ int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& r
             c.step = PairDownCall::kTable;
             c.nodes = P.pat_nodes + r.pat0;
             c.count = r.count;
-            fn(p, c, L.vw, L.g, sm_count(), s);
+            fn(p, c, L.vw, pair_lanes(L, false), sm_count(), s);
             c.step = PairDownCall::kGather;
             p.base0 = static_cast<unsigned>(r.pat0);
             p.group_begin = r.g0;
@@ -115,15 +140,15 @@ int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& r
             p.items = static_cast<unsigned>(r.items);
             p.groups_per_item = r.groups_per_item;
             p.part_begin = i > 0 ? 1 : 0;
-            p.work = work + i * L.ntiles;
-            fn(p, c, L.vw, L.g, sm_count(), s);
+            p.work = work + i * run.tiles;
+            fn(p, c, L.vw, pair_lanes(L, false), sm_count(), s);
             launches += 2;
             if (run.slots == 0) continue;
             c.step = PairDownCall::kFinish;
             c.parts = r.items + p.part_begin;
             c.onto = i + 1 == run.ranges.size();
             if (c.onto || c.parts > 1) {
-                fn(p, c, L.vw, L.g, sm_count(), s);
+                fn(p, c, L.vw, pair_lanes(L, false), sm_count(), s);
                 launches++;
             }
         }
@@ -152,8 +177,12 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
     int launches = 0;
     // Lanes per row for the gathers from the height-0 rows: as many as leave the columns of one tile
     // in L2 (float64 K=64 on 200,000 rows: 102 MB at once, 60% L2 hits and 13.4 ms; in two tiles 11.3)
-    int g = L.g;
-    while (g > 1 && P.h0 * g * 16 > kPairSourceBytes) g /= 2;
+    const int all = pair_lanes(L, true);
+    int g = all;
+    if (P.h0 * g * 16 > kPairSourceBytes) {
+        g = L.g;
+        while (g > 1 && P.h0 * g * 16 > kPairSourceBytes) g /= 2;
+    }
     const size_t rowBytes = static_cast<size_t>(L.stride) * L.ssize;
     for (const PairUpRun::Range& r : run.ranges) {
         const PairPlan::Segment &a = P.segments[r.s0], &b = P.segments[r.s1];
@@ -174,7 +203,7 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
                 p.second = second ? 1 : 0;
                 p.stride = L.stride;
                 p.gate = gate;
-                        fn(p, L.vw, second ? L.g : g, s);
+                        fn(p, L.vw, second ? all : g, s);
             };
             switch (L.kind) {
             case Kind::U32: go(PairUpParams<uint32_t>{}, pair_up_u32); break;

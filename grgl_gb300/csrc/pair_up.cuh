@@ -11,6 +11,9 @@
 
 namespace grgx {
 
+// Lanes per list: those for the columns, or at least eight.
+constexpr int pair_list_lanes(int g) { return (g & (g - 1)) == 0 && g < 8 ? 8 : g; }
+
 // One warp takes 32 / L lists of about equal length, L = G lanes for the columns, at least eight:
 // with narrower rows the lanes left over share out the list (sub), and their sums are merged at the
 // end.  The lanes of a list load its ids together and pass them round.
@@ -26,21 +29,28 @@ namespace grgx {
 template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const PairUpParams<typename Op::S>& p) {
     using S = typename Op::S;
     using Acc = VecAcc<Op, VW>;
-    constexpr int L = G < 8 ? 8 : G;           // lanes per list
-    constexpr int STEPS = G < 8 ? 8 / G : 1;   // ids a lane loads at a time
-    constexpr int SLOTS = G * STEPS;           // rows a lane gathers from them
-    constexpr int FLUSH_EVERY = SLOTS >= 32 ? 1 : 32 / SLOTS;
+    constexpr int L = pair_list_lanes(G);
+    constexpr bool kOdd = (G & (G - 1)) != 0;
+    constexpr int STEPS = kOdd ? 4 : (G < 8 ? 8 / G : 1);  // ids a lane loads at a time
+    constexpr int SLOTS = G * STEPS;                       // rows a lane gathers from them
+    static_assert(SLOTS % 8 == 0, "batches of eight");
+    constexpr int FLUSH_EVERY = SLOTS > 16 ? 1 : 32 / SLOTS;
     constexpr bool kChains = ChainTraits<Op>::kChains;
     const int lane = threadIdx.x & 31;
     const int gl = lane % L, sub = gl / G;
     const int col = blockIdx.y * (G * VW) + (lane % G) * VW;
     const bool colok = col < p.stride;
+    const bool inside = !kOdd || lane < 32 / L * L;  // (lanes past the last whole list have none)
     const long long r = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 / L) + lane / L;
     PairList list{0, 0, 0};
-    if (r < p.count) list = p.lists[r];
+    if (r < p.count && inside) list = p.lists[r];
     int most = list.len;
+    if constexpr (kOdd) {
+        most = __reduce_max_sync(FULL_MASK, most);
+    } else {
 #pragma unroll
-    for (int m = L; m < 32; m <<= 1) most = max(most, __shfl_xor_sync(FULL_MASK, most, m));
+        for (int m = L; m < 32; m <<= 1) most = max(most, __shfl_xor_sync(FULL_MASK, most, m));
+    }
     const uint32_t* ids = p.adj + list.e0;
     const char* src = reinterpret_cast<const char*>(p.src + (colok ? col : 0));
     const unsigned rowBytes = static_cast<unsigned>(p.stride * sizeof(S));
@@ -65,7 +75,7 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const
 #pragma unroll
             for (int t = 0; t < 8; t++) {
                 const int s = (t0 + t) / G, u = (t0 + t) % G;
-                const uint32_t id = __shfl_sync(FULL_MASK, raw[s], lane / L * L + sub * G + u);
+                const uint32_t id = __shfl_sync(FULL_MASK, raw[s], (lane / L * L + sub * G + u) & 31);
                 if (static_cast<int>(id) >= 0) {
                     Vec<S, VW>::ld(reinterpret_cast<const S*>(src + (unsigned long long)id * rowBytes), v[t]);
                 } else {
@@ -74,6 +84,7 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const
                 }
             }
             acc.template add_block<8>(v);
+            if (kChains && SLOTS > 32 && t0 % 32 == 24) acc.flush();  // a run is 32 additions at most
         }
         if (kChains && ++rounds == FLUSH_EVERY) {
             rounds = 0;
@@ -81,11 +92,11 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const
         }
     }
 #pragma unroll
-    for (int m = G; m < L; m <<= 1) {
+    for (int m = G; m < L; m <<= 1) {  // (none where L = G)
         const auto t = acc.shfl_xor(m);
         acc.merge(t);
     }
-    if (r >= p.count || sub != 0 || !colok) return;
+    if (r >= p.count || !inside || sub != 0 || !colok) return;
     if (list.out >= 0 && p.state != nullptr) {
         typename Op::A* d = static_cast<typename Op::A*>(p.state) + (long long)list.out * p.stride + col;
 #pragma unroll
@@ -105,7 +116,7 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const
 }
 
 template <class Op, int VW, int G>
-__global__ void __launch_bounds__(256, 4) pair_up_kernel(const PairUpParams<typename Op::S> p) {
+__global__ void __launch_bounds__(256, (G & (G - 1)) ? 3 : 4) pair_up_kernel(const PairUpParams<typename Op::S> p) {
     if constexpr (std::is_base_of<AddF64S, Op>::value) {
         if (p.gate != nullptr && *p.gate != 0) {
             pair_up<AddF64, VW, G>(as_f64(p));
@@ -116,7 +127,7 @@ __global__ void __launch_bounds__(256, 4) pair_up_kernel(const PairUpParams<type
 }
 
 template <class Op, int VW, int G> void pair_up_as(const PairUpParams<typename Op::S>& p, cudaStream_t s) {
-    constexpr int perBlock = 8 * (32 / (G < 8 ? 8 : G));
+    constexpr int perBlock = 8 * (32 / pair_list_lanes(G));
     const dim3 grid(static_cast<unsigned>((p.count + perBlock - 1) / perBlock),
                     static_cast<unsigned>((p.stride / VW + G - 1) / G));
     pair_up_kernel<Op, VW, G><<<grid, 256, 0, s>>>(p);
@@ -135,7 +146,9 @@ template <class Op, int VW, int G> void pair_up_as(const PairUpParams<typename O
     GRGX_PAIR_UP_CASE(OP, 4, 4)  \
     GRGX_PAIR_UP_CASE(OP, 4, 8)  \
     GRGX_PAIR_UP_CASE(OP, 4, 16) \
-    GRGX_PAIR_UP_CASE(OP, 4, 32)
+    GRGX_PAIR_UP_CASE(OP, 4, 32) \
+    GRGX_PAIR_UP_CASE(OP, 4, 6)  \
+    GRGX_PAIR_UP_CASE(OP, 4, 10)
 #define GRGX_PAIR_UP8(OP)        \
     GRGX_PAIR_UP_CASE(OP, 1, 1)  \
     GRGX_PAIR_UP_CASE(OP, 2, 1)  \
@@ -143,6 +156,8 @@ template <class Op, int VW, int G> void pair_up_as(const PairUpParams<typename O
     GRGX_PAIR_UP_CASE(OP, 2, 4)  \
     GRGX_PAIR_UP_CASE(OP, 2, 8)  \
     GRGX_PAIR_UP_CASE(OP, 2, 16) \
-    GRGX_PAIR_UP_CASE(OP, 2, 32)
+    GRGX_PAIR_UP_CASE(OP, 2, 32) \
+    GRGX_PAIR_UP_CASE(OP, 2, 6)  \
+    GRGX_PAIR_UP_CASE(OP, 2, 10)
 
 }  // namespace grgx

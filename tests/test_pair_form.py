@@ -88,6 +88,23 @@ def test_pair_up_matches_oracle(env, dt, K):
     _check(og, V, UP, gx.matmul(g, V, UP))
 
 
+# rows of 3, 5, 6, 9 and 10 vectors, whose lanes are no power of two (10 tiles of 3 lanes in a warp)
+@pytest.mark.parametrize("dt,K", [(np.int32, 11), (np.int32, 18), (np.float32, 9), (np.float32, 20), (np.float32, 23),
+                                  (np.float32, 36), (np.float32, 40), (np.float64, 5), (np.float64, 10), (np.float64, 11),
+                                  (np.float64, 18), (np.float64, 20), (np.int64, 19), (np.bool_, 320)])
+def test_pair_form_odd_lanes(env, dt, K):
+    gx, g, og = env
+    for direction, cols in ((DOWN, g.num_mutations), (UP, g.num_samples)):
+        V = _rand(np.random.default_rng(K), dt, (K, cols))
+        _check(og, V, direction, gx.matmul(g, V, direction))
+    # as many rows as fill the ids' tiles exactly, and a few more
+    for N in (128, 131, 256):
+        small = gx.window_tree_grg(N, 900, seed=N)
+        pg, po = _both(gx, small, ploidy=1)
+        V = _rand(np.random.default_rng(N), dt, (K, pg.num_mutations))
+        _check(po, V, DOWN, gx.matmul(pg, V, DOWN))
+
+
 def test_pair_up_options(env):
     gx, g, og = env
     rng = np.random.default_rng(3)
