@@ -1,7 +1,7 @@
 // Seed and gather kernels: moving K x cols row-major matrices (the reference's I/O layout,
 // grg.h:1341-1517) into and out of the node-major value rows the sweep works on.
 //
-// Both directions use 32 x 32 shared-memory tiles so that the global reads and writes are
+// Except for few columns (narrow_io) both directions use 32 x 32 shared-memory tiles so that the global reads and writes are
 // coalesced on both sides of the transpose.  Element conversion between the I/O type and the
 // storage type follows the accumulation kinds of ops.cuh: narrow integers are widened to 32
 // bits (residues mod 2^bits are preserved) and truncated on output.
@@ -126,6 +126,61 @@ __global__ void store_cols_kernel(const typename Store<IO>::S* __restrict__ vals
     }
 }
 
+// Few columns (narrow_io): a thread per row, whose vectors of node values stay in L1 between a warp's
+// columns.  Bound by the launch and one pass over the rows.
+template <typename IO, int VW>
+__global__ void load_rows_narrow_kernel(const IO* __restrict__ src, long long K, long long ld, long long R, int mode,
+                                        long long div, const uint32_t* __restrict__ tab,
+                                        typename Store<IO>::S* __restrict__ dst, long long stride, int add) {
+    using S = typename Store<IO>::S;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= R) return;
+    const long long col = (mode == MAP_DIV) ? i / div : (mode == MAP_TABLE ? (long long)tab[i] : i);
+    S* d = dst + i * stride;
+    for (long long k0 = 0; k0 < stride; k0 += VW) {
+        S v[VW];
+#pragma unroll
+        for (int j = 0; j < VW; j++) v[j] = (k0 + j < K) ? to_s<IO>(src[(k0 + j) * ld + col]) : S(0);
+        if (add) {
+#pragma unroll
+            for (int j = 0; j < VW; j++)
+                if (k0 + j < K) d[k0 + j] = s_add<S>(d[k0 + j], v[j]);
+        } else {
+            Vec<S, VW>::st(d + k0, v);
+        }
+    }
+}
+
+template <typename IO, int VW>
+__global__ void store_cols_narrow_kernel(const typename Store<IO>::S* __restrict__ vals, long long stride, long long K,
+                                         long long C, int mode, long long fold, const uint32_t* __restrict__ tab,
+                                         IO* __restrict__ out, long long ld, int add) {
+    using S = typename Store<IO>::S;
+    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= C) return;
+    const long long node = (mode == MAP_TABLE) ? (long long)tab[c] : (mode == MAP_FOLD ? c * fold : c);
+    const bool has = mode != MAP_TABLE || node != (long long)kInvalid;
+    for (long long k0 = 0; k0 < K; k0 += VW) {
+        S v[VW];
+#pragma unroll
+        for (int j = 0; j < VW; j++) v[j] = S(0);
+        if (has) Vec<S, VW>::ld(vals + node * stride + k0, v);
+        for (long long p = 1; mode == MAP_FOLD && p < fold; p++) {
+            S t[VW];
+            Vec<S, VW>::ld(vals + (node + p) * stride + k0, t);
+#pragma unroll
+            for (int j = 0; j < VW; j++) v[j] = s_add<S>(v[j], t[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < VW; j++) {
+            if (k0 + j >= K) break;
+            IO* o = out + (k0 + j) * ld + c;
+            const IO x = from_s<IO>(v[j]);
+            *o = add ? io_add<IO>(*o, x) : x;
+        }
+    }
+}
+
 template <typename IO>
 __global__ void init_vector_kernel(const IO* __restrict__ init, long long K, long long n,
                                    typename Store<IO>::S* __restrict__ vals, long long stride) {
@@ -192,6 +247,13 @@ template <typename IO>
 void load_rows_t(const void* src, long long K, long long ld, long long R, int mode, long long div, const uint32_t* tab,
                  void* dst, long long stride, int add, cudaStream_t s) {
     if (R <= 0) return;
+    if (narrow_io(K, R, sizeof(typename Store<IO>::S))) {
+        narrow_vec<sizeof(typename Store<IO>::S)>(stride, [&](auto vw) {
+            load_rows_narrow_kernel<IO, decltype(vw)::value><<<(unsigned)((R + 255) / 256), 256, 0, s>>>(
+                static_cast<const IO*>(src), K, ld, R, mode, div, tab, static_cast<typename Store<IO>::S*>(dst), stride, add);
+        });
+        return;
+    }
     const dim3 grid((unsigned)((R + 31) / 32), (unsigned)((stride + 31) / 32));
     load_rows_kernel<IO><<<grid, dim3(32, 8), 0, s>>>(static_cast<const IO*>(src), K, ld, R, mode, div, tab,
                                                       static_cast<typename Store<IO>::S*>(dst), stride, add);
@@ -201,6 +263,13 @@ template <typename IO>
 void store_cols_t(const void* vals, long long stride, long long K, long long C, int mode, long long fold,
                   const uint32_t* tab, void* out, long long ld, int add, cudaStream_t s) {
     if (C <= 0 || K <= 0) return;
+    if (narrow_io(K, C, sizeof(typename Store<IO>::S))) {
+        narrow_vec<sizeof(typename Store<IO>::S)>(stride, [&](auto vw) {
+            store_cols_narrow_kernel<IO, decltype(vw)::value><<<(unsigned)((C + 255) / 256), 256, 0, s>>>(
+                static_cast<const typename Store<IO>::S*>(vals), stride, K, C, mode, fold, tab, static_cast<IO*>(out), ld, add);
+        });
+        return;
+    }
     const dim3 grid((unsigned)((C + 31) / 32), (unsigned)((K + 31) / 32));
     store_cols_kernel<IO><<<grid, dim3(32, 8), 0, s>>>(static_cast<const typename Store<IO>::S*>(vals), stride, K,
                                                        C, mode, fold, tab, static_cast<IO*>(out), ld, add);

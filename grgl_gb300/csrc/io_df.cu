@@ -176,6 +176,80 @@ __global__ void store_cols_df_kernel(const DF* __restrict__ vals, long long stri
     }
 }
 
+// Few columns: a thread per row (load_rows_narrow_kernel, io.cu).
+template <int VW>
+__global__ void load_rows_narrow_df_kernel(const double* __restrict__ src, long long K, long long ld, long long R, int mode,
+                                           long long div, const uint32_t* __restrict__ tab, DF* __restrict__ dst,
+                                           long long stride, int add, const unsigned long long* __restrict__ rowmax,
+                                           const int* gate) {
+    const bool native = gate != nullptr && *gate != 0;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= R) return;
+    const long long col = (mode == MAP_DIV) ? i / div : (mode == MAP_TABLE ? (long long)tab[i] : i);
+    for (long long k0 = 0; k0 < stride; k0 += VW) {
+        const long long e = i * stride + k0;
+        double x[VW];
+#pragma unroll
+        for (int j = 0; j < VW; j++) x[j] = (k0 + j < K) ? src[(k0 + j) * ld + col] : 0.0;
+        if (native) {
+            double* d = reinterpret_cast<double*>(dst) + e;
+#pragma unroll
+            for (int j = 0; j < VW; j++) d[j] = (add && k0 + j < K) ? d[j] + x[j] : (add ? d[j] : x[j]);
+            continue;
+        }
+        DF v[VW];
+        if (add) ld_plain<DF, VW>(dst + e, v);
+#pragma unroll
+        for (int j = 0; j < VW; j++) {
+            const DF t = (k0 + j < K) ? split_scaled(x[j], row_exp(rowmax, k0 + j)) : DF{0.f, 0.f};
+            if (!add) v[j] = t;
+            else if (k0 + j < K) v[j] = AddF64S::split(AddF64S::value(v[j]) + AddF64S::value(t));
+        }
+        Vec<DF, VW>::st(dst + e, v);
+    }
+}
+
+template <int VW>
+__global__ void store_cols_narrow_df_kernel(const DF* __restrict__ vals, long long stride, long long K, long long C, int mode,
+                                            long long fold, const uint32_t* __restrict__ tab, double* __restrict__ out,
+                                            long long ld, int add, const unsigned long long* __restrict__ rowmax,
+                                            const int* gate) {
+    const bool native = gate != nullptr && *gate != 0;
+    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= C) return;
+    const long long node = (mode == MAP_TABLE) ? (long long)tab[c] : (mode == MAP_FOLD ? c * fold : c);
+    const bool has = mode != MAP_TABLE || node != (long long)kInvalid;
+    auto row = [&](long long nd, long long k0, double* v) {
+        if (native) {
+            Vec<double, VW>::ld(reinterpret_cast<const double*>(vals) + nd * stride + k0, v);
+        } else {
+            DF t[VW];
+            Vec<DF, VW>::ld(vals + nd * stride + k0, t);
+#pragma unroll
+            for (int j = 0; j < VW; j++) v[j] = AddF64S::value(t[j]);
+        }
+    };
+    for (long long k0 = 0; k0 < K; k0 += VW) {
+        double v[VW];
+#pragma unroll
+        for (int j = 0; j < VW; j++) v[j] = 0.0;
+        if (has) row(node, k0, v);
+        for (long long p = 1; mode == MAP_FOLD && p < fold; p++) {
+            double t[VW];
+            row(node + p, k0, t);
+#pragma unroll
+            for (int j = 0; j < VW; j++) v[j] += t[j];
+        }
+#pragma unroll
+        for (int j = 0; j < VW; j++) {
+            if (k0 + j >= K) break;
+            double* o = out + (k0 + j) * ld + c;
+            const double x = native ? v[j] : v[j] * pow2(row_exp(rowmax, k0 + j));
+            *o = add ? *o + x : x;
+        }
+    }
+}
+
 __global__ void init_vector_df_kernel(const double* __restrict__ init, long long K, long long n, DF* __restrict__ vals,
                                       long long stride, const unsigned long long* __restrict__ rowmax,
                                       const int* gate) {
@@ -233,6 +307,13 @@ void launch_load_rows_df(const double* src, long long K, long long ld, long long
                          const uint32_t* tab, void* dst, long long stride, int add,
                          const unsigned long long* rowmax, cudaStream_t s, const int* gate) {
     if (R <= 0) return;
+    if (narrow_io(K, R, sizeof(DF))) {
+        narrow_vec<8>(stride, [&](auto vw) {
+            load_rows_narrow_df_kernel<decltype(vw)::value><<<(unsigned)((R + 255) / 256), 256, 0, s>>>(
+                src, K, ld, R, mode, div, tab, static_cast<DF*>(dst), stride, add, rowmax, gate);
+        });
+        return;
+    }
     const dim3 grid((unsigned)((R + 31) / 32), (unsigned)((stride + 31) / 32));
     load_rows_df_kernel<<<grid, dim3(32, 8), 0, s>>>(src, K, ld, R, mode, div, tab, static_cast<DF*>(dst), stride,
                                                      add, rowmax, gate);
@@ -242,6 +323,13 @@ void launch_store_cols_df(const void* vals, long long stride, long long K, long 
                           const uint32_t* tab, double* out, long long ld, int add,
                           const unsigned long long* rowmax, cudaStream_t s, const int* gate) {
     if (C <= 0 || K <= 0) return;
+    if (narrow_io(K, C, sizeof(DF))) {
+        narrow_vec<8>(stride, [&](auto vw) {
+            store_cols_narrow_df_kernel<decltype(vw)::value><<<(unsigned)((C + 255) / 256), 256, 0, s>>>(
+                static_cast<const DF*>(vals), stride, K, C, mode, fold, tab, out, ld, add, rowmax, gate);
+        });
+        return;
+    }
     const dim3 grid((unsigned)((C + 31) / 32), (unsigned)((K + 31) / 32));
     store_cols_df_kernel<<<grid, dim3(32, 8), 0, s>>>(static_cast<const DF*>(vals), stride, K, C, mode, fold, tab,
                                                       out, ld, add, rowmax, gate);

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "sweep.cuh"
 
@@ -124,6 +125,27 @@ void pair_up_f64s(const PairUpParams<DF>& p, int vw, int g, cudaStream_t s);
 
 // Column-map modes of the transposing loads/stores.
 enum MapMode { MAP_IDENT = 0, MAP_DIV = 1, MAP_TABLE = 2, MAP_FOLD = 3 };
+
+// Loads and stores of few columns take a thread per row instead of tiles of 32 columns, which do 32 columns'
+// work for them.  Whole products, tiles against threads per row, in us: 200,000 samples and 250,000
+// mutations, int32 UP K=1 403 / 381, K=8 1199 / 1181, K=20 1853 / 1833, float64 DOWN K=1 490 / 436, K=20 3010 /
+// 3000; 60,000 and 100,000, float64 UP K=8 365 / 349, K=20 601 / 596.  With fewer rows the threads are too
+// few to hide a long row: 20,000 and 50,000, float64 DOWN K=4 101 / 95, K=20 204 / 209; 1,000 and 10,000, K=4
+// 63 / 61, K=8 63 / 65, int32 DOWN K=8 45 / 44, K=20 50 / 50.
+inline bool narrow_io(long long K, long long rows, size_t size) {
+    return K * static_cast<long long>(size) <= 48 || (K <= 20 && rows >= 60000);
+}
+// Calls f with the elements per vector of a row of `stride` elements of Size bytes (choose_layout).
+template <size_t Size, typename F> void narrow_vec(long long stride, F&& f) {
+    if (stride == 1) {
+        f(std::integral_constant<int, 1>{});
+    } else if constexpr (Size == 4) {
+        if (stride == 2) f(std::integral_constant<int, 2>{});
+        else f(std::integral_constant<int, 4>{});
+    } else {
+        f(std::integral_constant<int, 2>{});
+    }
+}
 
 // dst[i*stride + k] (=, or += when add) IO->S(src[k*ld + col(i)]) for i < R, k < K; columns
 // K..stride-1 are zeroed when assigning.  col(i) = i, i/div, or tab[i].
