@@ -271,6 +271,8 @@ struct PairUpRun {
     };
     std::vector<Range> ranges;
     size_t table_bytes = 0;
+    size_t source_bytes = 0;  // behind the table: the height-0 rows by column tiles, or none
+    size_t bytes() const { return table_bytes + source_bytes; }
 };
 PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit);
 // Writes every node's sum over its height-0 children to vals (onto it when rmw), or leaves it in

@@ -113,6 +113,7 @@ template <typename S> struct PairUpParams {
     void* state;   // when set, accumulators (Op::A)
     int second;    // the sources are rows of the table
     long long stride;
+    long long src_stride, tile_step;  // elements from a source row to the next, from a column tile to the next
     const int* gate;  // as SweepParams::gate
 };
 void pair_up_u32(const PairUpParams<uint32_t>& p, int vw, int g, cudaStream_t s);

@@ -758,7 +758,7 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
                                   : dsplit ? static_cast<size_t>(h0) * L.stride * std::max(L.asize, 8)
                                            : 0;
         void* state = stateBytes ? sc.get(stateBytes) : nullptr;
-        void* ptable = (dpair || upair) ? sc.get(dpair ? prun.table_bytes : urun.table_bytes) : nullptr;
+        void* ptable = (dpair || upair) ? sc.get(dpair ? prun.table_bytes : urun.bytes()) : nullptr;
         void* pparts = prun.slots ? sc.get(prun.part_bytes) : nullptr;
         // counters per launch and per heavy row: enough column tiles for any launch shape
         const int TS = std::max(max_tiles(L), prun.tiles);

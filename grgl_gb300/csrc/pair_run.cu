@@ -20,8 +20,9 @@ constexpr long long kPairItemBytes = 96LL << 20;
 // that make an item worth its sum's trip through memory.
 constexpr long long kPairItemsPerWarp = 8;
 constexpr int kPairMinGroups = 16;
-// UP: bytes of the height-0 rows' columns that a launch gathers from at a time.
-constexpr long long kPairSourceBytes = 56LL << 20;
+// UP: bytes of the height-0 rows' columns that a launch gathers from at a time (100 MB: float32 K=128 on
+// 200,000 rows 3.95 ms against 3.63, 50 to 72 MB the same).
+constexpr long long kPairSourceBytes = 64LL << 20;
 // Most of a call's scratch unless a scope says less.
 constexpr uint64_t kPairScratch = 6ULL << 30;
 
@@ -48,6 +49,38 @@ int pair_lanes(const Layout& L, bool up) {
         if (cost(g) <= (both ? 0.801 : 0.701) * cost(L.g) && cost(g) < cost(best)) best = g;
     }
     return best;
+}
+
+// Lanes per row for UP's gathers from the height-0 rows: as many as leave the columns of one tile
+// in L2 (float64 K=64 on 200,000 rows: 102 MB at once, 60% L2 hits and 13.4 ms; in two tiles 11.3;
+// float32 K=32 on 1,000,000: tiles of 32 MB 4.1, of 64 MB 2.7).
+int source_lanes(const Layout& L, long long h0) {
+    int g = pair_lanes(L, true);
+    if (h0 * g * 16 > kPairSourceBytes) {
+        g = L.g;
+        while (g > 1 && h0 * g * 16 > kPairSourceBytes) g /= 2;
+    }
+    return g;
+}
+
+// Tiles that are not whole 128-byte lines bring their neighbours' parts of the lines into L2: the rows'
+// columns are laid out tile by tile first where they don't all fit there.  UP on 1,000,000 samples and 50,000
+// mutations in ms, from the rows as they are in 56 MB tiles, laid out in 64 MB tiles, and the split form:
+// float32 K=32 9.2, 2.7 and 6.4, K=128 40.6, 10.4 and 18.0; float64 K=32 18.9, 6.3 and 11.3.  400,000 and
+// 100,000: float32 K=96 8.2, 6.2 and 13.0; 200,000 and 100,000: 3.5, 3.4 and 6.7.
+bool tile_sources(const Layout& L, long long h0) {
+    const long long rowBytes = L.stride * L.ssize, tileBytes = source_lanes(L, h0) * 16LL;
+    return L.vw * L.ssize == 16 && tileBytes < rowBytes && h0 * rowBytes > kPairSourceBytes &&
+           (tileBytes % 128 != 0 || rowBytes % 128 != 0);
+}
+
+// dst[tile][row][lanes] from src[row][vecs], vectors of 16 bytes.  One pass over the rows: DRAM-bound.
+__global__ void pair_source_kernel(const uint4* __restrict__ src, long long rows, int vecs, int lanes, uint4* __restrict__ dst) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rows * vecs; i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / vecs;
+        const int v = static_cast<int>(i - r * vecs), tile = v / lanes;
+        dst[(tile * rows + r) * lanes + v - tile * lanes] = src[i];
+    }
 }
 
 template <typename F> void by_kind(const Layout& L, F&& f) {
@@ -168,6 +201,11 @@ PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit) {
         s0 = s1;
     }
     if (run.table_bytes > limit) run.ranges.clear();
+    if (tile_sources(L, dp->pair.h0)) {
+        const long long g = source_lanes(L, dp->pair.h0), tiles = (L.stride / L.vw + g - 1) / g;
+        const size_t bytes = static_cast<size_t>(tiles * g * dp->pair.h0) * 16;
+        if (run.table_bytes + bytes <= limit) run.source_bytes = bytes;
+    }
     return run;
 }
 
@@ -175,13 +213,12 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
                    int rmw, cudaStream_t s, const int* gate) {
     const PairPlan& P = dp->pair;
     int launches = 0;
-    // Lanes per row for the gathers from the height-0 rows: as many as leave the columns of one tile
-    // in L2 (float64 K=64 on 200,000 rows: 102 MB at once, 60% L2 hits and 13.4 ms; in two tiles 11.3)
-    const int all = pair_lanes(L, true);
-    int g = all;
-    if (P.h0 * g * 16 > kPairSourceBytes) {
-        g = L.g;
-        while (g > 1 && P.h0 * g * 16 > kPairSourceBytes) g /= 2;
+    const int all = pair_lanes(L, true), g = source_lanes(L, P.h0);
+    char* const tiled = run.source_bytes ? static_cast<char*>(table) + run.table_bytes : nullptr;
+    if (tiled) {
+        pair_source_kernel<<<sm_count() * 8, 256, 0, s>>>(static_cast<const uint4*>(vals), P.h0,
+                                                          static_cast<int>(L.stride / L.vw), g, reinterpret_cast<uint4*>(tiled));
+        launches++;
     }
     const size_t rowBytes = static_cast<size_t>(L.stride) * L.ssize;
     for (const PairUpRun::Range& r : run.ranges) {
@@ -195,7 +232,10 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
                 p.lists = list;
                 p.count = count;
                 p.adj = adj;
-                p.src = reinterpret_cast<decltype(p.src)>(second ? t : static_cast<char*>(vals));
+                p.src = reinterpret_cast<decltype(p.src)>(second ? t : tiled ? tiled : static_cast<char*>(vals));
+                const int lanes = second ? all : g;
+                p.src_stride = !second && tiled ? static_cast<long long>(g) * L.vw : L.stride;
+                p.tile_step = (!second && tiled ? P.h0 : 1) * lanes * L.vw;
                 p.table = reinterpret_cast<decltype(p.table)>(t);
                 p.dst = reinterpret_cast<decltype(p.dst)>(nodes);
                 p.rmw = rmw;
@@ -203,7 +243,7 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
                 p.second = second ? 1 : 0;
                 p.stride = L.stride;
                 p.gate = gate;
-                        fn(p, L.vw, second ? all : g, s);
+                fn(p, L.vw, lanes, s);
             };
             switch (L.kind) {
             case Kind::U32: go(PairUpParams<uint32_t>{}, pair_up_u32); break;

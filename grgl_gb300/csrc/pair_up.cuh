@@ -52,8 +52,9 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const
         for (int m = L; m < 32; m <<= 1) most = max(most, __shfl_xor_sync(FULL_MASK, most, m));
     }
     const uint32_t* ids = p.adj + list.e0;
-    const char* src = reinterpret_cast<const char*>(p.src + (colok ? col : 0));
-    const unsigned rowBytes = static_cast<unsigned>(p.stride * sizeof(S));
+    // (lanes past the last column read with the tile's first lane: another tile's columns would take up L2)
+    const char* src = reinterpret_cast<const char*>(p.src + blockIdx.y * p.tile_step + (colok ? (lane % G) * VW : 0));
+    const unsigned rowBytes = static_cast<unsigned>(p.src_stride * sizeof(S));
     Acc acc;
     acc.zero();
     uint32_t next[STEPS];

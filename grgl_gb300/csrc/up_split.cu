@@ -565,7 +565,7 @@ bool use_up_split(grgx_graph* g, DevicePlan* dp, const Layout& L) {
         if (it != dp->split_choice.end()) {
             want = it->second;  // measured by grgx_autotune on this graph
         } else {
-            // the height-0 rows outgrow L2, or a single 4-byte column (the staged passes)
+            // the height-0 rows outgrow L2, or a single 4-byte column (the staged lists)
             const long long src0 = static_cast<long long>(dp->level_begin[1]);
             want = static_cast<uint64_t>(src0) * static_cast<uint64_t>(L.stride) * L.ssize > split_threshold_bytes() ||
                    (staged_layout(L) && split_threshold_bytes() < (1ull << 62));
@@ -585,7 +585,7 @@ bool use_down_split(grgx_graph* g, DevicePlan* dp, const Layout& L) {
         const int mode = g_down_mode.load();
         if (mode != 0) want = (mode == 1);
         else if (it != dp->down_split_choice.end()) want = it->second;  // measured by grgx_autotune
-        else want = staged_layout(L);  // a single 4-byte column: the staged passes
+        else want = staged_layout(L);  // a single 4-byte column: the staged lists
     }
     if (!want) return false;
     ensure_down_split(g, dp);

@@ -216,3 +216,25 @@ def test_pair_form_within_a_servers_memory(env, dt):
             V = _rand(np.random.default_rng(6), dt, (12, cols))
             got, _ = srv.result(srv.submit(gid, V, direction), timeout=60.0)
             _check(og, V, direction, got)
+
+
+@pytest.mark.parametrize("dt", [np.int32, np.int64, np.float32, np.float64])
+def test_pair_up_sources_by_column_tiles(cuda_ok, dt):
+    """Rows wider than L2 holds in tiles of less than a line: the last tile is partial; float64 also with
+    rows that take the FP64 path."""
+    import grgl_gb300 as gx
+
+    _pair_mode(1)
+    try:
+        g, og = _both(gx, gx.window_tree_grg(500_002, 1_500, seed=5))
+        K = 36 if np.dtype(dt).itemsize == 4 else 18  # 144 bytes a row: tiles of 64, 64 and 16
+        V = _rand(np.random.default_rng(2), dt, (K, g.num_samples))
+        for wide in (False, True) if dt == np.float64 else (False,):
+            if wide:
+                V[:, ::2] *= 1e-200
+            W = V.astype(np.float64) if V.dtype.kind == "f" else V
+            ref = oracle.matmul(og, W, UP)
+            scale = oracle.matmul(og, np.abs(W), UP)
+            assert_matches(gx.matmul(g, V, UP).astype(ref.dtype), ref, scale, rtol=1e-6 if dt == np.float32 else 1e-12)
+    finally:
+        _pair_mode(0)
