@@ -111,7 +111,7 @@ template <typename S> struct PairUpParams {
     S* dst;        // the nodes' rows of sums (added onto when rmw), or
     int rmw;
     void* state;   // when set, accumulators (Op::A)
-    int second;    // the sources are rows of the table
+    int second;    // sums for nodes (0: pattern rows)
     long long stride;
     long long src_stride, tile_step;  // elements from a source row to the next, from a column tile to the next
     const int* gate;  // as SweepParams::gate

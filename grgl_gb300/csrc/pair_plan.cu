@@ -255,6 +255,20 @@ __global__ void node_pairs_kernel(const uint2* __restrict__ nodes, long long row
     }
 }
 
+// The lists' ids: the children below h0 of the UP rows' edges from[i].x .. from[i].y - 1 (whose first ids
+// carry a row mark).
+__global__ void few_ids_kernel(const PairList* __restrict__ lists, const longlong2* __restrict__ from, long long count,
+                               unsigned h0, const uint32_t* __restrict__ adj, uint32_t* __restrict__ out) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
+        const PairList l = lists[i];
+        int k = 0;
+        for (long long x = from[i].x; x < from[i].y && k < l.len; x++) {
+            const uint32_t id = adj[x] & 0x7fffffffu;
+            if (id < h0) out[l.e0 + k++] = id;
+        }
+    }
+}
+
 // The runs, as first positions (with the end), from each position's predecessor.
 std::vector<int> cut_runs(const std::vector<int>& pv) {
     std::vector<int> start;
@@ -317,6 +331,7 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
     // position of each UP row in the sequence; a node's patterns are all of its own segment
     std::vector<unsigned> posOf(d.up_off.size(), 0);
     for (long long q = 0; q < Q; q++) posOf[P.seq[q]] = static_cast<unsigned>(q);
+    auto few = [&](long long q) { return P.low[P.seq[q]] <= kPairFew; };
     auto position = [&](unsigned node) { return node == INVALID_NODE ? INVALID_NODE : posOf[node - h0]; };
     std::vector<PairPlan::Segment> segments(nseg + 1);
     std::vector<long long> edge0(nseg + 1, 0), sub0(nseg + 1, 0), nedge0(nseg + 1, 0);
@@ -333,6 +348,7 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
         for (long long q = first_position(s); q < first_position(s + 1); q++) {
             const long long n = pieces_of(deg[q]);
             nedge0[s + 1] += deg[q];
+            if (few(q)) continue;
             next.node0 += n;
             next.top0 += n > 1;
             sub0[s + 1] += n > 1 ? n : 0;
@@ -371,7 +387,7 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
         e = nedge0[s];
         long long node = a.node0, top = a.top0, sub = sub0[s];
         for (long long q = first_position(s); q < first_position(s + 1); q++) {
-            const long long n = pieces_of(deg[q]);
+            const long long n = few(q) ? 0 : pieces_of(deg[q]);
             if (n > 1) topLists[top++] = {sub, static_cast<int>(n), P.seq[q]};
             for (long long i = 0; i < n; i++) {
                 cut(&nodeLists[node++], e, deg[q], n, i, n > 1 ? ~static_cast<int>(row) : P.seq[q]);
@@ -383,6 +399,18 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
         longest_first(nodeLists.data() + a.node0, static_cast<size_t>(node - a.node0));
     });
 
+    std::vector<PairList> fewLists;
+    for (long long q = 0; q < Q; q++)
+        if (few(q)) fewLists.push_back({0, static_cast<int>(P.low[P.seq[q]]), P.seq[q]});
+    longest_first(fewLists.data(), fewLists.size());
+    std::vector<longlong2> fewFrom(fewLists.size());
+    long long fewEdges = 0;
+    for (size_t i = 0; i < fewLists.size(); i++) {
+        fewFrom[i] = {static_cast<long long>(d.up_off[fewLists[i].out]), static_cast<long long>(d.up_off[fewLists[i].out + 1])};
+        fewLists[i].e0 = fewEdges;
+        fewEdges += fewLists[i].len;
+    }
+
     const uint2* dRowNodes = tmp.copy(rowNodes);
     unsigned *keys = tmp.get<unsigned>(2 * rows), *vals = tmp.get<unsigned>(2 * rows);
     unsigned *keys2 = tmp.get<unsigned>(2 * rows), *vals2 = tmp.get<unsigned>(2 * rows);
@@ -393,6 +421,15 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
     sort_pairs(tmp, keys, vals, keys2, vals2, 2 * rows, bits);
     uint32_t* adj = tmp.get<uint32_t>(ne);
     GRGX_CUDA(cudaMemcpyAsync(adj, vals, ne * sizeof(uint32_t), cudaMemcpyDeviceToDevice, cudaStreamLegacy));
+    if (!fewLists.empty()) {
+        P.few_lists = tmp.copy(fewLists);
+        P.few_adj = tmp.get<uint32_t>(fewEdges);
+        const longlong2* from = tmp.copy(fewFrom);
+        few_ids_kernel<<<blocks_for(static_cast<long long>(fewLists.size()), 256), 256>>>(
+            P.few_lists, from, static_cast<long long>(fewLists.size()), static_cast<unsigned>(h0), d.up.adj, P.few_adj);
+        GRGX_CUDA(cudaGetLastError());
+    }
+    P.nfew = static_cast<long long>(fewLists.size());
     P.pat_lists = tmp.copy(patLists);
     P.node_lists = tmp.copy(nodeLists);
     P.top_lists = tmp.copy(topLists);
@@ -406,6 +443,10 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
     tmp.keep(d, P.pat_lists, patLists.size() * sizeof(PairList));
     tmp.keep(d, P.node_lists, nodeLists.size() * sizeof(PairList));
     tmp.keep(d, P.top_lists, topLists.size() * sizeof(PairList));
+    if (P.nfew > 0) {
+        tmp.keep(d, P.few_lists, fewLists.size() * sizeof(PairList));
+        tmp.keep(d, P.few_adj, fewEdges * sizeof(uint32_t));
+    }
     P.segments = std::move(segments);
 }
 
@@ -627,6 +668,19 @@ std::vector<unsigned> count_low_children(DevicePlan& d) {
     GRGX_CUDA(cudaGetLastError());
     GRGX_CUDA(cudaMemcpy(low.data(), dLow, R * sizeof(unsigned), cudaMemcpyDeviceToHost));
     return low;
+}
+
+void pair_counts(grgx_graph* g, bool down, uint64_t out[4]) {
+    const DevicePlan* dp = ensure_device_plan(g);
+    std::lock_guard<std::mutex> lk(g->mu);
+    const PairPlan& P = dp->pair;
+    const bool built = P.usable && (down ? P.down_built : P.up_built);
+    uint64_t low = 0;
+    for (unsigned c : P.low) low += c;
+    out[0] = built ? P.h0 : 0;
+    out[1] = built ? P.nblk : 0;
+    out[2] = built ? P.npat : 0;
+    out[3] = built ? low : 0;
 }
 
 void set_pair_mode(int mode) { g_pair_mode.store(mode); }

@@ -33,6 +33,11 @@ constexpr double kPairMaxCost = 0.9;
 // UP: lists (a pattern's height-0 nodes, a node's table rows) are summed in pieces of at most this
 // many, each with a row of its own in the table; it bounds how long one group of lanes works on one.
 constexpr long long kPairPiece = 256;
+// UP: nodes with at most this many height-0 children sum them directly, with the nodes' own additions.  Over
+// pattern rows, which compensated float32 rounds, such nodes ended up to 1.3e-7 of sum |terms| off, directly
+// 6.0e-8 as in the sweep (N=200,000, M=250,000, K=8, N(0,1) inputs; float64 7.7e-15 and 3.7e-15).  They hold few
+// of the edges: 1277 and 1261 us there, float32 K=40 3052 and 3065, N=20,000, M=50,000 203 and 208.
+constexpr unsigned kPairFew = 32;
 // Blocks whose lists are sorted by length together, longest first (the order they are launched in).
 constexpr long long kPairSegment = 64;
 
@@ -72,6 +77,10 @@ struct PairPlan {
     std::vector<Segment> segments;                // + the end
     PairList *pat_lists = nullptr, *node_lists = nullptr, *top_lists = nullptr;
     uint32_t *pat_adj = nullptr, *node_adj = nullptr, *top_adj = nullptr;
+    // nodes of few height-0 children: lists of those, by length
+    long long nfew = 0;
+    PairList* few_lists = nullptr;
+    uint32_t* few_adj = nullptr;
 };
 
 }  // namespace grgx

@@ -221,21 +221,22 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
         launches++;
     }
     const size_t rowBytes = static_cast<size_t>(L.stride) * L.ssize;
+    bool few = P.nfew > 0;  // (with the first range)
     for (const PairUpRun::Range& r : run.ranges) {
         const PairPlan::Segment &a = P.segments[r.s0], &b = P.segments[r.s1];
         // table rows count from the first segment's first one, the nodes' from height 1 on
         char* t = static_cast<char*>(table) - static_cast<size_t>(a.row0) * rowBytes;
         char* nodes = static_cast<char*>(vals) + static_cast<size_t>(P.h0) * rowBytes;
-        auto lists = [&](const PairList* list, long long count, const uint32_t* adj, bool second) {
+        auto lists = [&](const PairList* list, long long count, const uint32_t* adj, bool second, bool rows) {
             if (count == 0) return;
             auto go = [&](auto p, auto fn) {
                 p.lists = list;
                 p.count = count;
                 p.adj = adj;
-                p.src = reinterpret_cast<decltype(p.src)>(second ? t : tiled ? tiled : static_cast<char*>(vals));
-                const int lanes = second ? all : g;
-                p.src_stride = !second && tiled ? static_cast<long long>(g) * L.vw : L.stride;
-                p.tile_step = (!second && tiled ? P.h0 : 1) * lanes * L.vw;
+                p.src = reinterpret_cast<decltype(p.src)>(!rows ? t : tiled ? tiled : static_cast<char*>(vals));
+                const int lanes = rows ? g : all;
+                p.src_stride = rows && tiled ? static_cast<long long>(g) * L.vw : L.stride;
+                p.tile_step = (rows && tiled ? P.h0 : 1) * lanes * L.vw;
                 p.table = reinterpret_cast<decltype(p.table)>(t);
                 p.dst = reinterpret_cast<decltype(p.dst)>(nodes);
                 p.rmw = rmw;
@@ -256,9 +257,11 @@ int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, 
             }
             launches++;
         };
-        lists(P.pat_lists + a.pat0, b.pat0 - a.pat0, P.pat_adj, false);
-        lists(P.node_lists + a.node0, b.node0 - a.node0, P.node_adj, true);
-        lists(P.top_lists + a.top0, b.top0 - a.top0, P.top_adj, true);
+        lists(P.pat_lists + a.pat0, b.pat0 - a.pat0, P.pat_adj, false, true);
+        if (few) lists(P.few_lists, P.nfew, P.few_adj, true, true);
+        few = false;
+        lists(P.node_lists + a.node0, b.node0 - a.node0, P.node_adj, true, false);
+        lists(P.top_lists + a.top0, b.top0 - a.top0, P.top_adj, true, false);
     }
     return launches;
 }
