@@ -117,6 +117,26 @@ def alg_bytes(stats, K, s, direction):
     return E * 4 + (n + 1) * 8 + E * K * s + n * K * s + K * (cols_in + cols_out) * s + 8 * M
 
 
+def gathered_bytes(gx, g, E, K, s, direction):
+    """Bytes one traversal gathers: an id and a row of K values per edge; in pair form (one gather per
+    block and height-0 node, and those that make and use the pattern rows) what that form reads."""
+    import ctypes
+
+    from grgl_gb300 import _lib
+
+    row, out = K * s, (ctypes.c_uint64 * 4)()
+    _lib.check(_lib.lib().grgx_debug_pair_counts(g._h, direction, out))
+    h0, blocks, patterns, low = (int(x) for x in out)
+    if direction == UP and row == 4:
+        blocks = 0  # single 4-byte columns stay with the lists per node
+    if blocks == 0:
+        return E * (4 + row)
+    rest = (E - low) * (4 + row)
+    if direction == DOWN:
+        return rest + blocks * h0 * (2 + row) + patterns * (8 + 2 * row)
+    return rest + (blocks * h0 + 2 * patterns) * (4 + row)
+
+
 class Clocks:
     """nvidia-smi sampling during the timed region."""
 
@@ -409,7 +429,7 @@ def cold_start(gx, torch, g):
 def large_graph(gx, torch, args, l2_peak):
     """The large window-tree graph (N=1,000,000 haplotypes, a variant prefix sized to 2-4e9 edges):
     float32 compensated and float64 at K in {16, 64, 256}, both directions, device inputs.  Each
-    entry: sweep device time (CUDA events), edge*K/s, gathered GB/s (edge ids + one row per edge)
+    entry: sweep device time (CUDA events), edge*K/s, gathered GB/s (gathered_bytes)
     against the L2 read ceiling measured in this run, and the float32 result's max error against
     the float64 result, relative to the sum of |terms| per output (|V| X); the float64 result is
     checked against native FP64 accumulation at K=16.  Then float32 and float64 K=16 products in
@@ -446,7 +466,7 @@ def large_graph(gx, torch, args, l2_peak):
                     res = gx.matmul(g, V, d)
                 t = gx.last_timing()
                 s = V.element_size()
-                gath = E * (4 + K * s) / (t["sweep_ms"] / 1e3) / 1e9
+                gath = gathered_bytes(gx, g, E, K, s, d) / (t["sweep_ms"] / 1e3) / 1e9
                 rows.append({"dtype": "float64" if s == 8 else "float32", "K": K, "dir": "UP" if d == UP else "DOWN",
                              "sweep_ms": t["sweep_ms"], "total_ms": t["total_ms"],
                              "edgeK_per_s": E * K / (t["sweep_ms"] / 1e3),
@@ -464,7 +484,8 @@ def large_graph(gx, torch, args, l2_peak):
     gx.set_timing(False)
     units = sum(E * r["K"] for r in rows)
     secs = sum(r["sweep_ms"] for r in rows) / 1e3
-    gbytes = sum(E * (4 + r["K"] * (8 if r["dtype"] == "float64" else 4)) for r in rows)
+    gbytes = sum(gathered_bytes(gx, g, E, r["K"], 8 if r["dtype"] == "float64" else 4, UP if r["dir"] == "UP" else DOWN)
+                 for r in rows)
     # a batched mix on the same graph: 64 requests, K ~ U{1..128}, UP/DOWN 50/50, compensated
     # float32, stacked into shared traversals (wall clock around the whole batch)
     reqs = []
@@ -480,7 +501,7 @@ def large_graph(gx, torch, args, l2_peak):
     torch.cuda.synchronize()
     t_b = time.perf_counter() - t0
     b_units = sum(E * V.shape[0] for V, _ in reqs)
-    b_bytes = sum(E * (4 + 4 * V.shape[0]) for V, _ in reqs)
+    b_bytes = sum(gathered_bytes(gx, g, E, V.shape[0], 4, d) for V, d in reqs)
     batched = {"requests": len(reqs), "columns": int(sum(V.shape[0] for V, _ in reqs)), "seconds": t_b,
                "edgeK_per_s": b_units / t_b, "gathered_GBps": b_bytes / t_b / 1e9,
                "l2_frac": b_bytes / t_b / 1e9 / l2_peak,
@@ -493,7 +514,7 @@ def large_graph(gx, torch, args, l2_peak):
         og = oracle_graph(g)
         parity = parity_vs_oracle(gx, torch, g, og, [(np.float32, 16, UP), (np.float32, 16, DOWN),
                                                      (np.float64, 16, UP), (np.float64, 16, DOWN)], seed=17)
-        parity["graph"] = "this graph (UP runs in split form above 2^31 edges)"
+        parity["graph"] = "this graph (more than 2^31 edges)"
         del og
     del g
     torch.cuda.empty_cache()
@@ -716,7 +737,7 @@ def main():
             t = gx.last_timing()
             rec = {"dtype": str(dt), "K": K, "dir": "UP" if d == UP else "DOWN", "total_ms": t["total_ms"],
                    "sweep_ms": t["sweep_ms"], "edgeK_per_s": E * K / (t["sweep_ms"] / 1e3),
-                   "gathered_GBps": E * (4 + K * dt.itemsize) / (t["sweep_ms"] / 1e3) / 1e9,
+                   "gathered_GBps": gathered_bytes(gx, g, E, K, dt.itemsize, d) / (t["sweep_ms"] / 1e3) / 1e9,
                    "launches": t["launches"]}
             print(json.dumps(rec), flush=True)
         return
@@ -781,14 +802,14 @@ def main():
 
     # ---- ceilings of the sweep kernel over the timed region -----------------------------------
     # The gathers are served by L2 (the node rows a level gathers are reused across its warps),
-    # so the bound is L2 read bandwidth: edge ids + one gathered row per edge, per launch, against
+    # so the bound is L2 read bandwidth: ids + gathered rows (gathered_bytes), per launch, against
     # the L2 -> SM read bandwidth measured in this run.  Beside it, the DRAM bytes ncu counts
     # (a capture of the same step on a quarter-size graph, scaled by edges) against the HBM peak.
     E = shard_stats["edges"]
     sweep_ms = sum(t["sweep_ms"] for *_, t in records)
     sweep_s_step = sweep_ms / args.steps / 1e3
     launches = sum(t["launches"] for *_, t in records)
-    gathered = sum(E * (4 + K * dt.itemsize) for dt, K, d, _ in records) / args.steps
+    gathered = sum(gathered_bytes(gx, g, E, K, dt.itemsize, d) for dt, K, d, _ in records) / args.steps
     abytes = sum(alg_bytes(shard_stats, K, dt.itemsize, d) for dt, K, d, _ in records) / args.steps
     compulsory = sum(E * 4 + (shard_stats["nodes"] + 1) * 8 + 2 * shard_stats["nodes"] * K * dt.itemsize
                      for dt, K, d, _ in records) / args.steps
@@ -814,15 +835,16 @@ def main():
         rates = [E * 4 / (ms_ / 1e3) / 1e9 for _, _, ms_ in k1]
         id_stream = {"achieved": statistics.fmean(rates), "peak": hbm_peak, "unit": "GB/s",
                      "frac": statistics.fmean(rates) / hbm_peak,
-                     "what": "K=1 matmuls: the 4-byte edge-id stream (E x 4 bytes, read once from HBM) / sweep "
-                             "time; the part of the step HBM itself bounds"}
+                     "what": "K=1 matmuls: 4 bytes per edge / sweep time (the pair form and the staged lists read 2 "
+                             "per gather instead)"}
     roofline = {
-        "bound": "l2", "kernel": "grgx::sweep_kernel",
+        "bound": "l2", "kernel": "grgx::pair_down_kernel, grgx::pair_up_kernel, grgx::sweep_kernel",
         "achieved": gathered / sweep_s_step / 1e9, "peak": l2_peak, "unit": "GB/s",
         "frac": gathered / sweep_s_step / 1e9 / l2_peak,
         "traffic": traffic, "traffic_source": traffic_src,
-        "what": "edge ids + one gathered row per edge (E x (4 + K x s) bytes per matmul) over the step's sweep "
-                "launches / their CUDA-event time, against the L2 -> SM read bandwidth measured in this run",
+        "what": "ids + gathered rows of the form each matmul takes (pair form: one row per block and height-0 node "
+                "plus the pattern rows' own; otherwise E x (4 + K x s) bytes) over the step's sweep launches / their "
+                "CUDA-event time, against the L2 -> SM read bandwidth measured in this run",
         "peak_source": "grgx_measure_l2_bandwidth in this run (an L2-resident buffer read by every SM); the "
                        "ncu cross-check is in profiles/l2_ceiling_small.md",
         "sweep_ms_per_step": sweep_s_step * 1e3,

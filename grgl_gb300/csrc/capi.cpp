@@ -30,6 +30,7 @@ void set_up_split(long long block, unsigned long long thresholdBytes);
 void set_down_split_mode(int mode);
 void set_staged(bool on);
 void set_pair_mode(int mode);
+void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
 void* host_alloc(uint64_t bytes);
 void host_free(void* b);
 std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags);
@@ -457,6 +458,15 @@ extern "C" void grgx_debug_split_forms(int down_mode, int staged) {
 // Test hook (not part of the public header): pair form by its rules (0), wherever possible (1) or
 // never (2); a graph's form is decided on the first call that may use it.
 extern "C" void grgx_debug_pair_form(int mode) { grgx::set_pair_mode(mode); }
+
+// Measurement hook (not part of the public header): what the pair form gathers.  out: height-0 nodes,
+// blocks, patterns and height-0 edges; zeros while no call of this direction has taken the form.
+extern "C" grgx_status grgx_debug_pair_counts(grgx_graph* g, int direction, uint64_t out[4]) {
+    return guarded([&] {
+        GRGX_CHECK(g && out, GRGX_ERR_API_MISUSE, "null argument");
+        grgx::pair_counts(g, direction == GRGX_DIRECTION_DOWN, out);
+    });
+}
 
 grgx_status grgx_collect_timings(grgx_timing* out, uint64_t capacity, uint64_t* count) {
     return guarded([&] {

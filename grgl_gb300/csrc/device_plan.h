@@ -242,6 +242,8 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
 // server's worker lowers it to what its batch has reserved (PairScratchScope).
 size_t pair_scratch_limit();
 void set_pair_mode(int mode);
+// out: height-0 nodes, blocks, patterns, height-0 edges of a direction in pair form (zeros: not in use).
+void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
 // The launches of a DOWN call in pair form, sized for layout L: a table of pattern rows per range
 // of blocks, and per range the sums of its items.  With several ranges the first sum carries what
 // the ranges before added up.
