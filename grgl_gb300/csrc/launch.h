@@ -92,6 +92,8 @@ void pair_down_u32(const PairDownParams<uint32_t>& p, PairDownCall& c, int vw, i
 void pair_down_xor(const PairDownParams<uint32_t>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
 void pair_down_u64(const PairDownParams<unsigned long long>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
 void pair_down_f64(const PairDownParams<double>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_f32c1(const PairDownParams<float>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
+void pair_down_f32cx(const PairDownParams<float>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
 void pair_down_f32c(const PairDownParams<float>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
 void pair_down_f32(const PairDownParams<float>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);
 void pair_down_f64s(const PairDownParams<DF>& p, PairDownCall& c, int vw, int g, int sms, cudaStream_t s);

@@ -130,6 +130,8 @@ struct AddF32C {
 // The same with PRE edges pre-summed in plain float32 where the sweep's block path pre-sums
 // kF32PreSum (vecacc.cuh).
 template <int PRE> struct AddF32CPre : AddF32C {};
+// ... and with pattern rows that keep the error of their sum (DOWN in pair form).
+struct AddF32CX : AddF32C {};
 
 // Float64 on GB300 without the FP64 pipe in the inner loop.  Node values are stored as a
 // float pair (hi + lo, 48 significant bits) of the value scaled by 2^-e_k per input row k, so

@@ -28,12 +28,13 @@ template <> struct PairPart<AddF64SD> {
 
 // Pattern row elements.  A pair of rows is summed in storage precision: compensated float32 rounds
 // it once, like the first level of the sweep's plain pre-sums (vecacc.cuh); float pairs keep 48
-// bits.  A single compensated column has no pre-sums in the sweep and keeps the pair's error here.
+// bits.  A single compensated column, and the columns of short rows (AddF32CX), have no pre-sums in the
+// sweep and keep the pair's error here.
 template <class Op, int VW> struct PairTable {
     using T = typename Op::S;
     static __device__ __forceinline__ T sum(typename Op::S a, typename Op::S b) {
         if constexpr (std::is_base_of<AddF64S, Op>::value) return df_add(a, b);
-        else if constexpr (std::is_same<Op, AddF32C>::value) return __fadd_rn(a, b);
+        else if constexpr (std::is_base_of<AddF32C, Op>::value) return __fadd_rn(a, b);
         else {
             typename Op::A t = Op::zero();
             Op::add(t, a);
@@ -42,7 +43,7 @@ template <class Op, int VW> struct PairTable {
         }
     }
 };
-template <> struct PairTable<AddF32C, 1> {
+struct PairTableExact {
     using T = F32Pair;
     static __device__ __forceinline__ T sum(float a, float b) {
         T t;
@@ -50,7 +51,19 @@ template <> struct PairTable<AddF32C, 1> {
         return t;
     }
 };
+template <> struct PairTable<AddF32C, 1> : PairTableExact {};
+template <> struct PairTable<AddF32CX, 2> : PairTableExact {};
 template <typename T, int VW> struct TableVec : Vec<T, VW> {};
+template <> struct TableVec<F32Pair, 2> {
+    static __device__ __forceinline__ void ld(const F32Pair* p, F32Pair* v) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+        v[0] = {t.x, t.y};
+        v[1] = {t.z, t.w};
+    }
+    static __device__ __forceinline__ void st(F32Pair* p, const F32Pair* v) {
+        *reinterpret_cast<float4*>(p) = make_float4(v[0].hi, v[0].lo, v[1].hi, v[1].lo);
+    }
+};
 template <> struct TableVec<F32Pair, 1> {
     static __device__ __forceinline__ void ld(const F32Pair* p, F32Pair* v) {
         const float2 t = __ldg(reinterpret_cast<const float2*>(p));

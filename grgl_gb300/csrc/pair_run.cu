@@ -83,13 +83,41 @@ __global__ void pair_source_kernel(const uint4* __restrict__ src, long long rows
     }
 }
 
-template <typename F> void by_kind(const Layout& L, F&& f) {
+// How compensated float32 adds DOWN pattern rows.  The sweep pre-sums four edges only in batches of
+// edges without a row start, so the shorter the rows (two edges per block) and the fewer the columns, the
+// fewer plain additions its sums pass.  Norm of the error against float64, 1e-8 of the norm, N(0,1) inputs, sweep
+// / rounded pattern rows pre-summed / one at a time / with their error:
+//   200,000 samples and 3,000 variants (15 blocks), K=8 5.4 / 6.4 / 5.8 / 5.2, K=64 6.1 / 6.3 / 5.7 / -
+//   100,000 and 20,000 (100),    K=4 5.7 / 6.9 / 6.2 / 5.1, K=32 6.3 / 6.6 / 5.8 / -, K=64 6.4 / 6.5 / 5.8 / -
+//   200,000 and 250,000 (1,250), K=8 6.4 / 6.5 / 5.8 / -,   K=16 6.5 / 6.5 / 5.9 / -, K=64 6.4 / 6.3 / - / -
+// Microseconds: 100,000 and 20,000 K=8 240 / 92 / 90 / 105, K=64 662 / 239 / 279 / -; 200,000 and 250,000 K=8 2260 /
+// 850 / 858 / -, K=16 2757 / 1166 / 1329 / -.  The kind that stays at or below the sweep's error is taken.
+enum class DownSums { kPreSum, kSingle, kExact };
+DownSums down_sums(const Layout& L, const PairPlan& P) {
+    if (L.kind != Kind::F32C || L.vw == 1) return DownSums::kPreSum;
+    const long long work = P.nblk * L.stride;
+    if (work <= 800) return DownSums::kExact;
+    return work < 10000 || L.stride <= 8 ? DownSums::kSingle : DownSums::kPreSum;
+}
+
+// The layout that the DOWN pair kernels run with: pattern rows with their error take two columns a lane.
+Layout down_layout(Layout L, const PairPlan& P) {
+    if (down_sums(L, P) != DownSums::kExact) return L;
+    L.vw = 2;
+    const long long vecs = L.stride / 2;
+    L.g = 1;
+    while (L.g < 32 && L.g < vecs) L.g *= 2;
+    return L;
+}
+
+template <typename F> void by_kind(const Layout& L, DownSums sums, F&& f) {
     switch (L.kind) {
     case Kind::U32: f(PairDownParams<uint32_t>{}, pair_down_u32); break;
     case Kind::XOR: f(PairDownParams<uint32_t>{}, pair_down_xor); break;
     case Kind::U64: f(PairDownParams<unsigned long long>{}, pair_down_u64); break;
     case Kind::F64: f(PairDownParams<double>{}, pair_down_f64); break;
-    case Kind::F32C: f(PairDownParams<float>{}, pair_down_f32c); break;
+    case Kind::F32C: f(PairDownParams<float>{}, sums == DownSums::kExact ? pair_down_f32cx
+                                                    : sums == DownSums::kSingle ? pair_down_f32c1 : pair_down_f32c); break;
     case Kind::F32: f(PairDownParams<float>{}, pair_down_f32); break;
     case Kind::F64S: f(PairDownParams<DF>{}, pair_down_f64s); break;
     }
@@ -101,13 +129,15 @@ PairScratchScope::PairScratchScope(uint64_t bytes) : saved_(t_limit) { t_limit =
 PairScratchScope::~PairScratchScope() { t_limit = saved_; }
 size_t pair_scratch_limit() { return static_cast<size_t>(t_limit); }
 
-PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit) {
+PairDownRun pair_down_run(const Layout& call, const DevicePlan* dp, size_t limit) {
     const PairPlan& P = dp->pair;
+    const Layout L = down_layout(call, P);
+    const DownSums sums = down_sums(call, P);
     PairDownRun run;
     const int lanes = pair_lanes(L, false);
     run.tiles = static_cast<int>((L.stride / L.vw + lanes - 1) / lanes);
     PairDownCall shape;
-    by_kind(L, [&](auto p, auto fn) { fn(p, shape, L.vw, pair_lanes(L, false), sm_count(), nullptr); });
+    by_kind(L, sums, [&](auto p, auto fn) { fn(p, shape, L.vw, pair_lanes(L, false), sm_count(), nullptr); });
     const size_t rowBytes = static_cast<size_t>(L.stride) * shape.table_bytes;
     const size_t slotBytes = static_cast<size_t>(P.h0) * L.stride * shape.part_bytes;
     const size_t tableMost = std::min(kPairTableBytes, limit / 3);
@@ -143,11 +173,12 @@ PairDownRun pair_down_run(const Layout& L, const DevicePlan* dp, size_t limit) {
     return run;
 }
 
-int launch_pair_down(const Layout& L, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
+int launch_pair_down(const Layout& call, const DevicePlan* dp, const PairDownRun& run, void* vals, void* table, void* parts,
                      unsigned* work, cudaStream_t s, const int* gate) {
     const PairPlan& P = dp->pair;
+    const Layout L = down_layout(call, P);
     int launches = 0;
-    by_kind(L, [&](auto p, auto fn) {
+    by_kind(L, down_sums(call, P), [&](auto p, auto fn) {
         PairDownCall c;
         fn(p, c, L.vw, pair_lanes(L, false), sm_count(), s);
         p.ids = reinterpret_cast<const uint2*>(P.ids);

@@ -213,10 +213,15 @@ template <int NP, int PRE = kF32PreSum> struct PackedF32C {
         }
     }
     // Four pattern rows, each the rounded sum of two edges: two at a time in plain float32, so the
-    // edges pass the same two rounding levels before a TwoSum as four edges do in add_block.
+    // edges pass the same two rounding levels before a TwoSum as four edges do in add_block (PRE 1: one at a time).
     __device__ __forceinline__ void add_pairs(const float (*v)[2 * NP]) {
 #pragma unroll
         for (int u = 0; u < 4; u += 2) {
+            if constexpr (PRE == 1) {
+                add(v[u]);
+                add(v[u + 1]);
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < NP; j++)
                 add_pair2(j, add2(make_float2(v[u][2 * j], v[u][2 * j + 1]),
@@ -267,6 +272,15 @@ template <int NP, int PRE = kF32PreSum> struct PackedF32C {
 };
 template <> struct VecAcc<AddF32C, 2> : PackedF32C<1> {};
 template <> struct VecAcc<AddF32C, 4> : PackedF32C<2> {};
+template <> struct VecAcc<AddF32CX, 2> : PackedF32C<1, 1> {
+    __device__ __forceinline__ void add_pairs(const F32Pair (*v)[2]) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            add_pair2(0, make_float2(v[u][0].hi, v[u][1].hi));
+            lo[0] = add2(lo[0], make_float2(v[u][0].lo, v[u][1].lo));
+        }
+    }
+};
 template <int PRE> struct VecAcc<AddF32CPre<PRE>, 1> : VecAcc<AddF32C, 1> {};
 template <int PRE> struct VecAcc<AddF32CPre<PRE>, 2> : PackedF32C<1, PRE> {};
 template <int PRE> struct VecAcc<AddF32CPre<PRE>, 4> : PackedF32C<2, PRE> {};

@@ -238,3 +238,20 @@ def test_pair_up_sources_by_column_tiles(cuda_ok, dt):
             assert_matches(gx.matmul(g, V, UP).astype(ref.dtype), ref, scale, rtol=1e-6 if dt == np.float32 else 1e-12)
     finally:
         _pair_mode(0)
+
+
+@pytest.mark.parametrize("blocks,K", [(15, 2), (15, 7), (15, 52), (15, 56), (101, 4), (101, 8), (101, 96), (101, 100), (1, 130)])
+def test_pair_down_compensated_sums(cuda_ok, blocks, K):
+    """Compensated float32 over pattern rows with their error (blocks x columns up to 800, the last in tiles of
+    64 columns), one at a time, and pre-summed (from 10,000): within 1e-6 of sum |terms|."""
+    import grgl_gb300 as gx
+
+    _pair_mode(1)
+    try:
+        g, og = _both(gx, gx.window_tree_grg(2_002, blocks * 200, seed=3))
+        V = _rand(np.random.default_rng(K), np.float32, (K, g.num_mutations))
+        W = V.astype(np.float64)
+        assert_matches(gx.matmul(g, V, DOWN).astype(np.float64), oracle.matmul(og, W, DOWN),
+                       oracle.matmul(og, np.abs(W), DOWN), rtol=1e-6)
+    finally:
+        _pair_mode(0)
