@@ -825,7 +825,7 @@ def main():
         tf = json.loads(tfile.read_text())
         if tf.get("dram_bytes_per_step") and tf.get("graph", {}).get("edges"):
             traffic = tf["dram_bytes_per_step"] * E / tf["graph"]["edges"]
-            traffic_src = (f"ncu dram__bytes_read.sum + dram__bytes_write.sum over every sweep launch of one step on "
+            traffic_src = (f"ncu dram__bytes_read.sum + dram__bytes_write.sum over every traversal launch of one step on "
                            f"the N={tf['graph']['samples']}, M={tf['graph']['mutations']} graph "
                            f"(E={tf['graph']['edges']}), scaled by edges x{E / tf['graph']['edges']:.2f} "
                            "(profiles/sweep_traffic.json)")
