@@ -31,6 +31,7 @@ void set_down_split_mode(int mode);
 void set_staged(bool on);
 void set_pair_mode(int mode);
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
+const void* pair_analysis(grgx_graph* g);
 void* host_alloc(uint64_t bytes);
 void host_free(void* b);
 std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags);
@@ -465,6 +466,14 @@ extern "C" grgx_status grgx_debug_pair_counts(grgx_graph* g, int direction, uint
     return guarded([&] {
         GRGX_CHECK(g && out, GRGX_ERR_API_MISUSE, "null argument");
         grgx::pair_counts(g, direction == GRGX_DIRECTION_DOWN, out);
+    });
+}
+
+// Test hook (not part of the public header): where the pair form's analysis is held; null without one.
+extern "C" grgx_status grgx_debug_pair_analysis(grgx_graph* g, const void** out) {
+    return guarded([&] {
+        GRGX_CHECK(g && out, GRGX_ERR_API_MISUSE, "null argument");
+        *out = grgx::pair_analysis(g);
     });
 }
 

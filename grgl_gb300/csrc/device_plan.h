@@ -244,6 +244,8 @@ size_t pair_scratch_limit();
 void set_pair_mode(int mode);
 // out: height-0 nodes, blocks, patterns, height-0 edges of a direction in pair form (zeros: not in use).
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
+// Where the analysis that calls read without the graph's lock is held (null: none; tests).
+const void* pair_analysis(grgx_graph* g);
 // The launches of a DOWN call in pair form, sized for layout L: a table of pattern rows per range
 // of blocks, and per range the sums of its items.  With several ranges the first sum carries what
 // the ranges before added up.

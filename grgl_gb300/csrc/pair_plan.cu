@@ -649,6 +649,8 @@ void build_pair_plan(DevicePlan& d, bool down) {
         build_up_lists(d, tmp, patBase, counts, upAdj, upEdges, nodes);
         P.up_built = true;
     }
+    // (the second direction's build finds the same numbers: calls of the first one are reading them)
+    if (P.usable) return;
     P.h0 = h0;
     P.nblk = nblk;
     P.npat = npat;
@@ -681,6 +683,12 @@ void pair_counts(grgx_graph* g, bool down, uint64_t out[4]) {
     out[1] = built ? P.nblk : 0;
     out[2] = built ? P.npat : 0;
     out[3] = built ? low : 0;
+}
+
+const void* pair_analysis(grgx_graph* g) {
+    const DevicePlan* dp = ensure_device_plan(g);
+    std::lock_guard<std::mutex> lk(g->mu);
+    return dp->pair.usable ? dp->pair.pat_base.data() : nullptr;
 }
 
 void set_pair_mode(int mode) { g_pair_mode.store(mode); }

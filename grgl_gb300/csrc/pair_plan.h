@@ -50,6 +50,8 @@ struct PairBlock {
 struct PairPlan {
     bool tried = false;   // the analysis ran (once per graph)
     bool usable = false;  // ... and found the form worth using
+    // Written once, before `usable` is set: calls read these after use_pair_form has let go of the graph's
+    // lock, also while another thread's first call of the other direction builds that direction's arrays.
     long long h0 = 0;     // height-0 nodes (new ids 0 .. h0-1)
     long long nblk = 0;
     long long npat = 0;

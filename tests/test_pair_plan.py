@@ -1,0 +1,77 @@
+"""The life of a graph's pair form (pair_plan.h): what the first call of each direction builds and what it
+leaves alone, on several threads, and where it cannot be built."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+from tests.test_pair_form import DOWN, UP, _both, _check, _pair_mode, _rand
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def env(cuda_ok):
+    import grgl_gb300 as gx
+
+    _pair_mode(1)
+    gx.set_graph_replay(False)
+    try:
+        yield (gx, *_both(gx, gx.window_tree_grg(3001, 20300, seed=97), ploidy=1))
+    finally:
+        gx.set_graph_replay(True)
+        _pair_mode(0)
+
+
+def _analysis(g):
+    from grgl_gb300 import _lib
+
+    out = ctypes.c_void_p()
+    _lib.check(_lib.lib().grgx_debug_pair_analysis(g._h, ctypes.byref(out)))
+    return out.value
+
+
+def _input(g, direction, dt, K, seed=0):
+    return _rand(np.random.default_rng(seed), dt, (K, g.num_samples if direction == UP else g.num_mutations))
+
+
+@pytest.mark.parametrize("first", [DOWN, UP])
+def test_second_direction_leaves_the_analysis_in_place(env, first):
+    """Calls of the first direction read it without the graph's lock."""
+    gx, g, og = env
+    gx.matmul(g, _input(g, first, np.int32, 6), first)
+    before = _analysis(g)
+    assert before
+    V = _input(g, 3 - first, np.int32, 6)
+    _check(og, V, 3 - first, gx.matmul(g, V, 3 - first))
+    assert _analysis(g) == before
+
+
+@pytest.mark.parametrize("first", [DOWN, UP])
+def test_first_calls_of_both_directions_on_several_threads(env, first):
+    """Products of one direction run while another thread's first call builds the other."""
+    gx, g, og = env
+    gx.matmul(g, _input(g, first, np.float64, 3), first)  # this direction is built
+    started, errs = threading.Event(), []
+
+    def work(i):
+        try:
+            for k in range(6):
+                d = first if i else 3 - first
+                V = _input(g, d, (np.int32, np.float64)[i % 2], 3 + i, seed=10 * i + k)
+                if i:
+                    started.set()
+                else:
+                    started.wait()
+                _check(og, V, d, gx.matmul(g, V, d))
+        except Exception as e:  # reported below
+            errs.append(e)
+            started.set()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errs, errs
