@@ -32,6 +32,7 @@ void set_staged(bool on);
 void set_pair_mode(int mode);
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
 const void* pair_analysis(grgx_graph* g);
+long long set_plan_alloc(long long pass, long long refuse);
 void* host_alloc(uint64_t bytes);
 void host_free(void* b);
 std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags);
@@ -476,6 +477,10 @@ extern "C" grgx_status grgx_debug_pair_analysis(grgx_graph* g, const void** out)
         *out = grgx::pair_analysis(g);
     });
 }
+
+// Test hook (not part of the public header): lets `pass` more allocations of plan memory succeed and fails
+// the `refuse` after them as out of memory (pass -1: none); returns how many have failed since the last call.
+extern "C" long long grgx_debug_plan_alloc(long long pass, long long refuse) { return grgx::set_plan_alloc(pass, refuse); }
 
 grgx_status grgx_collect_timings(grgx_timing* out, uint64_t capacity, uint64_t* count) {
     return guarded([&] {

@@ -143,6 +143,31 @@ int max_tiles(const Layout& L);
 // K >= 4 eight-byte values) take the fine chunking, narrower rows -- whose chunks cost little
 // each, so that more of them only adds per-chunk work (the staged single-column passes lose
 // 10-20%) -- the coarse one.  The split copies' members are empty until they are built.
+// Device memory of a plan (cudaMalloc).  set_plan_alloc (tests): `pass` more allocations are made, `refuse`
+// after them fail as out of memory (pass -1: none fail); returns how many have failed since the last call.
+void* plan_alloc(size_t bytes);
+long long set_plan_alloc(long long pass, long long refuse);
+// What a build adds to a plan is handed over when it has succeeded: freed again unless kept.
+class PlanAddition {
+  public:
+    explicit PlanAddition(DevicePlan& d) : d_(d), count_(d.allocs.size()), bytes_(d.bytes) {}
+    ~PlanAddition() {
+        if (kept_) return;
+        for (size_t i = count_; i < d_.allocs.size(); i++) cudaFree(d_.allocs[i]);
+        d_.allocs.resize(count_);
+        d_.bytes = bytes_;
+    }
+    void keep() { kept_ = true; }
+    PlanAddition(const PlanAddition&) = delete;
+    PlanAddition& operator=(const PlanAddition&) = delete;
+
+  private:
+    DevicePlan& d_;
+    size_t count_;
+    uint64_t bytes_;
+    bool kept_ = false;
+};
+
 struct SweepCSRs {
     const DevCSR* up;
     const DevCSR* down;

@@ -36,14 +36,36 @@ void destroy_device_plan(DevicePlan* p) {
 }
 
 namespace {
+std::atomic<long long> g_alloc_pass{-1}, g_alloc_refuse{0}, g_alloc_refused{0};  // (tests)
+}
+
+void* plan_alloc(size_t bytes) {
+    if (g_alloc_pass.load() >= 0 && g_alloc_pass.fetch_sub(1) <= 0) {
+        g_alloc_pass.store(0);
+        if (g_alloc_refuse.fetch_sub(1) > 0) {
+            g_alloc_refused++;
+            throw Error(GRGX_ERR_OUT_OF_MEMORY, "plan memory refused by a test");
+        }
+    }
+    void* p = nullptr;
+    GRGX_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 1)));
+    return p;
+}
+
+long long set_plan_alloc(long long pass, long long refuse) {
+    g_alloc_refuse.store(refuse);
+    g_alloc_pass.store(pass);
+    return g_alloc_refused.exchange(0);
+}
+
+namespace {
 
 static_assert(sizeof(Chunk) == sizeof(ChunkDev), "chunk layout");
 static_assert(sizeof(HeavyRow) == sizeof(HeavyDev), "heavy layout");
 
 template <typename T> T* upload(DevicePlan& d, const std::vector<T>& v) {
     if (v.empty()) return nullptr;
-    void* p = nullptr;
-    GRGX_CUDA(cudaMalloc(&p, v.size() * sizeof(T)));
+    void* p = plan_alloc(v.size() * sizeof(T));
     d.allocs.push_back(p);
     d.bytes += v.size() * sizeof(T);
     GRGX_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));

@@ -37,8 +37,7 @@ constexpr long long kMaxPairs = 49152;
 struct Temps {
     std::vector<void*> ptrs;
     template <typename T> T* get(size_t count) {
-        void* p = nullptr;
-        GRGX_CUDA(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
+        void* p = plan_alloc(count * sizeof(T));
         ptrs.push_back(p);
         return static_cast<T*>(p);
     }
@@ -451,38 +450,41 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
 }
 
 // Everything about the form that needs one pass over the height-0 edges: the analysis on the first
-// call (which may find the form not worth using), and the arrays of the direction asked for.
-void build_pair_plan(DevicePlan& d, bool down) {
+// call, and the arrays of the direction asked for.  False: the form is not worth using, or impossible.
+// What a build that fails leaves behind is at most the finished analysis, for the next one.
+bool build_pair_plan(DevicePlan& d, bool down) {
     PairPlan& P = d.pair;
-    const bool first = !P.tried, forced = g_pair_mode.load() == 1;
-    P.tried = true;
-    if (d.num_levels < 2 || d.up_off.size() < 2) return;
+    const bool forced = g_pair_mode.load() == 1 || P.usable;
+    if (d.num_levels < 2 || d.up_off.size() < 2) return false;
     const long long h0 = static_cast<long long>(d.level_begin[1]);
     const long long n = static_cast<long long>(d.level_begin[d.num_levels]);
     const long long R = n - h0;
     // 16-bit matrix entries and 32-bit positions; small graphs stay as they are
-    if (d.up_off.back() < (forced ? 1 : kPairMinEdges) || h0 > 0x3fffffff) return;
+    if (d.up_off.back() < (forced ? 1 : kPairMinEdges) || h0 > 0x3fffffff) return false;
     const unsigned H = static_cast<unsigned>(h0);
     Temps tmp;
     const long long* dOff = reinterpret_cast<long long*>(tmp.copy(d.up_off));
-    if (first) {
-        P.low = count_low_children(d);
+    if (P.seq.empty()) {
+        std::vector<unsigned> low = count_low_children(d);
         std::vector<uint32_t> old2new(n);
         GRGX_CUDA(cudaMemcpy(old2new.data(), d.old2new, n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
         // the nodes with height-0 children, in original id order
+        std::vector<int> seq;
         for (long long v = 0; v < n; v++) {
             const long long r = static_cast<long long>(old2new[v]) - h0;
-            if (r >= 0 && P.low[r]) P.seq.push_back(static_cast<int>(r));
+            if (r >= 0 && low[r]) seq.push_back(static_cast<int>(r));
         }
+        P.low = std::move(low);
+        P.seq = std::move(seq);
     }
     const long long Q = static_cast<long long>(P.seq.size());
     std::vector<long long> cum(1, 0);
     for (int r : P.seq) cum.push_back(cum.back() + P.low[r]);
     const long long E0 = cum.back();
-    if (Q == 0 || E0 < (forced ? 1 : kPairMinEdges) || 2 * E0 < d.up_off.back()) return;
+    if (Q == 0 || E0 < (forced ? 1 : kPairMinEdges) || 2 * E0 < d.up_off.back()) return false;
     const int* dRow = tmp.copy(P.seq);
 
-    if (first) {
+    if (P.blocks.empty()) {
         // ---- runs: stretches of at least 6 average haplotype sets, one thread block each -----------
         const long long S =
             std::max<long long>(1, std::min<long long>({2LL * sm_count(), E0 / h0 / 6, (1LL << 30) / h0 + 1, Q}));
@@ -503,25 +505,28 @@ void build_pair_plan(DevicePlan& d, bool down) {
             GRGX_CUDA(cudaGetLastError());
             GRGX_CUDA(cudaMemcpy(pv.data(), dPv, Q * sizeof(int), cudaMemcpyDeviceToHost));
         }
-        P.run = cut_runs(pv);
+        std::vector<int> run = cut_runs(pv);
         // ---- blocks --------------------------------------------------------------------------------
-        const int nruns = static_cast<int>(P.run.size()) - 1;
+        const int nruns = static_cast<int>(run.size()) - 1;
+        std::vector<PairBlock> blocks;
         for (int r = 0; r < nruns;) {
-            PairBlock B{r, P.run[r], 0, P.run[r + 1] - P.run[r], 0};
-            if (r + 1 < nruns && (B.n0 + 1LL) * (P.run[r + 2] - P.run[r + 1] + 1) <= kMaxPairs) {
-                B.q1 = P.run[r + 1];
-                B.n1 = P.run[r + 2] - P.run[r + 1];
+            PairBlock B{r, run[r], 0, run[r + 1] - run[r], 0};
+            if (r + 1 < nruns && (B.n0 + 1LL) * (run[r + 2] - run[r + 1] + 1) <= kMaxPairs) {
+                B.q1 = run[r + 1];
+                B.n1 = run[r + 2] - run[r + 1];
             }
             r += B.n1 ? 2 : 1;
-            P.blocks.push_back(B);
+            blocks.push_back(B);
         }
+        P.run = std::move(run);
+        P.blocks = std::move(blocks);
     }
     const std::vector<int>& run = P.run;
     const std::vector<PairBlock>& blocks = P.blocks;
     const int nruns = static_cast<int>(run.size()) - 1;
     const long long nblk = static_cast<long long>(blocks.size());
     const double edges = static_cast<double>(E0);
-    if (!forced && static_cast<double>(nblk) * h0 > kPairMaxCost * edges) return;
+    if (!forced && static_cast<double>(nblk) * h0 > kPairMaxCost * edges) return false;
 
     // ---- patterns, a batch of blocks at a time -------------------------------------------------------
     std::vector<int> runOf(Q), seqNode(Q);
@@ -589,7 +594,7 @@ void build_pair_plan(DevicePlan& d, bool down) {
         if (patBase.back() >= 0x7fffffffLL ||
             (!forced && b0 == 0 && nb * h0 + kPairPatternCost * static_cast<double>(total) >
                                        kPairMaxCost * static_cast<double>(cum[run[run1]] - cum[run[run0]])))
-            return;
+            return false;
         GRGX_CUDA(cudaMemcpy(dBase, rel.data(), nb * sizeof(unsigned), cudaMemcpyHostToDevice));
         out.patBase = dBase;
         parts.push_back({tmp.get<uint2>(total), total});
@@ -621,9 +626,9 @@ void build_pair_plan(DevicePlan& d, bool down) {
     unsigned long long set = 0;
     GRGX_CUDA(cudaMemcpy(&set, dSet, sizeof(set), cudaMemcpyDeviceToHost));
     // every edge has its entry: no height-0 node has two parents in one run, or the same one twice
-    if (static_cast<long long>(set) != E0) return;
+    if (static_cast<long long>(set) != E0) return false;
     const long long npat = patBase.back();
-    if (!forced && nblk * h0 + kPairPatternCost * static_cast<double>(npat) > kPairMaxCost * edges) return;
+    if (!forced && nblk * h0 + kPairPatternCost * static_cast<double>(npat) > kPairMaxCost * edges) return false;
 
     uint2* nodes = tmp.get<uint2>(npat);
     long long at = 0;
@@ -650,12 +655,13 @@ void build_pair_plan(DevicePlan& d, bool down) {
         P.up_built = true;
     }
     // (the second direction's build finds the same numbers: calls of the first one are reading them)
-    if (P.usable) return;
+    if (P.usable) return true;
     P.h0 = h0;
     P.nblk = nblk;
     P.npat = npat;
     P.pat_base = std::move(patBase);
     P.usable = true;
+    return true;
 }
 
 }  // namespace
@@ -704,18 +710,21 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
     if (!down && L.stride == 1 && (L.kind == Kind::F32C || (staged_layout(L) && up_split_possible(dp)))) return false;
     std::lock_guard<std::mutex> lk(g->mu);
     PairPlan& P = dp->pair;
-    bool& built = down ? P.down_built : P.up_built;
-    if (!P.tried || (P.usable && !built)) {
+    bool& tried = down ? P.down_tried : P.up_tried;
+    for (int attempt = 0; attempt < 2 && !tried && !P.refused; attempt++) {
         try {
-            build_pair_plan(*dp, down);
+            P.refused = !build_pair_plan(*dp, down);
+            tried = true;
         } catch (const Error& e) {
-            // no memory for it: the other forms need none of this
+            tried = e.code != GRGX_ERR_OUT_OF_MEMORY || attempt > 0;
             if (e.code != GRGX_ERR_OUT_OF_MEMORY) throw;
             cudaGetLastError();
-            P.usable = P.usable && (P.down_built || P.up_built);
+            // Once more with the memory the pool keeps between calls.  Then the direction stays with the
+            // other forms, which need none of this: every further call would wait for the same failure.
+            if (!tried) trim_pool();
         }
     }
-    return P.usable && built;
+    return down ? P.down_built : P.up_built;
 }
 
 }  // namespace grgx

@@ -48,8 +48,9 @@ struct PairBlock {
 };
 
 struct PairPlan {
-    bool tried = false;   // the analysis ran (once per graph)
-    bool usable = false;  // ... and found the form worth using
+    bool refused = false;  // the analysis found the form not worth using (decided once per graph)
+    bool usable = false;   // ... or worth it, and the arrays of some direction are built
+    bool down_tried = false, up_tried = false;  // a build of the direction has succeeded or failed for good
     // Written once, before `usable` is set: calls read these after use_pair_form has let go of the graph's
     // lock, also while another thread's first call of the other direction builds that direction's arrays.
     long long h0 = 0;     // height-0 nodes (new ids 0 .. h0-1)

@@ -179,8 +179,7 @@ DevCSR upload_pull(DevicePlan& d, const PullCSR& P, void* adj, long long E, cons
                    const std::vector<long long>* blockRows) {
     auto up = [&](const auto& v) -> void* {
         if (v.empty()) return nullptr;
-        void* p = nullptr;
-        BL_CUDA(cudaMalloc(&p, v.size() * sizeof(v[0])));
+        void* p = plan_alloc(v.size() * sizeof(v[0]));
         d.allocs.push_back(p);
         d.bytes += v.size() * sizeof(v[0]);
         BL_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
@@ -275,6 +274,7 @@ long long block_layout(PullCSR& P0, const std::vector<uint32_t>& seg, long long 
 // Internal edges: one level per UP level (heights 1..H-1), plus the finish lists.
 void build_up_internal(DevicePlan& d, const std::vector<unsigned>& low) {
     if (d.up_int_built) return;
+    PlanAddition added(d);
     const long long src0 = static_cast<long long>(d.level_begin[1]);
     const long long R = static_cast<long long>(d.level_begin[d.num_levels]) - src0;
     const std::vector<int64_t>& off = d.up_off;
@@ -306,10 +306,10 @@ void build_up_internal(DevicePlan& d, const std::vector<unsigned>& low) {
     const long long EI = offI.back();
     void *dOff = nullptr, *dDst = nullptr, *out = nullptr, *dFin = nullptr;
     try {
-        BL_CUDA(cudaMalloc(&dOff, (R + 1) * sizeof(long long)));
-        BL_CUDA(cudaMalloc(&dDst, std::max<long long>(R, 1) * sizeof(long long)));
-        BL_CUDA(cudaMalloc(&out, std::max<long long>(EI, 1) * sizeof(uint32_t)));
-        BL_CUDA(cudaMalloc(&dFin, std::max<size_t>(fin.size(), 1) * sizeof(int)));
+        dOff = plan_alloc((R + 1) * sizeof(long long));
+        dDst = plan_alloc(R * sizeof(long long));
+        out = plan_alloc(static_cast<size_t>(EI) * sizeof(uint32_t));
+        dFin = plan_alloc(fin.size() * sizeof(int));
         BL_CUDA(cudaMemcpy(dOff, off.data(), (R + 1) * sizeof(long long), cudaMemcpyHostToDevice));
         BL_CUDA(cudaMemcpy(dDst, dstI.data(), R * sizeof(long long), cudaMemcpyHostToDevice));
         if (!fin.empty()) BL_CUDA(cudaMemcpy(dFin, fin.data(), fin.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -333,6 +333,7 @@ void build_up_internal(DevicePlan& d, const std::vector<unsigned>& low) {
     d.fin = static_cast<int*>(dFin);
     d.fin_begin = finBegin;
     d.up_int_built = true;
+    added.keep();
 }
 
 namespace {

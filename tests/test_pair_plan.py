@@ -75,3 +75,55 @@ def test_first_calls_of_both_directions_on_several_threads(env, first):
     for t in threads:
         t.join()
     assert not errs, errs
+
+
+def _refuse(skip, count):
+    """Fails `count` allocations of plan memory after `skip` more; returns how many have failed since the last call."""
+    from grgl_gb300 import _lib
+
+    fn = _lib.lib().grgx_debug_plan_alloc
+    fn.restype = ctypes.c_longlong
+    fn.argtypes = [ctypes.c_longlong, ctypes.c_longlong]
+    return fn(skip, count)
+
+
+def _built(g, direction):
+    from grgl_gb300 import _lib
+
+    out = (ctypes.c_uint64 * 4)()
+    _lib.check(_lib.lib().grgx_debug_pair_counts(g._h, direction, out))
+    return out[1] > 0
+
+
+@pytest.mark.parametrize("second", [False, True])
+@pytest.mark.parametrize("direction", [DOWN, UP])
+def test_out_of_memory_in_a_build(env, direction, second):
+    """Every allocation of a build fails in turn: once, and the build is made again; then for good, and calls of
+    the direction take the other forms, without building again or keeping memory."""
+    gx, g, og = env
+    V, W = (_input(g, d, np.int32, 6) for d in (direction, 3 - direction))
+    a = g.export_arrays()
+    skip, failed, kept = 0, True, set()
+    while failed:
+        for count in (1, 1 << 40):
+            h = gx.from_csr(g.num_samples, 1, a["down_off"], a["down_adj"], a["mut_node"]).upload()
+            if second:
+                gx.matmul(h, W, 3 - direction)
+            bytes0 = h.info()["device_bytes"]
+            try:
+                _refuse(skip, count)
+                _check(og, V, direction, gx.matmul(h, V, direction))
+                failed = _refuse(skip, count)
+                assert failed <= 2
+                assert _built(h, direction) == (failed < 2)
+                if failed == 2:
+                    kept.add(h.info()["device_bytes"] - bytes0)
+                _check(og, V, direction, gx.matmul(h, V, direction))
+                assert _refuse(-1, 0) == 0
+            finally:
+                _refuse(-1, 0)
+            _check(og, W, 3 - direction, gx.matmul(h, W, 3 - direction))
+            assert _built(h, 3 - direction)
+        skip += 1
+    # (the UP edges between inner nodes, once complete, serve the split form too)
+    assert skip > 10 and 0 in kept and len(kept) == (1 if direction == DOWN else 2)
