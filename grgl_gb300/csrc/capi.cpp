@@ -32,6 +32,7 @@ void set_staged(bool on);
 void set_pair_mode(int mode);
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
 const void* pair_analysis(grgx_graph* g);
+void set_pair_rows(long long most);
 long long set_plan_alloc(long long pass, long long refuse);
 void* host_alloc(uint64_t bytes);
 void host_free(void* b);
@@ -477,6 +478,9 @@ extern "C" grgx_status grgx_debug_pair_analysis(grgx_graph* g, const void** out)
         *out = grgx::pair_analysis(g);
     });
 }
+
+// Test hook (not part of the public header): UP keeps the other forms from this many rows of pair tables on.
+extern "C" void grgx_debug_pair_rows(long long most) { grgx::set_pair_rows(most); }
 
 // Test hook (not part of the public header): lets `pass` more allocations of plan memory succeed and fails
 // the `refuse` after them as out of memory (pass -1: none); returns how many have failed since the last call.

@@ -267,6 +267,7 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
 // server's worker lowers it to what its batch has reserved (PairScratchScope).
 size_t pair_scratch_limit();
 void set_pair_mode(int mode);
+void set_pair_rows(long long most);  // UP table rows from which that direction keeps the other forms (tests)
 // out: height-0 nodes, blocks, patterns, height-0 edges of a direction in pair form (zeros: not in use).
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
 // Where the analysis that calls read without the graph's lock is held (null: none; tests).

@@ -28,6 +28,7 @@ namespace grgx {
 namespace {
 
 std::atomic<int> g_pair_mode{0};  // 0 by the rules below, 1 wherever possible, 2 never
+std::atomic<long long> g_most_rows{kPairMostRows};
 
 constexpr int kThreads = 1024;
 // Possible pairs of one block: a counter each in shared memory (192 KB).
@@ -291,8 +292,9 @@ void sort_pairs(Temps& tmp, unsigned*& keys, unsigned*& vals, unsigned* keys2, u
     tmp.release(t);
 }
 
-// The UP lists, by segments: the patterns' pieces (a table row each), the nodes' table rows.
-void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& patBase, const std::vector<unsigned>& counts,
+// The UP lists, by segments: the patterns' pieces (a table row each), the nodes' table rows.  False: more
+// rows than lists can number.
+bool build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& patBase, const std::vector<unsigned>& counts,
                     uint32_t* patAdj, long long patEdges, const uint2* nodes) {
     PairPlan& P = d.pair;
     const long long h0 = static_cast<long long>(d.level_begin[1]);
@@ -364,7 +366,8 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
         segments[s + 1].top0 += segments[s].top0;
     }
     const long long rows = segments.back().row0, ne = nedge0.back();
-    GRGX_CHECK(edge0.back() == patEdges && rows < 0x3fffffffLL, GRGX_ERR_UNSUPPORTED, "pair form too large");
+    GRGX_CHECK(edge0.back() == patEdges, GRGX_ERR_CUDA, "pair form edge count mismatch");
+    if (rows >= g_most_rows.load()) return false;
     std::vector<PairList> patLists(segments.back().pat0), nodeLists(segments.back().node0), topLists(segments.back().top0);
     std::vector<uint2> rowNodes(rows, uint2{INVALID_NODE, INVALID_NODE});
     std::vector<uint32_t> topAdj(sub0.back());
@@ -447,10 +450,12 @@ void build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
         tmp.keep(d, P.few_adj, fewEdges * sizeof(uint32_t));
     }
     P.segments = std::move(segments);
+    return true;
 }
 
 // Everything about the form that needs one pass over the height-0 edges: the analysis on the first
-// call, and the arrays of the direction asked for.  False: the form is not worth using, or impossible.
+// call, and the arrays of the direction asked for (none where only that direction is too large for them).
+// False: the form is not worth using, or impossible.
 // What a build that fails leaves behind is at most the finished analysis, for the next one.
 bool build_pair_plan(DevicePlan& d, bool down) {
     PairPlan& P = d.pair;
@@ -651,7 +656,7 @@ bool build_pair_plan(DevicePlan& d, bool down) {
         P.down_built = true;
     } else {
         build_up_internal(d, P.low);
-        build_up_lists(d, tmp, patBase, counts, upAdj, upEdges, nodes);
+        if (!build_up_lists(d, tmp, patBase, counts, upAdj, upEdges, nodes)) return true;
         P.up_built = true;
     }
     // (the second direction's build finds the same numbers: calls of the first one are reading them)
@@ -696,6 +701,8 @@ const void* pair_analysis(grgx_graph* g) {
     std::lock_guard<std::mutex> lk(g->mu);
     return dp->pair.usable ? dp->pair.pat_base.data() : nullptr;
 }
+
+void set_pair_rows(long long most) { g_most_rows.store(most); }
 
 void set_pair_mode(int mode) { g_pair_mode.store(mode); }
 

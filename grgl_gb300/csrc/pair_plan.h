@@ -38,6 +38,8 @@ constexpr long long kPairPiece = 256;
 // 6.0e-8 as in the sweep (N=200,000, M=250,000, K=8, N(0,1) inputs; float64 7.7e-15 and 3.7e-15).  They hold few
 // of the edges: 1277 and 1261 us there, float32 K=40 3052 and 3065, N=20,000, M=50,000 203 and 208.
 constexpr unsigned kPairFew = 32;
+// UP: a list's destination row, or the complement of a table row, is an int.
+constexpr long long kPairMostRows = 0x3fffffff;
 // Blocks whose lists are sorted by length together, longest first (the order they are launched in).
 constexpr long long kPairSegment = 64;
 

@@ -127,3 +127,22 @@ def test_out_of_memory_in_a_build(env, direction, second):
         skip += 1
     # (the UP edges between inner nodes, once complete, serve the split form too)
     assert skip > 10 and 0 in kept and len(kept) == (1 if direction == DOWN else 2)
+
+
+@pytest.mark.parametrize("first", [DOWN, UP])
+def test_more_table_rows_than_lists_can_number(env, first):
+    """UP takes another form then; DOWN, whose patterns have no such rows, keeps the pair form."""
+    from grgl_gb300 import _lib
+
+    gx, g, og = env
+    fn = _lib.lib().grgx_debug_pair_rows
+    fn.restype = None
+    fn.argtypes = [ctypes.c_longlong]
+    fn(1000)
+    try:
+        for direction in (first, 3 - first):
+            V = _input(g, direction, np.int32, 6)
+            _check(og, V, direction, gx.matmul(g, V, direction))
+            assert _built(g, direction) == (direction == DOWN)
+    finally:
+        fn(0x3fffffff)
