@@ -1,7 +1,10 @@
 // The C ABI (include/grgx.h): exception-free wrappers over the host graph, the plan and the
 // matmul orchestration.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
+#include <functional>
+#include <new>
 #include <string>
 
 #include "grgx_internal.h"
@@ -476,6 +479,19 @@ extern "C" grgx_status grgx_debug_pair_analysis(grgx_graph* g, const void** out)
     return guarded([&] {
         GRGX_CHECK(g && out, GRGX_ERR_API_MISUSE, "null argument");
         *out = grgx::pair_analysis(g);
+    });
+}
+
+// Test hook (not part of the public header): n items on the build's host threads, adding their numbers to *sum;
+// item `fails` throws bad_alloc.
+extern "C" grgx_status grgx_debug_run_threads(long long n, long long fails, long long* sum) {
+    return guarded([&] {
+        std::atomic<long long> s{0};
+        grgx::run_threads(n, [&](long long i) {
+            if (i == fails) throw std::bad_alloc();
+            s += i;
+        });
+        *sum = s;
     });
 }
 

@@ -3,6 +3,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
@@ -125,6 +126,10 @@ struct HostPlan {
 };
 
 std::unique_ptr<HostPlan> build_plan(const HostGraph& g);
+
+// fn(0) .. fn(n - 1) on up to 32 host threads; what the first failing one throws is thrown here, when all threads
+// have ended (a thread that cannot be started leaves its share to this one).
+void run_threads(long long n, const std::function<void(long long)>& fn);
 
 // Stages of the plan shared by the host builder (build_plan) and the device builder
 // (plan_device.cu), which computes heights, the renumbering, the UP adjacency and the parent

@@ -18,7 +18,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cub/device/device_radix_sort.cuh>
-#include <thread>
+#include <new>
 #include <vector>
 
 #include "device_plan.h"
@@ -319,16 +319,6 @@ bool build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
         return s * kPairSegment < nblk ? static_cast<long long>(P.blocks[s * kPairSegment].q0) : Q;
     };
     auto pieces_of = [](long long c) { return (c + kPairPiece - 1) / kPairPiece; };
-    auto threaded = [&](auto&& fn) {
-        const long long T = std::min<long long>(nseg, std::max(1u, std::min(32u, std::thread::hardware_concurrency())));
-        std::vector<std::thread> pool;
-        for (long long t = 1; t < T; t++)
-            pool.emplace_back([&, t] {
-                for (long long s = t; s < nseg; s += T) fn(s);
-            });
-        for (long long s = 0; s < nseg; s += T) fn(s);
-        for (std::thread& th : pool) th.join();
-    };
     // position of each UP row in the sequence; a node's patterns are all of its own segment
     std::vector<unsigned> posOf(d.up_off.size(), 0);
     for (long long q = 0; q < Q; q++) posOf[P.seq[q]] = static_cast<unsigned>(q);
@@ -337,7 +327,7 @@ bool build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
     std::vector<PairPlan::Segment> segments(nseg + 1);
     std::vector<long long> edge0(nseg + 1, 0), sub0(nseg + 1, 0), nedge0(nseg + 1, 0);
     std::vector<unsigned> deg(Q, 0);
-    threaded([&](long long s) {
+    run_threads(nseg, [&](long long s) {
         PairPlan::Segment& next = segments[s + 1];
         for (long long p = first_pattern(s); p < first_pattern(s + 1); p++) {
             const long long n = pieces_of(counts[p]);
@@ -371,7 +361,7 @@ bool build_up_lists(DevicePlan& d, Temps& tmp, const std::vector<long long>& pat
     std::vector<PairList> patLists(segments.back().pat0), nodeLists(segments.back().node0), topLists(segments.back().top0);
     std::vector<uint2> rowNodes(rows, uint2{INVALID_NODE, INVALID_NODE});
     std::vector<uint32_t> topAdj(sub0.back());
-    threaded([&](long long s) {
+    run_threads(nseg, [&](long long s) {
         const PairPlan::Segment& a = segments[s];
         long long e = edge0[s], row = a.row0, at = a.pat0;
         auto cut = [](PairList* out, long long e, long long c, long long n, long long i, int dst) {
@@ -720,14 +710,16 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
     bool& tried = down ? P.down_tried : P.up_tried;
     for (int attempt = 0; attempt < 2 && !tried && !P.refused; attempt++) {
         try {
-            P.refused = !build_pair_plan(*dp, down);
             tried = true;
+            P.refused = !build_pair_plan(*dp, down);
+        } catch (const std::bad_alloc&) {
+            // host memory: the other forms need little of it
         } catch (const Error& e) {
-            tried = e.code != GRGX_ERR_OUT_OF_MEMORY || attempt > 0;
             if (e.code != GRGX_ERR_OUT_OF_MEMORY) throw;
             cudaGetLastError();
             // Once more with the memory the pool keeps between calls.  Then the direction stays with the
             // other forms, which need none of this: every further call would wait for the same failure.
+            tried = attempt > 0;
             if (!tried) trim_pool();
         }
     }

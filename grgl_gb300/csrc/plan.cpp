@@ -16,9 +16,11 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <exception>
 #include <cstdio>
 #include <cstdlib>
 #include <functional>
+#include <mutex>
 #include <numeric>
 #include <thread>
 
@@ -47,6 +49,32 @@ void parallel_for(uint64_t n, const std::function<void(uint64_t, uint64_t, int)>
 }
 
 }  // namespace
+
+void run_threads(long long n, const std::function<void(long long)>& fn) {
+    std::atomic<long long> next{0};
+    std::mutex mu;
+    std::exception_ptr failed;
+    auto work = [&] {
+        for (long long i; (i = next.fetch_add(1)) < n;) {
+            try {
+                fn(i);
+            } catch (...) {
+                std::lock_guard<std::mutex> lk(mu);
+                if (!failed) failed = std::current_exception();
+                next.store(n);
+            }
+        }
+    };
+    std::vector<std::thread> pool;
+    const long long threads = std::min<long long>(n, std::min(host_threads(), 32));
+    try {
+        for (long long t = 1; t < threads; t++) pool.emplace_back(work);
+    } catch (...) {
+    }
+    work();
+    for (std::thread& th : pool) th.join();
+    if (failed) std::rethrow_exception(failed);
+}
 
 // Chunk target (the coarse chunking): SMs x 128 chunks per level -- about four per resident warp
 // of the sweep kernel (32 warps per SM) -- never fewer than 64 edges per chunk; the fine chunking
