@@ -275,6 +275,7 @@ long long block_layout(PullCSR& P0, const std::vector<uint32_t>& seg, long long 
 void build_up_internal(DevicePlan& d, const std::vector<unsigned>& low) {
     if (d.up_int_built) return;
     PlanAddition added(d);
+    const PlanDeviceScope planSms(sm_count());
     const long long src0 = static_cast<long long>(d.level_begin[1]);
     const long long R = static_cast<long long>(d.level_begin[d.num_levels]) - src0;
     const std::vector<int64_t>& off = d.up_off;
