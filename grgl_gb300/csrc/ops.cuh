@@ -128,7 +128,7 @@ struct AddF32C {
 };
 
 // The same with PRE edges pre-summed in plain float32 where the sweep's block path pre-sums
-// kF32PreSum (vecacc.cuh).
+// kF32PreSum (1: none are), or kF32Ordered (vecacc.cuh).
 template <int PRE> struct AddF32CPre : AddF32C {};
 // ... and with pattern rows that keep the error of their sum (DOWN in pair form).
 struct AddF32CX : AddF32C {};

@@ -27,7 +27,7 @@ template <> struct PairPart<AddF64SD> {
 };
 
 // Pattern row elements.  A pair of rows is summed in storage precision: compensated float32 rounds
-// it once, like the first level of the sweep's plain pre-sums (vecacc.cuh); float pairs keep 48
+// it once, which takes the place of the sweep's plain pre-sums (vecacc.cuh); float pairs keep 48
 // bits.  A single compensated column, and the columns of short rows (AddF32CX), have no pre-sums in the
 // sweep and keep the pair's error here.
 template <class Op, int VW> struct PairTable {
@@ -308,6 +308,8 @@ template <class Op, int VW, int G> void pair_down_as(PairDownParams<typename Op:
     GRGX_PAIR_CASE(OP, VWV, 10)
 #define GRGX_PAIR4(OP)                                                                              \
     GRGX_PAIR_CASE(OP, 1, 1)                                                                        \
+    GRGX_PAIR_WIDE4(OP)
+#define GRGX_PAIR_WIDE4(OP)                                                                         \
     GRGX_PAIR_CASE(OP, 2, 1)                                                                        \
     GRGX_PAIR_CASE(OP, 4, 1)                                                                        \
     GRGX_PAIR_CASE(OP, 4, 2)                                                                        \

@@ -85,19 +85,22 @@ __global__ void pair_source_kernel(const uint4* __restrict__ src, long long rows
 
 // How compensated float32 adds DOWN pattern rows.  The sweep pre-sums four edges only in batches of
 // edges without a row start, so the shorter the rows (two edges per block) and the fewer the columns, the
-// fewer plain additions its sums pass.  Norm of the error against float64, 1e-8 of the norm, N(0,1) inputs, sweep
-// / rounded pattern rows pre-summed / one at a time / with their error:
-//   200,000 samples and 3,000 variants (15 blocks), K=8 5.4 / 6.4 / 5.8 / 5.2, K=64 6.1 / 6.3 / 5.7 / -
-//   100,000 and 20,000 (100),    K=4 5.7 / 6.9 / 6.2 / 5.1, K=32 6.3 / 6.6 / 5.8 / -, K=64 6.4 / 6.5 / 5.8 / -
-//   200,000 and 250,000 (1,250), K=8 6.4 / 6.5 / 5.8 / -,   K=16 6.5 / 6.5 / 5.9 / -, K=64 6.4 / 6.3 / - / -
-// Microseconds: 100,000 and 20,000 K=8 240 / 92 / 90 / 105, K=64 662 / 239 / 279 / -; 200,000 and 250,000 K=8 2260 /
-// 850 / 858 / -, K=16 2757 / 1166 / 1329 / -.  The kind that stays at or below the sweep's error is taken.
-enum class DownSums { kPreSum, kSingle, kExact };
+// fewer plain additions its sums pass.  Norm of the error against float64, 1e-8 of the norm, sweep / rounded
+// pattern rows by FastTwoSum / by TwoSum / rows with their error; N(0,1) inputs, then standardized products:
+//   200,000 samples and 3,000 variants (15 blocks), K=48 5.9 / - / - / 4.9 and 6.38 / - / - / 5.77, K=64 5.9 / - /
+//     5.6 / - and 6.39 / - / 6.42 / -
+//   200,000 and 10,000 (50),     K=18 6.0 / 5.7 / 5.6 / - and 7.17 / 7.35 / 7.12 / -
+//   100,000 and 20,000 (100),    K=12 6.5 / 6.1 / 6.0 / - and 7.36 / 7.45 / 7.28 / -, K=100 6.8 / 5.9 / - / - and 8.2 / 7.5
+//   200,000 and 250,000 (1,250), K=6 6.5 / - / 6.0 / - and 8.2 / - / 7.5 / -, K=12 6.4 / 5.8 / 5.9 / - and 8.2 / 7.6 / - / -
+// Microseconds: 100,000 and 20,000 K=8 240 / - / 90 / 105, K=64 662 / 231 / 274 / -; 200,000 and 250,000 K=8 2260 / - /
+// 858 / -, K=16 2757 / 1147 / 1329 / -.  The fastest kind that stays at or below the sweep's error in both is
+// taken.  (Two rows pre-summed before a TwoSum take as long as two FastTwoSums and leave 6.4 where those leave 5.8.)
+enum class DownSums { kOrdered, kSingle, kExact };
 DownSums down_sums(const Layout& L, const PairPlan& P) {
-    if (L.kind != Kind::F32C || L.vw == 1) return DownSums::kPreSum;
+    if (L.kind != Kind::F32C || L.vw == 1) return DownSums::kOrdered;
     const long long work = P.nblk * L.stride;
-    if (work <= 800) return DownSums::kExact;
-    return work < 10000 || L.stride <= 8 ? DownSums::kSingle : DownSums::kPreSum;
+    if (work <= 1000) return DownSums::kExact;
+    return work < 10000 || L.stride <= 8 ? DownSums::kSingle : DownSums::kOrdered;
 }
 
 // The layout that the DOWN pair kernels run with: pattern rows with their error take two columns a lane.

@@ -175,6 +175,11 @@ template <> struct VecAcc<AddF64S, 1> {
 // u = 2^-24, for a quarter of the TwoSums of one per edge; steps with a row boundary keep one
 // TwoSum per edge.
 constexpr int kF32PreSum = 4;
+// No pre-sum: a FastTwoSum (Dekker, Numer. Math. 18, 1971) of running sum and addend per edge, four
+// operations as one of two edges behind a pre-sum has.  Its error term is exact where the sum is not the
+// smaller of the two -- nearly always once a few edges are in it -- and otherwise off by at most the rounding
+// that a plain addition has.
+constexpr int kF32Ordered = 0;
 
 // Compensated float32, columns in pairs; PRE edges are pre-summed in add_block.
 template <int NP, int PRE = kF32PreSum> struct PackedF32C {
@@ -193,40 +198,41 @@ template <int NP, int PRE = kF32PreSum> struct PackedF32C {
 #pragma unroll
         for (int j = 0; j < NP; j++) add_pair2(j, make_float2(v[2 * j], v[2 * j + 1]));
     }
+    __device__ __forceinline__ void add_ordered(const float* v) {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            const float2 x = make_float2(v[2 * j], v[2 * j + 1]), s = add2(hi[j], x);
+            lo[j] = add2(lo[j], sub2(x, sub2(s, hi[j])));
+            hi[j] = s;
+        }
+    }
     template <int N> __device__ __forceinline__ void add_block(const float (*v)[2 * NP]) {
-        static_assert(N % PRE == 0 && (PRE == 1 || PRE == 2 || PRE == 4), "block of whole pre-sums");
+        if constexpr (PRE == kF32PreSum) {
+            static_assert(N % PRE == 0 && PRE == 4, "block of whole pre-sums");
 #pragma unroll
-        for (int u = 0; u < N; u += PRE) {
+            for (int u = 0; u < N; u += PRE) {
 #pragma unroll
-            for (int j = 0; j < NP; j++) {
-                float2 t = make_float2(v[u][2 * j], v[u][2 * j + 1]);
-                if constexpr (PRE == 2) {
-                    t = add2(t, make_float2(v[u + 1][2 * j], v[u + 1][2 * j + 1]));
-                } else if constexpr (PRE == 4) {
+                for (int j = 0; j < NP; j++) {
+                    const float2 a = make_float2(v[u][2 * j], v[u][2 * j + 1]);
                     const float2 b = make_float2(v[u + 1][2 * j], v[u + 1][2 * j + 1]);
                     const float2 c = make_float2(v[u + 2][2 * j], v[u + 2][2 * j + 1]);
                     const float2 d = make_float2(v[u + 3][2 * j], v[u + 3][2 * j + 1]);
-                    t = add2(add2(t, b), add2(c, d));
+                    add_pair2(j, add2(add2(a, b), add2(c, d)));
                 }
-                add_pair2(j, t);
+            }
+        } else {
+            static_assert(PRE == 1 || PRE == kF32Ordered, "no other pre-sums");
+#pragma unroll
+            for (int u = 0; u < N; u++) {
+                if constexpr (PRE == 1) add(v[u]);
+                else add_ordered(v[u]);
             }
         }
     }
-    // Four pattern rows, each the rounded sum of two edges: two at a time in plain float32, so the
-    // edges pass the same two rounding levels before a TwoSum as four edges do in add_block (PRE 1: one at a time).
+    // Four pattern rows of the pair form, each the rounded sum of two edges.
     __device__ __forceinline__ void add_pairs(const float (*v)[2 * NP]) {
-#pragma unroll
-        for (int u = 0; u < 4; u += 2) {
-            if constexpr (PRE == 1) {
-                add(v[u]);
-                add(v[u + 1]);
-                continue;
-            }
-#pragma unroll
-            for (int j = 0; j < NP; j++)
-                add_pair2(j, add2(make_float2(v[u][2 * j], v[u][2 * j + 1]),
-                                  make_float2(v[u + 1][2 * j], v[u + 1][2 * j + 1])));
-        }
+        static_assert(PRE == 1 || PRE == kF32Ordered, "a pattern row is a pre-sum already");
+        add_block<4>(v);
     }
     __device__ __forceinline__ void merge(const PackedF32C& o) {
 #pragma unroll

@@ -1,0 +1,58 @@
+"""Compensated float32 in pair form is at least as near to the float64 product as the sweep over edges, which
+the pair form takes the place of: the norm of the error over all outputs, plain and standardized products."""
+import numpy as np
+import pytest
+
+from tests.test_pair_form import DOWN, UP, _pair_mode
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def graphs(cuda_ok):
+    import grgl_gb300 as gx
+
+    made = {}
+
+    def get(N, M):
+        if (N, M) not in made:
+            made.clear()
+            made[N, M] = gx.window_tree_grg(N, M, seed=42).upload()
+        return made[N, M]
+
+    gx.set_graph_replay(False)
+    try:
+        yield gx, get
+    finally:
+        gx.set_graph_replay(True)
+        _pair_mode(0)
+
+
+# blocks x columns of every kind of DOWN sum (pair_run.cu), and the narrow and wide ends of UP
+@pytest.mark.parametrize("N,M,direction,K", [
+    (20_000, 250_000, DOWN, 6), (20_000, 250_000, DOWN, 9), (20_000, 250_000, DOWN, 12), (20_000, 250_000, DOWN, 24),
+    (20_000, 250_000, UP, 2), (20_000, 250_000, UP, 6), (20_000, 250_000, UP, 33),
+    (100_000, 20_000, DOWN, 12), (100_000, 20_000, DOWN, 100), (200_000, 3_000, DOWN, 48), (200_000, 3_000, DOWN, 64)])
+@pytest.mark.parametrize("standardized", [False, True])
+def test_errors_at_or_below_the_sweeps(graphs, N, M, direction, K, standardized):
+    import torch
+
+    gx, get = graphs
+    g = get(N, M)
+    product = gx.matmul_standardized if standardized else gx.matmul
+
+    def error(mode, x, exact):
+        _pair_mode(mode)
+        got = product(g, x, direction).double()
+        return float((got - exact).square().sum()), float(exact.square().sum())
+
+    total = {1: 0.0, 2: 0.0}
+    for seed in range(4):
+        torch.manual_seed(seed)
+        x = torch.randn((K, g.num_samples if direction == UP else g.num_mutations), device="cuda")
+        _pair_mode(2)
+        exact = product(g, x.double(), direction, f64_native=True)
+        for mode in total:
+            e, n = error(mode, x, exact)
+            total[mode] += e / n
+    assert total[1] <= total[2], (np.sqrt(total[1] / 4), np.sqrt(total[2] / 4))
