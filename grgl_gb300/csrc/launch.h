@@ -76,6 +76,7 @@ template <typename S> struct PairDownParams {
     long long rows, stride, groups;
     unsigned base0, tiles, items;
     int group_begin, group_end, groups_per_item, part_begin;
+    int long_runs;       // float pairs: runs of eight rows (0: of four)
     const int* gate;  // as SweepParams::gate
 };
 // What a pair_down_* call does, and what its kShape step answers.

@@ -263,5 +263,27 @@ struct AddF64S {
 struct AddF64SD : AddF64S {};
 // ... and with no runs: every addition is normalised (df_add).
 struct AddF64SN : AddF64SD {};
+// Sum of float pairs as three floats of falling size, whose additions are exact but for the last float's.
+struct DFSum {
+    float t0, t1, t2;
+    __device__ __forceinline__ void fold(DF x) {
+        float s, e, f, g;
+        AddF32C::two_sum(t0, x.hi, s, e);
+        t0 = s;
+        AddF32C::two_sum(t1, x.lo, s, f);
+        AddF32C::two_sum(s, e, t1, g);
+        t2 = __fadd_rn(t2, __fadd_rn(f, g));
+    }
+    // ... rounded to a pair
+    __device__ __forceinline__ DF pair() const {
+        float s, e;
+        AddF32C::two_sum(t0, t1, s, e);
+        e = __fadd_rn(e, t2);
+        const float h = __fadd_rn(s, e);
+        return {h, __fsub_rn(e, __fsub_rn(h, s))};
+    }
+};
+// ... and with short runs folded into such sums (DOWN in pair form).
+struct AddF64ST : AddF64S {};
 
 }  // namespace grgx

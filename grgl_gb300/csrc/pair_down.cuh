@@ -13,17 +13,26 @@
 
 namespace grgx {
 
-// Accumulated sum of one item as it is kept between kernels: compensated sums stay pairs, a
-// float-pair run becomes the double it stands for.
+// Accumulated sum of one item as it is kept between kernels: compensated sums stay pairs, float pairs' sums
+// become pairs again.
 template <class Op> struct PairPart {
     using T = typename Op::A;
-    static __device__ __forceinline__ T of(const typename Op::A& a) { return a; }
-    static __device__ __forceinline__ void merge(typename Op::A& a, const T& x) { Op::merge(a, x); }
+    using Sum = typename Op::A;
+    static __device__ __forceinline__ Sum zero() { return Op::zero(); }
+    static __device__ __forceinline__ T of(const Sum& a) { return a; }
+    static __device__ __forceinline__ void merge(Sum& a, const T& x) { Op::merge(a, x); }
+    static __device__ __forceinline__ typename Op::S finish_onto(typename Op::S base, const Sum& a) { return Op::finish_onto(base, a); }
 };
-template <> struct PairPart<AddF64SD> {
-    using T = double;
-    static __device__ __forceinline__ T of(const F64Run& a) { return a.acc + AddF64S::run_value(a); }
-    static __device__ __forceinline__ void merge(F64Run& a, const T& x) { a.acc += x; }
+template <> struct PairPart<AddF64ST> {
+    using T = DF;
+    using Sum = DFSum;
+    static __device__ __forceinline__ Sum zero() { return {0.0f, 0.0f, 0.0f}; }
+    static __device__ __forceinline__ T of(const Sum& a) { return a.pair(); }
+    static __device__ __forceinline__ void merge(Sum& a, const T& x) { a.fold(x); }
+    static __device__ __forceinline__ DF finish_onto(DF base, Sum a) {
+        a.fold(base);
+        return a.pair();
+    }
 };
 
 // Pattern row elements.  A pair of rows is summed in storage precision: compensated float32 rounds
@@ -138,7 +147,7 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(con
     using Part = PairPart<Op>;
     constexpr int NG = 32 / G, ROWS = kPairRows;
     static_assert(NG * ROWS <= kPairTile, "a warp's rows end within the padded ids");
-    constexpr bool kChains = ChainTraits<Op>::kChains;
+    constexpr bool kRuns = std::is_same<Op, AddF64ST>::value;
     const int lane = threadIdx.x & 31;
     // (lanes without a column or past the last whole row follow along on the warp's first row)
     const int col = blockIdx.y * (G * VW) + (lane % G) * VW;
@@ -186,11 +195,27 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(con
                 for (int u = 0; u < 4; u++)
                     TableVec<T, VW>::ld(reinterpret_cast<const T*>(table + (unsigned long long)k[u] * rowBytes), v[r][u]);
             }
+            if constexpr (kRuns) {
+                if ((q - q0) & 1 & p.long_runs) {
 #pragma unroll
-            for (int r = 0; r < ROWS; r++) acc[r].add_pairs(v[r]);
-            if (kChains && ((q - q0) & 7) == 7) {
+                    for (int r = 0; r < ROWS; r++) acc[r].add_rows(v[r]);
+                } else {
 #pragma unroll
-                for (int r = 0; r < ROWS; r++) acc[r].flush();
+                    for (int r = 0; r < ROWS; r++) acc[r].start_rows(v[r]);
+                }
+                if ((q - q0) & 1 | !p.long_runs) {
+#pragma unroll
+                    for (int r = 0; r < ROWS; r++) acc[r].fold();
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < ROWS; r++) acc[r].add_pairs(v[r]);
+            }
+        }
+        if constexpr (kRuns) {
+            if ((q1 - q0) & 1 & p.long_runs) {
+#pragma unroll
+                for (int r = 0; r < ROWS; r++) acc[r].fold();
             }
         }
         if (!active) continue;
@@ -203,7 +228,7 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(con
                 S* d = p.vals + row * p.stride + col;
                 ld_plain<S, VW>(d, base);
 #pragma unroll
-                for (int i = 0; i < VW; i++) out[i] = Op::finish_onto(base[i], acc[r].get(i));
+                for (int i = 0; i < VW; i++) out[i] = Part::finish_onto(base[i], acc[r].get(i));
                 Vec<S, VW>::st(d, out);
             } else {
                 typename Part::T* d = static_cast<typename Part::T*>(p.parts) +
@@ -232,16 +257,16 @@ __device__ __forceinline__ void pair_finish(typename PairPart<Op>::T* __restrict
                                             long long stride, typename Op::S* __restrict__ vals) {
     const long long total = rows * stride;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
-        typename Op::A a = Op::zero();
+        typename PairPart<Op>::Sum a = PairPart<Op>::zero();
         for (int j = 0; j < count; j++) PairPart<Op>::merge(a, parts[j * total + x]);
         if (vals == nullptr) {
             parts[x] = PairPart<Op>::of(a);
             continue;
         }
         if constexpr (std::is_same<typename Op::S, DF>::value)
-            df_put(vals, x, stride, Op::finish_onto(df_get(vals, x, stride), a));
+            df_put(vals, x, stride, PairPart<Op>::finish_onto(df_get(vals, x, stride), a));
         else
-            vals[x] = Op::finish_onto(vals[x], a);
+            vals[x] = PairPart<Op>::finish_onto(vals[x], a);
     }
 }
 
@@ -250,7 +275,7 @@ __global__ void pair_finish_kernel(typename PairPart<Op>::T* parts, int count, l
                                    typename Op::S* vals, const int* gate) {
     if constexpr (kHasF64<Op>) {
         if (gate != nullptr && *gate != 0) {
-            pair_finish<AddF64>(parts, count, rows, stride, reinterpret_cast<double*>(vals));
+            pair_finish<AddF64>(reinterpret_cast<double*>(parts), count, rows, stride, reinterpret_cast<double*>(vals));
             return;
         }
     }

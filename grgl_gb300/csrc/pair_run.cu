@@ -23,6 +23,8 @@ constexpr int kPairMinGroups = 16;
 // UP: bytes of the height-0 rows' columns that a launch gathers from at a time (100 MB: float32 K=128 on
 // 200,000 rows 3.95 ms against 3.63, 50 to 72 MB the same).
 constexpr long long kPairSourceBytes = 64LL << 20;
+// Blocks from which float64 sums eight pattern rows between folds, not four (error and time: pair_down_f64s.cu).
+constexpr long long kPairLongRuns = 50;
 // Most of a call's scratch unless a scope says less.
 constexpr uint64_t kPairScratch = 6ULL << 30;
 
@@ -194,6 +196,7 @@ int launch_pair_down(const Layout& call, const DevicePlan* dp, const PairDownRun
         p.groups = (P.nblk + 3) / 4;
         p.tiles = static_cast<unsigned>((P.h0 + c.rows_per_warp - 1) / c.rows_per_warp);
         p.gate = gate;
+        p.long_runs = P.nblk >= kPairLongRuns;
         for (size_t i = 0; i < run.ranges.size(); i++) {
             const PairDownRun::Range& r = run.ranges[i];
             c.step = PairDownCall::kTable;

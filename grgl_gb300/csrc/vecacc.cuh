@@ -159,7 +159,6 @@ template <> struct VecAcc<AddF64S, 1> {
             if ((u & 3) == 3) settle();
         }
     }
-    __device__ __forceinline__ void add_pairs(const DF (*v)[1]) { add_block<4>(v); }
     __device__ __forceinline__ void merge(const VecAcc& o) { AddF64S::merge(a[0], o.a[0]); }
     __device__ __forceinline__ VecAcc shfl_xor(int m) const { return {{AddF64S::shfl_xor(a[0], m)}}; }
     __device__ __forceinline__ VecAcc shfl_up(int d) const { return {{AddF64S::shfl_up(a[0], d)}}; }
@@ -320,7 +319,6 @@ template <int NP> struct PackedF64S {
             if ((u & 3) == 3) settle();
         }
     }
-    __device__ __forceinline__ void add_pairs(const DF (*v)[2 * NP]) { add_block<4>(v); }
     __device__ __forceinline__ void settle() {
 #pragma unroll
         for (int j = 0; j < NP; j++) {
@@ -399,8 +397,8 @@ __device__ __forceinline__ void df_add2(float2& ahi, float2& alo, float2 bhi, fl
 }
 
 // float64 as float pairs with the runs folded into a normalised float pair: no FP64 instruction
-// until the sum is read.  The low part is renormalised every two additions, not four (2% of the
-// time of a wide product): mean errors of products in pair form stay 15-20% below the sweep's.
+// until the sum is read (UP in pair form).  The low part is renormalised every two additions, not four (2% of
+// the time of a wide product): mean errors of UP products stay 15-20% below the sweep's.
 template <int NP> struct PackedF64SD {
     float2 hi[NP], lo[NP], thi[NP], tlo[NP];
     __device__ __forceinline__ void zero() {
@@ -423,7 +421,6 @@ template <int NP> struct PackedF64SD {
             if (u & 1) settle();
         }
     }
-    __device__ __forceinline__ void add_pairs(const DF (*v)[2 * NP]) { add_block<4>(v); }
     __device__ __forceinline__ void settle() {
 #pragma unroll
         for (int j = 0; j < NP; j++) {
@@ -481,11 +478,93 @@ template <> struct VecAcc<AddF64SD, 1> : PackedF64SD<1> {
             if ((u & 2) != 0) settle();
         }
     }
-    __device__ __forceinline__ void add_pairs(const DF (*v)[1]) { add_block<4>(v); }
     __device__ __forceinline__ DF pair(int) const { return df_add(Base::pair(0), Base::pair(1)); }
     __device__ __forceinline__ F64Run get(int) const {
         const F64Run a = Base::get(0), b = Base::get(1);
         return {a.acc + b.acc + AddF64S::run_value(b), a.hi, a.lo};
+    }
+};
+
+// float64 as float pairs in runs of four or eight rows, each run folded into a DFSum: a run's first row is its
+// start, the pair is renormalised after four, and no FP64 instruction is needed at all (FP64 conversions and
+// additions run at about two lanes per clock and SM).  A run's low parts are rounded relative to its sum,
+// so the run's length sets the error: see pair_down_f64s.cu.
+template <int NP> struct PackedF64ST {
+    float2 hi[NP], lo[NP], t0[NP], t1[NP], t2[NP];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int j = 0; j < NP; j++) t0[j] = t1[j] = t2[j] = make_float2(0.0f, 0.0f);
+    }
+    __device__ __forceinline__ void start(const DF* v) {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            hi[j] = make_float2(v[2 * j].hi, v[2 * j + 1].hi);
+            lo[j] = make_float2(v[2 * j].lo, v[2 * j + 1].lo);
+        }
+    }
+    __device__ __forceinline__ void add(const DF* v) {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            float2 s, e;
+            two_sum2(hi[j], make_float2(v[2 * j].hi, v[2 * j + 1].hi), s, e);
+            lo[j] = add2(lo[j], add2(e, make_float2(v[2 * j].lo, v[2 * j + 1].lo)));
+            hi[j] = s;
+        }
+    }
+    __device__ __forceinline__ void settle() {
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            const float2 h = add2(hi[j], lo[j]);
+            lo[j] = sub2(lo[j], sub2(h, hi[j]));
+            hi[j] = h;
+        }
+    }
+    __device__ __forceinline__ void fold() {  // (DFSum::fold)
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            float2 s, e, f, g;
+            two_sum2(t0[j], hi[j], s, e);
+            t0[j] = s;
+            two_sum2(t1[j], lo[j], s, f);
+            two_sum2(s, e, t1[j], g);
+            t2[j] = add2(t2[j], add2(f, g));
+        }
+    }
+    // Four rows that start a run, and four more.
+    __device__ __forceinline__ void start_rows(const DF (*v)[2 * NP]) {
+        start(v[0]);
+#pragma unroll
+        for (int u = 1; u < 4; u++) add(v[u]);
+        settle();
+    }
+    __device__ __forceinline__ void add_rows(const DF (*v)[2 * NP]) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) add(v[u]);
+    }
+    __device__ __forceinline__ DFSum get(int i) const {
+        return {lane_of(t0[i >> 1], i), lane_of(t1[i >> 1], i), lane_of(t2[i >> 1], i)};
+    }
+};
+template <> struct VecAcc<AddF64ST, 2> : PackedF64ST<1> {};
+// One column: two rows at a time, one in each half.
+template <> struct VecAcc<AddF64ST, 1> : PackedF64ST<1> {
+    using Base = PackedF64ST<1>;
+    __device__ __forceinline__ void start_rows(const DF (*v)[1]) {
+        const DF a[2] = {v[0][0], v[1][0]}, b[2] = {v[2][0], v[3][0]};
+        start(a);
+        add(b);
+    }
+    __device__ __forceinline__ void add_rows(const DF (*v)[1]) {
+        const DF a[2] = {v[0][0], v[1][0]}, b[2] = {v[2][0], v[3][0]};
+        add(a);
+        add(b);
+    }
+    __device__ __forceinline__ DFSum get(int) const {
+        DFSum a = Base::get(0);
+        const DFSum b = Base::get(1);
+        a.fold(DF{b.t0, b.t1});
+        a.t2 = __fadd_rn(a.t2, b.t2);
+        return a;
     }
 };
 

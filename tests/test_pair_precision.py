@@ -56,3 +56,29 @@ def test_errors_at_or_below_the_sweeps(graphs, N, M, direction, K, standardized)
             e, n = error(mode, x, exact)
             total[mode] += e / n
     assert total[1] <= total[2], (np.sqrt(total[1] / 4), np.sqrt(total[2] / 4))
+
+
+# (short rows, whose sums take runs of four pattern rows; many blocks; few and many columns)
+@pytest.mark.parametrize("N,M,direction,K", [
+    (20_000, 50_000, DOWN, 1), (20_000, 50_000, DOWN, 3), (20_000, 50_000, DOWN, 9), (20_000, 50_000, DOWN, 64),
+    (20_000, 50_000, UP, 1), (20_000, 50_000, UP, 6), (20_000, 50_000, UP, 33),
+    (100_000, 20_000, DOWN, 2), (100_000, 20_000, DOWN, 18), (200_000, 3_000, DOWN, 2), (200_000, 3_000, DOWN, 6)])
+@pytest.mark.parametrize("inputs", ["normal", "positive", "standardized"])
+def test_float64_errors_at_or_below_the_sweeps(graphs, N, M, direction, K, inputs):
+    import torch
+
+    gx, get = graphs
+    g = get(N, M)
+    product = gx.matmul_standardized if inputs == "standardized" else gx.matmul
+    total = {1: 0.0, 2: 0.0}
+    for seed in range(4):
+        torch.manual_seed(seed)
+        x = torch.randn((K, g.num_samples if direction == UP else g.num_mutations), device="cuda", dtype=torch.float64)
+        if inputs == "positive":
+            x = x.abs()
+        _pair_mode(2)
+        exact = product(g, x, direction, f64_native=True)
+        for mode in total:
+            _pair_mode(mode)
+            total[mode] += float((product(g, x, direction) - exact).square().sum() / exact.square().sum())
+    assert total[1] <= total[2], (np.sqrt(total[1] / 4), np.sqrt(total[2] / 4))
