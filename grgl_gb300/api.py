@@ -593,7 +593,8 @@ def autotune(grg: GRG, dtype, rows: int, direction, *, f32_compensated: bool = T
     """Measure every launch shape on each level of one traversal of ``grg`` for ``rows`` x cols
     inputs of ``dtype`` in ``direction`` and record the winners in the process-wide shape table
     (keyed on the level's width, mean degree, the storage kind and K).  Returns the per-level
-    report.  Later calls on any graph whose levels match an entry run the tuned shape."""
+    report.  Later calls on any graph whose levels match an entry run the tuned shape, and calls
+    on ``grg`` of this row width the form (unsplit, split or pair) that was fastest."""
     code = _DTYPE_CODES[np.dtype(dtype)]
     need = ctypes.c_uint64()
     buf = ctypes.create_string_buffer(1 << 16)

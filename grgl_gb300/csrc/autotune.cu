@@ -10,9 +10,10 @@
 // resident graph (CUDA events around the level's launch, best of two after a warm launch) --
 // the deep variant at the default lanes, then halvings of the lanes per row while each keeps
 // winning -- and records the winner when it beats the default by more than 2%.  Levels with
-// under 0.5% of the traversal's edges keep the default.  For UP on graphs where the split form
-// (up_split.cu) is possible it tunes both forms and records, for this graph and (storage kind,
-// stride), the one whose tuned sweep is faster.  Calls on any graph then look up every
+// under 0.5% of the traversal's edges, and levels of short rows, keep the default.  On graphs where the split
+// form (up_split.cu) is possible it tunes both forms and records, for this graph and (storage kind,
+// stride), the one whose tuned sweep is faster; where calls would take the pair form (pair_plan.h) it times
+// that as well and records whether it is the fastest.  Calls on any graph then look up every
 // level's key; levels without an entry run the default shape.  Shapes change only the order in
 // which a row's float terms are added (integer results are bit-exact with any shape).
 #include <cuda_runtime.h>
@@ -145,10 +146,10 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
     const Layout L = choose_layout(dtype, static_cast<long long>(rows), (flags & GRGX_FLAG_F32_PLAIN) != 0,
                                    (flags & GRGX_FLAG_F64_NATIVE) != 0);
     const bool down = (direction == GRGX_DIRECTION_DOWN);
-    // the CSRs a call of this shape sweeps; for UP both forms when the split form is possible,
-    // so the faster one is recorded for this graph
-    // (for DOWN too: the height-0 level in parent blocks, the levels above it as usual; a single
-    // 4-byte column's split form runs on lists in shared memory, which has one shape)
+    // the CSRs a call of this shape sweeps; both forms when the split form is possible, so the faster one is
+    // recorded for this graph (for DOWN the height-0 level in parent blocks, the levels above it as usual; a
+    // single 4-byte column's split form runs on lists in shared memory, which has one shape), and the pair
+    // form's levels beside its own launches, which have one shape too
     struct Pass {
         const DevCSR* c;
         int mode;
@@ -156,6 +157,7 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
         long long stateBase;
         bool skipLast;  // the CSR's last level is left to the next pass
         bool staged = false;  // the CSR's levels are one launch of staged lists
+        bool pair = false;    // the height-0 edges over patterns; the CSR's levels (c) are the next pass
     };
     const bool staged = staged_layout(L);
     std::vector<std::vector<Pass>> forms;
@@ -176,19 +178,34 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
             forms.push_back({{cs.up0b, 1, "split: height-0 block", dp->split_src, false, staged && dp->up_staged.slots > 0},
                              {cs.up_int, 2, "split: level", dp->split_src, false}});
     }
+    const bool split = forms.size() > 1;
+    clear_pair_choice(g, dp, L, down);
+    const bool upState = !down && L.kind == Kind::F32C;  // (as matmul_once)
+    const size_t upStateBytes = upState ? static_cast<size_t>(g->host->num_nodes - h0) * L.stride * L.asize : 0;
+    PairDownRun prun;
+    PairUpRun urun;
+    if (use_pair_form(g, dp, L, down)) {
+        if (down) prun = pair_down_run(L, dp, pair_scratch_limit());
+        else if (upStateBytes < pair_scratch_limit()) urun = pair_up_run(L, dp, pair_scratch_limit() - upStateBytes);
+        const SweepCSRs cs = sweep_csrs(dp, L);
+        const DevCSR* levels = down ? cs.down : cs.up_int;
+        if (!prun.ranges.empty() || !urun.ranges.empty())
+            forms.push_back({{levels, 0, "pair: height-0 patterns", 0, false, false, true},
+                             {levels, upState ? 2 : 0, "pair: level", h0, down}});
+    }
+    bool pair = forms.size() > (split ? 2u : 1u);
     long long maxPieces = 0, maxHeavy = 0;
     for (const auto& f : forms)
         for (const Pass& ps : f) {
             maxPieces = std::max(maxPieces, ps.c->n_pieces);
             maxHeavy = std::max(maxHeavy, ps.c->n_heavy);
         }
-    const bool needState = forms.size() > 1;
     const int maxT = max_tiles(L);
     const size_t n = g->host->num_nodes;
     cudaStream_t s = nullptr;
     GRGX_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    void *vals = nullptr, *partials = nullptr, *state = nullptr, *slots = nullptr;
-    unsigned* counters = nullptr;
+    void *vals = nullptr, *partials = nullptr, *state = nullptr, *slots = nullptr, *ptable = nullptr, *pparts = nullptr;
+    unsigned *counters = nullptr, *pwork = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     std::ostringstream rep;
     auto release = [&] {
@@ -196,6 +213,9 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
         if (partials) cudaFree(partials);
         if (state) cudaFree(state);
         if (slots) cudaFree(slots);
+        if (ptable) cudaFree(ptable);
+        if (pparts) cudaFree(pparts);
+        if (pwork) cudaFree(pwork);
         if (counters) cudaFree(counters);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
@@ -206,8 +226,8 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
         GRGX_CUDA(cudaMalloc(&vals, std::max<size_t>(valBytes, 16)));
         GRGX_CUDA(cudaMemsetAsync(vals, 0, valBytes, s));
         GRGX_CUDA(cudaMalloc(&partials, std::max<size_t>(static_cast<size_t>(maxPieces) * L.stride * L.asize, 16)));
-        if (needState) {
-            const size_t stateRows = down ? static_cast<size_t>(h0) : n - static_cast<size_t>(dp->split_src);
+        if (split || (pair && upState)) {
+            const size_t stateRows = down ? static_cast<size_t>(h0) : n - static_cast<size_t>(h0);
             const size_t stateBytes = stateRows * L.stride * std::max(L.asize, 8);
             GRGX_CUDA(cudaMalloc(&state, std::max<size_t>(stateBytes, 16)));
             GRGX_CUDA(cudaMemsetAsync(state, 0, stateBytes, s));
@@ -254,19 +274,44 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
             }
             return best;
         };
+        const size_t pworkBytes = std::max<size_t>(prun.ranges.size() * prun.tiles, 1) * sizeof(unsigned);
+        if (pair && (cudaMalloc(&ptable, std::max<size_t>(down ? prun.table_bytes : urun.bytes(), 16)) != cudaSuccess ||
+                     cudaMalloc(&pparts, std::max<size_t>(prun.part_bytes, 16)) != cudaSuccess ||
+                     cudaMalloc(&pwork, pworkBytes) != cudaSuccess)) {
+            // no memory for the pair form's scratch beside the other forms': calls decide by the rules
+            cudaGetLastError();
+            forms.pop_back();
+            pair = false;
+        }
+        auto time_pair = [&] {
+            float best = 1e30f;
+            for (int rep_i = 0; rep_i < 3; rep_i++) {
+                GRGX_CUDA(cudaMemsetAsync(pwork, 0, pworkBytes, s));
+                GRGX_CUDA(cudaEventRecord(e0, s));
+                if (down) launch_pair_down(L, dp, prun, vals, ptable, pparts, pwork, s, nullptr);
+                else launch_pair_up(L, dp, urun, vals, ptable, upState ? state : nullptr, 0, s, nullptr);
+                GRGX_CUDA(cudaEventRecord(e1, s));
+                GRGX_CUDA(cudaEventSynchronize(e1));
+                GRGX_CUDA(cudaGetLastError());
+                float ms = 0;
+                GRGX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+                if (rep_i > 0) best = std::min(best, ms);
+            }
+            return best;
+        };
         const std::vector<int> gs = candidate_g(L);
         std::vector<double> formBest;
         for (const auto& form : forms) {
             long long totalEdges = 0;
-            for (const Pass& ps : form) totalEdges += ps.c->n_edges;
+            for (const Pass& ps : form) totalEdges += ps.pair ? 0 : ps.c->n_edges;
             double totDefault = 0, totBest = 0;
             for (const Pass& ps : form) {
                 cur = ps.c;
                 curMode = ps.mode;
                 curBase = ps.stateBase;
                 const DevCSR& c = *ps.c;
-                if (ps.staged) {
-                    const float t = time_staged();
+                if (ps.staged || ps.pair) {
+                    const float t = ps.pair ? time_pair() : time_staged();
                     totDefault += t;
                     totBest += t;
                     continue;
@@ -276,8 +321,8 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
                     const LevelShape def = default_shape(L);
                     const float tDef = time_shape(lvl, def);
                     totDefault += tDef;
-                    // levels under 0.5% of the traversal's edges keep the default
-                    if (c.level_edges[lvl] * 200 < totalEdges) {
+                    // levels under 0.5% of the traversal's edges, and those with one shape, keep the default
+                    if (c.level_edges[lvl] * 200 < totalEdges || (lvl < c.level_alone.size() && c.level_alone[lvl])) {
                         totBest += tDef;
                         continue;
                     }
@@ -316,23 +361,27 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
                 }
             }
             char tail[160];
-            const bool splitForm = (&form != &forms[0]);
+            const bool pairForm = pair && &form == &forms.back(), splitForm = !pairForm && &form != &forms[0];
             std::snprintf(tail, sizeof(tail), "%s %.4f ms tuned, %.4f ms default\n",
-                          forms.size() > 1 ? (splitForm ? "split sweep" : "unsplit sweep") : "sweep", totBest,
-                          totDefault);
+                          pairForm    ? "pair sweep"
+                          : splitForm ? "split sweep"
+                          : split     ? "unsplit sweep"
+                                      : "sweep",
+                          totBest, totDefault);
             rep << tail;
             formBest.push_back(totBest);
         }
-        if (forms.size() > 1) {
-            const bool split = formBest[1] < 0.98 * formBest[0];
-            if (down) {
-                set_down_split_choice(g, dp, L, split);
-                rep << (split ? "DOWN runs in split form for this shape\n" : "DOWN runs unsplit for this shape\n");
-            } else {
-                set_up_split_choice(g, dp, L, split);
-                rep << (split ? "UP runs in split form for this shape\n" : "UP runs unsplit for this shape\n");
-            }
+        const bool splitWins = split && formBest[1] < 0.98 * formBest[0];
+        if (split) {
+            if (down) set_down_split_choice(g, dp, L, splitWins);
+            else set_up_split_choice(g, dp, L, splitWins);
         }
+        // (the form of the rules is kept where another one is no more than 2% faster)
+        const bool pairWins = pair && !(formBest[splitWins ? 1 : 0] < 0.98 * formBest.back());
+        if (pair) set_pair_choice(g, dp, L, down, pairWins);
+        if (split || pair)
+            rep << (down ? "DOWN" : "UP")
+                << (pairWins ? " runs in pair form" : splitWins ? " runs in split form" : " runs unsplit") << " for this shape\n";
     } catch (...) {
         release();
         throw;

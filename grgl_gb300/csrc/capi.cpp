@@ -36,6 +36,7 @@ void set_pair_mode(int mode);
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
 const void* pair_analysis(grgx_graph* g);
 void set_pair_rows(long long most);
+int call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags, int pair);
 long long set_plan_alloc(long long pass, long long refuse);
 void* host_alloc(uint64_t bytes);
 void host_free(void* b);
@@ -479,6 +480,16 @@ extern "C" grgx_status grgx_debug_pair_analysis(grgx_graph* g, const void** out)
     return guarded([&] {
         GRGX_CHECK(g && out, GRGX_ERR_API_MISUSE, "null argument");
         *out = grgx::pair_analysis(g);
+    });
+}
+
+// Test hook (not part of the public header): the form a call takes, 0 unsplit, 1 split, 2 pair; `pair` 0 or 1
+// first records a measured choice against or for the pair form (-1: none).
+extern "C" grgx_status grgx_debug_call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags, int pair,
+                                            int* form) {
+    return guarded([&] {
+        GRGX_CHECK(g && form, GRGX_ERR_API_MISUSE, "null argument");
+        *form = grgx::call_form(g, dtype, rows, direction, flags, pair);
     });
 }
 

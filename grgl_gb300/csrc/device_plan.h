@@ -93,6 +93,7 @@ struct DevicePlan {
     long long n_fin_down = 0;
     bool down_split_built = false;
     std::map<std::pair<int, long long>, bool> down_split_choice;
+    std::map<std::pair<int, long long>, bool> up_pair_choice, down_pair_choice;  // pair form or not, measured
     PairPlan pair;                       // pair form of the height-0 edges, on first use (use_pair_form)
     std::vector<int64_t> down_off;       // DOWN row offsets (host copy)
     long long down_h0_row = 0;           // first DOWN row of height 0
@@ -267,6 +268,9 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
 // server's worker lowers it to what its batch has reserved (PairScratchScope).
 size_t pair_scratch_limit();
 void set_pair_mode(int mode);
+// What grgx_autotune measured for L's (storage kind, stride) on this graph; clear_pair_choice: the rules again.
+void set_pair_choice(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, bool pair);
+void clear_pair_choice(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
 void set_pair_rows(long long most);  // UP table rows from which that direction keeps the other forms (tests)
 // out: height-0 nodes, blocks, patterns, height-0 edges of a direction in pair form (zeros: not in use).
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);

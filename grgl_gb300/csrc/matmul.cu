@@ -1021,6 +1021,16 @@ void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols
     }
 }
 
+int call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags, int pair) {
+    DevicePlan* dp = ensure_device_plan(g);
+    const Layout L = choose_layout(dtype, static_cast<long long>(rows), (flags & GRGX_FLAG_F32_PLAIN) != 0,
+                                   (flags & GRGX_FLAG_F64_NATIVE) != 0);
+    const bool down = direction == GRGX_DIRECTION_DOWN;
+    if (pair >= 0) set_pair_choice(g, dp, L, down, pair != 0);
+    if (use_pair_form(g, dp, L, down)) return 2;
+    return (down ? use_down_split(g, dp, L) : use_up_split(g, dp, L)) ? 1 : 0;
+}
+
 // ---- captured CUDA graphs of whole calls (small graphs) ----------------------------------------
 
 struct GraphEntry {

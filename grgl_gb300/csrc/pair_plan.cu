@@ -696,6 +696,16 @@ void set_pair_rows(long long most) { g_most_rows.store(most); }
 
 void set_pair_mode(int mode) { g_pair_mode.store(mode); }
 
+void set_pair_choice(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, bool pair) {
+    std::lock_guard<std::mutex> lk(g->mu);
+    (down ? dp->down_pair_choice : dp->up_pair_choice)[{static_cast<int>(L.kind), L.stride}] = pair;
+}
+
+void clear_pair_choice(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
+    std::lock_guard<std::mutex> lk(g->mu);
+    (down ? dp->down_pair_choice : dp->up_pair_choice).erase({static_cast<int>(L.kind), L.stride});
+}
+
 bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
     const int mode = g_pair_mode.load();
     if (mode == 2) return false;
@@ -706,6 +716,9 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
     // N=200,000, M=250,000); compensated sums would lose the pattern rows' roundings.
     if (!down && L.stride == 1 && (L.kind == Kind::F32C || (staged_layout(L) && up_split_possible(dp)))) return false;
     std::lock_guard<std::mutex> lk(g->mu);
+    const auto& choice = down ? dp->down_pair_choice : dp->up_pair_choice;
+    const auto chosen = choice.find({static_cast<int>(L.kind), L.stride});
+    if (mode == 0 && chosen != choice.end() && !chosen->second) return false;
     PairPlan& P = dp->pair;
     bool& tried = down ? P.down_tried : P.up_tried;
     for (int attempt = 0; attempt < 2 && !tried && !P.refused; attempt++) {

@@ -146,3 +146,45 @@ def test_more_table_rows_than_lists_can_number(env, first):
             assert _built(g, direction) == (direction == DOWN)
     finally:
         fn(0x3fffffff)
+
+
+def _form(g, dt, K, direction, pair=-1):
+    """The form a call takes; `pair` 0 or 1: with that measured choice recorded."""
+    from grgl_gb300 import _lib
+    from grgl_gb300.api import _DTYPE_CODES
+
+    out = ctypes.c_int()
+    fn = _lib.lib().grgx_debug_call_form
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_uint32, ctypes.c_int,
+                   ctypes.POINTER(ctypes.c_int)]
+    _lib.check(fn(g._h, _DTYPE_CODES[np.dtype(dt)], K, direction, 0, pair, ctypes.byref(out)))
+    return ("unsplit", "in split form", "in pair form")[out.value]
+
+
+@pytest.mark.parametrize("direction", [DOWN, UP])
+def test_autotune_chooses_among_all_forms(cuda_ok, direction):
+    """The form it reports is the one that calls take, also against the rules, and results hold in any."""
+    import grgl_gb300 as gx
+
+    g = gx.window_tree_grg(40_000, 9_000, seed=5).upload()  # 3.6e6 edges, two blocks of samples
+    try:
+        for dt, K in ((np.int32, 6), (np.int32, 1), (np.float32, 9), (np.float64, 20)):
+            V = _input(g, direction, dt, K)
+            exact = gx.matmul(g, V.astype(np.float64), direction, f64_native=True)
+            by_rule = _form(g, dt, K, direction)
+            report = gx.autotune(g, dt, K, direction)
+            form = _form(g, dt, K, direction)
+            assert report.splitlines()[-1].endswith(f"runs {form} for this shape")
+            assert ("pair sweep" in report) == (by_rule == "in pair form")
+            for pair in (0, 1):
+                assert (_form(g, dt, K, direction, pair) == "in pair form") == (pair == 1 and by_rule == "in pair form")
+                gx.set_graph_replay(False)
+                got = gx.matmul(g, V, direction)
+                gx.set_graph_replay(True)
+                scale = gx.matmul(g, np.abs(V).astype(np.float64), direction, f64_native=True)
+                assert np.all(np.abs(got - exact) <= {4: 1e-6, 8: 1e-12}[V.itemsize] * scale)
+            report = gx.autotune(g, dt, K, direction)  # (measured again, whatever was recorded)
+            assert report.splitlines()[-1].endswith(f"runs {_form(g, dt, K, direction)} for this shape")
+    finally:
+        gx.autotune_clear()
+        gx.set_graph_replay(True)
