@@ -180,18 +180,15 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
     }
     const bool split = forms.size() > 1;
     clear_pair_choice(g, dp, L, down);
-    const bool upState = !down && L.kind == Kind::F32C;  // (as matmul_once)
-    const size_t upStateBytes = upState ? static_cast<size_t>(g->host->num_nodes - h0) * L.stride * L.asize : 0;
-    PairDownRun prun;
-    PairUpRun urun;
-    if (use_pair_form(g, dp, L, down)) {
-        if (down) prun = pair_down_run(L, dp, pair_scratch_limit());
-        else if (upStateBytes < pair_scratch_limit()) urun = pair_up_run(L, dp, pair_scratch_limit() - upStateBytes);
+    const PairRuns pruns = pair_runs(g, dp, L, down);
+    const PairDownRun& prun = pruns.down;
+    const PairUpRun& urun = pruns.up;
+    const bool upState = pruns.up_state_bytes > 0;
+    if (!prun.ranges.empty() || !urun.ranges.empty()) {
         const SweepCSRs cs = sweep_csrs(dp, L);
         const DevCSR* levels = down ? cs.down : cs.up_int;
-        if (!prun.ranges.empty() || !urun.ranges.empty())
-            forms.push_back({{levels, 0, "pair: height-0 patterns", 0, false, false, true},
-                             {levels, upState ? 2 : 0, "pair: level", h0, down}});
+        forms.push_back({{levels, 0, "pair: height-0 patterns", 0, false, false, true},
+                         {levels, upState ? 2 : 0, "pair: level", h0, down}});
     }
     bool pair = forms.size() > (split ? 2u : 1u);
     long long maxPieces = 0, maxHeavy = 0;

@@ -36,7 +36,8 @@ void set_pair_mode(int mode);
 void pair_counts(grgx_graph* g, bool down, uint64_t out[4]);
 const void* pair_analysis(grgx_graph* g);
 void set_pair_rows(long long most);
-int call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags, int pair);
+int call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags, int pair, int* ranges);
+void set_pair_scratch(uint64_t bytes);
 long long set_plan_alloc(long long pass, long long refuse);
 void* host_alloc(uint64_t bytes);
 void host_free(void* b);
@@ -489,7 +490,19 @@ extern "C" grgx_status grgx_debug_call_form(grgx_graph* g, int dtype, uint64_t r
                                             int* form) {
     return guarded([&] {
         GRGX_CHECK(g && form, GRGX_ERR_API_MISUSE, "null argument");
-        *form = grgx::call_form(g, dtype, rows, direction, flags, pair);
+        int ranges = 0;
+        *form = grgx::call_form(g, dtype, rows, direction, flags, pair, &ranges);
+    });
+}
+
+// Test hook (not part of the public header): the tables that a call in pair form makes one after the other, when its
+// scratch is limited to `limit` bytes (for this thread's calls from now on; 0: as always).
+extern "C" grgx_status grgx_debug_pair_ranges(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags,
+                                              uint64_t limit, int* ranges) {
+    return guarded([&] {
+        GRGX_CHECK(g && ranges, GRGX_ERR_API_MISUSE, "null argument");
+        grgx::set_pair_scratch(limit);
+        grgx::call_form(g, dtype, rows, direction, flags, -1, ranges);
     });
 }
 

@@ -309,6 +309,16 @@ struct PairUpRun {
     size_t bytes() const { return table_bytes + source_bytes; }
 };
 PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit);
+// A call's pair form within this thread's scratch limit: its direction's launches, without ranges where it
+// takes another form.
+struct PairRuns {
+    PairUpRun up;
+    PairDownRun down;
+    // UP: compensated float32 keeps the sums as pairs until a node's other children are added; every other
+    // kind adds them onto the node's value
+    size_t up_state_bytes = 0;
+};
+PairRuns pair_runs(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
 // Writes every node's sum over its height-0 children to vals (onto it when rmw), or leaves it in
 // `state` where one is given.
 int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, void* vals, void* table, void* state,

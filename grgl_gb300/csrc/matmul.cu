@@ -728,19 +728,12 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
         // passes, then the other edges level by level (up_split.cu)
         // UP in pair form: the height-0 edges over patterns first (pair_plan.h), the others level by
         // level from the sums, as in split form
-        PairUpRun urun;
-        size_t upStateBytes = 0;
-        if (!down && pairForm && use_pair_form(g, dp, L, false)) {
-            // compensated float32 keeps the sums as pairs until a node's other children are added;
-            // every other kind adds them onto the node's value
-            upStateBytes = L.kind == Kind::F32C ? static_cast<size_t>(n - dp->pair.h0) * L.stride * L.asize : 0;
-            if (upStateBytes < pair_scratch_limit()) urun = pair_up_run(L, dp, pair_scratch_limit() - upStateBytes);
-        }
+        const PairRuns pruns = pairForm ? pair_runs(g, dp, L, down) : PairRuns{};
+        const PairUpRun& urun = pruns.up;
         const bool upair = !urun.ranges.empty();
         const bool split = !down && !upair && use_up_split(g, dp, L);
         // DOWN: the height-0 level over patterns (pair_plan.h), or in parent blocks (up_split.cu)
-        PairDownRun prun;
-        if (down && pairForm && use_pair_form(g, dp, L, true)) prun = pair_down_run(L, dp, pair_scratch_limit());
+        const PairDownRun& prun = pruns.down;
         const bool dpair = !prun.ranges.empty();
         const bool dsplit = down && !dpair && use_down_split(g, dp, L);
         // coarse or fine chunking for this row width (the split copies are built by now)
@@ -776,7 +769,7 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
         void* slots = staged ? sc.get(slotBytes) : nullptr;
         const size_t stateBytes = staged   ? (split && L.kind == Kind::F32C ? static_cast<size_t>(n - h0) * L.asize : 0)
                                   : split  ? static_cast<size_t>(n - dp->split_src) * L.stride * std::max(L.asize, 8)
-                                  : upair  ? upStateBytes
+                                  : upair  ? pruns.up_state_bytes
                                   : dsplit ? static_cast<size_t>(h0) * L.stride * std::max(L.asize, 8)
                                            : 0;
         void* state = stateBytes ? sc.get(stateBytes) : nullptr;
@@ -1021,13 +1014,15 @@ void matmul_direct(grgx_graph* g, int dtype, const void* input, uint64_t in_cols
     }
 }
 
-int call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags, int pair) {
+int call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t flags, int pair, int* ranges) {
     DevicePlan* dp = ensure_device_plan(g);
     const Layout L = choose_layout(dtype, static_cast<long long>(rows), (flags & GRGX_FLAG_F32_PLAIN) != 0,
                                    (flags & GRGX_FLAG_F64_NATIVE) != 0);
     const bool down = direction == GRGX_DIRECTION_DOWN;
     if (pair >= 0) set_pair_choice(g, dp, L, down, pair != 0);
-    if (use_pair_form(g, dp, L, down)) return 2;
+    const PairRuns runs = pair_runs(g, dp, L, down);
+    *ranges = static_cast<int>(down ? runs.down.ranges.size() : runs.up.ranges.size());
+    if (*ranges > 0) return 2;
     return (down ? use_down_split(g, dp, L) : use_up_split(g, dp, L)) ? 1 : 0;
 }
 

@@ -132,6 +132,7 @@ template <typename F> void by_kind(const Layout& L, DownSums sums, F&& f) {
 
 PairScratchScope::PairScratchScope(uint64_t bytes) : saved_(t_limit) { t_limit = std::min(bytes, kPairScratch); }
 PairScratchScope::~PairScratchScope() { t_limit = saved_; }
+void set_pair_scratch(uint64_t bytes) { t_limit = bytes ? std::min(bytes, kPairScratch) : kPairScratch; }
 size_t pair_scratch_limit() { return static_cast<size_t>(t_limit); }
 
 PairDownRun pair_down_run(const Layout& call, const DevicePlan* dp, size_t limit) {
@@ -244,6 +245,19 @@ PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit) {
         if (run.table_bytes + bytes <= limit) run.source_bytes = bytes;
     }
     return run;
+}
+
+PairRuns pair_runs(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
+    PairRuns r;
+    if (!use_pair_form(g, dp, L, down)) return r;
+    const size_t limit = pair_scratch_limit();
+    if (down) {
+        r.down = pair_down_run(L, dp, limit);
+        return r;
+    }
+    if (L.kind == Kind::F32C) r.up_state_bytes = static_cast<size_t>(g->host->num_nodes - dp->pair.h0) * L.stride * L.asize;
+    if (r.up_state_bytes < limit) r.up = pair_up_run(L, dp, limit - r.up_state_bytes);
+    return r;
 }
 
 int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, void* vals, void* table, void* state,

@@ -188,3 +188,73 @@ def test_autotune_chooses_among_all_forms(cuda_ok, direction):
     finally:
         gx.autotune_clear()
         gx.set_graph_replay(True)
+
+
+@pytest.mark.parametrize("N,M", [(3001, 20300), (128, 900), (131, 900), (256, 900), (2002, 200), (2002, 20200)])
+def test_graphs_of_the_form_tests_take_it(env, N, M):
+    """The oracle comparisons of the pair form (test_pair_form.py) are of that form."""
+    gx = env[0]
+    g, og = _both(gx, gx.window_tree_grg(N, M, seed=N), ploidy=1)
+    for direction in (DOWN, UP):
+        for dt, K in ((np.int32, 2), (np.float32, 33), (np.float64, 1)):
+            V = _input(g, direction, dt, K)
+            _check(og, V, direction, gx.matmul(g, V, direction))
+            assert _form(g, dt, K, direction) == "in pair form" and _built(g, direction)
+
+
+def test_duplicate_children_take_another_form(env):
+    """A height-0 node that is the same node's child twice has no single pattern."""
+    import oracle
+
+    gx = env[0]
+    arrays = dict(down_off=np.array([0] * 35 + [4, 6, 9], dtype=np.uint64),
+                  down_adj=np.array([0, 1, 1, 2, 1, 33, 3, 34, 35], dtype=np.uint32), mut_node=np.arange(37, dtype=np.uint32))
+    g, og = gx.from_csr(34, 1, *arrays.values()), oracle.OracleGraph(num_samples=34, ploidy=1, **arrays)
+    for direction in (DOWN, UP):
+        V = _input(g, direction, np.int32, 2)
+        _check(og, V, direction, gx.matmul(g, V, direction))
+        assert _form(g, np.int32, 2, direction) == "unsplit" and not _built(g, direction)
+
+
+def _ranges(g, dt, K, direction, limit):
+    from grgl_gb300 import _lib
+    from grgl_gb300.api import _DTYPE_CODES
+
+    out = ctypes.c_int()
+    fn = _lib.lib().grgx_debug_pair_ranges
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64,
+                   ctypes.POINTER(ctypes.c_int)]
+    _lib.check(fn(g._h, _DTYPE_CODES[np.dtype(dt)], K, direction, 0, limit, ctypes.byref(out)))
+    return out.value
+
+
+@pytest.fixture(scope="module")
+def many_blocks(cuda_ok):
+    """300 blocks: five segments of UP lists."""
+    import grgl_gb300 as gx
+
+    _pair_mode(1)
+    try:
+        yield _both(gx, gx.window_tree_grg(2002, 60_000, seed=3), ploidy=1)
+    finally:
+        _pair_mode(0)
+
+
+# kinds with state between UP's tables and levels, and without; columns in one tile and several
+@pytest.mark.parametrize("dt,K", [(np.int32, 12), (np.int64, 3), (np.float32, 40), (np.float64, 1), (np.float64, 18), (np.bool_, 70)])
+@pytest.mark.parametrize("direction", [DOWN, UP])
+def test_several_tables(env, many_blocks, direction, dt, K):
+    """With little scratch the patterns' rows are made in parts, whose sums are carried on."""
+    gx, (g, og) = env[0], many_blocks
+    V = _input(g, direction, dt, K)
+    seen = set()
+    try:
+        for shift in range(40, 11, -1):
+            for limit in (1 << shift, 3 << (shift - 2)):
+                n = _ranges(g, dt, K, direction, limit)
+                if n not in seen:
+                    seen.add(n)
+                    _check(og, V, direction, gx.matmul(g, V, direction))
+    finally:
+        _ranges(g, dt, K, direction, 0)
+    assert {0, 1, 2} <= seen and max(seen) >= 3, seen
