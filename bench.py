@@ -119,7 +119,8 @@ def alg_bytes(stats, K, s, direction):
 
 def gathered_bytes(gx, g, E, K, s, direction):
     """Bytes one traversal gathers: an id and a row of K values per edge; in pair form (one gather per
-    block and height-0 node, and those that make and use the pattern rows) what that form reads."""
+    block and height-0 node, and those that make and use the pattern rows) what that form reads; the 16-bit ids
+    alone for UP's single 4-byte columns, whose values are gathered from shared memory."""
     import ctypes
 
     from grgl_gb300 import _lib
@@ -128,7 +129,7 @@ def gathered_bytes(gx, g, E, K, s, direction):
     _lib.check(_lib.lib().grgx_debug_pair_counts(g._h, direction, out))
     h0, blocks, patterns, low = (int(x) for x in out)
     if direction == UP and row == 4:
-        blocks = 0  # single 4-byte columns stay with the lists per node
+        return E * 2
     if blocks == 0:
         return E * (4 + row)
     rest = (E - low) * (4 + row)
@@ -829,14 +830,6 @@ def main():
                            f"the N={tf['graph']['samples']}, M={tf['graph']['mutations']} graph "
                            f"(E={tf['graph']['edges']}), scaled by edges x{E / tf['graph']['edges']:.2f} "
                            "(profiles/sweep_traffic.json)")
-    k1 = [(dt, d, t["sweep_ms"]) for dt, K, d, t in records if K == 1]
-    id_stream = None
-    if k1:
-        rates = [E * 4 / (ms_ / 1e3) / 1e9 for _, _, ms_ in k1]
-        id_stream = {"achieved": statistics.fmean(rates), "peak": hbm_peak, "unit": "GB/s",
-                     "frac": statistics.fmean(rates) / hbm_peak,
-                     "what": "K=1 matmuls: 4 bytes per edge / sweep time (the pair form and the staged lists read 2 "
-                             "per gather instead)"}
     roofline = {
         "bound": "l2", "kernel": "grgx::pair_down_kernel, grgx::pair_up_kernel, grgx::sweep_kernel",
         "achieved": gathered / sweep_s_step / 1e9, "peak": l2_peak, "unit": "GB/s",
@@ -851,7 +844,6 @@ def main():
         "hbm": {"achieved": None if traffic is None else traffic / sweep_s_step / 1e9, "peak": hbm_peak,
                 "unit": "GB/s", "frac": None if traffic is None else traffic / sweep_s_step / 1e9 / hbm_peak,
                 "peak_source": hbm_src, "what": "measured DRAM bytes (scaled ncu capture) / sweep time"},
-        "edge_id_stream": id_stream,
         "gather_model_GBps": abytes / sweep_s_step / 1e9,
         "gather_model_note": "the survey's algorithmic bytes (ids, offsets, one row per edge, one row per node, "
                              "I/O) / sweep time: exceeds the HBM peak because L2 serves the row gathers; not a "
