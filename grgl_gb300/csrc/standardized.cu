@@ -164,10 +164,14 @@ void ensure_stats(grgx_graph* g, DevicePlan* dp, cudaStream_t s) {
     matmul_impl(g, GRGX_I32, ones, N, 1, GRGX_DIRECTION_UP, counts, M, 0, 0, nullptr, GRGX_INIT_ZERO, nullptr,
                 GRGX_FLAG_DEVICE_POINTERS | GRGX_FLAG_OVERWRITE, s);
     double *freq = nullptr, *inv = nullptr;
-    GRGX_CUDA(cudaMalloc(&freq, std::max<long long>(M, 1) * sizeof(double)));
-    dp->allocs.push_back(freq);
-    GRGX_CUDA(cudaMalloc(&inv, std::max<long long>(M, 1) * sizeof(double)));
-    dp->allocs.push_back(inv);
+    {
+        // (the plan's list of memory is the graph's: another thread may be building a form)
+        std::lock_guard<std::mutex> plan(g->mu);
+        GRGX_CUDA(cudaMalloc(&freq, std::max<long long>(M, 1) * sizeof(double)));
+        dp->allocs.push_back(freq);
+        GRGX_CUDA(cudaMalloc(&inv, std::max<long long>(M, 1) * sizeof(double)));
+        dp->allocs.push_back(inv);
+    }
     stats_kernel<<<grid_for(M), 256, 0, s>>>(counts, M, static_cast<double>(N), freq, inv);
     GRGX_CUDA(cudaFreeAsync(ones, s));
     GRGX_CUDA(cudaFreeAsync(counts, s));
