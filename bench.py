@@ -754,7 +754,7 @@ def main():
             levels_tuned += sum(1 for ln in rep.splitlines() if " rows " in ln)
             for ln in rep.splitlines():
                 if ln.startswith("UP runs"):
-                    up_form[f"{np.dtype(dt).name}:{K}"] = "split" if "split form" in ln else "unsplit"
+                    up_form[f"{np.dtype(dt).name}:{K}"] = next((f for f in ("split", "pair") if f"{f} form" in ln), "unsplit")
         torch.cuda.synchronize()
         table = gx.autotune_table()
         tune = {"seconds": time.perf_counter() - t0, "levels_tuned": levels_tuned,
