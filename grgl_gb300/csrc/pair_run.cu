@@ -101,7 +101,7 @@ enum class DownSums { kOrdered, kSingle, kExact };
 DownSums down_sums(const Layout& L, const PairPlan& P) {
     if (L.kind != Kind::F32C || L.vw == 1) return DownSums::kOrdered;
     const long long work = P.nblk * L.stride;
-    if (work <= 1000) return DownSums::kExact;
+    if (work <= (P.nblk <= 50 ? 1000 : 800)) return DownSums::kExact;
     return work < 10000 || L.stride <= 8 ? DownSums::kSingle : DownSums::kOrdered;
 }
 

@@ -140,11 +140,13 @@ template <class Op, int VW, int G> void pair_up_as(const PairUpParams<typename O
         return;                        \
     }
 #define GRGX_PAIR_UP4(OP)        \
+    GRGX_PAIR_UP_CASE(OP, 4, 4)  \
+    GRGX_PAIR_UP4_BUT4(OP)
+#define GRGX_PAIR_UP4_BUT4(OP)   \
     GRGX_PAIR_UP_CASE(OP, 1, 1)  \
     GRGX_PAIR_UP_CASE(OP, 2, 1)  \
     GRGX_PAIR_UP_CASE(OP, 4, 1)  \
     GRGX_PAIR_UP_CASE(OP, 4, 2)  \
-    GRGX_PAIR_UP_CASE(OP, 4, 4)  \
     GRGX_PAIR_UP_CASE(OP, 4, 8)  \
     GRGX_PAIR_UP_CASE(OP, 4, 16) \
     GRGX_PAIR_UP_CASE(OP, 4, 32) \

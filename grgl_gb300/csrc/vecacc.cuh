@@ -220,11 +220,18 @@ template <int NP, int PRE = kF32PreSum> struct PackedF32C {
                 }
             }
         } else {
-            static_assert(PRE == 1 || PRE == kF32Ordered, "no other pre-sums");
+            static_assert(N % 2 == 0 && (PRE == 1 || PRE == 2 || PRE == kF32Ordered), "no other pre-sums");
 #pragma unroll
             for (int u = 0; u < N; u++) {
-                if constexpr (PRE == 1) add(v[u]);
-                else add_ordered(v[u]);
+                if constexpr (PRE == 1) {
+                    add(v[u]);
+                } else if constexpr (PRE == 2) {
+#pragma unroll
+                    for (int j = 0; u % 2 == 0 && j < NP; j++)
+                        add_pair2(j, add2(make_float2(v[u][2 * j], v[u][2 * j + 1]), make_float2(v[u + 1][2 * j], v[u + 1][2 * j + 1])));
+                } else {
+                    add_ordered(v[u]);
+                }
             }
         }
     }
