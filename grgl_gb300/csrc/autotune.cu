@@ -180,7 +180,7 @@ std::string autotune_impl(grgx_graph* g, int dtype, uint64_t rows, int direction
     }
     const bool split = forms.size() > 1;
     clear_pair_choice(g, dp, L, down);
-    const PairRuns pruns = pair_runs(g, dp, L, down);
+    const PairRuns pruns = pair_runs(g, dp, L, down, nullptr);
     const PairDownRun& prun = pruns.down;
     const PairUpRun& urun = pruns.up;
     const bool upState = pruns.up_state_bytes > 0;

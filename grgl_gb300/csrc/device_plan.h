@@ -261,9 +261,9 @@ void build_staged(DevicePlan& d, StagedLists& T, const std::vector<uint32_t>& se
 void set_down_split_mode(int mode);
 bool down_split_forced();
 
-// Whether a call with layout L runs in pair form (pair_plan.h); builds the form on the first call
-// that may use it.  set_pair_mode: 0 by the rules, 1 wherever possible, 2 never (tests).
-bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
+// Whether a call with layout L on stream s runs in pair form (pair_plan.h); builds the form on the first call
+// that may use it, unless s is being captured into a CUDA graph.  set_pair_mode: 0 by the rules, 1 wherever possible, 2 never (tests).
+bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, cudaStream_t s);
 // Scratch the pair form of a call on this thread may take beyond what the other forms need; a
 // server's worker lowers it to what its batch has reserved (PairScratchScope).
 size_t pair_scratch_limit();
@@ -318,7 +318,7 @@ struct PairRuns {
     // kind adds them onto the node's value
     size_t up_state_bytes = 0;
 };
-PairRuns pair_runs(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down);
+PairRuns pair_runs(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, cudaStream_t s);
 // Writes every node's sum over its height-0 children to vals (onto it when rmw), or leaves it in
 // `state` where one is given.
 int launch_pair_up(const Layout& L, const DevicePlan* dp, const PairUpRun& run, void* vals, void* table, void* state,

@@ -728,7 +728,7 @@ void matmul_once(grgx_graph* g, int dtype, const void* input, uint64_t in_cols, 
         // passes, then the other edges level by level (up_split.cu)
         // UP in pair form: the height-0 edges over patterns first (pair_plan.h), the others level by
         // level from the sums, as in split form
-        const PairRuns pruns = pairForm ? pair_runs(g, dp, L, down) : PairRuns{};
+        const PairRuns pruns = pairForm ? pair_runs(g, dp, L, down, s) : PairRuns{};
         const PairUpRun& urun = pruns.up;
         const bool upair = !urun.ranges.empty();
         const bool split = !down && !upair && use_up_split(g, dp, L);
@@ -1020,7 +1020,7 @@ int call_form(grgx_graph* g, int dtype, uint64_t rows, int direction, uint32_t f
                                    (flags & GRGX_FLAG_F64_NATIVE) != 0);
     const bool down = direction == GRGX_DIRECTION_DOWN;
     if (pair >= 0) set_pair_choice(g, dp, L, down, pair != 0);
-    const PairRuns runs = pair_runs(g, dp, L, down);
+    const PairRuns runs = pair_runs(g, dp, L, down, nullptr);
     *ranges = static_cast<int>(down ? runs.down.ranges.size() : runs.up.ranges.size());
     if (*ranges > 0) return 2;
     return (down ? use_down_split(g, dp, L) : use_up_split(g, dp, L)) ? 1 : 0;

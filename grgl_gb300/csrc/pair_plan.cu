@@ -706,7 +706,22 @@ void clear_pair_choice(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down
     (down ? dp->down_pair_choice : dp->up_pair_choice).erase({static_cast<int>(L.kind), L.stride});
 }
 
-bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
+namespace {
+// While alive, this thread's allocations and synchronous copies neither fail for nor end another thread's
+// stream capture.
+class RelaxedCapture {
+  public:
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+  private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+}  // namespace
+
+bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, cudaStream_t s) {
     const int mode = g_pair_mode.load();
     if (mode == 2) return false;
     // (a split form asked for by its test hooks)
@@ -721,6 +736,13 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
     if (mode == 0 && chosen != choice.end() && !chosen->second) return false;
     PairPlan& P = dp->pair;
     bool& tried = down ? P.down_tried : P.up_tried;
+    if (!tried && !P.refused) {
+        // A call that an application captures into a CUDA graph takes another form, as a build's allocations and
+        // copies cannot be captured; a capture on another thread is none of this build's business.
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+    }
+    const RelaxedCapture relaxed;
     for (int attempt = 0; attempt < 2 && !tried && !P.refused; attempt++) {
         try {
             tried = true;

@@ -247,9 +247,9 @@ PairUpRun pair_up_run(const Layout& L, const DevicePlan* dp, size_t limit) {
     return run;
 }
 
-PairRuns pair_runs(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down) {
+PairRuns pair_runs(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, cudaStream_t s) {
     PairRuns r;
-    if (!use_pair_form(g, dp, L, down)) return r;
+    if (!use_pair_form(g, dp, L, down, s)) return r;
     const size_t limit = pair_scratch_limit();
     if (down) {
         r.down = pair_down_run(L, dp, limit);

@@ -258,3 +258,47 @@ def test_several_tables(env, many_blocks, direction, dt, K):
     finally:
         _ranges(g, dt, K, direction, 0)
     assert {0, 1, 2} <= seen and max(seen) >= 3, seen
+
+
+@pytest.mark.parametrize("direction", [DOWN, UP])
+def test_first_call_inside_an_applications_capture(env, direction):
+    """It takes a form that needs no build, and a later call the pair form; the captured graph stays right."""
+    import torch
+
+    gx, g, og = env
+    V = _input(g, direction, np.float64, 6)
+    x = torch.zeros(V.shape, dtype=torch.float64, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = gx.matmul(g, x, direction)
+    assert not _built(g, direction)
+    x.copy_(torch.from_numpy(V))
+    graph.replay()
+    _check(og, V, direction, out.cpu().numpy())
+    _check(og, V, direction, gx.matmul(g, V, direction))
+    assert _built(g, direction)
+    graph.replay()
+    _check(og, V, direction, out.cpu().numpy())
+    del graph
+
+
+@pytest.mark.parametrize("direction", [DOWN, UP])
+def test_build_beside_an_applications_capture(env, direction):
+    """A first call on another thread, while this one captures."""
+    import torch
+
+    gx, g, og = env
+    V = _input(g, direction, np.int32, 6)
+    got = []
+    x = torch.ones(1000, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = x + 1
+        t = threading.Thread(target=lambda: got.append(_form(g, np.int32, 6, direction)))
+        t.start()
+        t.join()
+        z = y * 2
+    graph.replay()
+    assert got == ["in pair form"] and float(z.sum()) == 4000.0
+    _check(og, V, direction, gx.matmul(g, V, direction))
