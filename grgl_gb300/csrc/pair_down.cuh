@@ -125,8 +125,8 @@ __global__ void pair_table_kernel(const uint2* nodes, long long count, const typ
 
 // Rows per group of lanes: a warp covers (32 / G) * kPairRows rows, four blocks of each at a time,
 // so eight gathers are in flight per lane.  Four rows (sixteen gathers, two blocks of threads per
-// SM instead of three) ran within 3% either way for int32 and wide float64 and slower for the rest
-// (float32 K=64 4.29 against 4.11 ms, float64 K=8 1.92 against 1.66 ms; N=200,000, M=250,000).
+// SM instead of three), with the kernel's first version, ran within 3% either way for int32 and wide float64
+// and slower for the rest (float32 K=64 4.29 against 4.11 ms, float64 K=8 1.92 against 1.66 ms; N=200,000, M=250,000).
 constexpr int kPairRows = 2;
 
 // Bound by the L2 -> SM reads of its gathers when rows are wide (float32 K=64: 16-17 TB/s of pattern
@@ -134,8 +134,8 @@ constexpr int kPairRows = 2;
 // of gather instructions for the narrowest rows, whose tables mostly sit in L1.  It takes half the
 // gathers of a sweep over edges, has no row boundaries to look for (each row has exactly one
 // pattern per block), and reads one byte of ids per edge.  DOWN products on N=200,000, M=250,000
-// before and after: int32 K=1 0.65 -> 0.34 ms (staged split passes before), float32 K=9 2.38 ->
-// 1.32, float32 K=64 7.87 -> 4.1, float64 K=64 16.6 -> 9.3 ms.
+// before and now: int32 K=1 0.65 -> 0.28 ms (staged split passes before), float32 K=9 2.38 ->
+// 1.18, float32 K=64 7.87 -> 3.63, float64 K=64 16.6 -> 8.06 ms.
 //
 // One warp per item (a share of the blocks x a tile of rows).  A row's columns are spread over G
 // lanes as in the sweep; each lane loads its rows' ids of four blocks (8 bytes) and gathers the

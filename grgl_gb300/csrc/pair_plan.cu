@@ -727,7 +727,7 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, cu
     // (a split form asked for by its test hooks)
     if (mode == 0 && (down ? down_split_forced() : split_threshold_bytes() != kDefaultSplitThreshold)) return false;
     // UP, a single 4-byte column: gathers from the height-0 values run at about one per SM clock
-    // however narrow, and the staged lists at five edges per clock (int32 0.43 ms against 1.0,
+    // however narrow, and the staged lists at five edges per clock (int32 0.38 ms against 1.0,
     // N=200,000, M=250,000); compensated sums would lose the pattern rows' roundings.
     if (!down && L.stride == 1 && (L.kind == Kind::F32C || (staged_layout(L) && up_split_possible(dp)))) return false;
     std::lock_guard<std::mutex> lk(g->mu);

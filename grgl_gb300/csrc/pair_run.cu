@@ -13,8 +13,8 @@ namespace {
 constexpr size_t kPairTableBytes = 1ULL << 30;
 // A share of the blocks (item) covers at most this much of a table.  The warps of a launch take
 // the items of one share before those of the next, so about this much is gathered from at a time
-// and mostly stays in L2 (float32 K=64, N=200,000, M=250,000, a 650 MB table: 4.08 ms at 96 MB,
-// 4.29 at 48 MB, 4.57 unshared).
+// and mostly stays in L2 (N=200,000, M=250,000, K=64, at 96 MB / 48 / 192 / unshared, ms: float32, a 650 MB table, 3.63 /
+// 3.84 / 3.78 / 3.86; int32 3.16 / 3.23 / 3.46 / 3.56; float64 8.06 / 8.27 / 7.90 / 8.44, K=32 4.01 / 4.12 / 4.14 / 4.29).
 constexpr long long kPairItemBytes = 96LL << 20;
 // Items per resident warp that even out the launch's end, and the fewest groups of four blocks
 // that make an item worth its sum's trip through memory.

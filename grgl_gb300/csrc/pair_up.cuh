@@ -19,7 +19,7 @@ constexpr int pair_list_lanes(int g) { return (g & (g - 1)) == 0 && g < 8 ? 8 : 
 // end.  The lanes of a list load its ids together and pass them round.
 //
 // Bound by the L2 -> SM reads of its gathers and the packed additions when rows are wide (float32
-// K=64: 58% of L2 throughput, 68% of the FP32 pipe that takes packed instructions; its sources miss
+// K=64: 68% of L2 throughput, 65% of the FP32 pipe that takes packed instructions; its sources miss
 // L1 throughout), by L1's rate of about one random row per clock when they are narrow.  The sweep
 // over the same lists walks every row boundary (a quarter of the patterns hold a single height-0
 // node) through its reductions: on N=200,000, M=250,000 float32 K=64 took 7.4 ms that way, 8.1

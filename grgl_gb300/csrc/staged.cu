@@ -34,7 +34,7 @@ constexpr long long kStagedListCost = 100;
 // about 3.4 times, so about 9 edges per SM and clock is the most; the packed compensated additions
 // and the id arithmetic take about as long (74% of the shared-memory pipe, 53% of the issue slots).
 // UP K=1 on N=200,000, M=250,000 before (one launch per block, rows found from head bits in chunks,
-// each row merged into its state per block) and after: float32 0.87 -> 0.46 ms, int32 0.63 -> 0.43.
+// each row merged into its state per block) and now: float32 0.87 -> 0.42 ms, int32 0.63 -> 0.38.
 template <class Op>
 __global__ void __launch_bounds__(kStagedThreads, 1) staged_kernel(const StagedPart* __restrict__ parts,
                                                                    const PairList* __restrict__ lists,
