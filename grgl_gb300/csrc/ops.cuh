@@ -82,6 +82,16 @@ struct AddF32 {
     static __device__ __forceinline__ S finish_onto(S base, const A& a) { return base + a; }
 };
 
+// Plain floats in the pair form, where one lane adds up all of a row: the additions are grouped (GroupedAcc,
+// vecacc.cuh).
+struct AddF32G : AddF32 {};
+struct AddF64G : AddF64 {};
+// ... without runs, whose registers the float-pair path beside it needs
+struct AddF64T : AddF64 {};
+template <class Op> constexpr bool kGrouped = false;
+template <> inline constexpr bool kGrouped<AddF32G> = true;
+template <> inline constexpr bool kGrouped<AddF64G> = true;
+
 // Compensated float: the running sum is hi + lo with |lo| <= ulp(hi)/2.  TwoSum (Knuth,
 // TAOCP vol. 2, 4.2.2) gives the exact rounding error of each addition; the errors are
 // collected in lo and folded back when the node value is rounded to float.

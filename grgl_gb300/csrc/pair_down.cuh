@@ -116,7 +116,7 @@ __global__ void pair_table_kernel(const uint2* nodes, long long count, const typ
                                   typename PairTable<Op, VW>::T* table, const int* gate) {
     if constexpr (kHasF64<Op>) {
         if (gate != nullptr && *gate != 0) {
-            pair_table<AddF64, VW>(nodes, count, reinterpret_cast<const double*>(vals), stride, reinterpret_cast<double*>(table));
+            pair_table<AddF64T, VW>(nodes, count, reinterpret_cast<const double*>(vals), stride, reinterpret_cast<double*>(table));
             return;
         }
     }
@@ -207,6 +207,18 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(con
 #pragma unroll
                     for (int r = 0; r < ROWS; r++) acc[r].fold();
                 }
+            } else if constexpr (kGrouped<Op>) {
+                if ((q - q0) & 1) {
+#pragma unroll
+                    for (int r = 0; r < ROWS; r++) acc[r].add_rows(v[r]);
+                    if (((q - q0) & 7) == 7) {
+#pragma unroll
+                        for (int r = 0; r < ROWS; r++) acc[r].flush();
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < ROWS; r++) acc[r].hold_rows(v[r]);
+                }
             } else {
 #pragma unroll
                 for (int r = 0; r < ROWS; r++) acc[r].add_pairs(v[r]);
@@ -216,6 +228,13 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_down(con
             if ((q1 - q0) & 1 & p.long_runs) {
 #pragma unroll
                 for (int r = 0; r < ROWS; r++) acc[r].fold();
+            }
+        }
+        if constexpr (kGrouped<Op>) {
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) {
+                if ((q1 - q0) & 1) acc[r].add_held();
+                acc[r].seal();
             }
         }
         if (!active) continue;
@@ -244,7 +263,7 @@ template <class Op, int VW, int G>
 __global__ void __launch_bounds__(256, 3) pair_down_kernel(const PairDownParams<typename Op::S> p) {
     if constexpr (kHasF64<Op>) {
         if (p.gate != nullptr && *p.gate != 0) {
-            pair_down<AddF64, VW, G>(as_f64(p));
+            pair_down<AddF64T, VW, G>(as_f64(p));
             return;
         }
     }
@@ -275,7 +294,7 @@ __global__ void pair_finish_kernel(typename PairPart<Op>::T* parts, int count, l
                                    typename Op::S* vals, const int* gate) {
     if constexpr (kHasF64<Op>) {
         if (gate != nullptr && *gate != 0) {
-            pair_finish<AddF64>(reinterpret_cast<double*>(parts), count, rows, stride, reinterpret_cast<double*>(vals));
+            pair_finish<AddF64T>(reinterpret_cast<double*>(parts), count, rows, stride, reinterpret_cast<double*>(vals));
             return;
         }
     }

@@ -92,6 +92,7 @@ template <class Op, int VW, int G> __device__ __forceinline__ void pair_up(const
             acc.flush();
         }
     }
+    if constexpr (kGrouped<Op>) acc.seal();
 #pragma unroll
     for (int m = G; m < L; m <<= 1) {  // (none where L = G)
         const auto t = acc.shfl_xor(m);
@@ -120,7 +121,7 @@ template <class Op, int VW, int G>
 __global__ void __launch_bounds__(256, (G & (G - 1)) ? 3 : 4) pair_up_kernel(const PairUpParams<typename Op::S> p) {
     if constexpr (std::is_base_of<AddF64S, Op>::value) {
         if (p.gate != nullptr && *p.gate != 0) {
-            pair_up<AddF64, VW, G>(as_f64(p));
+            pair_up<AddF64T, VW, G>(as_f64(p));
             return;
         }
     }

@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_kernel(const StagedP
             }
             acc.template add_block<8>(v);
         }
+        if constexpr (kGrouped<Op>) acc.seal();
 #pragma unroll
         for (int m = 1; m < 8; m <<= 1) {
             const auto t = acc.shfl_xor(m);
@@ -166,7 +167,7 @@ int launch_staged(Kind kind, const StagedLists& T, void* vals, void* sums, void*
     case Kind::U32: return run_staged<AddU32>(T, vals, sums, state, stateBase, rmw, s);
     case Kind::XOR: return run_staged<XorU32>(T, vals, sums, state, stateBase, rmw, s);
     case Kind::F32C: return run_staged<AddF32C>(T, vals, sums, state, stateBase, rmw, s);
-    case Kind::F32: return run_staged<AddF32>(T, vals, sums, state, stateBase, rmw, s);
+    case Kind::F32: return run_staged<AddF32G>(T, vals, sums, state, stateBase, rmw, s);
     default: return 0;
     }
 }

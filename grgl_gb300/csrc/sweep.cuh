@@ -212,6 +212,8 @@ template <> struct ChainTraits<AddF64S> {
     static constexpr bool kChains = true;
 };
 template <> struct ChainTraits<AddF64SD> : ChainTraits<AddF64S> {};
+template <> struct ChainTraits<AddF32G> : ChainTraits<AddF64S> {};
+template <> struct ChainTraits<AddF64G> : ChainTraits<AddF64S> {};
 
 // Chunk tail: the warp's last row sum is written, or -- a piece of a heavy row -- published as a
 // partial; the last piece to finish (atomic ticket) adds all of them up in piece order.

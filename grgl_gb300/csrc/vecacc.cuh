@@ -492,6 +492,81 @@ template <> struct VecAcc<AddF64SD, 1> : PackedF64SD<1> {
     }
 };
 
+// Plain floats and doubles, grouped: the rows of a block as a tree, and (RUNS) blocks in runs, runs onto the sum.
+// Error and time: pair_down_f32.cu.
+template <class Op, int VW, bool RUNS> struct GroupedAcc {
+    using S = typename Op::S;
+    S run[VW], sum[RUNS ? VW : 1], held[RUNS ? VW : 1];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < VW; i++) run[i] = S(0);
+        if constexpr (RUNS) {
+#pragma unroll
+            for (int i = 0; i < VW; i++) sum[i] = S(0);
+        }
+    }
+    template <int N> static __device__ __forceinline__ S tree(const S (*v)[VW], int i) {
+        static_assert((N & (N - 1)) == 0, "a whole tree");
+        S t[N];
+#pragma unroll
+        for (int u = 0; u < N; u++) t[u] = v[u][i];
+#pragma unroll
+        for (int n = N / 2; n > 0; n /= 2) {
+#pragma unroll
+            for (int u = 0; u < n; u++) t[u] = t[2 * u] + t[2 * u + 1];
+        }
+        return t[0];
+    }
+    template <int N> __device__ __forceinline__ void add_block(const S (*v)[VW]) {
+#pragma unroll
+        for (int i = 0; i < VW; i++) run[i] += tree<N>(v, i);
+    }
+    __device__ __forceinline__ void add_pairs(const S (*v)[VW]) { add_block<4>(v); }
+    // Four rows whose sum waits for the next four's.
+    __device__ __forceinline__ void hold_rows(const S (*v)[VW]) {
+#pragma unroll
+        for (int i = 0; i < VW; i++) held[i] = tree<4>(v, i);
+    }
+    __device__ __forceinline__ void add_rows(const S (*v)[VW]) {
+#pragma unroll
+        for (int i = 0; i < VW; i++) run[i] += held[i] + tree<4>(v, i);
+    }
+    __device__ __forceinline__ void add_held() {
+#pragma unroll
+        for (int i = 0; i < VW; i++) run[i] += held[i];
+    }
+    __device__ __forceinline__ void flush() {
+        if constexpr (RUNS) {
+#pragma unroll
+            for (int i = 0; i < VW; i++) {
+                sum[i] += run[i];
+                run[i] = S(0);
+            }
+        }
+    }
+    // No more blocks: the sum is whole from here on.
+    __device__ __forceinline__ void seal() {
+        if constexpr (RUNS) {
+#pragma unroll
+            for (int i = 0; i < VW; i++) run[i] += sum[i];
+        }
+    }
+    __device__ __forceinline__ void merge(const GroupedAcc& o) {
+#pragma unroll
+        for (int i = 0; i < VW; i++) run[i] += o.run[i];
+    }
+    __device__ __forceinline__ GroupedAcc shfl_xor(int m) const {
+        GroupedAcc r;
+#pragma unroll
+        for (int i = 0; i < VW; i++) r.run[i] = Op::shfl_xor(run[i], m);
+        return r;
+    }
+    __device__ __forceinline__ S get(int i) const { return run[i]; }
+};
+template <int VW> struct VecAcc<AddF32G, VW> : GroupedAcc<AddF32G, VW, true> {};
+template <int VW> struct VecAcc<AddF64G, VW> : GroupedAcc<AddF64G, VW, true> {};
+template <int VW> struct VecAcc<AddF64T, VW> : GroupedAcc<AddF64T, VW, false> {};
+
 // float64 as float pairs in runs of four or eight rows, each run folded into a DFSum: a run's first row is its
 // start, the pair is renormalised after four, and no FP64 instruction is needed at all (FP64 conversions and
 // additions run at about two lanes per clock and SM).  A run's low parts are rounded relative to its sum,

@@ -82,3 +82,34 @@ def test_float64_errors_at_or_below_the_sweeps(graphs, N, M, direction, K, input
             _pair_mode(mode)
             total[mode] += float((product(g, x, direction) - exact).square().sum() / exact.square().sum())
     assert total[1] <= total[2], (np.sqrt(total[1] / 4), np.sqrt(total[2] / 4))
+
+
+@pytest.mark.parametrize("N,M,direction,K", [
+    (20_000, 50_000, DOWN, 2), (20_000, 50_000, DOWN, 18), (20_000, 50_000, UP, 2), (20_000, 50_000, UP, 18),
+    (100_000, 20_000, DOWN, 3), (100_000, 20_000, DOWN, 33), (100_000, 20_000, UP, 9), (100_000, 20_000, UP, 64)])
+def test_plain_sums_near_the_sweeps(graphs, N, M, direction, K):
+    """Plain float32 and FP64 sums of one lane per row, grouped: within 1.25 times the sweep's error (whose terms are
+    spread over lanes), where sums one by one have up to three times it.  FP64's error is taken against inputs in
+    two halves whose sums are exact."""
+    import torch
+
+    gx, get = graphs
+    g = get(N, M)
+    total = {(m, dt): 0.0 for m in (1, 2) for dt in (torch.float32, torch.float64)}
+    for seed in range(4):
+        torch.manual_seed(seed)
+        x = torch.randn((K, g.num_samples if direction == UP else g.num_mutations), device="cuda", dtype=torch.float64)
+        high = (x * 2**22).round() / 2**22
+        low = ((x - high) * 2**48).round() / 2**48
+        _pair_mode(2)
+        H, L = (gx.matmul(g, v, direction, f64_native=True) for v in (high, low))
+        x32 = x.float()
+        exact32 = gx.matmul(g, x32.double(), direction, f64_native=True)
+        for mode in (1, 2):
+            _pair_mode(mode)
+            e = (gx.matmul(g, high + low, direction, f64_native=True) - H) - L
+            total[mode, torch.float64] += float(e.square().sum() / H.square().sum())
+            e = gx.matmul(g, x32, direction, f32_compensated=False).double() - exact32
+            total[mode, torch.float32] += float(e.square().sum() / exact32.square().sum())
+    for dt in (torch.float32, torch.float64):
+        assert total[1, dt] <= 1.25**2 * total[2, dt], (dt, np.sqrt(total[1, dt] / 4), np.sqrt(total[2, dt] / 4))
