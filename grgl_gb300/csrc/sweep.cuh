@@ -480,6 +480,10 @@ __device__ __forceinline__ void short_row(const SweepParams<typename Op::S>& p, 
                 acc.a[i].hi = r.hi;
                 acc.a[i].lo = r.lo;
             }
+        } else if constexpr (std::is_same<Op, AddF32>::value || std::is_same<Op, AddF64>::value) {
+            // plain sums: the batch as a tree (what lies past the row's end is zero)
+#pragma unroll
+            for (int i = 0; i < VW; i++) acc.a[i] += (v[0][i] + v[1][i]) + (v[2][i] + v[3][i]);
         } else {
 #pragma unroll
             for (int u = 0; u < kShortBatch; u++)

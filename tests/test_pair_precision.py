@@ -113,3 +113,21 @@ def test_plain_sums_near_the_sweeps(graphs, N, M, direction, K):
             total[mode, torch.float32] += float(e.square().sum() / exact32.square().sum())
     for dt in (torch.float32, torch.float64):
         assert total[1, dt] <= 1.25**2 * total[2, dt], (dt, np.sqrt(total[1, dt] / 4), np.sqrt(total[2, dt] / 4))
+
+
+def test_plain_sums_of_short_rows(cuda_ok):
+    """Rows of eight edges, one group of lanes each, four edges at a time as a tree.  The same sums of N(0,1) values in
+    numpy leave 0.80 u of the norm as trees of four and 0.94 u one by one (u = 2^-24): the line lies between."""
+    import torch
+
+    import grgl_gb300 as gx
+
+    rng = np.random.default_rng(4)
+    N, rows, d = 3000, 12000, 8
+    adj = np.sort(np.stack([rng.choice(N, size=d, replace=False) for _ in range(rows)])).astype(np.uint32)
+    off = np.concatenate([np.zeros(N, dtype=np.uint64), np.arange(rows + 1, dtype=np.uint64) * d])
+    g = gx.from_csr(N, 1, off, adj.ravel(), np.arange(N, N + rows, dtype=np.uint32)).upload()
+    x = torch.from_numpy(rng.standard_normal((8, N)).astype(np.float32)).cuda()
+    exact = x.double()[:, torch.from_numpy(adj.astype(np.int64)).cuda()].sum(-1)
+    got = gx.matmul(g, x, UP, f32_compensated=False).double()
+    assert float((got - exact).norm() / exact.norm()) <= 0.87 * 2.0**-24
