@@ -736,14 +736,15 @@ bool use_pair_form(grgx_graph* g, DevicePlan* dp, const Layout& L, bool down, cu
     if (mode == 0 && chosen != choice.end() && !chosen->second) return false;
     PairPlan& P = dp->pair;
     bool& tried = down ? P.down_tried : P.up_tried;
-    if (!tried && !P.refused) {
-        // A call that an application captures into a CUDA graph takes another form, as a build's allocations and
-        // copies cannot be captured; a capture on another thread is none of this build's business.
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
-    }
+    if (tried || P.refused) return down ? P.down_built : P.up_built;
+    // A call that an application captures into a CUDA graph takes another form, as a build's allocations and
+    // copies cannot be captured; a capture on another thread is none of this build's business.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    const cudaError_t asked = cudaStreamIsCapturing(s, &capturing);
+    if (asked != cudaSuccess) cudaGetLastError();  // (the legacy stream, beside a blocking stream's capture)
+    if (asked != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
     const RelaxedCapture relaxed;
-    for (int attempt = 0; attempt < 2 && !tried && !P.refused; attempt++) {
+    for (int attempt = 0; attempt < 2 && !tried; attempt++) {
         try {
             tried = true;
             P.refused = !build_pair_plan(*dp, down);
